@@ -1,8 +1,10 @@
-"""In-tree build of the CUDA library (nvcc, sm_100a only).
+"""In-tree build of the CUDA library (nvcc, sm_100a only) and of the torch host module.
 
-``build()`` compiles every ``csrc/*.cu`` into ``lib/libflexgemm_b200.so`` next
-to the package, so the binary travels with a copy of the source tree.  It is
-incremental: an object is rebuilt only when its source or a header is newer.
+``build()`` compiles every ``csrc/*.cu`` into ``lib/libflexgemm_b200.so`` and
+``csrc/host/fgb_torch.cpp`` (g++, against torch's headers) into
+``lib/_fgb_torch.so`` next to the package, so the binaries travel with a copy of
+the source tree.  It is incremental: a file is rebuilt only when its source or a
+header is newer.
 """
 import os
 import shutil
@@ -14,6 +16,8 @@ INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflexgemm_b200.so")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
+HOST_SRC = os.path.join(CSRC, "host", "fgb_torch.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "_fgb_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -33,6 +37,24 @@ def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
 
 
+def _build_host(force: bool):
+    """Command and process of the torch host module's build, or None when it is up to date."""
+    newest = _newest([HOST_SRC] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE) if f.endswith(".h")])
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= newest:
+        return None
+    import sysconfig
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + os.path.join(tdir, "include"), "-I" + os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_path("include"), HOST_SRC, "-o", HOST_PATH,
+           "-L" + os.path.join(tdir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+           "-L" + os.path.join(cuda, "lib64"), "-lcudart"]
+    return cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -42,6 +64,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     hdr_time = _newest(headers)
     objs, rebuilt = [], False
     procs = []
+    host = _build_host(force)
     for src in sources:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ_DIR, src[:-3] + ".o")
@@ -61,6 +84,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed: %s\n%s" % (" ".join(cmd), r.stdout))
+    if host is not None:
+        out, _ = host[1].communicate()
+        if host[1].returncode != 0:
+            raise RuntimeError("host module build failed: %s\n%s" % (" ".join(host[0]), out))
     return LIB_PATH
 
 

@@ -17,6 +17,15 @@ F16, BF16, F32_TF32, F32_IEEE = 0, 1, 2, 3
 _P = c_void_p
 _PROTOTYPES = {
     "fgb_version": (c_char_p, []),
+    "fgb_status_set_mirror": (c_int, [_P, _P]),
+    "fgb_conv_call_workspace_bytes": (c_int64, [_P, c_int]),
+    "fgb_conv_call_fprop": (c_int, [_P, _P]),
+    "fgb_conv_call_dgrad": (c_int, [_P, _P]),
+    "fgb_wgrad_call_workspace_bytes": (c_int64, [_P]),
+    "fgb_wgrad_call_run": (c_int, [_P, _P]),
+    "fgb_resize_rows": (c_int, [_P, _P, c_int64, c_int64, c_int64, c_int64, _P]),
+    "fgb_subm_cache_scratch_bytes": (c_int64, [_P]),
+    "fgb_subm_cache_build": (c_int, [_P, _P]),
     "fgb_error_string": (c_char_p, [c_int]),
     "fgb_selftest_device_tables": (c_int, []),
     "fgb_fetch_words_async": (c_int, [_P, _P, c_int64, _P]),

@@ -1,6 +1,44 @@
-// Version and error strings of the C ABI.
+// Version and error strings of the C ABI, and the host-visible copies of status words.
+#include <atomic>
+#include <mutex>
+
 #include "fgb_common.cuh"
 #include "fgb_device.cuh"
+
+namespace fgb {
+namespace {
+struct MirrorEntry {
+  std::atomic<const int32_t*> status{nullptr};
+  std::atomic<int32_t*> mirror{nullptr};
+};
+MirrorEntry g_mirrors[kMaxDevices];  // one status word per device in practice; filled from the front, never emptied
+std::mutex g_mirror_mu;
+}  // namespace
+
+int32_t* status_mirror(const int32_t* status) {
+  if (status == nullptr) return nullptr;
+  for (MirrorEntry& e : g_mirrors) {
+    const int32_t* s = e.status.load(std::memory_order_acquire);
+    if (s == status) return e.mirror.load(std::memory_order_acquire);
+    if (s == nullptr) return nullptr;
+  }
+  return nullptr;
+}
+}  // namespace fgb
+
+extern "C" int fgb_status_set_mirror(const int32_t* status, int32_t* mirror) {
+  using namespace fgb;
+  if (status == nullptr) return FGB_E_NULL;
+  std::lock_guard<std::mutex> lock(g_mirror_mu);
+  for (MirrorEntry& e : g_mirrors) {
+    const int32_t* s = e.status.load(std::memory_order_acquire);
+    if (s != nullptr && s != status) continue;
+    e.mirror.store(mirror, std::memory_order_release);
+    e.status.store(status, std::memory_order_release);
+    return FGB_OK;
+  }
+  return FGB_E_SIZE;
+}
 
 extern "C" const char* fgb_version(void) { return "flexgemm_b200 0.1.0 (sm_100a)"; }
 

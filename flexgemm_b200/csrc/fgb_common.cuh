@@ -21,6 +21,17 @@ __device__ __forceinline__ void report(int32_t* status, int32_t code) {
   if (status != nullptr) atomicCAS(status, 0, code);
 }
 
+// Host-visible copy of a device status word (fgb_status_set_mirror): kernels that find or set a code there store it to
+// the mirror as well, so that the host looks at the state of the device by reading its own memory -- no copy, event or
+// launch per call.  status_mirror() is the launch code's lookup: null when the word has no mirror.
+int32_t* status_mirror(const int32_t* status);
+__device__ __forceinline__ void mirror_code(int32_t* mirror, int32_t code) {
+  if (mirror != nullptr) {
+    *reinterpret_cast<volatile int32_t*>(mirror) = code;
+    __threadfence_system();
+  }
+}
+
 inline int elem_bytes(int dtype) {
   switch (dtype) {
     case FGB_F16:
@@ -35,6 +46,7 @@ inline int elem_bytes(int dtype) {
 }
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+inline int64_t align256(int64_t x) { return (x + 255) & ~int64_t(255); }
 
 // fprop / dgrad of a small input (fewer work items than SMs) split every item's offsets into shares that run as
 // separate items into fp32 slabs (fgb_igemm.cu): the number of shares for n output rows x nout channels on the current

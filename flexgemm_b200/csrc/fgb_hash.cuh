@@ -103,7 +103,7 @@ struct Grid3 {
   }
 };
 
-// one thread per voxel, 16-byte coordinate loads
+// 16-byte coordinate loads; the grid may be smaller than the rows ask for (where the kernel often has nothing to do)
 // `unsorted` (may be null): device word, 0 when the sorted-input path builds the map instead -- then the table is not needed
 template <int kKeyBits>
 __global__ void __launch_bounds__(kMapBlock) hash_insert_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g,
@@ -112,11 +112,11 @@ __global__ void __launch_bounds__(kMapBlock) hash_insert_kernel(const int4* __re
   chain_release();
   chain_wait();
   if (unsorted != nullptr && *unsorted == 0u) return;
-  const uint32_t i = blockIdx.x * kMapBlock + threadIdx.x;
-  if (i >= n) return;
-  const int4 c = __ldg(&coords[i]);
   const auto table = make_table<kKeyBits>(table_mem, slots);
-  if (!table.insert(g.template key<kKeyBits>(c.x, c.y, c.z, c.w), i)) report(status, FGB_S_TABLE_FULL);
+  for (uint64_t i = blockIdx.x * uint64_t(kMapBlock) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kMapBlock) {
+    const int4 c = __ldg(&coords[i]);
+    if (!table.insert(g.template key<kKeyBits>(c.x, c.y, c.z, c.w), static_cast<uint32_t>(i))) report(status, FGB_S_TABLE_FULL);
+  }
 }
 
 }  // namespace fgb

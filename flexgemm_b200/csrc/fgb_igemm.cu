@@ -42,6 +42,7 @@
 #include "fgb_common.cuh"
 #include "fgb_device.cuh"
 #include "fgb_precision.cuh"
+#include "fgb_sort.cuh"
 #include "fgb_umma.cuh"
 
 namespace fgb {
@@ -86,6 +87,7 @@ struct IgemmParams {
   int acc_sets;              // accumulator pairs that fit in TMEM (1 or 2)
   uint32_t idesc;
   int32_t* status;
+  int32_t* status_mirror;    // host-visible copy of *status, or null
 };
 
 // what the fused epilogue adds (a kernel parameter of its own: the plain kernel's parameter block, and with it its
@@ -225,7 +227,10 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
   // A kernel that already reported a soft error makes the rest of the grid a
   // no-op.  One thread reads the word so that the whole CTA takes the same branch.
   __shared__ int s_skip;
-  if (threadIdx.x == 0) s_skip = p.status != nullptr && *reinterpret_cast<volatile const int32_t*>(p.status) != 0;
+  if (threadIdx.x == 0) {
+    s_skip = p.status != nullptr ? *reinterpret_cast<volatile const int32_t*>(p.status) : 0;
+    if (s_skip != 0 && blockIdx.x == 0) mirror_code(p.status_mirror, s_skip);
+  }
   __syncthreads();
   if (s_skip) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -583,7 +588,10 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512u);
   }
-  if (tid == 0 && ctl->abort_flag) report(p.status, FGB_S_WAIT_TIMEOUT);
+  if (tid == 0 && ctl->abort_flag) {
+    report(p.status, FGB_S_WAIT_TIMEOUT);
+    mirror_code(p.status_mirror, FGB_S_WAIT_TIMEOUT);
+  }
 }
 
 // ------------------------------------------------------------------ block schedule
@@ -591,28 +599,85 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
 // cost of a block being the number of (tile, offset) products it runs.  One CTA;
 // a counting sort over the 65 possible costs.  Blocks of equal cost may come out
 // in any order: the order only decides which SM computes a block, never a result.
-__global__ void __launch_bounds__(1024) block_schedule_kernel(const uint32_t* __restrict__ masks, uint32_t num_tiles, uint32_t nb,
-                                                              uint32_t* __restrict__ order) {
-  __shared__ uint32_t s_count[65];
-  __shared__ uint32_t s_start[65];
-  const int t = threadIdx.x;
-  if (t < 65) s_count[t] = 0;
+// Costs of a block of two tiles lie in 0 .. 64.  Blocks of equal cost mostly stand together (the rows are sorted by
+// mask), so a warp takes its places by one atomic per distinct cost, not per block.
+struct ScheduleSmem {
+  uint32_t count[65], start[65];
+};
+__device__ __forceinline__ void block_schedule(ScheduleSmem& sm, const uint32_t* masks, uint32_t num_tiles, uint32_t nb,
+                                               uint32_t* __restrict__ order) {
+  const int t = threadIdx.x, lane = t & 31;
+  if (t < 65) sm.count[t] = 0;
   __syncthreads();
-  auto cost_of = [&](uint32_t b) {
+  auto cost_of = [&](uint32_t b) {  // the masks may have been written by other CTAs of this launch: loads that bypass L1
     const uint32_t t0 = 2 * b;
-    return __popc(__ldg(&masks[t0])) + (t0 + 1 < num_tiles ? __popc(__ldg(&masks[t0 + 1])) : 0);
+    return __popc(__ldcg(&masks[t0])) + (t0 + 1 < num_tiles ? __popc(__ldcg(&masks[t0 + 1])) : 0);
   };
-  for (uint32_t b = t; b < nb; b += 1024) atomicAdd(&s_count[cost_of(b)], 1u);
+  auto take = [&](uint32_t* counters, uint32_t b) -> uint32_t {  // whole warps call it; a place for every lane with b < nb
+    const bool ok = b < nb;
+    const int c = ok ? cost_of(b) : 65;
+    const unsigned peers = __match_any_sync(0xffffffffu, c);
+    const int leader = __ffs(peers) - 1;
+    uint32_t base = 0;
+    if (ok && lane == leader) base = atomicAdd(&counters[c], static_cast<uint32_t>(__popc(peers)));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    return base + static_cast<uint32_t>(__popc(peers & ((1u << lane) - 1u)));
+  };
+  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) take(sm.count, b0 + lane);
   __syncthreads();
   if (t == 0) {
     uint32_t acc = 0;
     for (int c = 64; c >= 0; --c) {
-      s_start[c] = acc;
-      acc += s_count[c];
+      sm.start[c] = acc;
+      acc += sm.count[c];
     }
   }
   __syncthreads();
-  for (uint32_t b = t; b < nb; b += 1024) order[atomicAdd(&s_start[cost_of(b)], 1u)] = b;
+  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) {
+    const uint32_t pos = take(sm.start, b0 + lane);
+    if (b0 + lane < nb) order[pos] = b0 + lane;
+  }
+}
+__global__ void __launch_bounds__(1024) block_schedule_kernel(const uint32_t* __restrict__ masks, uint32_t num_tiles, uint32_t nb,
+                                                              uint32_t* __restrict__ order) {
+  __shared__ ScheduleSmem sm;
+  block_schedule(sm, masks, num_tiles, nb, order);
+}
+
+// Tile masks (one warp per tile of 128 sorted rows) and, by the CTA that ends last, the block schedule: one launch.
+__global__ void __launch_bounds__(1024) tile_plan_kernel(const int32_t* __restrict__ gray, const int64_t* __restrict__ sorted_idx, uint32_t n,
+                                                         uint32_t num_tiles, uint32_t* masks, uint32_t* __restrict__ order,
+                                                         uint32_t* counter) {
+  __shared__ ScheduleSmem sm;
+  __shared__ bool s_last;
+  chain_release();
+  chain_wait();
+  const uint32_t tile = blockIdx.x * 32 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (tile < num_tiles) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < kTileM; i += 32) {
+      const uint64_t r = uint64_t(tile) * kTileM + i + lane;
+      if (r < n) m |= static_cast<uint32_t>(__ldg(&gray[__ldg(&sorted_idx[r])]));
+    }
+    m = __reduce_or_sync(0xffffffffu, m);
+    if (lane == 0) masks[tile] = m;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  block_schedule(sm, masks, num_tiles, (num_tiles + 1) / 2, order);
+}
+
+cudaError_t launch_tile_plan(const int32_t* gray, const int64_t* sorted_idx, int64_t n, uint32_t* tile_masks, uint32_t* block_order,
+                             uint32_t* counter, cudaStream_t s) {
+  const uint32_t tiles = static_cast<uint32_t>(ceil_div(n, kTileM));
+  return launch_chained(tile_plan_kernel, dim3(static_cast<unsigned>(ceil_div(tiles, 32))), dim3(1024), 0, s, gray, sorted_idx,
+                        static_cast<uint32_t>(n), tiles, tile_masks, block_order, counter);
 }
 
 // ------------------------------------------------------------------ weight re-layout for dgrad
@@ -651,6 +716,20 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
+// Calls `encode`, and once more with the device's context bound when the thread has none yet: the encoder is a driver
+// call and, unlike the runtime's, does not bind the context of the device by itself (a thread of the autograd engine may
+// come here before it has made any runtime call).
+template <typename Encode>
+static int encode_tmap(Encode encode) {
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    const int dev = current_device();
+    if (dev < 0 || cudaSetDevice(dev) != cudaSuccess) return FGB_E_DRIVER;
+    r = encode();
+  }
+  return r == CUDA_SUCCESS ? FGB_OK : FGB_E_DRIVER;
+}
+
 // 3-D map over w[nout][V][kc]; box = 128 bytes of kc x 1 offset x bn rows, 128B swizzle
 int make_weight_tmap(CUtensorMap* map, const void* w, int nout, int V, int kc, int bn, int dtype) {
   EncodeTiledFn fn = encode_tiled_fn();
@@ -663,9 +742,10 @@ int make_weight_tmap(CUtensorMap* map, const void* w, int nout, int V, int kc, i
   cuuint64_t strides[2] = {cuuint64_t(kc) * eb, cuuint64_t(V) * kc * eb};
   cuuint32_t box[3] = {cuuint32_t(128 / eb), 1u, cuuint32_t(bn)};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, dt, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return encode_tmap([&] {
+    return fn(map, dt, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FGB_OK : FGB_E_DRIVER;
+  });
 }
 
 // 3-D map over the weight as stored, w[Co][V][Ci] of 16-bit elements, for dgrad: box = 64 input channels (128 bytes) x 1
@@ -678,9 +758,10 @@ int make_weight_tmap_mn(CUtensorMap* map, const void* w, int Co, int V, int Ci, 
   cuuint64_t strides[2] = {cuuint64_t(Ci) * 2, cuuint64_t(V) * Ci * 2};
   cuuint32_t box[3] = {64u, 1u, 64u};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, dt, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return encode_tmap([&] {
+    return fn(map, dt, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FGB_OK : FGB_E_DRIVER;
+  });
 }
 
 // 2-D map over rows[n_rows][row_elems] of 16-bit elements; box = 128 bytes of one row, 128B swizzle (the box TMA
@@ -692,10 +773,11 @@ int make_rows_tmap(CUtensorMap* map, const void* rows, int64_t n_rows, int row_e
   cuuint64_t strides[1] = {cuuint64_t(row_elems) * 2};
   cuuint32_t box[2] = {64u, 1u};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(rows), dims, strides, box, estr,
+  return encode_tmap([&] {
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(rows), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FGB_OK : FGB_E_DRIVER;
+  });
 }
 
 static int pick_bn(int nout) {
@@ -762,6 +844,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) splitk_rows_reduce_kernel(const float* __restrict__ partial, int splits, int64_t elems, int nout,
                                                                  const T* __restrict__ bias, T* __restrict__ out) {
   const int64_t e = (blockIdx.x * int64_t(256) + threadIdx.x) * 4;
+  chain_release();
+  chain_wait();  // the slabs are complete
   if (e >= elems) return;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int sp = 0; sp < splits; ++sp) {
@@ -833,6 +917,7 @@ int run_igemm(const void* x, const void* w, const void* bias, const uint32_t* nb
   const bool b_mn = (flip & 2) != 0;  // the weight operand as stored for the other direction: w [kc, V, nout]
   p.idesc = make_idesc(fmt, kTileM, p.bn, 0, b_mn ? 1 : 0);
   p.status = status;
+  p.status_mirror = status_mirror(status);
   if (!ticket) return FGB_E_NULL;
   // the work counter starts at zero; a caller that launches kernels of its own right before this one zeroes it ahead of
   // them, so that the conv kernel follows a kernel in the stream and its chained launch takes effect
@@ -854,17 +939,22 @@ int run_igemm(const void* x, const void* w, const void* bias, const uint32_t* nb
   if (rc != FGB_OK || p.splits == 1) return rc;
   const int64_t elems = n * nout;
   const unsigned grid = static_cast<unsigned>(ceil_div(elems, 1024));
+  const float* part = partial;
+  cudaError_t e;
   switch (dtype) {
     case FGB_F16:
-      splitk_rows_reduce_kernel<__half><<<grid, 256, 0, s>>>(partial, p.splits, elems, nout, static_cast<const __half*>(bias), static_cast<__half*>(out));
+      e = launch_chained(splitk_rows_reduce_kernel<__half>, dim3(grid), dim3(256), 0, s, part, p.splits, elems, nout,
+                         static_cast<const __half*>(bias), static_cast<__half*>(out));
       break;
     case FGB_BF16:
-      splitk_rows_reduce_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(partial, p.splits, elems, nout, static_cast<const __nv_bfloat16*>(bias),
-                                                                    static_cast<__nv_bfloat16*>(out));
+      e = launch_chained(splitk_rows_reduce_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, s, part, p.splits, elems, nout,
+                         static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out));
       break;
     default:
-      splitk_rows_reduce_kernel<float><<<grid, 256, 0, s>>>(partial, p.splits, elems, nout, static_cast<const float*>(bias), static_cast<float*>(out));
+      e = launch_chained(splitk_rows_reduce_kernel<float>, dim3(grid), dim3(256), 0, s, part, p.splits, elems, nout,
+                         static_cast<const float*>(bias), static_cast<float*>(out));
   }
+  if (e != cudaSuccess) return cuda_status(e);
   return launch_status();
 }
 
@@ -907,21 +997,22 @@ namespace fgb {
 static int fprop_impl(const void* feats, const void* weight, const void* bias, const uint32_t* neighbor_map, const int64_t* sorted_idx,
                       const uint32_t* tile_masks, const uint32_t* block_order, void* out, int64_t n, int64_t n_src, int Ci, int Co, int V,
                       int dtype, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream, int act = FGB_ACT_NONE,
-                      const void* residual = nullptr, void* preact = nullptr) {
+                      const void* residual = nullptr, void* preact = nullptr, uint32_t* zeroed_ticket = nullptr) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n < 0 || n_src < 0 || Ci <= 0 || Co <= 0 || V < 1 || V > 32) return FGB_E_SIZE;
   if (n == 0) return FGB_OK;
   if (!workspace) return FGB_E_NULL;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
   if (workspace_bytes < kWsHeader) return FGB_E_WORKSPACE;
-  uint32_t* ticket = static_cast<uint32_t*>(workspace);
+  // the work counter: a zeroed word of the caller's, or the workspace's first word (zeroed here)
+  uint32_t* ticket = zeroed_ticket ? zeroed_ticket : static_cast<uint32_t*>(workspace);
   char* scratch = static_cast<char*>(workspace) + kWsHeader;
   const bool fused = act != FGB_ACT_NONE || residual != nullptr || preact != nullptr;  // the fused epilogue is never split
   const int64_t part_bytes = fused ? 0 : igemm_partial_bytes(n, Co, V);
   if (dtype != FGB_F32_IEEE) {
     if (workspace_bytes < kWsHeader + part_bytes) return FGB_E_WORKSPACE;
     return run_igemm(feats, weight, bias, neighbor_map, sorted_idx, tile_masks, block_order, ticket, out, n, Ci, Co, V, dtype, 0, status, s,
-                     part_bytes ? reinterpret_cast<float*>(scratch) : nullptr, act, residual, preact);
+                     part_bytes ? reinterpret_cast<float*>(scratch) : nullptr, act, residual, preact, zeroed_ticket != nullptr);
   }
   // fp32-accurate: one TF32 run over the tripled channel dimension
   if (!feats || !weight) return FGB_E_NULL;
@@ -936,7 +1027,7 @@ static int fprop_impl(const void* feats, const void* weight, const void* bias, c
   rc = launch_split3(static_cast<const float*>(weight), w3, int64_t(Co) * V, Ci, kSplitWeights, s);
   if (rc != FGB_OK) return rc;
   return run_igemm(x3, w3, bias, neighbor_map, sorted_idx, tile_masks, block_order, ticket, out, n, 3 * Ci, Co, V, FGB_F32_TF32, 0, status, s,
-                   part, act, residual, preact);
+                   part, act, residual, preact, zeroed_ticket != nullptr);
 }
 
 }  // namespace fgb
@@ -969,18 +1060,27 @@ extern "C" int fgb_subm_conv_fprop_fused(const void* feats, const void* weight, 
 
 namespace fgb {
 
+// 16-bit types read the weight as it is stored, [Co][V][Ci], as an MN-major operand (rows = reduction channels): no
+// re-layout pass.  Column tiles narrower than one 64-channel chunk, and the 32-bit types (whose MN-major layout TMA
+// does not produce), go through the re-laid-out copy.
+static bool dgrad_as_stored(int Ci, int eb) {
+  return eb == 2 && !g_dgrad_relayout.load(std::memory_order_relaxed) && pick_bn(Ci) % 64 == 0;
+}
+
 // n rows of the map / of `grad_feats`; n_src rows of `grad_out`; mirror = the map is the forward map of a submanifold
 // conv, whose row for offset v is the backward map's row for offset V-1-v
 static int dgrad_impl(const void* grad_out, const void* weight, const uint32_t* neighbor_map, const int64_t* sorted_idx,
                       const uint32_t* tile_masks, const uint32_t* block_order, void* grad_feats, int64_t n, int64_t n_src, int Ci, int Co,
-                      int V, int dtype, int mirror, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
+                      int V, int dtype, int mirror, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream,
+                      uint32_t* zeroed_ticket = nullptr) {
   const int eb = elem_bytes(dtype);
   if (eb == 0) return FGB_E_DTYPE;
   if (n < 0 || n_src < 0 || Ci <= 0 || Co <= 0 || V < 1 || V > 32) return FGB_E_SIZE;
   if (n == 0) return FGB_OK;
   if (!weight || !workspace) return FGB_E_NULL;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
-  const int64_t wt_bytes = align256(int64_t(Ci) * V * Co * eb);
+  const bool as_stored = dgrad_as_stored(Ci, eb);
+  const int64_t wt_bytes = as_stored && zeroed_ticket != nullptr ? 0 : align256(int64_t(Ci) * V * Co * eb);
   const bool ieee = dtype == FGB_F32_IEEE;
   const int64_t w3_bytes = ieee ? align256(int64_t(Ci) * V * 3 * Co * 4) : 0;
   const int64_t g3_bytes = ieee ? align256(n_src * 3 * Co * 4) : 0;
@@ -988,16 +1088,13 @@ static int dgrad_impl(const void* grad_out, const void* weight, const uint32_t* 
   if (workspace_bytes < kWsHeader + wt_bytes + w3_bytes + g3_bytes + part_bytes) return FGB_E_WORKSPACE;
   float* part = part_bytes ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWsHeader + wt_bytes + w3_bytes + g3_bytes) : nullptr;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  uint32_t* ticket = static_cast<uint32_t*>(workspace);
+  uint32_t* ticket = zeroed_ticket ? zeroed_ticket : static_cast<uint32_t*>(workspace);
   char* wt = static_cast<char*>(workspace) + kWsHeader;
-  // 16-bit types read the weight as it is stored, [Co][V][Ci], as an MN-major operand (rows = reduction channels): no
-  // re-layout pass.  Column tiles narrower than one 64-channel chunk, and the 32-bit types (whose MN-major layout TMA
-  // does not produce), go through the re-laid-out copy.
-  if (eb == 2 && !g_dgrad_relayout.load(std::memory_order_relaxed) && pick_bn(Ci) % 64 == 0)
+  if (as_stored)
     return run_igemm(grad_out, weight, nullptr, neighbor_map, sorted_idx, tile_masks, block_order, ticket, grad_feats, n, Co, Ci, V, dtype,
-                     mirror | 2, status, s, part);
+                     mirror | 2, status, s, part, FGB_ACT_NONE, nullptr, nullptr, zeroed_ticket != nullptr);
   dim3 grid(static_cast<unsigned>(ceil_div(Ci, 32)), static_cast<unsigned>(ceil_div(Co, 32)), V);
-  {
+  if (zeroed_ticket == nullptr) {
     const cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t), s);  // ahead of the re-layout: see run_igemm
     if (e != cudaSuccess) return cuda_status(e);
   }
@@ -1037,4 +1134,29 @@ extern "C" int fgb_sparse_conv_dgrad(const void* grad_out, const void* weight, c
                                      int64_t workspace_bytes, int32_t* status, void* stream) {
   return fgb::dgrad_impl(grad_out, weight, neighbor_map_bwd, sorted_idx_bwd, tile_masks_bwd, block_order_bwd, grad_feats, n_in, n_out, Ci,
                          Co, V, dtype, 0, workspace, workspace_bytes, status, stream);
+}
+
+// ------------------------------------------------------------------ one-struct calls
+extern "C" int64_t fgb_conv_call_workspace_bytes(const fgb_conv_call* c, int pass) {
+  using fgb::align256;
+  if (!c) return FGB_E_NULL;
+  // pass 0: c->n output rows, c->n_src feature rows; pass 1: c->n rows of grad_feats, c->n_src rows of grad_out
+  if (pass == 0) return fgb_sparse_conv_workspace_bytes(0, c->n, c->n_src, c->ci, c->co, c->v, c->dtype, 1);
+  const int64_t bytes = fgb_sparse_conv_workspace_bytes(1, c->n_src, c->n, c->ci, c->co, c->v, c->dtype, 1);
+  const int eb = fgb::elem_bytes(c->dtype);
+  // no room for the re-laid-out weight where it is not made
+  return bytes > 0 && fgb::dgrad_as_stored(c->ci, eb) ? bytes - align256(int64_t(c->ci) * c->v * c->co * eb) : bytes;
+}
+
+extern "C" int fgb_conv_call_fprop(const fgb_conv_call* c, void* stream) {
+  if (!c) return FGB_E_NULL;
+  return fgb::fprop_impl(c->x, c->weight, c->bias, c->neighbor_map, c->sorted_idx, c->tile_masks, c->block_order, c->out, c->n, c->n_src,
+                         c->ci, c->co, c->v, c->dtype, c->workspace, c->workspace_bytes, c->status, stream, FGB_ACT_NONE, nullptr, nullptr,
+                         c->counters);
+}
+
+extern "C" int fgb_conv_call_dgrad(const fgb_conv_call* c, void* stream) {
+  if (!c) return FGB_E_NULL;
+  return fgb::dgrad_impl(c->x, c->weight, c->neighbor_map, c->sorted_idx, c->tile_masks, c->block_order, c->out, c->n, c->n_src, c->ci,
+                         c->co, c->v, c->dtype, c->mirror, c->workspace, c->workspace_bytes, c->status, stream, c->counters);
 }

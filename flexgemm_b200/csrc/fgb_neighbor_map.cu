@@ -33,6 +33,7 @@
 #include "fgb_common.cuh"
 #include "fgb_device.cuh"
 #include "fgb_hash.cuh"
+#include "fgb_sort.cuh"
 
 namespace fgb {
 
@@ -53,19 +54,72 @@ struct Stencil {
 // holds the input voxels, the probed coordinate is coords[i] * stride - padding
 // + k * dilation, and every hit is also scattered into the backward map
 // nbr_bwd[input row, v] = output row (when nbr_bwd is non-null).
+struct HashLookupSmem {
+  int4 coord[kMapBlock];
+  int4 delta[32];  // (dx, dy, dz) of each offset: no divisions in the item loop
+  uint32_t gray[kMapBlock];
+  uint32_t count[32];
+};
+
+// What the map kernels hand on: the map and everything that later passes need from it.
+struct MapOut {
+  uint32_t* nbr;           // [n, V]
+  int32_t* gray;           // [n]
+  int32_t* binary;         // [n]
+  uint32_t* block_counts;  // [V, nblk]
+  uint32_t* digit_hist;    // the sort's digit histograms (fgb_sort.cuh), or null
+  uint32_t nblk;
+};
+
+__device__ __forceinline__ uint32_t gray_to_binary(uint32_t x) {  // prefix xor from the top bit down
+  x ^= x >> 1;
+  x ^= x >> 2;
+  x ^= x >> 4;
+  x ^= x >> 8;
+  x ^= x >> 16;
+  return x;
+}
+
+// Writes the codes of the CTA's voxels and, where the sort follows, adds them to its digit histograms (which saves the
+// sort's own pass over the codes): runs of equal codes in a warp -- neighbouring voxels mostly share theirs -- count once
+// in shared memory, and the CTA's non-zero bins go to the global histograms.
+__device__ __forceinline__ void emit_codes(const MapOut& o, uint32_t n0, uint32_t nv, int V, uint32_t gray, uint32_t* s_hist) {
+  const int t = threadIdx.x, lane = t & 31;
+  const uint32_t binary = gray_to_binary(gray);
+  if (t < nv) {
+    o.gray[n0 + t] = static_cast<int32_t>(gray);
+    o.binary[n0 + t] = static_cast<int32_t>(binary);
+  }
+  if (o.digit_hist == nullptr) return;  // uniform
+  const int passes = sort_passes_of(V);
+  __syncthreads();  // s_hist lies over what the lookup has used
+  for (int i = t; i < passes * kSortDigits; i += kMapBlock) s_hist[i] = 0;
+  __syncthreads();
+  const uint32_t key = sort_key_of(binary, V);
+  const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+  const bool ok = t < nv;
+  const unsigned valid = __ballot_sync(0xffffffffu, ok);
+  const unsigned heads = __ballot_sync(0xffffffffu, ok && (lane == 0 || key != prev));
+  if (heads >> lane & 1u) {
+    const unsigned later = heads & ~((2u << lane) - 1u);
+    const uint32_t len = static_cast<uint32_t>((later != 0u ? __ffs(later) - 1 : __popc(valid)) - lane);
+    for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kSortDigits + sort_digit_of(key, p)], len);
+  }
+  __syncthreads();
+  for (int i = t; i < passes * kSortDigits; i += kMapBlock) {
+    const uint32_t c = s_hist[i];
+    if (c != 0u) atomicAdd(&o.digit_hist[i], c);
+  }
+}
+
 template <int kKeyBits, bool kGeneral>
-__global__ void __launch_bounds__(kMapBlock)
-    subm_lookup_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, void* table_mem, uint32_t slots,
-                       uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_bwd, int32_t* __restrict__ gray_out,
-                       int32_t* __restrict__ binary_out, uint32_t* __restrict__ block_counts, uint32_t nblk,
-                       const uint32_t* __restrict__ unsorted) {
-  chain_release();
-  chain_wait();
-  if (unsorted != nullptr && *unsorted == 0u) return;  // the sorted-input kernel builds the map
-  __shared__ int4 s_coord[kMapBlock];
-  __shared__ uint32_t s_gray[kMapBlock];
-  __shared__ uint32_t s_count[32];
-  __shared__ int4 s_delta[32];  // (dx, dy, dz) of each offset: no divisions in the item loop
+__device__ __forceinline__ void hash_lookup(HashLookupSmem& sm, const int4* __restrict__ coords, uint32_t n, const Grid3& g,
+                                            const Stencil& st, void* table_mem, uint32_t slots, const MapOut& o,
+                                            uint32_t* __restrict__ nbr_bwd) {
+  int4* s_coord = sm.coord;
+  int4* s_delta = sm.delta;
+  uint32_t* s_gray = sm.gray;
+  uint32_t* s_count = sm.count;
   const uint32_t n0 = blockIdx.x * kMapBlock;
   const uint32_t nv = min(static_cast<uint32_t>(kMapBlock), n - n0);
   const int t = threadIdx.x;
@@ -88,7 +142,7 @@ __global__ void __launch_bounds__(kMapBlock)
   const auto table = make_table<kKeyBits>(table_mem, slots);
   const int centre = V >> 1;  // all kernel extents are odd
   const uint32_t items = nv * V;
-  uint32_t* out = nbr + static_cast<size_t>(n0) * V;
+  uint32_t* out = o.nbr + static_cast<size_t>(n0) * V;
   // item = lv * V + v walks t, t + 256, ...: (lv, v) advance by (256 / V, 256 % V) with a carry
   const uint32_t step_lv = kMapBlock / V;
   const int step_v = kMapBlock % V;
@@ -121,25 +175,42 @@ __global__ void __launch_bounds__(kMapBlock)
     }
   }
   __syncthreads();
-  if (t < nv) {
-    const uint32_t gray = s_gray[t];
-    uint32_t binary = gray;  // Gray -> binary: prefix xor from the top bit down
-    binary ^= binary >> 1;
-    binary ^= binary >> 2;
-    binary ^= binary >> 4;
-    binary ^= binary >> 8;
-    binary ^= binary >> 16;
-    gray_out[n0 + t] = static_cast<int32_t>(gray);
-    binary_out[n0 + t] = static_cast<int32_t>(binary);
-  }
-  if (t < V) block_counts[static_cast<size_t>(t) * nblk + blockIdx.x] = s_count[t];
+  if (t < V) o.block_counts[static_cast<size_t>(t) * o.nblk + blockIdx.x] = s_count[t];
+  emit_codes(o, n0, nv, V, t < nv ? s_gray[t] : 0u, reinterpret_cast<uint32_t*>(&sm));
 }
 
+static size_t hash_smem_bytes(int V) {  // the lookup's own, and the digit histograms that lie over it in the end
+  return std::max(sizeof(HashLookupSmem), size_t(sort_passes_of(V)) * kSortDigits * sizeof(uint32_t));
+}
+
+// generic sparse conv: rows = output voxels, table = input voxels
+template <int kKeyBits>
+__global__ void __launch_bounds__(kMapBlock)
+    sparse_lookup_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, void* table_mem, uint32_t slots, MapOut o,
+                         uint32_t* __restrict__ nbr_bwd) {
+  chain_release();
+  chain_wait();
+  extern __shared__ __align__(16) uint8_t s_map_mem[];
+  hash_lookup<kKeyBits, true>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), coords, n, g, st, table_mem, slots, o, nbr_bwd);
+}
+
+// What a build leaves for the host (besides the tensors): see block_scan_kernel.
+struct ScanFinish {
+  uint32_t* done;               // zeroed word: count of finished CTAs; null = leave the totals as they are
+  const uint32_t* unsorted;     // copied to seg[V + 1] when not null
+  const int32_t* build_status;  // copied to seg[V + 2] when not null
+  uint32_t* host_words;         // mapped pinned memory [V + 3], then the sequence word; null = not wanted
+  uint32_t host_seq;
+};
+
 // CTA v turns block_counts[v, :] into exclusive offsets in place and leaves the
-// total of offset v in seg[v + 1].  With `finish` the CTA that ends last also turns the totals into the segment table
-// (what seg_prefix_kernel does as a launch of its own); seg[0] counts the finished CTAs and must be 0 on entry.
+// total of offset v in seg[v + 1].  With `fin.done` the CTA that ends last also turns the totals into the segment table
+// (what seg_prefix_kernel does as a launch of its own), adds the key-order word and the build's status behind it, and --
+// fin.host_words -- stores all of them straight into host memory, a sequence number last: the host reads the pair count
+// by watching that word.  (Against a copy and an event in the stream: two driver calls and about 5 us less, and the
+// kernels after the scan stay chained.)
 __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__ block_counts, uint32_t nblk, uint32_t* __restrict__ seg,
-                                                          bool finish) {
+                                                          ScanFinish fin) {
   chain_release();
   chain_wait();
   __shared__ uint32_t s_warp[32];
@@ -178,16 +249,27 @@ __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__
   }
   if (t == 0) {
     seg[blockIdx.x + 1] = s_carry;
-    if (finish) {
+    if (fin.done != nullptr) {
       __threadfence();
-      if (atomicAdd(&seg[0], 1u) == gridDim.x - 1) {  // every total is written
+      if (atomicAdd(fin.done, 1u) == gridDim.x - 1) {  // every total is written
         __threadfence();
+        const uint32_t V = gridDim.x;
         uint32_t acc = 0;
-        for (uint32_t v = 1; v <= gridDim.x; ++v) {
+        for (uint32_t v = 1; v <= V; ++v) {
           acc += *reinterpret_cast<volatile uint32_t*>(&seg[v]);
           seg[v] = acc;
         }
         seg[0] = 0;
+        if (fin.unsorted != nullptr) seg[V + 1] = *fin.unsorted;
+        if (fin.build_status != nullptr) seg[V + 2] = static_cast<uint32_t>(*fin.build_status);
+        if (fin.host_words != nullptr) {
+          volatile uint32_t* h = fin.host_words;
+          h[V] = acc;
+          h[V + 1] = seg[V + 1];
+          h[V + 2] = seg[V + 2];
+          __threadfence_system();
+          h[V + 3] = fin.host_seq;
+        }
       }
     }
   }
@@ -262,17 +344,10 @@ __global__ void __launch_bounds__(256) table_clear_kernel(uint32_t* __restrict__
 // The kernel is bound by instruction issue, not by memory, so the common stencil (3x3x3, dilation 1: kUnit) gets an
 // instance whose extents are compile-time constants (divisions by 9 and 3 become multiplies, the target loop unrolls),
 // and column indices are 32-bit (the table has fewer than 2^32 entries by construction).
-template <int kKeyBits, bool kUnit>
-__global__ void __launch_bounds__(kMapBlock)
-    subm_column_lookup_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, const uint2* __restrict__ col_table,
-                              uint32_t* __restrict__ nbr, int32_t* __restrict__ gray_out, int32_t* __restrict__ binary_out,
-                              uint32_t* __restrict__ block_counts, uint32_t nblk, const uint32_t* __restrict__ unsorted) {
-  chain_release();
-  chain_wait();
-  if (*unsorted != 0u) return;  // the hash kernels build the map
-  extern __shared__ __align__(16) uint32_t s_nbr[];  // [kMapBlock * V]
-  __shared__ int4 s_coord[kMapBlock];                // (column index, x, y, z)
-  __shared__ uint32_t s_count[32];
+template <bool kUnit>
+__device__ __forceinline__ void column_lookup(uint32_t* s_nbr /* [kMapBlock * V] */, int4* s_coord /* (column index, x, y, z) */,
+                                              uint32_t* s_count, uint32_t* s_hist, const int4* __restrict__ coords, uint32_t n,
+                                              const Grid3& g, const Stencil& st, const uint2* __restrict__ col_table, const MapOut& o) {
   const int Kw = kUnit ? 3 : st.Kw, Kh = kUnit ? 3 : st.Kh, Kd = kUnit ? 3 : st.Kd;
   const int Dw = kUnit ? 1 : st.Dw, Dh = kUnit ? 1 : st.Dh, Dd = kUnit ? 1 : st.Dd;
   const int V = kUnit ? 27 : st.V;
@@ -352,69 +427,101 @@ __global__ void __launch_bounds__(kMapBlock)
   __syncthreads();
   {
     // the CTA's map rows leave as 16-byte pieces (a block starts 256 * V * 4 bytes after the previous one)
-    uint32_t* out = nbr + static_cast<size_t>(n0) * V;
+    uint32_t* out = o.nbr + static_cast<size_t>(n0) * V;
     const uint32_t words = nv * V;
     const uint32_t vecs = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? words >> 2 : 0u;  // a map that is only 4-byte aligned goes word by word
     for (uint32_t i = t; i < vecs; i += kMapBlock) reinterpret_cast<uint4*>(out)[i] = reinterpret_cast<const uint4*>(s_nbr)[i];
     for (uint32_t i = vecs * 4 + t; i < words; i += kMapBlock) out[i] = s_nbr[i];
   }
-  if (t < nv) {
-    uint32_t binary = gray;
-    binary ^= binary >> 1;
-    binary ^= binary >> 2;
-    binary ^= binary >> 4;
-    binary ^= binary >> 8;
-    binary ^= binary >> 16;
-    gray_out[n0 + t] = static_cast<int32_t>(gray);
-    binary_out[n0 + t] = static_cast<int32_t>(binary);
+  if (t < V) o.block_counts[static_cast<size_t>(t) * o.nblk + blockIdx.x] = s_count[t];
+  emit_codes(o, n0, nv, V, gray, s_hist);
+}
+
+// The submanifold map: one kernel with both lookups, so that the path that is not taken costs neither a launch nor a
+// pass of empty CTAs (20 us at 5.3 M voxels).  *unsorted decides (see column_index_kernel); null = the hash table.
+static size_t map_smem_bytes(int V) {
+  const size_t tile = size_t(kMapBlock) * V * sizeof(uint32_t) + kMapBlock * sizeof(int4) + 32 * sizeof(uint32_t);
+  return std::max(tile, hash_smem_bytes(V));
+}
+template <int kKeyBits, bool kUnit>
+__global__ void __launch_bounds__(kMapBlock)
+    subm_map_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, const uint2* __restrict__ col_table, void* table_mem,
+                    uint32_t slots, MapOut o, const uint32_t* __restrict__ unsorted) {
+  chain_release();
+  extern __shared__ __align__(16) uint8_t s_map_mem[];
+  chain_wait();
+  if (unsorted == nullptr || *unsorted != 0u) {
+    hash_lookup<kKeyBits, false>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), coords, n, g, st, table_mem, slots, o, nullptr);
+  } else {
+    int4* s_coord = reinterpret_cast<int4*>(s_map_mem);
+    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_coord + kMapBlock);
+    column_lookup<kUnit>(s_count + 32, s_coord, s_count, reinterpret_cast<uint32_t*>(s_map_mem), coords, n, g, st, col_table, o);
   }
-  if (t < V) block_counts[static_cast<size_t>(t) * nblk + blockIdx.x] = s_count[t];
+}
+
+// Memory of a build, and where its kernels leave things
+struct BuildMem {
+  uint2* columns;          // [B * W * H] or null: no table-free path
+  void* table;             // hash table; may share its memory with `columns`
+  bool table_cleared;      // the hash table is filled with ones already and apart from the columns
+  uint32_t slots;
+  uint32_t* seg;           // [V + 1] (+ the key-order word and the build's status, see ScanFinish)
+  uint32_t* unsorted;      // zeroed word, or null without the table-free path
+  int32_t* build_status;   // zeroed word or null
+  ScanFinish fin;
+};
+
+template <int kKeyBits>
+static cudaError_t launch_build(const int4* c4, uint32_t n, const Grid3& g, const Stencil& st, uint64_t columns, const BuildMem& m,
+                                const MapOut& o, cudaStream_t s) {
+  LaunchErrors chain;
+  const unsigned nblk = o.nblk;
+  if (m.columns != nullptr)
+    chain.add(launch_chained(column_index_kernel<kKeyBits>, dim3(static_cast<unsigned>(ceil_div(n, 256))), dim3(256), 0, s, c4, n, g, columns,
+                             m.columns, m.unsorted));
+  const uint32_t* unsorted = m.unsorted;
+  if (!m.table_cleared) {
+    const size_t words = static_cast<size_t>(fgb_hash_table_bytes(m.slots, kKeyBits)) / 4;
+    const unsigned grid = static_cast<unsigned>(std::min<size_t>(ceil_div(static_cast<int64_t>(words), 256 * 8), 148 * 16));
+    chain.add(launch_chained(table_clear_kernel, dim3(grid > 0 ? grid : 1), dim3(256), 0, s, static_cast<uint32_t*>(m.table), words, unsorted));
+  }
+  const unsigned igrid = std::min<unsigned>(nblk, 148 * 8);
+  chain.add(launch_chained(hash_insert_kernel<kKeyBits>, dim3(igrid), dim3(kMapBlock), 0, s, c4, n, g, m.table, m.slots, m.build_status, unsorted));
+  const bool unit = st.Kw == 3 && st.Kh == 3 && st.Kd == 3 && st.Dw == 1 && st.Dh == 1 && st.Dd == 1;
+  const uint2* cols = m.columns;
+  if (unit)
+    chain.add(launch_chained(subm_map_kernel<kKeyBits, true>, dim3(nblk), dim3(kMapBlock), map_smem_bytes(st.V), s, c4, n, g, st, cols, m.table,
+                             m.slots, o, unsorted));
+  else
+    chain.add(launch_chained(subm_map_kernel<kKeyBits, false>, dim3(nblk), dim3(kMapBlock), map_smem_bytes(st.V), s, c4, n, g, st, cols, m.table,
+                             m.slots, o, unsorted));
+  chain.add(launch_chained(block_scan_kernel, dim3(st.V), dim3(1024), 0, s, o.block_counts, nblk, m.seg, m.fin));
+  return chain.first;
 }
 
 template <int kKeyBits>
 static int build_impl(const int32_t* coords, uint32_t n, int B, Grid3 g, Stencil st, void* table, uint32_t slots, uint32_t* nbr,
                       int32_t* gray, int32_t* binary, uint32_t* block_counts, uint32_t* seg, int32_t* status, cudaStream_t s) {
-  const uint32_t nblk = static_cast<uint32_t>(ceil_div(n, kMapBlock));
-  const int4* c4 = reinterpret_cast<const int4*>(coords);
   const size_t table_bytes = static_cast<size_t>(fgb_hash_table_bytes(slots, kKeyBits));
-  const size_t table_words = table_bytes / 4;
-  const unsigned clear_grid = static_cast<unsigned>(std::min<size_t>(ceil_div(static_cast<int64_t>(table_words), 256 * 8), 148 * 16));
   // The sorted-input path needs one 8-byte entry per (b, x, y) column and keeps them in the caller's table memory; the
   // map tile of a CTA must fit shared memory.  seg[V + 1] carries the device-side decision between the two paths (0 =
   // rows in key order, the table-free path built the map) and stays there for the pair-list kernel.
   const uint64_t columns = static_cast<uint64_t>(B > 0 ? B : 0) * g.W * g.H;
   const bool try_sorted = columns > 0 && columns * sizeof(uint2) <= table_bytes;
-  uint32_t* unsorted = try_sorted ? seg + st.V + 1 : nullptr;
-  {
-    // seg[0] = 0: the scan's count of finished CTAs; seg[V + 1]: the key-order word
-    cudaError_t e = cudaMemsetAsync(seg, 0, (st.V + 2) * sizeof(uint32_t), s);
-    if (e == cudaSuccess && !try_sorted) e = cudaMemsetAsync(seg + st.V + 1, 1, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return cuda_status(e);
-  }
-  if (try_sorted) {
-    cudaError_t e = cudaMemsetAsync(table, 0xFF, columns * sizeof(uint2), s);
-    if (e != cudaSuccess) return cuda_status(e);
-    column_index_kernel<kKeyBits><<<static_cast<unsigned>(ceil_div(n, 256)), 256, 0, s>>>(c4, n, g, columns, static_cast<uint2*>(table), unsorted);
-  }
-  // from here on every kernel is chained to the one before it (fgb_device.cuh): the launches overlap the kernels' tails
-  LaunchErrors chain;
-  chain.add(launch_chained(table_clear_kernel, dim3(clear_grid > 0 ? clear_grid : 1), dim3(256), 0, s, static_cast<uint32_t*>(table),
-                           table_words, unsorted));
-  chain.add(launch_chained(hash_insert_kernel<kKeyBits>, dim3(nblk), dim3(kMapBlock), 0, s, c4, n, g, table, slots, status, unsorted));
-  chain.add(launch_chained(subm_lookup_kernel<kKeyBits, false>, dim3(nblk), dim3(kMapBlock), 0, s, c4, n, g, st, table, slots, nbr,
-                           static_cast<uint32_t*>(nullptr), gray, binary, block_counts, nblk, unsorted));
-  if (try_sorted) {
-    const size_t smem = size_t(kMapBlock) * st.V * sizeof(uint32_t);
-    const bool unit = st.Kw == 3 && st.Kh == 3 && st.Kd == 3 && st.Dw == 1 && st.Dh == 1 && st.Dd == 1;
-    if (unit)
-      chain.add(launch_chained(subm_column_lookup_kernel<kKeyBits, true>, dim3(nblk), dim3(kMapBlock), smem, s, c4, n, g, st,
-                               static_cast<const uint2*>(table), nbr, gray, binary, block_counts, nblk, unsorted));
-    else
-      chain.add(launch_chained(subm_column_lookup_kernel<kKeyBits, false>, dim3(nblk), dim3(kMapBlock), smem, s, c4, n, g, st,
-                               static_cast<const uint2*>(table), nbr, gray, binary, block_counts, nblk, unsorted));
-  }
-  chain.add(launch_chained(block_scan_kernel, dim3(st.V), dim3(1024), 0, s, block_counts, nblk, seg, true));
-  return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
+  // seg[0] = 0: the scan's count of finished CTAs; seg[V + 1]: the key-order word
+  cudaError_t e = cudaMemsetAsync(seg, 0, (st.V + 2) * sizeof(uint32_t), s);
+  if (e == cudaSuccess && !try_sorted) e = cudaMemsetAsync(seg + st.V + 1, 1, sizeof(uint32_t), s);
+  if (e == cudaSuccess && try_sorted) e = cudaMemsetAsync(table, 0xFF, columns * sizeof(uint2), s);
+  if (e != cudaSuccess) return cuda_status(e);
+  BuildMem m{};
+  m.columns = try_sorted ? static_cast<uint2*>(table) : nullptr;
+  m.table = table, m.slots = slots, m.seg = seg;
+  m.unsorted = try_sorted ? seg + st.V + 1 : nullptr;
+  m.build_status = status;
+  m.fin.done = seg;
+  const MapOut o{nbr, gray, binary, block_counts, nullptr, static_cast<uint32_t>(ceil_div(n, kMapBlock))};
+  e = launch_build<kKeyBits>(reinterpret_cast<const int4*>(coords), n, g, st, columns, m, o, s);
+  return e != cudaSuccess ? cuda_status(e) : launch_status();
 }
 
 // generic sparse conv: table over the input voxels, rows = output voxels
@@ -426,9 +533,9 @@ static int build_general_impl(const int32_t* in_coords, uint32_t n_in, const int
     hash_insert_kernel<kKeyBits><<<static_cast<unsigned>(ceil_div(n_in, kMapBlock)), kMapBlock, 0, s>>>(
         reinterpret_cast<const int4*>(in_coords), n_in, g, table, slots, status, nullptr);
   const uint32_t nblk = static_cast<uint32_t>(ceil_div(n_out, kMapBlock));
-  subm_lookup_kernel<kKeyBits, true><<<nblk, kMapBlock, 0, s>>>(reinterpret_cast<const int4*>(out_coords), n_out, g, st, table, slots,
-                                                               nbr, nbr_bwd, gray, binary, block_counts, nblk, nullptr);
-  block_scan_kernel<<<st.V, 1024, 0, s>>>(block_counts, nblk, seg, false);
+  const MapOut o{nbr, gray, binary, block_counts, nullptr, nblk};
+  sparse_lookup_kernel<kKeyBits><<<nblk, kMapBlock, hash_smem_bytes(st.V), s>>>(reinterpret_cast<const int4*>(out_coords), n_out, g, st, table, slots, o, nbr_bwd);
+  block_scan_kernel<<<st.V, 1024, 0, s>>>(block_counts, nblk, seg, ScanFinish{});
   seg_prefix_kernel<<<1, 32, 0, s>>>(seg, st.V);
   return launch_status();
 }
@@ -454,14 +561,8 @@ __global__ void __launch_bounds__(256) gray_from_map_kernel(const uint32_t* __re
   __syncthreads();
   if (t < nv) {
     const uint32_t gray = s_gray[t];
-    uint32_t binary = gray;
-    binary ^= binary >> 1;
-    binary ^= binary >> 2;
-    binary ^= binary >> 4;
-    binary ^= binary >> 8;
-    binary ^= binary >> 16;
     gray_out[n0 + t] = static_cast<int32_t>(gray);
-    binary_out[n0 + t] = static_cast<int32_t>(binary);
+    binary_out[n0 + t] = static_cast<int32_t>(gray_to_binary(gray));
   }
 }
 
@@ -502,6 +603,113 @@ extern "C" int fgb_subm_build_neighbor_map(const int32_t* coords, int64_t n, int
                           binary_code, block_counts, valid_signal_seg, status, s);
   return build_impl<64>(coords, static_cast<uint32_t>(n), B, g, st, table, static_cast<uint32_t>(slots), neighbor_map, gray_code,
                         binary_code, block_counts, valid_signal_seg, status, s);
+}
+
+namespace fgb {
+// Scratch of fgb_subm_cache_build: one block whose first part starts as zeros (one memset for the whole build: key-order
+// word, build status, counters, the sort's histograms and look-back words), whose second starts as ones (column table
+// and, below kClearWithTable, the hash table), and working arrays that start as anything.
+struct CacheScratch {
+  SortLayout sort;
+  size_t words_off, hist_off, lookback_off, zero_bytes;   // zeros: [0, zero_bytes)
+  size_t columns_off, table_off, ones_off, ones_bytes;
+  size_t codes_off, sort_off, total;
+  bool try_sorted, table_cleared;
+};
+// Clearing the hash table along with the columns saves a kernel per build; for tables above this size the clearing
+// itself (13 us for the 85 MB of 5.3 M voxels, and the L2 it sweeps) costs more than the launch, and rows in key order
+// do not need it.
+constexpr size_t kClearWithTable = size_t(16) << 20;
+
+static CacheScratch cache_scratch(int64_t n, int64_t B, int64_t W, int64_t H, int V, int64_t slots, int key_bits) {
+  CacheScratch c{};
+  c.sort = sort_layout(n);
+  const size_t table_bytes = static_cast<size_t>(fgb_hash_table_bytes(slots, key_bits));
+  const uint64_t columns = static_cast<uint64_t>(B > 0 ? B : 0) * W * H;
+  c.try_sorted = columns > 0 && columns * sizeof(uint2) <= table_bytes;
+  c.table_cleared = table_bytes <= kClearWithTable;
+  c.words_off = 0;                                   // [0] key-order word [1] build status [2] scan counter [3] plan counter
+  c.hist_off = 256;
+  c.lookback_off = c.hist_off + align256((kSortMaxPasses * kSortDigits + kSortMaxPasses) * 4);
+  c.zero_bytes = c.lookback_off + align256(int64_t(sort_passes_of(V)) * c.sort.tiles * kSortDigits * 4);
+  c.ones_off = c.zero_bytes;
+  const size_t col_bytes = c.try_sorted ? align256(static_cast<int64_t>(columns * sizeof(uint2))) : 0;
+  c.columns_off = c.ones_off;
+  c.table_off = c.table_cleared ? c.ones_off + col_bytes : c.ones_off;  // a large table shares the columns' memory
+  c.ones_bytes = col_bytes + (c.table_cleared ? table_bytes : 0);
+  const size_t end = std::max(c.ones_off + col_bytes, c.table_off + table_bytes);
+  c.codes_off = align256(static_cast<int64_t>(end));
+  c.sort_off = c.codes_off + align256(n * 4);
+  c.total = c.sort_off + c.sort.buffer_bytes;
+  return c;
+}
+
+static int check_map_call(const fgb_map_call* c) {
+  if (!c) return FGB_E_NULL;
+  if (c->n < 0 || c->n >= (int64_t(1) << 30)) return FGB_E_SIZE;
+  if (c->b < 0 || c->w <= 0 || c->h <= 0 || c->d <= 0) return FGB_E_SIZE;
+  int64_t V = 1;
+  for (int i = 0; i < 3; ++i) {
+    if (c->k[i] <= 0 || !(c->k[i] & 1) || c->dil[i] <= 0) return FGB_E_SIZE;
+    V *= c->k[i];
+    if (V > 32) return FGB_E_SIZE;
+  }
+  if (c->key_bits != 32 && c->key_bits != 64) return FGB_E_DTYPE;
+  if (c->slots < c->n || c->slots < 1 || c->slots >= (int64_t(1) << 31)) return FGB_E_SIZE;
+  return FGB_OK;
+}
+}  // namespace fgb
+
+extern "C" int64_t fgb_subm_cache_scratch_bytes(const fgb_map_call* c) {
+  using namespace fgb;
+  const int rc = check_map_call(c);
+  if (rc != FGB_OK) return rc;
+  return static_cast<int64_t>(cache_scratch(c->n, c->b, c->w, c->h, c->k[0] * c->k[1] * c->k[2], c->slots, c->key_bits).total);
+}
+
+extern "C" int fgb_subm_cache_build(const fgb_map_call* c, void* stream) {
+  using namespace fgb;
+  int rc = check_map_call(c);
+  if (rc != FGB_OK) return rc;
+  const int V = c->k[0] * c->k[1] * c->k[2];
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!c->meta) return FGB_E_NULL;
+  if (c->n == 0) return cuda_status(cudaMemsetAsync(c->meta, 0, (V + 3) * sizeof(uint32_t), s));
+  if (!c->coords || !c->scratch || !c->neighbor_map || !c->gray_code || !c->sorted_idx || !c->tile_masks || !c->block_order || !c->block_offsets)
+    return FGB_E_NULL;
+  if ((reinterpret_cast<uintptr_t>(c->coords) & 15) || (reinterpret_cast<uintptr_t>(c->scratch) & 255)) return FGB_E_ALIGN;
+  const CacheScratch L = cache_scratch(c->n, c->b, c->w, c->h, V, c->slots, c->key_bits);
+  if (c->scratch_bytes < static_cast<int64_t>(L.total)) return FGB_E_WORKSPACE;
+  char* mem = static_cast<char*>(c->scratch);
+  uint32_t* words = reinterpret_cast<uint32_t*>(mem + L.words_off);
+  uint32_t* hist = reinterpret_cast<uint32_t*>(mem + L.hist_off);
+  cudaError_t e = cudaMemsetAsync(mem, 0, L.zero_bytes, s);
+  if (e == cudaSuccess && !L.try_sorted) e = cudaMemsetAsync(words, 1, 4, s);  // no table-free path: "not in key order"
+  if (e == cudaSuccess && L.ones_bytes > 0) e = cudaMemsetAsync(mem + L.ones_off, 0xFF, L.ones_bytes, s);
+  if (e != cudaSuccess) return cuda_status(e);
+  const uint32_t n = static_cast<uint32_t>(c->n);
+  const Grid3 g{c->w, c->h, c->d};
+  const Stencil st{c->k[0], c->k[1], c->k[2], c->dil[0], c->dil[1], c->dil[2], V};
+  BuildMem m{};
+  m.columns = L.try_sorted ? reinterpret_cast<uint2*>(mem + L.columns_off) : nullptr;
+  m.table = mem + L.table_off;
+  m.table_cleared = L.table_cleared;
+  m.slots = static_cast<uint32_t>(c->slots);
+  m.seg = c->meta;
+  m.unsorted = L.try_sorted ? words : nullptr;
+  m.build_status = reinterpret_cast<int32_t*>(words + 1);
+  m.fin = ScanFinish{words + 2, words, m.build_status, c->host_words, c->host_seq};
+  int32_t* codes = reinterpret_cast<int32_t*>(mem + L.codes_off);
+  const MapOut o{c->neighbor_map, c->gray_code, codes, c->block_offsets, hist, static_cast<uint32_t>(ceil_div(c->n, kMapBlock))};
+  const uint64_t columns = static_cast<uint64_t>(c->b) * c->w * c->h;
+  const int4* c4 = reinterpret_cast<const int4*>(c->coords);
+  e = c->key_bits == 32 ? launch_build<32>(c4, n, g, st, columns, m, o, s) : launch_build<64>(c4, n, g, st, columns, m, o, s);
+  if (e != cudaSuccess) return cuda_status(e);
+  e = launch_sort_passes(codes, c->n, V, c->sorted_idx, mem + L.sort_off, L.sort, hist, reinterpret_cast<uint32_t*>(mem + L.lookback_off),
+                         c->status, s);
+  if (e != cudaSuccess) return cuda_status(e);
+  e = launch_tile_plan(c->gray_code, c->sorted_idx, c->n, c->tile_masks, c->block_order, words + 3, s);
+  return e != cudaSuccess ? cuda_status(e) : launch_status();
 }
 
 extern "C" int fgb_sparse_build_neighbor_map(const int32_t* in_coords, int64_t n_in, const int32_t* out_coords, int64_t n_out, int W,

@@ -22,6 +22,5 @@ int launch_split3(const float* src, float* dst, int64_t rows, int C, SplitMode m
 // hi[i] = tf32(src[i]), lo[i] = src[i] - hi[i]
 int launch_split2(const float* src, float* hi, float* lo, int64_t count, cudaStream_t s);
 
-inline int64_t align256(int64_t x) { return (x + 255) & ~int64_t(255); }
 
 }  // namespace fgb

@@ -21,14 +21,14 @@
 
 #include "fgb_common.cuh"
 #include "fgb_device.cuh"
+#include "fgb_sort.cuh"
 
 namespace fgb {
 
-constexpr int kDigitBits = 9;
-constexpr int kDigits = 1 << kDigitBits;   // 512
+constexpr int kDigitBits = kSortDigitBits;
+constexpr int kDigits = kSortDigits;
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortMaxPasses = 4;          // 32 bits / 9
 constexpr uint32_t kFlagAggregate = 1u << 30, kFlagPrefix = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr uint32_t kLookbackPolls = 1u << 22;   // of >= 32 ns each: far beyond any legitimate wait
 
@@ -206,38 +206,29 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 }
 
-struct SortLayout {
-  size_t keys_a, vals_a, keys_b, vals_b, control, status, total;
-  uint32_t tiles;
-  int items;
-};
-
 // Tiles of 4096 keys for long inputs (the per-tile bookkeeping -- 512 counters published and looked back over the
 // earlier tiles -- is then small beside the keys), of 2048 keys up to 400 k keys (measured: 52 against 58 us at 164 k keys,
 // 79 against 76 us at 660 k) and of 1024 keys for very short inputs, so that more CTAs share the work.
-static SortLayout sort_layout(int64_t n) {
-  auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+SortLayout sort_layout(int64_t n) {
   SortLayout L;
   L.items = n <= (int64_t(1) << 15) ? 4 : n <= 400000 ? 8 : 16;
   L.tiles = static_cast<uint32_t>(ceil_div(n > 0 ? n : 1, int64_t(kSortThreads) * L.items));
-  const size_t arr = align(size_t(n) * 4);
+  const size_t arr = align256(n * 4);
   L.keys_a = 0, L.vals_a = arr, L.keys_b = 2 * arr, L.vals_b = 3 * arr;
-  L.control = 4 * arr;                                                     // histograms [4][512], then the tickets [4]
-  L.status = L.control + align((kSortMaxPasses * kDigits + kSortMaxPasses) * 4);
-  L.total = L.status + align(size_t(kSortMaxPasses) * L.tiles * kDigits * 4);
+  L.buffer_bytes = 4 * arr;
   return L;
 }
 
 template <int kItems>
-static cudaError_t launch_pass(int pass, int passes, const int32_t* codes, char* ws, const SortLayout& L, uint32_t n, uint32_t flip, int64_t* out,
-                        int32_t* err, cudaStream_t s) {
+static cudaError_t launch_pass(int pass, int passes, const int32_t* codes, char* ws, const SortLayout& L, uint32_t n, uint32_t flip,
+                               int64_t* out, uint32_t* hist_all, uint32_t* lookback, int32_t* err, cudaStream_t s) {
   uint32_t* ka = reinterpret_cast<uint32_t*>(ws + L.keys_a);
   uint32_t* va = reinterpret_cast<uint32_t*>(ws + L.vals_a);
   uint32_t* kb = reinterpret_cast<uint32_t*>(ws + L.keys_b);
   uint32_t* vb = reinterpret_cast<uint32_t*>(ws + L.vals_b);
-  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.control) + pass * kDigits;
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(ws + L.control) + kSortMaxPasses * kDigits + pass;
-  uint32_t* status = reinterpret_cast<uint32_t*>(ws + L.status) + size_t(pass) * L.tiles * kDigits;
+  const uint32_t* hist = hist_all + pass * kDigits;
+  uint32_t* ticket = hist_all + kSortMaxPasses * kDigits + pass;
+  uint32_t* status = lookback + size_t(pass) * L.tiles * kDigits;
   // passes alternate between the two buffer pairs: pass 0 writes a, pass 1 reads a and writes b, ...
   const uint32_t* kin = (pass & 1) ? ka : kb;
   const uint32_t* vin = (pass & 1) ? va : vb;
@@ -245,23 +236,39 @@ static cudaError_t launch_pass(int pass, int passes, const int32_t* codes, char*
   uint32_t* vout = (pass & 1) ? vb : va;
   const int shift = pass * kDigitBits;
   const bool first = pass == 0, last = pass == passes - 1;
-  cudaError_t rc;
-  if (first && last)
-    rc = launch_chained(sort_pass_kernel<kItems, true, true>, dim3(L.tiles), dim3(kSortThreads), 0, s, codes, kin, vin, kout, vout, out, n, shift, flip, hist, ticket, status, err);
-  else if (first)
-    rc = launch_chained(sort_pass_kernel<kItems, true, false>, dim3(L.tiles), dim3(kSortThreads), 0, s, codes, kin, vin, kout, vout, out, n, shift, flip, hist, ticket, status, err);
-  else if (last)
-    rc = launch_chained(sort_pass_kernel<kItems, false, true>, dim3(L.tiles), dim3(kSortThreads), 0, s, codes, kin, vin, kout, vout, out, n, shift, flip, hist, ticket, status, err);
-  else
-    rc = launch_chained(sort_pass_kernel<kItems, false, false>, dim3(L.tiles), dim3(kSortThreads), 0, s, codes, kin, vin, kout, vout, out, n, shift, flip, hist, ticket, status, err);
-  return rc;
+  auto kernel = first && last ? sort_pass_kernel<kItems, true, true>
+                : first       ? sort_pass_kernel<kItems, true, false>
+                : last        ? sort_pass_kernel<kItems, false, true>
+                              : sort_pass_kernel<kItems, false, false>;
+  return launch_chained(kernel, dim3(L.tiles), dim3(kSortThreads), 0, s, codes, kin, vin, kout, vout, out, n, shift, flip, hist, ticket, status,
+                        err);
 }
+
+cudaError_t launch_sort_passes(const int32_t* codes, int64_t n, int key_bits, int64_t* sorted_idx, char* buffers, const SortLayout& L,
+                               uint32_t* hist, uint32_t* lookback, int32_t* err, cudaStream_t s) {
+  const int passes = sort_passes_of(key_bits);
+  const uint32_t flip = sort_flip_of(key_bits), n32 = static_cast<uint32_t>(n);
+  for (int pass = 0; pass < passes; ++pass) {
+    const cudaError_t e = L.items == 16 ? launch_pass<16>(pass, passes, codes, buffers, L, n32, flip, sorted_idx, hist, lookback, err, s)
+                          : L.items == 8 ? launch_pass<8>(pass, passes, codes, buffers, L, n32, flip, sorted_idx, hist, lookback, err, s)
+                                         : launch_pass<4>(pass, passes, codes, buffers, L, n32, flip, sorted_idx, hist, lookback, err, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// workspace of the stand-alone call: buffers, histograms and tickets, look-back words
+static size_t sort_control_off(const SortLayout& L) { return L.buffer_bytes; }
+static size_t sort_lookback_off(const SortLayout& L) {
+  return sort_control_off(L) + align256((kSortMaxPasses * kDigits + kSortMaxPasses) * 4);
+}
+static size_t sort_total(const SortLayout& L) { return sort_lookback_off(L) + align256(int64_t(kSortMaxPasses) * L.tiles * kDigits * 4); }
 
 }  // namespace fgb
 
 extern "C" int64_t fgb_pp_sorted_idx_workspace_bytes(int64_t n) {
   if (n < 0 || n >= (int64_t(1) << 30)) return FGB_E_SIZE;
-  return static_cast<int64_t>(fgb::sort_layout(n).total);
+  return static_cast<int64_t>(fgb::sort_total(fgb::sort_layout(n)));
 }
 
 extern "C" int fgb_pp_sorted_idx(const int32_t* binary_code, int64_t n, int key_bits, int64_t* sorted_idx, void* workspace,
@@ -273,27 +280,19 @@ extern "C" int fgb_pp_sorted_idx(const int32_t* binary_code, int64_t n, int key_
   if (!binary_code || !sorted_idx || !workspace) return FGB_E_NULL;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
   const SortLayout L = sort_layout(n);
-  if (workspace_bytes < static_cast<int64_t>(L.total)) return FGB_E_WORKSPACE;
+  if (workspace_bytes < static_cast<int64_t>(sort_total(L))) return FGB_E_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
-  const int passes = (key_bits + kDigitBits - 1) / kDigitBits;
-  // Codes with fewer than 32 significant bits are non-negative; with 32 bits they are signed, and flipping the top
-  // bit makes the unsigned digit order the signed order.
-  const uint32_t flip = key_bits == 32 ? 0x80000000u : 0u;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + sort_control_off(L));
   // histograms, tickets and the look-back words start at zero
-  int rc = cuda_status(cudaMemsetAsync(ws + L.control, 0, L.total - L.control, s));
+  int rc = cuda_status(cudaMemsetAsync(hist, 0, sort_total(L) - sort_control_off(L), s));
   if (rc != FGB_OK) return rc;
   // keys per CTA of the histogram: 1024 up to 400 k keys, 2048 beyond (measured: 42 / 43.5 / 46.5 us for the whole sort at
   // 164 k keys with 1024 / 2048 / 4096; 70.5 / 68.7 / 70.6 us at 660 k), at most eight CTAs per SM
   const unsigned hist_grid = static_cast<unsigned>(std::min<int64_t>(ceil_div(n, n <= 400000 ? 1024 : 2048), 148 * 8));
-  sort_histogram_kernel<<<hist_grid, kSortThreads, 0, s>>>(binary_code, static_cast<uint32_t>(n), passes, flip,
-                                                          reinterpret_cast<uint32_t*>(ws + L.control));
-  for (int pass = 0; pass < passes; ++pass) {
-    cudaError_t e;
-    if (L.items == 16) e = launch_pass<16>(pass, passes, binary_code, ws, L, static_cast<uint32_t>(n), flip, sorted_idx, status, s);
-    else if (L.items == 8) e = launch_pass<8>(pass, passes, binary_code, ws, L, static_cast<uint32_t>(n), flip, sorted_idx, status, s);
-    else e = launch_pass<4>(pass, passes, binary_code, ws, L, static_cast<uint32_t>(n), flip, sorted_idx, status, s);
-    if (e != cudaSuccess) return cuda_status(e);
-  }
-  return launch_status();
+  sort_histogram_kernel<<<hist_grid, kSortThreads, 0, s>>>(binary_code, static_cast<uint32_t>(n), sort_passes_of(key_bits), sort_flip_of(key_bits),
+                                                          hist);
+  const cudaError_t e = launch_sort_passes(binary_code, n, key_bits, sorted_idx, ws, L, hist, reinterpret_cast<uint32_t*>(ws + sort_lookback_off(L)),
+                                           status, s);
+  return e != cudaSuccess ? cuda_status(e) : launch_status();
 }

@@ -63,7 +63,12 @@ struct WgradParams {
   uint32_t idesc;
   uint32_t tmem_cols;
   int order;      // unit enumeration: 0 = offset-major, 1 = chunk-major
+  const char* bias_src;   // [bias_rows, Co] matrix whose column sums are wanted (the bias gradient), or null
+  int64_t bias_rows;
+  float* bias_partial;    // [bias_ctas, Co]
+  int bias_ctas;
   int32_t* status;
+  int32_t* status_mirror;
 };
 
 struct WgradSmem {
@@ -168,12 +173,61 @@ __host__ __device__ __forceinline__ uint32_t wg_band_share(uint32_t nkb, uint32_
   return base + (q < rem ? 1u : 0u);
 }
 
+// Column sums of this CTA's share of the rows of `src` ([rows, Co], Co * sizeof(T) a multiple of 16), written to
+// partial[cta, :].  Run by the 128 threads of the epilogue warps while the CTA's pipeline fills and runs: they have
+// nothing else to do until the accumulator is complete, so the bias gradient costs no launch and next to no time
+// (before: a kernel pair on a side stream with its fork and join, 24 + 12 us beside the conv kernels at N = 164 k,
+// C = 256, and five driver calls).  A thread owns one 16-byte column of every nrg-th row, four rows in flight.
+template <typename T>
+__device__ __forceinline__ void bias_share(const T* __restrict__ src, int64_t rows, int Co, float* __restrict__ partial, int cta, int ctas,
+                                           float* s_acc /* [128 * 16 / sizeof(T)] */, int tid) {
+  constexpr int kVec = 16 / sizeof(T);
+  const int64_t per = (rows + ctas - 1) / ctas;
+  const int64_t r0 = cta * per, r1 = min(rows, r0 + per);
+  const int ncg = Co / kVec;
+  for (int cg0 = 0; cg0 < ncg; cg0 += 128) {
+    const int n_here = min(128, ncg - cg0), nrg = 128 / n_here;
+    const int cg = tid % n_here, rg = tid / n_here;  // threads with rg == nrg have no rows
+    float acc[4][kVec];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) acc[u][i] = 0.f;
+    if (rg < nrg) {
+      for (int64_t r = r0 + rg; r < r1; r += 4 * nrg) {
+        uint4 w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          w[u] = r + u * nrg < r1 ? __ldg(reinterpret_cast<const uint4*>(src + (r + u * nrg) * Co) + cg0 + cg) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const T* e = reinterpret_cast<const T*>(&w[u]);
+#pragma unroll
+          for (int i = 0; i < kVec; ++i) acc[u][i] += static_cast<float>(e[i]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) s_acc[tid * kVec + i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    for (int c = tid; c < n_here * kVec; c += 128) {
+      float sum = 0.f;
+      for (int k = 0; k < nrg; ++k) sum += s_acc[k * n_here * kVec + c];  // fixed order
+      partial[size_t(cta) * Co + cg0 * kVec + c] = sum;
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+  }
+}
+
 // kRows = pairs of a stage / 32 = pair rows per gather thread.  kBanded: the CTA walks its share of every row band (see
 // above); otherwise one contiguous run of k-blocks of its offset's list, without the per-band tables in the gather loop
 // (that loop's bookkeeping alone costs 2-3 % where bands bring nothing).
-template <int kElem, int kRows, bool kBanded>
+template <int kDtype, int kRows, bool kBanded>
 __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradParams p) {
-  constexpr bool kTF32 = (kElem == 4);
+  constexpr bool kTF32 = (kDtype == FGB_F32_TF32);
+  constexpr int kElem = kTF32 ? 4 : 2;
+  using T = typename std::conditional<kTF32, float, typename std::conditional<kDtype == FGB_F16, __half, __nv_bfloat16>::type>::type;
+  __shared__ float s_bias[128 * 16 / sizeof(T)];
   constexpr int kUmmaK = 32 / kElem;      // 16 for 16-bit types, 8 for tf32
   constexpr int kChunkElems = 128 / kElem;
   // MN-major operands: 16-bit types use the plain 128-byte swizzle (8-row K groups, 1024 B apart);
@@ -201,8 +255,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     const uint32_t ukb = wg_plan_unit_kb(p.seg, p.V, p.kb, static_cast<uint32_t>(p.target_units), lane);
     int v = -1, j = -1;
     if (lane == 0) {
-      const bool skip = p.status != nullptr && *reinterpret_cast<volatile const int32_t*>(p.status) != 0;
-      if (skip || !wg_find_unit(p.seg, p.V, p.kb, static_cast<int>(ukb), p.order, bid, &v, &j)) v = j = -1;
+      const int32_t skip = p.status != nullptr ? *reinterpret_cast<volatile const int32_t*>(p.status) : 0;
+      if (skip != 0 && blockIdx.x == 0) mirror_code(p.status_mirror, skip);
+      if (skip != 0 || !wg_find_unit(p.seg, p.V, p.kb, static_cast<int>(ukb), p.order, bid, &v, &j)) v = j = -1;
       ctl->unit_v = v, ctl->unit_j = j, ctl->unit_kb = static_cast<int>(ukb);
     }
     v = __shfl_sync(0xffffffffu, v, 0), j = __shfl_sync(0xffffffffu, j, 0);
@@ -241,7 +296,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
   }
   __syncthreads();
   const int v = ctl->unit_v, unit_j = ctl->unit_j, unit_kb = ctl->unit_kb;
-  if (v < 0) return;  // grid is sized for the worst case; also the no-op path after a soft error
+  const bool sums_bias = warp < 4 && p.bias_src != nullptr && blockIdx.x < static_cast<uint32_t>(p.bias_ctas);
+  if (v < 0) {  // grid is sized for the worst case; also the no-op path after a soft error
+    if (sums_bias) bias_share<T>(reinterpret_cast<const T*>(p.bias_src), p.bias_rows, p.Co, p.bias_partial, blockIdx.x, p.bias_ctas, s_bias, tid);
+    return;
+  }
   const int co0 = co_group * p.mt * 128;
   const int ci0 = ci_tile * p.bn;
   // contiguous walk: k-blocks [k_begin, k_begin + total) of the offset's list, full units and a shorter last one
@@ -383,6 +442,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     // and nothing is in flight), 16-byte pieces XOR-swizzled by the row, and come back so that eight consecutive
     // lanes hold one row's 128 contiguous bytes: every store instruction then writes four whole lines of the slab
     // instead of one 16-byte piece in each of 32 lines.
+    if (sums_bias) bias_share<T>(reinterpret_cast<const T*>(p.bias_src), p.bias_rows, p.Co, p.bias_partial, blockIdx.x, p.bias_ctas, s_bias, tid);
     const uint32_t slab = wg_slab_of(p.seg, p.kb, unit_kb, v, unit_j);
     mbar_wait(&ctl->acc_full, 0, abort_flag);
     tc_fence_after_sync();
@@ -422,16 +482,49 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, p.tmem_cols);
   }
-  if (tid == 0 && ctl->abort_flag) report(p.status, FGB_S_WAIT_TIMEOUT);
+  if (tid == 0 && ctl->abort_flag) {
+    report(p.status, FGB_S_WAIT_TIMEOUT);
+    mirror_code(p.status_mirror, FGB_S_WAIT_TIMEOUT);
+  }
+}
+
+// The bias gradient's last step: out[c] = sum over the CTAs' partial sums, in CTA order; 32 columns per CTA
+template <typename T>
+__device__ __forceinline__ void bias_finish(const float* __restrict__ partial, int ctas, int Co, int block, int blocks, T* __restrict__ out) {
+  __shared__ float s_acc[8][32];
+  const int lane = threadIdx.x & 31, rg = threadIdx.x >> 5;
+  for (int c0 = block * 32; c0 < Co; c0 += blocks * 32) {
+    const int c = c0 + lane;
+    float acc = 0.f;
+    if (c < Co) {
+#pragma unroll 4
+      for (int b = rg; b < ctas; b += 8) acc += partial[size_t(b) * Co + c];
+    }
+    s_acc[rg][lane] = acc;
+    __syncthreads();
+    if (rg == 0 && c < Co) {
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += s_acc[k][lane];
+      out[c] = static_cast<T>(sum);
+    }
+    __syncthreads();
+  }
 }
 
 // out[co, v, ci] = sum over the slabs of offset v, in slab order; written as dtype and/or fp32
 template <typename T>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, const uint32_t* __restrict__ seg, int kb,
                                                             int target_units, int Co, int V, int Ci, T* __restrict__ out,
-                                                            float* __restrict__ out_f32, int accumulate) {
+                                                            float* __restrict__ out_f32, int accumulate,
+                                                            const float* __restrict__ bias_partial, int bias_ctas, T* __restrict__ bias_out) {
   __shared__ int s_unit_kb;
   chain_release();
+  if (blockIdx.y == static_cast<unsigned>(V)) {  // the extra row of CTAs of a launch that also finishes the bias gradient
+    chain_wait();
+    bias_finish<T>(bias_partial, bias_ctas, Co, blockIdx.x, gridDim.x, bias_out);
+    return;
+  }
   // the plan depends on the segment table only (written by the cache build): it is made while the wgrad kernel runs
   if (threadIdx.x < 32) {
     const uint32_t ukb = wg_plan_unit_kb(seg, V, kb, static_cast<uint32_t>(target_units), threadIdx.x);
@@ -691,24 +784,41 @@ extern "C" int64_t fgb_sparse_conv_workspace_bytes(int pass, int64_t n_out, int6
 namespace fgb {
 // One launcher per kernel instance: the dynamic shared-memory limit is a property of (kernel, device), and all
 // instances share one function-pointer type, so the table must hang on the template arguments, not on the type.
-template <int kElem, int kRows, bool kBanded>
+template <int kDtype, int kRows, bool kBanded>
 static int launch_wgrad_instance(int64_t grid, size_t smem, const WgradParams& p, cudaStream_t s) {
   static PerDeviceTable configured;
-  const int rc = ensure_dynamic_smem(configured, subm_wgrad_kernel<kElem, kRows, kBanded>, smem);
+  const int rc = ensure_dynamic_smem(configured, subm_wgrad_kernel<kDtype, kRows, kBanded>, smem);
   if (rc != FGB_OK) return rc;
-  subm_wgrad_kernel<kElem, kRows, kBanded><<<static_cast<unsigned>(grid), kWgThreads, smem, s>>>(p);
+  subm_wgrad_kernel<kDtype, kRows, kBanded><<<static_cast<unsigned>(grid), kWgThreads, smem, s>>>(p);
   return launch_status();
 }
-template <int kElem, int kRows>
+template <int kDtype>
 static int launch_wgrad(int64_t grid, size_t smem, const WgradParams& p, cudaStream_t s) {
-  return p.bands > 1 ? launch_wgrad_instance<kElem, kRows, true>(grid, smem, p, s) : launch_wgrad_instance<kElem, kRows, false>(grid, smem, p, s);
+  const bool banded = p.bands > 1;
+  switch (p.kb / 32) {
+    case 4:
+      return banded ? launch_wgrad_instance<kDtype, 4, true>(grid, smem, p, s) : launch_wgrad_instance<kDtype, 4, false>(grid, smem, p, s);
+    case 2:
+      return banded ? launch_wgrad_instance<kDtype, 2, true>(grid, smem, p, s) : launch_wgrad_instance<kDtype, 2, false>(grid, smem, p, s);
+    default:
+      return banded ? launch_wgrad_instance<kDtype, 1, true>(grid, smem, p, s) : launch_wgrad_instance<kDtype, 1, false>(grid, smem, p, s);
+  }
 }
+
+// bias gradient computed along with the weight gradient: source rows, result, and room for the CTAs' partial sums
+struct BiasJob {
+  const void* src = nullptr;
+  int64_t rows = 0;
+  float* partial = nullptr;  // [kBiasCtas, Co]
+  void* out = nullptr;
+};
+constexpr int kBiasCtas = 148;  // the CTAs of a launch's first wave share the rows
 
 // one wgrad pass over operands of element type `dtype` (never FGB_F32_IEEE): partial slabs, then the ordered sum
 static int wgrad_pass(const void* grad_out, const void* feats, const uint32_t* vs_i, const uint32_t* vs_o, const uint32_t* seg,
                       const uint32_t* block_offsets, void* grad_weight, float* grad_weight_f32, int64_t n_out, int64_t n_in,
                       int64_t n_pairs, int Ci, int Co, int V, int dtype, int splitk, float* slabs, int accumulate, int32_t* status,
-                      cudaStream_t s) {
+                      cudaStream_t s, const BiasJob& bias = BiasJob()) {
   const int eb = elem_bytes(dtype);
   const WgradPlan w = plan_wgrad(Ci, Co, eb);
   WgradParams p;
@@ -731,26 +841,34 @@ static int wgrad_pass(const void* grad_out, const void* feats, const uint32_t* v
   p.tmem_cols = w.tmem_cols;
   p.order = 0;  // offset-major: measured faster than chunk-major on B200 (chunk-major makes every SM stream the same rows at once)
   p.status = status;
+  p.status_mirror = status_mirror(status);
   const int64_t grid = max_units * w.co_groups * w.ci_tiles;
   if (grid > 0x7FFFFFFF) return FGB_E_SIZE;
-  const int rows = w.kb / 32;
-  int rc;
-  if (eb == 2) rc = rows == 4 ? launch_wgrad<2, 4>(grid, w.smem, p, s) : rows == 2 ? launch_wgrad<2, 2>(grid, w.smem, p, s) : launch_wgrad<2, 1>(grid, w.smem, p, s);
-  else rc = rows == 4 ? launch_wgrad<4, 4>(grid, w.smem, p, s) : rows == 2 ? launch_wgrad<4, 2>(grid, w.smem, p, s) : launch_wgrad<4, 1>(grid, w.smem, p, s);
+  p.bias_src = static_cast<const char*>(bias.src);
+  p.bias_rows = bias.rows;
+  p.bias_partial = bias.partial;
+  p.bias_ctas = static_cast<int>(std::min<int64_t>(grid, kBiasCtas));
+  int rc = dtype == FGB_F16    ? launch_wgrad<FGB_F16>(grid, w.smem, p, s)
+           : dtype == FGB_BF16 ? launch_wgrad<FGB_BF16>(grid, w.smem, p, s)
+                               : launch_wgrad<FGB_F32_TF32>(grid, w.smem, p, s);
   if (rc != FGB_OK) return rc;
-  const dim3 rgrid(static_cast<unsigned>(ceil_div(int64_t(Co) * Ci, 1024)), static_cast<unsigned>(V));
+  const dim3 rgrid(static_cast<unsigned>(ceil_div(int64_t(Co) * Ci, 1024)), static_cast<unsigned>(V + (bias.src != nullptr ? 1 : 0)));
+  const float* slabs_in = slabs;
+  const float* bias_in = bias.partial;
   switch (dtype) {
     case FGB_F16:
-      rc = cuda_status(launch_chained(splitk_reduce_kernel<__half>, rgrid, dim3(256), 0, s, static_cast<const float*>(slabs), seg, p.kb,
-                                      p.target_units, Co, V, Ci, static_cast<__half*>(grad_weight), grad_weight_f32, 0));
+      rc = cuda_status(launch_chained(splitk_reduce_kernel<__half>, rgrid, dim3(256), 0, s, slabs_in, seg, p.kb, p.target_units, Co, V, Ci,
+                                      static_cast<__half*>(grad_weight), grad_weight_f32, 0, bias_in, p.bias_ctas, static_cast<__half*>(bias.out)));
       break;
     case FGB_BF16:
-      rc = cuda_status(launch_chained(splitk_reduce_kernel<__nv_bfloat16>, rgrid, dim3(256), 0, s, static_cast<const float*>(slabs), seg,
-                                      p.kb, p.target_units, Co, V, Ci, static_cast<__nv_bfloat16*>(grad_weight), grad_weight_f32, 0));
+      rc = cuda_status(launch_chained(splitk_reduce_kernel<__nv_bfloat16>, rgrid, dim3(256), 0, s, slabs_in, seg, p.kb, p.target_units, Co, V,
+                                      Ci, static_cast<__nv_bfloat16*>(grad_weight), grad_weight_f32, 0, bias_in, p.bias_ctas,
+                                      static_cast<__nv_bfloat16*>(bias.out)));
       break;
     default:
-      rc = cuda_status(launch_chained(splitk_reduce_kernel<float>, rgrid, dim3(256), 0, s, static_cast<const float*>(slabs), seg, p.kb,
-                                      p.target_units, Co, V, Ci, static_cast<float*>(grad_weight), grad_weight_f32, accumulate));
+      rc = cuda_status(launch_chained(splitk_reduce_kernel<float>, rgrid, dim3(256), 0, s, slabs_in, seg, p.kb, p.target_units, Co, V, Ci,
+                                      static_cast<float*>(grad_weight), grad_weight_f32, accumulate, bias_in, p.bias_ctas,
+                                      static_cast<float*>(bias.out)));
   }
   return rc != FGB_OK ? rc : launch_status();
 }
@@ -764,12 +882,12 @@ extern "C" int fgb_subm_conv_wgrad(const void* grad_out, const void* feats, cons
                                grad_weight_f32, n, n, n_pairs, Ci, Co, V, dtype, splitk, workspace, workspace_bytes, status, stream);
 }
 
-extern "C" int fgb_sparse_conv_wgrad(const void* grad_out, const void* feats, const uint32_t* valid_signal_i,
+namespace fgb {
+static int wgrad_impl(const void* grad_out, const void* feats, const uint32_t* valid_signal_i,
                                      const uint32_t* valid_signal_o, const uint32_t* valid_signal_seg, const uint32_t* block_offsets,
                                      void* grad_weight, float* grad_weight_f32, int64_t n_out, int64_t n_in, int64_t n_pairs, int Ci,
                                      int Co, int V, int dtype, int splitk, void* workspace, int64_t workspace_bytes, int32_t* status,
-                                     void* stream) {
-  using namespace fgb;
+                                     void* stream, void* grad_bias = nullptr) {
   const int eb = elem_bytes(dtype);
   if (eb == 0) return FGB_E_DTYPE;
   if (n_out < 0 || n_in < 0 || n_pairs < 0 || n_pairs > n_out * V || Ci <= 0 || Co <= 0 || V < 1 || V > 32 || splitk < 1 || splitk > 1024)
@@ -782,12 +900,20 @@ extern "C" int fgb_sparse_conv_wgrad(const void* grad_out, const void* feats, co
        reinterpret_cast<uintptr_t>(grad_weight_f32)) & 15)
     return FGB_E_ALIGN;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
-  if (workspace_bytes < fgb_sparse_conv_workspace_bytes(2, n_out, n_in, Ci, Co, V, dtype, splitk)) return FGB_E_WORKSPACE;
+  const int64_t own_bytes = fgb_sparse_conv_workspace_bytes(2, n_out, n_in, Ci, Co, V, dtype, splitk);
+  BiasJob bias;
+  if (grad_bias != nullptr) {
+    bias.src = grad_out;
+    bias.rows = n_out;
+    bias.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + own_bytes);
+    bias.out = grad_bias;
+  }
+  if (workspace_bytes < own_bytes + (grad_bias != nullptr ? int64_t(kBiasCtas) * Co * 4 : 0)) return FGB_E_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* slabs = static_cast<float*>(workspace);
   if (dtype != FGB_F32_IEEE)
     return wgrad_pass(grad_out, feats, valid_signal_i, valid_signal_o, valid_signal_seg, block_offsets, grad_weight, grad_weight_f32,
-                      n_out, n_in, n_pairs, Ci, Co, V, dtype, splitk, slabs, 0, status, s);
+                      n_out, n_in, n_pairs, Ci, Co, V, dtype, splitk, slabs, 0, status, s, bias);
   // fp32-accurate: g_hi*x_hi + g_hi*x_lo + g_lo*x_hi, three passes adding into the fp32 output
   char* base = static_cast<char*>(workspace) + align256(int64_t(Ci) * V * Co * 4 * (int64_t(splitk) + 1));
   float* x_hi = reinterpret_cast<float*>(base);
@@ -803,10 +929,74 @@ extern "C" int fgb_sparse_conv_wgrad(const void* grad_out, const void* feats, co
   const float* xa[3] = {x_hi, x_lo, x_hi};
   for (int pass = 0; pass < 3; ++pass) {
     rc = wgrad_pass(ga[pass], xa[pass], valid_signal_i, valid_signal_o, valid_signal_seg, block_offsets, grad_weight, grad_weight_f32,
-                    n_out, n_in, n_pairs, Ci, Co, V, FGB_F32_TF32, splitk, slabs, pass > 0, status, s);
+                    n_out, n_in, n_pairs, Ci, Co, V, FGB_F32_TF32, splitk, slabs, pass > 0, status, s, pass == 0 ? bias : BiasJob());
     if (rc != FGB_OK) return rc;
   }
   return FGB_OK;
+}
+}  // namespace fgb
+
+extern "C" int fgb_sparse_conv_wgrad(const void* grad_out, const void* feats, const uint32_t* valid_signal_i,
+                                     const uint32_t* valid_signal_o, const uint32_t* valid_signal_seg, const uint32_t* block_offsets,
+                                     void* grad_weight, float* grad_weight_f32, int64_t n_out, int64_t n_in, int64_t n_pairs, int Ci,
+                                     int Co, int V, int dtype, int splitk, void* workspace, int64_t workspace_bytes, int32_t* status,
+                                     void* stream) {
+  return fgb::wgrad_impl(grad_out, feats, valid_signal_i, valid_signal_o, valid_signal_seg, block_offsets, grad_weight, grad_weight_f32,
+                         n_out, n_in, n_pairs, Ci, Co, V, dtype, splitk, workspace, workspace_bytes, status, stream);
+}
+
+extern "C" int64_t fgb_wgrad_call_workspace_bytes(const fgb_wgrad_call* c) {
+  if (!c) return FGB_E_NULL;
+  const int splitk = fgb_wgrad_default_splitk(c->n_pairs, c->ci, c->co, c->v, c->dtype);
+  if (splitk < 1) return splitk;
+  const int64_t own = fgb_sparse_conv_workspace_bytes(2, c->n_out, c->n_in, c->ci, c->co, c->v, c->dtype, splitk);
+  return own < 0 ? own : own + (c->grad_bias != nullptr ? int64_t(fgb::kBiasCtas) * c->co * 4 : 0);
+}
+
+extern "C" int fgb_wgrad_call_run(const fgb_wgrad_call* c, void* stream) {
+  if (!c) return FGB_E_NULL;
+  const int splitk = fgb_wgrad_default_splitk(c->n_pairs, c->ci, c->co, c->v, c->dtype);
+  if (splitk < 1) return splitk;
+  return fgb::wgrad_impl(c->grad_out, c->feats, c->valid_signal_i, c->valid_signal_o, c->valid_signal_seg, c->block_offsets, c->grad_weight,
+                         nullptr, c->n_out, c->n_in, c->n_pairs, c->ci, c->co, c->v, c->dtype, splitk, c->workspace, c->workspace_bytes,
+                         c->status, stream, c->grad_bias);
+}
+
+namespace fgb {
+// one thread per 2-byte (kUnit = uint16_t) or 4-byte word of the destination
+template <typename U>
+__global__ void __launch_bounds__(256) resize_rows_kernel(const U* __restrict__ src, U* __restrict__ dst, int64_t rows_in, int64_t words, int w_in,
+                                                          int w_out) {
+  chain_release();
+  chain_wait();
+  for (int64_t e = blockIdx.x * int64_t(256) + threadIdx.x; e < words; e += int64_t(gridDim.x) * 256) {
+    const int64_t r = e / w_out;
+    const int c = static_cast<int>(e - r * w_out);
+    dst[e] = c < w_in && r < rows_in ? src[r * w_in + c] : U(0);
+  }
+}
+}  // namespace fgb
+
+extern "C" int fgb_resize_rows(const void* src, void* dst, int64_t rows_in, int64_t rows_out, int64_t width_in, int64_t width_out, void* stream) {
+  using namespace fgb;
+  if (rows_in < 0 || rows_out < 0 || width_in < 0 || width_out < 0 || width_in > (1 << 30) || width_out > (1 << 30)) return FGB_E_SIZE;
+  if ((width_in | width_out) & 1) return FGB_E_ALIGN;
+  if (rows_out == 0 || width_out == 0) return FGB_OK;
+  if (!dst || (!src && rows_in > 0 && width_in > 0)) return FGB_E_NULL;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const bool wide = ((width_in | width_out | int64_t(reinterpret_cast<uintptr_t>(src)) | int64_t(reinterpret_cast<uintptr_t>(dst))) & 3) == 0;
+  const int unit = wide ? 4 : 2;
+  const int64_t words = rows_out * (width_out / unit);
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(ceil_div(words, 256), 148 * 16)));
+  const int w_in = static_cast<int>(width_in / unit), w_out = static_cast<int>(width_out / unit);
+  cudaError_t e;
+  if (wide)
+    e = launch_chained(resize_rows_kernel<uint32_t>, grid, dim3(256), 0, s, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst),
+                       rows_in, words, w_in, w_out);
+  else
+    e = launch_chained(resize_rows_kernel<uint16_t>, grid, dim3(256), 0, s, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst),
+                       rows_in, words, w_in, w_out);
+  return e != cudaSuccess ? cuda_status(e) : launch_status();
 }
 
 extern "C" int64_t fgb_bias_grad_workspace_bytes(int Co) { return Co <= 0 ? FGB_E_SIZE : int64_t(fgb::kBiasBlocks) * Co * 4; }

@@ -9,7 +9,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
-from .. import _cabi
+from .. import _cabi, _native
 from . import config
 
 _DTYPES = {torch.float16: _cabi.F16, torch.bfloat16: _cabi.BF16}
@@ -48,16 +48,21 @@ def _stream(device) -> int:
 # per-(device, stream) scratch and the device status word
 # --------------------------------------------------------------------------
 _scratch: Dict[tuple, torch.Tensor] = {}
-_status: Dict[int, torch.Tensor] = {}
 
-# Number of this library's own kernels launched so far.  Each wrapper adds the
-# number of kernels its C entry point launches.
-launch_count = 0
+# Kernels launched through the wrappers of this module; the native module counts its own.  ``launch_count`` (below) is
+# the number of this library's own kernels launched so far.
+_launches = 0
 
 
 def _count(k: int) -> None:
-    global launch_count
-    launch_count += k
+    global _launches
+    _launches += k
+
+
+def __getattr__(name: str):
+    if name == "launch_count":
+        return _launches + _native.ext().launches()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def workspace(device: torch.device, tag: str, nbytes: int) -> torch.Tensor:
@@ -76,11 +81,12 @@ def release_workspaces() -> None:
     _scratch.clear()
 
 
+def _device_index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
+
+
 def status_word(device: torch.device) -> torch.Tensor:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    if idx not in _status:
-        _status[idx] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status[idx]
+    return _native.ext().status_word(_device_index(device))
 
 
 def check_status(device: torch.device) -> None:
@@ -88,57 +94,26 @@ def check_status(device: torch.device) -> None:
     recorded a soft error."""
     word = status_word(device)
     code = int(word.item())
-    _status_pending.pop(_device_index(device), None)
     if code != 0:
+        torch.cuda.synchronize(device)   # kernels that still see the word would report it again
         word.zero_()
+        _native.ext().clear_mirror(_device_index(device))
         raise_for_status(code)
 
 
-def _device_index(device: torch.device) -> int:
-    return device.index if device.index is not None else torch.cuda.current_device()
-
-
-# device index -> (pinned host word, event recorded after the copy that fills it)
-_status_pending: Dict[int, tuple] = {}
-
-
 def poll_status(device: torch.device) -> None:
-    """Non-blocking look at the device status word, called by the conv wrappers
-    before they launch.
+    """Look at the device's soft errors, called by the conv wrappers before they launch.
 
     A kernel that hits a soft error (a bounded barrier wait that ran out, a full
-    hash table) records a code in the word and every later conv kernel on that
-    device returns at once while it is set, so the error must reach the caller:
-    this function queues a 4-byte copy of the word to pinned host memory and, on
-    a later call, once that copy has landed, looks at it.  A non-zero code clears
-    the word (so that the calls after the exception run normally) and raises
-    ``RuntimeError``.  Nothing here waits for the GPU; the error therefore
-    surfaces at the first conv call made after the device has reported it --
-    ``check_status`` is the synchronising variant."""
-    idx = _device_index(device)
-    entry = _status_pending.get(idx)
-    if entry is not None:
-        host, event = entry
-        if not event.query():
-            return  # the previous copy is still in flight: look again at the next call
-        code = int(host[0])
-        del _status_pending[idx]
-        if code != 0:
-            status_word(device).zero_()
-            raise_for_status(code)
-    else:
-        host = None
-    if host is None:
-        host = _status_host.get(idx)
-        if host is None:
-            host = _status_host[idx] = torch.zeros(1, dtype=torch.int32).pin_memory()
-    event = torch.cuda.Event()
-    host.copy_(status_word(device), non_blocking=True)
-    event.record(torch.cuda.current_stream(device))
-    _status_pending[idx] = (host, event)
-
-
-_status_host: Dict[int, torch.Tensor] = {}
+    hash table) records a code in the device status word and every later conv
+    kernel on that device returns at once while it is set, so the error must reach
+    the caller: the kernels store the code that they find or set to a word of
+    mapped host memory as well, and this function reads that word -- nothing is
+    queued and nothing waits.  A non-zero code clears the word (so that the calls
+    after the exception run normally) and raises ``RuntimeError``.  The error
+    therefore surfaces at the first conv call made after the device has reported
+    it; ``check_status`` is the synchronising variant."""
+    _native.ext().poll(_device_index(device))
 
 
 # --------------------------------------------------------------------------

@@ -15,7 +15,8 @@ from torch.autograd import Function
 
 from . import Algorithm
 from .. import spconv, utils
-from ... import kernels
+from ... import _native, kernels
+from ...kernels import config
 from .submanifold_conv3d import _MASKED, _gather_rows
 
 
@@ -253,6 +254,10 @@ class SparseConv3dFunction(Function):
             if not feats.is_cuda:
                 raise NotImplementedError("flexgemm_b200 kernels need CUDA tensors")
             assert weight.is_contiguous(), "Matrix weight must be contiguous"
+            out = _native.ext().conv(feats.detach(), weight.detach(), bias.detach() if bias is not None else None, neighbor_cache,
+                                     config.allow_tf32, True)
+            if out is not None:
+                return out
             tile = kernels.cuda.conv_tile_rows()
             return kernels.cuda.conv_fprop(
                 feats, weight.reshape(Co, V, Ci), bias.contiguous() if bias is not None else None,
@@ -282,6 +287,10 @@ class SparseConv3dFunction(Function):
             grad_output = grad_output.contiguous()
             assert feats.is_contiguous(), "Matrix input must be contiguous"
             assert weight.is_contiguous(), "Matrix weight must be contiguous"
+            got = _native.ext().conv_backward(grad_output, feats.detach(), weight.detach(), neighbor_cache, config.allow_tf32, True,
+                                              feats.requires_grad, weight.requires_grad, bias is not None and bias.requires_grad)
+            if got is not None:
+                return got
             w = weight.reshape(Co, V, Ci)
             join = None
             if bias is not None and bias.requires_grad:   # a small reduction: runs beside the conv kernels

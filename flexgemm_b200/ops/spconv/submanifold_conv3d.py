@@ -10,7 +10,8 @@ from torch.autograd import Function
 
 from . import Algorithm
 from .. import spconv, utils
-from ... import kernels
+from ... import _native, kernels
+from ...kernels import config
 
 _MASKED = (Algorithm.IMPLICIT_GEMM, Algorithm.IMPLICIT_GEMM_SPLITK,
            Algorithm.MASKED_IMPLICIT_GEMM, Algorithm.MASKED_IMPLICIT_GEMM_SPLITK)
@@ -92,38 +93,19 @@ class SubMConv3dFunction(Function):
         V = kernel_size[0] * kernel_size[1] * kernel_size[2]
         assert V <= 32, "Currently, the max kernel volume is 32 because kernel mask is encoded as uint32"
         assert all(int(k) % 2 == 1 for k in kernel_size), "Kernel extents must be odd"
-        n = coords.shape[0]
-        slots = max(int(spconv.HASHMAP_RATIO * n), n, 1)
-        table, key_bits = utils.init_table(shape, slots, coords.device)
-        built = kernels.cuda.subm_build_neighbor_map(coords, shape, kernel_size, dilation, table, key_bits, slots)
         if spconv.ALGORITHM == Algorithm.EXPLICIT_GEMM:
+            n = coords.shape[0]
+            slots = max(int(spconv.HASHMAP_RATIO * n), n, 1)
+            table, key_bits = utils.init_table(shape, slots, coords.device)
+            built = kernels.cuda.subm_build_neighbor_map(coords, shape, kernel_size, dilation, table, key_bits, slots)
             kernels.cuda.raise_for_status(int(built["meta"][-1].item()))
             return SubMConv3dNeighborCache(neighbor_map=built["neighbor_map"])
-
-        if needs_grad:
-            # The one host round trip of the build: the pair count sizes the lists, and
-            # the same copy brings the build's status word (hash table overflow).  The
-            # copy is queued before the sort so that the host wait overlaps the sort.
-            meta_host, copied = kernels.cuda.fetch_meta_async(built["meta"])
-        sorted_idx = kernels.cuda.sorted_idx_from_binary(built["binary_code"], V)
-        cache = SubMConv3dNeighborCache(neighbor_map=built["neighbor_map"], gray_code=built["gray_code"], sorted_idx=sorted_idx)
-        if needs_grad:
-            copied.synchronize()
-            kernels.cuda.raise_for_status(int(meta_host[-1]))
-            seg = built["valid_signal_seg"]
-            num_pairs = int(meta_host[V])
-            vs_i, vs_o = kernels.cuda.valid_signal(built["neighbor_map"], built["gray_code"], built["block_offsets"], seg, num_pairs,
-                                                   built["order_flag"])
-            cache["valid_signal_seg"] = seg
-            cache["valid_signal_i"] = vs_i
-            cache["valid_signal_o"] = vs_o
-            # not part of the reference's cache: where each 256-row block starts in every offset's pair list, which
-            # lets wgrad walk all lists in row bands that share L2
-            cache["pair_block_offsets"] = built["block_offsets"]
-        else:
-            # inference cache: nothing needs the host, so nothing synchronises; an
-            # overflowing table would show in this word, readable at any later time
-            cache["build_status"] = built["meta"][-1:]
+        utils.hashmap_key_bits(shape)   # raises for a grid that no key can hold
+        # map, row order, tile masks and schedule in one native call; the one host round trip of a training cache is the
+        # pair count that sizes the lists
+        cache = _native.ext().subm_cache(SubMConv3dNeighborCache, coords, tuple(int(s) for s in shape), tuple(int(k) for k in kernel_size),
+                                         tuple(int(d) for d in dilation), float(spconv.HASHMAP_RATIO), bool(needs_grad))
+        assert cache is not None, "coords should be an [N, 4] tensor"
         return cache
 
     @staticmethod
@@ -170,6 +152,10 @@ class SubMConv3dFunction(Function):
             if not feats.is_cuda:
                 raise NotImplementedError("flexgemm_b200 kernels need CUDA tensors")
             assert weight.is_contiguous(), "Matrix weight must be contiguous"
+            out = _native.ext().conv(feats.detach(), weight.detach(), bias.detach() if bias is not None else None, neighbor_cache,
+                                     config.allow_tf32, False)
+            if out is not None:
+                return out
             tile = kernels.cuda.conv_tile_rows()
             return kernels.cuda.conv_fprop(
                 feats, weight.reshape(Co, V, Ci), bias.contiguous() if bias is not None else None,
@@ -201,6 +187,10 @@ class SubMConv3dFunction(Function):
             grad_output = grad_output.contiguous()
             assert feats.is_contiguous(), "Matrix input must be contiguous"
             assert weight.is_contiguous(), "Matrix weight must be contiguous"
+            got = _native.ext().conv_backward(grad_output, feats.detach(), weight.detach(), neighbor_cache, config.allow_tf32, False,
+                                              feats.requires_grad, weight.requires_grad, bias is not None and bias.requires_grad)
+            if got is not None:
+                return got
             w = weight.reshape(Co, V, Ci)
             join = None
             if bias is not None and bias.requires_grad:   # a small reduction: runs beside the conv kernels
@@ -265,4 +255,9 @@ def sparse_submanifold_conv3d(feats: torch.Tensor, coords: torch.Tensor, shape: 
     Returns:
         (output [N, Co], neighbor_cache)
     """
+    if spconv.ALGORITHM in _MASKED:
+        got = _native.ext().subm_conv(SubMConv3dNeighborCache, feats, coords, shape, weight, bias, neighbor_cache, dilation,
+                                      spconv.HASHMAP_RATIO, config.allow_tf32)
+        if got is not None:
+            return got
     return SubMConv3dFunction.apply(feats, coords, shape, neighbor_cache, weight, bias, dilation)

@@ -50,6 +50,13 @@ extern "C" {
 #define FGB_ACT_NONE 0
 #define FGB_ACT_SILU 1  /* x * sigmoid(x) */
 
+/* Registers a host-visible copy of a device status word (mirror: a device
+ * pointer to mapped pinned memory, one int32; null = none).  The conv kernels
+ * launched with that status word store the code they find or set there to the
+ * mirror too, so a host sees a soft error by reading its own memory.  At most 64
+ * words. (No counterpart in the reference.) */
+int fgb_status_set_mirror(const int32_t* status, int32_t* mirror);
+
 const char* fgb_version(void);
 const char* fgb_error_string(int code);
 
@@ -524,6 +531,95 @@ int fgb_indice_weighted_sum_fwd(const void* feats, const uint32_t* indices, cons
  * in the feature dtype. */
 int fgb_indice_weighted_sum_bwd(const void* grad_out, const uint32_t* indices, const float* weight,
                                 float* grad_feats_f32, int64_t M, int64_t N, int C, int V, int dtype, void* stream);
+
+/* ------------------------------------------------------------------------
+ * One-struct calls of the conv passes (what the torch host code uses)
+ * --------------------------------------------------------------------- */
+
+/* The passes above with their arguments in one struct and two differences that
+ * save stream operations: the caller hands in `counters`, device words that are
+ * zero and that no other call uses (one word; a pool zeroed now and then costs
+ * nothing per call, where a memset per launch does), and the weight gradient
+ * call computes the bias gradient in the same two launches.
+ *
+ * fprop: x = feats [n_src, ci], out [n, co]; dgrad: x = grad_out [n_src, co],
+ * out = grad_feats [n, ci], mirror = 1 for the forward map of a submanifold conv,
+ * 0 for a backward map.  The map, order and masks have n rows. */
+typedef struct fgb_conv_call {
+  const void* x;
+  const void* weight;
+  const void* bias;
+  const uint32_t* neighbor_map;
+  const int64_t* sorted_idx;
+  const uint32_t* tile_masks;
+  const uint32_t* block_order;
+  void* out;
+  int64_t n, n_src;
+  int32_t ci, co, v, dtype, mirror;
+  void* workspace;
+  int64_t workspace_bytes;
+  uint32_t* counters;
+  int32_t* status;
+} fgb_conv_call;
+/* pass 0 = fprop, 1 = dgrad */
+int64_t fgb_conv_call_workspace_bytes(const fgb_conv_call* call, int pass);
+int fgb_conv_call_fprop(const fgb_conv_call* call, void* stream);
+int fgb_conv_call_dgrad(const fgb_conv_call* call, void* stream);
+
+/* Everything a submanifold conv needs of its coordinates, in one call: the map
+ * (fgb_subm_build_neighbor_map), sorted_idx (fgb_pp_sorted_idx), the masks of
+ * 128-row tiles and the block schedule, on one scratch block and two memsets.
+ * meta [v + 3] receives the segment table [v + 1], the key-order word and the
+ * build's status (FGB_S_TABLE_FULL); host_words, when not null, is mapped pinned
+ * memory [v + 4] whose words v .. v + 2 receive the pair count, the key-order word
+ * and the status, and then word v + 3 the value host_seq: a host that wants the
+ * pair count watches that word.  `status`: the device status word of the sort. */
+typedef struct fgb_map_call {
+  const int32_t* coords;
+  int64_t n;
+  int32_t b, w, h, d, k[3], dil[3], key_bits;
+  int64_t slots;
+  void* scratch;
+  int64_t scratch_bytes;
+  uint32_t* neighbor_map;
+  int32_t* gray_code;
+  int64_t* sorted_idx;
+  uint32_t* tile_masks;
+  uint32_t* block_order;
+  uint32_t* block_offsets;
+  uint32_t* meta;
+  uint32_t* host_words;
+  uint32_t host_seq;
+  int32_t* status;
+} fgb_map_call;
+int64_t fgb_subm_cache_scratch_bytes(const fgb_map_call* call);
+int fgb_subm_cache_build(const fgb_map_call* call, void* stream);
+
+/* grad_weight [co, v, ci] and, when grad_bias is not null, grad_bias [co], both
+ * of the element type `dtype`. */
+typedef struct fgb_wgrad_call {
+  const void* grad_out;
+  const void* feats;
+  const uint32_t* valid_signal_i;
+  const uint32_t* valid_signal_o;
+  const uint32_t* valid_signal_seg;
+  const uint32_t* block_offsets;
+  void* grad_weight;
+  void* grad_bias;
+  int64_t n_out, n_in, n_pairs;
+  int32_t ci, co, v, dtype;
+  void* workspace;
+  int64_t workspace_bytes;
+  int32_t* status;
+} fgb_wgrad_call;
+int64_t fgb_wgrad_call_workspace_bytes(const fgb_wgrad_call* call);
+int fgb_wgrad_call_run(const fgb_wgrad_call* call, void* stream);
+
+/* Rows of `width_in` bytes copied to rows of `width_out` bytes, cut or padded
+ * with zero bytes; rows from rows_in on are zero.  (Channel counts that do not make rows whole
+ * 16-byte pieces are padded on the way into the conv calls and cut on the way
+ * out.)  Widths must be multiples of 2. */
+int fgb_resize_rows(const void* src, void* dst, int64_t rows_in, int64_t rows_out, int64_t width_in, int64_t width_out, void* stream);
 
 /* ------------------------------------------------------------------------
  * Pipeline microbenchmark (no counterpart in the reference)

@@ -1,0 +1,85 @@
+"""The native host path against the library's single-purpose calls: cache build (map, order, masks, schedule, pair lists)
+at the edges of its tiles, the bias gradient computed along with the weight gradient, and padded channel counts."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import submconv_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def u32(t):
+    return t.cpu().view(torch.int32).numpy().view(np.uint32)
+
+
+@pytest.mark.parametrize("n,ksize,shuffle,volume", [(1, (3, 3, 3), False, 64), (127, (3, 3, 3), False, 64), (128, (3, 3, 3), True, 64),
+                                                    (257, (3, 1, 3), False, 64), (1025, (3, 3, 3), True, 64), (4097, (1, 1, 1), False, 64),
+                                                    (33000, (3, 3, 3), False, 64), (33000, (3, 3, 3), True, 2048),
+                                                    (3000, (1, 1, 31), False, 64)])
+def test_cache_build_matches_single_calls(n, ksize, shuffle, volume):
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import utils
+    from flexgemm_b200.ops.spconv import SubMConv3dFunction
+    g = torch.Generator().manual_seed(n)
+    flat = torch.randperm(64 ** 3, generator=g)[:n].sort().values
+    coords = torch.stack([flat * 0, flat // 4096, flat // 64 % 64, flat % 64], 1).int()
+    if shuffle:
+        coords = coords[torch.randperm(n, generator=g)]
+    coords = coords.to(DEV).contiguous()
+    shape = torch.Size((1, 8, volume, volume, volume))
+    V = ksize[0] * ksize[1] * ksize[2]
+    got = SubMConv3dFunction._compute_neighbor_cache(coords, shape, ksize, (1, 1, 1), True)
+    table, bits = utils.init_table(shape, max(2 * n, 1), DEV)
+    want = K.subm_build_neighbor_map(coords, shape, ksize, (1, 1, 1), table, bits, max(2 * n, 1))
+    seg = u32(want["valid_signal_seg"])
+    order = K.sorted_idx_from_binary(want["binary_code"], V)
+    vs_i, vs_o = K.valid_signal(want["neighbor_map"], want["gray_code"], want["block_offsets"], want["valid_signal_seg"], int(seg[V]))
+    masks = K.tile_masks(want["gray_code"], order, 128)
+    for name, ref in (("neighbor_map", want["neighbor_map"]), ("valid_signal_seg", want["valid_signal_seg"]), ("valid_signal_i", vs_i),
+                      ("valid_signal_o", vs_o), ("pair_block_offsets", want["block_offsets"]), ("tile_masks_128", masks)):
+        assert np.array_equal(u32(got[name]), u32(ref)), name
+    assert torch.equal(got["gray_code"], want["gray_code"]) and torch.equal(got["sorted_idx"], order)
+    # a schedule is any order of descending cost
+    m = u32(masks)
+    m = np.concatenate([m, np.zeros(len(m) % 2, np.uint32)]).reshape(-1, 2)
+    cost = np.array([bin(int(a)).count("1") + bin(int(b)).count("1") for a, b in m])
+    blocks = u32(got["block_order_128"])
+    assert np.array_equal(np.sort(blocks), np.arange(len(cost))) and np.all(np.diff(cost[blocks]) <= 0)
+    K.check_status(DEV)
+
+
+@pytest.mark.parametrize("res,ci,co,dtype", [(8, 8, 8, "float16"), (16, 6, 20, "bfloat16"), (16, 32, 136, "float16"), (8, 3, 1032, "float32"),
+                                             (24, 64, 2056, "bfloat16")])
+def test_gradients_with_bias_and_padding(res, ci, co, dtype):
+    """The bias sums are fp32 over at most a few thousand values and rounded once: within half a unit in the last place
+    of the type plus n * 2^-24 of the absolute sum; everything else within the library's 1e-2 of the oracle's maximum."""
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = orc.make_problem(res, ci, co, dtype, seed=res + co)
+    gout = torch.randn(coords.shape[0], co, generator=torch.Generator().manual_seed(1)).to(feats.dtype)
+    f, w, b = (t.to(DEV).requires_grad_(True) for t in (feats, weight, bias))
+    out, cache = spconv.sparse_submanifold_conv3d(f, coords.to(DEV), torch.Size(shape), w, b)
+    gf, gw, gb = torch.autograd.grad(out, (f, w, b), gout.to(DEV))
+    nbr = orc.neighbor_map(coords.numpy(), shape)
+    rf, rw, rb = orc.conv_backward(gout.double(), feats.double(), nbr, weight.double())
+    ro = orc.conv_forward(feats.double(), nbr, weight.double(), bias.double())
+    for got, want in ((out, ro), (gf, rf), (gw, rw)):
+        assert (got.detach().cpu().double() - want).abs().max() <= 1e-2 * want.abs().max()
+    ulp = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -24}[dtype]
+    bound = rb.abs() * ulp + gout.double().abs().sum(0) * 2.0 ** -24 * gout.shape[0] + 1e-7
+    assert torch.all((gb.cpu().double() - rb).abs() <= bound)
+    # the same through the Python autograd function
+    out2, _ = spconv.SubMConv3dFunction.apply(f, coords.to(DEV), torch.Size(shape), cache, w, b)
+    for x, y in zip((out2, *torch.autograd.grad(out2, (f, w, b), gout.to(DEV))), (out, gf, gw, gb)):
+        assert torch.equal(x, y)
+
+
+def test_inference_cache_has_no_pair_lists():
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = orc.make_problem(8, 16, 16, "float16", seed=3)
+    _, cache = spconv.sparse_submanifold_conv3d(feats.to(DEV), coords.to(DEV), torch.Size(shape), weight.to(DEV), bias.to(DEV))
+    w = weight.to(DEV).requires_grad_(True)
+    out, _ = spconv.sparse_submanifold_conv3d(feats.to(DEV), coords.to(DEV), torch.Size(shape), w, None, cache)
+    with pytest.raises(AttributeError, match="valid_signal_i"):
+        out.sum().backward()

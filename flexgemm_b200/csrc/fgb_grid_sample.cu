@@ -6,6 +6,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "fgb_common.cuh"
 #include "fgb_hash.cuh"
 
@@ -165,6 +167,283 @@ __global__ void __launch_bounds__(256) weighted_scatter_kernel(const T* __restri
   }
 }
 
+// ------------------------------------------------------------------ fused sample
+// Points around one voxel grid, features blended in one kernel.  A warp takes four points at a time: its 32 lanes look up
+// the 4 x 8 corners at once (the probes are dependent L2 loads: the latency is paid once per four points, and the map goes
+// to memory only where a backward pass will want it), then the points' feature rows are gathered with 16-byte loads, all
+// corners of a point in flight.  Narrow rows share the warp: kGroup lanes per point.  Bound: the gathered rows out of L2
+// (about four of eight corners exist near a surface: 2 GB at 10^6 points, C = 256 fp16).  Against the map kernel and a
+// gather that walked the corners one after the other (84 + 620 us): see the figure at fgb_grid_sample_fused.
+// kNearest: one corner, the voxel that contains the point; the four points of a warp are looked up by four lanes.
+template <typename T, int kVec>
+struct Pack;  // kVec consecutive elements as one load
+template <typename T>
+struct Pack<T, 8> { using Raw = uint4; };
+template <typename T>
+struct Pack<T, 4> { using Raw = typename std::conditional<sizeof(T) == 4, uint4, uint2>::type; };
+template <typename T, int kVec>
+__device__ __forceinline__ void fma_pack(float (&acc)[kVec], const typename Pack<T, kVec>::Raw& raw, float w) {
+  const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) acc[i] += w * static_cast<float>(e[i]);
+}
+template <typename T, int kVec>
+__device__ __forceinline__ typename Pack<T, kVec>::Raw round_pack(const float (&acc)[kVec]) {
+  typename Pack<T, kVec>::Raw raw;
+  T* e = reinterpret_cast<T*>(&raw);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) e[i] = static_cast<T>(acc[i]);
+  return raw;
+}
+
+constexpr int kSamplePoints = 4;  // points of a warp
+
+template <typename T, int kVec, int kKeyBits, bool kNearest, int kGroup>
+__global__ void __launch_bounds__(256) sample_kernel(const T* __restrict__ feats, const float* __restrict__ query, uint32_t points, uint32_t L,
+                                                     Grid3 g, void* table_mem, uint32_t slots, int C, T* __restrict__ out,
+                                                     uint32_t* __restrict__ neighbor, float* __restrict__ weight) {
+  using Raw = typename Pack<T, kVec>::Raw;
+  constexpr int kCorners = kNearest ? 1 : 8;
+  constexpr int kAtOnce = 32 / kGroup;  // points gathered side by side
+  chain_release();
+  chain_wait();
+  const int lane = threadIdx.x & 31;
+  const uint32_t p0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * kSamplePoints;
+  if (p0 >= points) return;  // whole warps
+  uint32_t nb = kInvalid;
+  float w = 0.f;
+  {
+    const uint32_t q = p0 + lane / kCorners;
+    if (lane < kSamplePoints * kCorners && q < points) {
+      const int b = static_cast<int>(q / L), k = lane % kCorners;
+      const float qx = __ldg(&query[3 * size_t(q)]), qy = __ldg(&query[3 * size_t(q) + 1]), qz = __ldg(&query[3 * size_t(q) + 2]);
+      int x, y, z;
+      if constexpr (kNearest) {
+        x = static_cast<int>(qx), y = static_cast<int>(qy), z = static_cast<int>(qz);
+      } else {
+        x = static_cast<int>(floorf(qx - 0.5f)) + (k & 1);
+        y = static_cast<int>(floorf(qy - 0.5f)) + ((k >> 1) & 1);
+        z = static_cast<int>(floorf(qz - 0.5f)) + ((k >> 2) & 1);
+      }
+      if (x >= 0 && x < g.W && y >= 0 && y < g.H && z >= 0 && z < g.D) {
+        nb = make_table<kKeyBits>(table_mem, slots).find(g.template key<kKeyBits>(b, x, y, z));
+        if (nb != kInvalid) {
+          if constexpr (kNearest) w = 1.f;
+          else w = (1.f - fabsf(qx - x - 0.5f)) * (1.f - fabsf(qy - y - 0.5f)) * (1.f - fabsf(qz - z - 0.5f));
+        }
+      }
+    }
+    if constexpr (!kNearest) {
+      // corner order of the sum as in the map kernel: the weights of a point are the same bits either way
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += __shfl_sync(0xffffffffu, w, (lane & 24) + k);
+      w *= 1.f / fmaxf(sum, 1e-12f);
+    }
+    if (neighbor != nullptr && lane < kSamplePoints * kCorners && q < points) {
+      neighbor[size_t(p0) * kCorners + lane] = nb;
+      if constexpr (!kNearest) weight[size_t(p0) * kCorners + lane] = w;
+    }
+  }
+  const int nv = C / kVec;
+#pragma unroll
+  for (int i = 0; i < kSamplePoints; i += (kAtOnce < kSamplePoints ? kAtOnce : kSamplePoints)) {
+    const int local = i + (kAtOnce == 1 ? 0 : lane / kGroup);
+    const bool mine = local < kSamplePoints && p0 + local < points;
+    uint32_t rows[kCorners];
+    float ws[kCorners];
+#pragma unroll
+    for (int k = 0; k < kCorners; ++k) {
+      rows[k] = __shfl_sync(0xffffffffu, nb, (local * kCorners + k) & 31);
+      ws[k] = __shfl_sync(0xffffffffu, w, (local * kCorners + k) & 31);
+    }
+    if (!mine) continue;
+    for (int c = lane % kGroup; c < nv; c += kGroup) {
+      Raw raw[kCorners];
+#pragma unroll
+      for (int k = 0; k < kCorners; ++k)
+        if (rows[k] != kInvalid) raw[k] = __ldg(reinterpret_cast<const Raw*>(feats + size_t(rows[k]) * C) + c);
+      float acc[kVec];
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) acc[j] = 0.f;
+#pragma unroll
+      for (int k = 0; k < kCorners; ++k)
+        if (rows[k] != kInvalid) fma_pack<T, kVec>(acc, raw[k], ws[k]);
+      __stcs(reinterpret_cast<Raw*>(out + size_t(p0 + local) * C) + c, round_pack<T, kVec>(acc));
+    }
+  }
+}
+
+// ------------------------------------------------------------------ gradient w.r.t. the features
+// grad_feats[r, :] = sum over the (point, corner) entries e with indices[e] == r of weight[e] * grad_out[point(e), :]
+//
+// As a gather: the entries are first grouped by voxel (count, place the groups, fill), then one warp per voxel reads the
+// gradient rows of its entries with 16-byte loads, sums in fp32 registers and writes the row once in the feature type.
+// Against fp32 atomics into a buffer that is zeroed before and converted after (10^6 points, C = 256 fp16 on the RES=256
+// shell: 2.05 ms + 28 + 35 us, all of it atomic traffic of 4 bytes per channel and corner) the gradient rows cross L2
+// as 2-byte values, and consecutive voxels share the points between them, so a row comes from HBM once.
+__global__ void __launch_bounds__(256) group_count_kernel(const uint32_t* __restrict__ indices, uint32_t entries, uint32_t* __restrict__ count,
+                                                          uint32_t* __restrict__ rank) {
+  chain_release();
+  chain_wait();
+  for (uint64_t e = blockIdx.x * uint64_t(256) + threadIdx.x; e < entries; e += uint64_t(gridDim.x) * 256) {
+    const uint32_t row = __ldg(&indices[e]);
+    if (row != kInvalid) rank[e] = atomicAdd(&count[row], 1u);
+  }
+}
+// start[r] = where the entries of voxel r go.  The groups of 1024 consecutive voxels stand together, in order; such
+// blocks take their places as they come (one atomic each), which no result depends on.
+__global__ void __launch_bounds__(1024) group_place_kernel(const uint32_t* __restrict__ count, uint32_t n, uint32_t* __restrict__ start,
+                                                           uint32_t* __restrict__ total) {
+  __shared__ uint32_t s_warp[32];
+  __shared__ uint32_t s_base;
+  chain_release();
+  chain_wait();
+  const uint32_t i = blockIdx.x * 1024u + threadIdx.x;
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const uint32_t x = i < n ? count[i] : 0u;
+  uint32_t inc = x;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += y;
+  }
+  if (lane == 31) s_warp[wi] = inc;
+  __syncthreads();
+  if (wi == 0) {
+    uint32_t ws = s_warp[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, ws, d);
+      if (lane >= d) ws += y;
+    }
+    s_warp[lane] = ws;
+    if (lane == 31) s_base = atomicAdd(total, ws);
+  }
+  __syncthreads();
+  if (i < n) start[i] = s_base + (wi ? s_warp[wi - 1] : 0u) + inc - x;
+}
+__global__ void __launch_bounds__(256) group_fill_kernel(const uint32_t* __restrict__ indices, const float* __restrict__ weight, uint32_t entries,
+                                                         int V, const uint32_t* __restrict__ start, const uint32_t* __restrict__ rank,
+                                                         uint2* __restrict__ grouped) {
+  chain_release();
+  chain_wait();
+  for (uint64_t e = blockIdx.x * uint64_t(256) + threadIdx.x; e < entries; e += uint64_t(gridDim.x) * 256) {
+    const uint32_t row = __ldg(&indices[e]);
+    if (row == kInvalid) continue;
+    const float w = weight != nullptr ? __ldg(&weight[e]) : 1.f;
+    grouped[__ldg(&start[row]) + __ldg(&rank[e])] = make_uint2(static_cast<uint32_t>(e / V), __float_as_uint(w));
+  }
+}
+// kWarps warps of a CTA share one voxel (1, or 8 where voxels have many entries); kGroup lanes cover a row, so 32 / kGroup
+// entries are read side by side.
+template <typename T, int kVec, int kWarps, int kGroup>
+__global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ grad_out, const uint2* __restrict__ grouped,
+                                                        const uint32_t* __restrict__ start, const uint32_t* __restrict__ count, uint32_t n, int C,
+                                                        T* __restrict__ grad_feats) {
+  using Raw = typename Pack<T, kVec>::Raw;
+  constexpr int kSide = 32 / kGroup;
+  __shared__ float s_acc[kWarps > 1 ? kWarps : 1][kWarps > 1 ? 32 * kVec : 1];
+  chain_release();
+  chain_wait();
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const uint32_t row = kWarps > 1 ? blockIdx.x : blockIdx.x * 8u + wi;
+  if (row >= n) return;  // whole warps; with kWarps > 1 whole CTAs
+  const uint32_t len = __ldg(&count[row]);
+  const uint2* list = grouped + (len ? __ldg(&start[row]) : 0u);
+  const int nv = C / kVec;
+  const int side = lane / kGroup;
+  const int share = kWarps > 1 ? wi : 0;
+  for (int c0 = 0; c0 < nv; c0 += kGroup) {
+    const int c = c0 + lane % kGroup;
+    float acc[kVec];
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) acc[i] = 0.f;
+    for (uint32_t base = share * 32u; base < len; base += kWarps * 32u) {
+      const uint32_t here = min(32u, len - base);
+      const uint2 e = lane < here ? __ldg(&list[base + lane]) : make_uint2(0, 0);
+#pragma unroll 4
+      for (uint32_t j0 = 0; j0 < here; j0 += kSide) {
+        const uint32_t j = j0 + side;
+        const uint32_t m = __shfl_sync(0xffffffffu, e.x, j & 31);
+        const float w = __uint_as_float(__shfl_sync(0xffffffffu, e.y, j & 31));
+        if (j < here && c < nv) fma_pack<T, kVec>(acc, __ldg(reinterpret_cast<const Raw*>(grad_out + size_t(m) * C) + c), w);
+      }
+    }
+#pragma unroll
+    for (int d = kGroup; d < 32; d <<= 1)
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], d);
+    if constexpr (kWarps > 1) {
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) s_acc[wi][lane * kVec + i] = acc[i];
+      __syncthreads();
+      if (wi == 0) {
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) {
+          acc[i] = 0.f;
+#pragma unroll
+          for (int k = 0; k < kWarps; ++k) acc[i] += s_acc[k][lane * kVec + i];
+        }
+      }
+      __syncthreads();
+    }
+    if ((kWarps == 1 || wi == 0) && side == 0 && c < nv) reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
+  }
+}
+
+// lanes for a row of nv packs: the next power of two, 8 .. 32
+static int group_lanes(int nv) { return nv <= 8 ? 8 : nv <= 16 ? 16 : 32; }
+
+template <typename T, int kVec, int kKeyBits, bool kNearest>
+static cudaError_t launch_sample(const void* feats, const float* query, uint32_t points, uint32_t L, Grid3 g, void* table, uint32_t slots, int C,
+                                 void* out, uint32_t* neighbor, float* weight, cudaStream_t s) {
+  const int lanes = group_lanes(C / kVec);
+  auto kernel = lanes == 8    ? sample_kernel<T, kVec, kKeyBits, kNearest, 8>
+                : lanes == 16 ? sample_kernel<T, kVec, kKeyBits, kNearest, 16>
+                              : sample_kernel<T, kVec, kKeyBits, kNearest, 32>;
+  return launch_chained(kernel, dim3(static_cast<unsigned>(ceil_div(points, 8 * kSamplePoints))), dim3(256), 0, s, static_cast<const T*>(feats),
+                        query, points, L, g, table, slots, C, static_cast<T*>(out), neighbor, weight);
+}
+template <typename T, int kVec>
+static cudaError_t launch_sample(int key_bits, bool nearest, const void* feats, const float* query, uint32_t points, uint32_t L, Grid3 g, void* table,
+                                 uint32_t slots, int C, void* out, uint32_t* neighbor, float* weight, cudaStream_t s) {
+  if (key_bits == 32)
+    return nearest ? launch_sample<T, kVec, 32, true>(feats, query, points, L, g, table, slots, C, out, neighbor, weight, s)
+                   : launch_sample<T, kVec, 32, false>(feats, query, points, L, g, table, slots, C, out, neighbor, weight, s);
+  return nearest ? launch_sample<T, kVec, 64, true>(feats, query, points, L, g, table, slots, C, out, neighbor, weight, s)
+                 : launch_sample<T, kVec, 64, false>(feats, query, points, L, g, table, slots, C, out, neighbor, weight, s);
+}
+
+template <typename T, int kVec>
+static cudaError_t launch_group_sum(bool shared_rows, const void* grad_out, const uint2* grouped, const uint32_t* start, const uint32_t* count,
+                                    uint32_t n, int C, void* grad_feats, cudaStream_t s) {
+  const int lanes = group_lanes(C / kVec);
+  auto kernel = shared_rows ? (lanes == 8    ? group_sum_kernel<T, kVec, 8, 8>
+                               : lanes == 16 ? group_sum_kernel<T, kVec, 8, 16>
+                                             : group_sum_kernel<T, kVec, 8, 32>)
+                            : (lanes == 8    ? group_sum_kernel<T, kVec, 1, 8>
+                               : lanes == 16 ? group_sum_kernel<T, kVec, 1, 16>
+                                             : group_sum_kernel<T, kVec, 1, 32>);
+  return launch_chained(kernel, dim3(shared_rows ? n : static_cast<unsigned>(ceil_div(n, 8))), dim3(256), 0, s, static_cast<const T*>(grad_out),
+                        grouped, start, count, n, C, static_cast<T*>(grad_feats));
+}
+
+struct GroupScratch {
+  size_t count_off, total_off, zero_bytes, start_off, rank_off, grouped_off, bytes;
+};
+static GroupScratch group_scratch(int64_t entries, int64_t n) {
+  GroupScratch g;
+  g.count_off = 0;
+  g.total_off = align256(n * 4);
+  g.zero_bytes = g.total_off + 256;
+  g.start_off = g.zero_bytes;
+  g.rank_off = g.start_off + align256(n * 4);
+  g.grouped_off = g.rank_off + align256(entries * 4);
+  g.bytes = g.grouped_off + align256(entries * 8);
+  return g;
+}
+
 static int check_table(const void* table, int64_t slots, int key_bits) {
   if (key_bits != 32 && key_bits != 64) return FGB_E_DTYPE;
   if (slots < 1 || slots >= (int64_t(1) << 31)) return FGB_E_SIZE;
@@ -295,4 +574,91 @@ extern "C" int fgb_indice_weighted_sum_bwd(const void* grad_out, const uint32_t*
   else
     weighted_scatter_kernel<float><<<g, 256, 0, s>>>(static_cast<const float*>(grad_out), indices, weight, grad_feats_f32, M, C, V);
   return launch_status();
+}
+
+extern "C" int fgb_grid_sample_fused(const int32_t* coords, int64_t n, const void* feats, const float* query, int64_t B, int64_t L, int W, int H,
+                                     int D, int C, int dtype, int trilinear, void* table, int64_t slots, int key_bits, int32_t* table_status,
+                                     void* out, uint32_t* neighbor, float* weight, void* stream) {
+  using namespace fgb;
+  if (!elem_code_ok(dtype)) return FGB_E_DTYPE;
+  if (n < 0 || n >= (int64_t(1) << 32) - 1 || B < 0 || L < 0 || B * L >= (int64_t(1) << 28) || W <= 0 || H <= 0 || D <= 0 || C <= 0) return FGB_E_SIZE;
+  if (C % 4) return FGB_E_ALIGN;
+  int rc = check_table(table, slots, key_bits);
+  if (rc != FGB_OK) return rc;
+  if (slots < n) return FGB_E_SIZE;
+  if (B * L == 0) return FGB_OK;
+  if ((n > 0 && (!coords || !feats)) || !query || !out || (neighbor != nullptr && trilinear && !weight)) return FGB_E_NULL;
+  if ((reinterpret_cast<uintptr_t>(coords) | reinterpret_cast<uintptr_t>(feats) | reinterpret_cast<uintptr_t>(out)) & 15) return FGB_E_ALIGN;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(table, 0xFF, static_cast<size_t>(fgb_hash_table_bytes(slots, key_bits)), s);
+  if (e != cudaSuccess) return cuda_status(e);
+  const Grid3 g{W, H, D};
+  const uint32_t sl = static_cast<uint32_t>(slots), points = static_cast<uint32_t>(B * L), l = static_cast<uint32_t>(L);
+  if (n > 0) {
+    const dim3 blocks(static_cast<unsigned>(ceil_div(n, kMapBlock)));
+    const int4* c4 = reinterpret_cast<const int4*>(coords);
+    const uint32_t* always = nullptr;
+    e = key_bits == 32 ? launch_chained(hash_insert_kernel<32>, blocks, dim3(kMapBlock), 0, s, c4, static_cast<uint32_t>(n), g, table, sl, table_status, always)
+                       : launch_chained(hash_insert_kernel<64>, blocks, dim3(kMapBlock), 0, s, c4, static_cast<uint32_t>(n), g, table, sl, table_status, always);
+    if (e != cudaSuccess) return cuda_status(e);
+  }
+  const bool nearest = trilinear == 0;
+  if (dtype == FGB_F16)
+    e = C % 8 == 0 ? launch_sample<__half, 8>(key_bits, nearest, feats, query, points, l, g, table, sl, C, out, neighbor, weight, s)
+                   : launch_sample<__half, 4>(key_bits, nearest, feats, query, points, l, g, table, sl, C, out, neighbor, weight, s);
+  else if (dtype == FGB_BF16)
+    e = C % 8 == 0 ? launch_sample<__nv_bfloat16, 8>(key_bits, nearest, feats, query, points, l, g, table, sl, C, out, neighbor, weight, s)
+                   : launch_sample<__nv_bfloat16, 4>(key_bits, nearest, feats, query, points, l, g, table, sl, C, out, neighbor, weight, s);
+  else
+    e = launch_sample<float, 4>(key_bits, nearest, feats, query, points, l, g, table, sl, C, out, neighbor, weight, s);
+  return e != cudaSuccess ? cuda_status(e) : launch_status();
+}
+
+extern "C" int64_t fgb_indice_weighted_sum_grad_bytes(int64_t M, int64_t N, int V) {
+  if (M < 0 || N < 0 || N >= (int64_t(1) << 32) - 1 || V < 1 || V > 64 || M * V >= (int64_t(1) << 32)) return FGB_E_SIZE;
+  return static_cast<int64_t>(fgb::group_scratch(M * V, N).bytes);
+}
+
+extern "C" int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t* indices, const float* weight, void* grad_feats, int64_t M,
+                                            int64_t N, int C, int V, int dtype, void* workspace, int64_t workspace_bytes, void* stream) {
+  using namespace fgb;
+  if (!elem_code_ok(dtype)) return FGB_E_DTYPE;
+  const int64_t bytes = fgb_indice_weighted_sum_grad_bytes(M, N, V);
+  if (bytes < 0 || C <= 0) return FGB_E_SIZE;
+  if (C % 4) return FGB_E_ALIGN;
+  if (N == 0) return FGB_OK;
+  if (!grad_feats || !workspace || (M > 0 && (!grad_out || !indices))) return FGB_E_NULL;
+  if ((reinterpret_cast<uintptr_t>(grad_out) | reinterpret_cast<uintptr_t>(grad_feats)) & 15) return FGB_E_ALIGN;
+  if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
+  if (workspace_bytes < bytes) return FGB_E_WORKSPACE;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const uint32_t entries = static_cast<uint32_t>(M * V), n = static_cast<uint32_t>(N);
+  const GroupScratch G = group_scratch(entries, N);
+  char* mem = static_cast<char*>(workspace);
+  uint32_t* count = reinterpret_cast<uint32_t*>(mem + G.count_off);
+  uint32_t* total = reinterpret_cast<uint32_t*>(mem + G.total_off);
+  uint32_t* start = reinterpret_cast<uint32_t*>(mem + G.start_off);
+  uint32_t* rank = reinterpret_cast<uint32_t*>(mem + G.rank_off);
+  uint2* grouped = reinterpret_cast<uint2*>(mem + G.grouped_off);
+  LaunchErrors chain;
+  chain.add(cudaMemsetAsync(mem, 0, G.zero_bytes, s));
+  if (entries > 0) {
+    const dim3 egrid(static_cast<unsigned>(std::min<int64_t>(ceil_div(entries, 256), 148 * 32)));
+    chain.add(launch_chained(group_count_kernel, egrid, dim3(256), 0, s, indices, entries, count, rank));
+    chain.add(launch_chained(group_place_kernel, dim3(static_cast<unsigned>(ceil_div(N, 1024))), dim3(1024), 0, s, static_cast<const uint32_t*>(count), n,
+                             start, total));
+    chain.add(launch_chained(group_fill_kernel, egrid, dim3(256), 0, s, indices, weight, entries, V, static_cast<const uint32_t*>(start),
+                             static_cast<const uint32_t*>(rank), grouped));
+  }
+  // many entries per voxel: the warps of a CTA share a voxel, else few warps would walk long lists
+  const bool shared_rows = entries / n >= 128u;
+  if (dtype == FGB_F16)
+    chain.add(C % 8 == 0 ? launch_group_sum<__half, 8>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s)
+                         : launch_group_sum<__half, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+  else if (dtype == FGB_BF16)
+    chain.add(C % 8 == 0 ? launch_group_sum<__nv_bfloat16, 8>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s)
+                         : launch_group_sum<__nv_bfloat16, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+  else
+    chain.add(launch_group_sum<float, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+  return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
 }

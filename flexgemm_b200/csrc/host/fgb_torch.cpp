@@ -45,7 +45,8 @@ using torch::autograd::variable_list;
   X(fgb_error_string) X(fgb_status_set_mirror) X(fgb_conv_call_workspace_bytes) X(fgb_conv_call_fprop)                \
   X(fgb_conv_call_dgrad) X(fgb_wgrad_call_workspace_bytes) X(fgb_wgrad_call_run) X(fgb_resize_rows)                   \
   X(fgb_bias_grad_workspace_bytes) X(fgb_subm_conv_bias_grad) X(fgb_subm_cache_scratch_bytes)                         \
-  X(fgb_subm_cache_build) X(fgb_pp_valid_signal) X(fgb_map_num_blocks)
+  X(fgb_subm_cache_build) X(fgb_pp_valid_signal) X(fgb_hash_table_bytes)                                    \
+  X(fgb_grid_sample_fused) X(fgb_indice_weighted_sum_grad_bytes) X(fgb_indice_weighted_sum_grad)
 struct Api {
 #define X(f) decltype(&::f) f = nullptr;
   FGB_TORCH_API(X)
@@ -807,6 +808,98 @@ PyObject* py_conv_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   FGB_END
 }
 
+// ------------------------------------------------------------------ grid sample
+Tensor run_sample_grad(const Tensor& grad_out /* [M, C] */, const Tensor& indices, const Tensor& weight, int64_t n, int64_t V) {
+  c10::cuda::CUDAGuard guard(grad_out.device());
+  const auto stream = c10::cuda::getCurrentCUDAStream(grad_out.device().index());
+  const int64_t M = grad_out.size(0), C = grad_out.size(1);
+  Tensor out = new_tensor({n, C}, grad_out.scalar_type(), grad_out.device());
+  const int64_t bytes = check_bytes(api.fgb_indice_weighted_sum_grad_bytes(M, n, static_cast<int>(V)), "fgb_indice_weighted_sum_grad_bytes");
+  const c10::DataPtr ws = scratch(bytes);
+  check(api.fgb_indice_weighted_sum_grad(ptr(grad_out), cptr<uint32_t>(indices), weight.defined() ? cptr<float>(weight) : nullptr,
+                                         n > 0 ? out.data_ptr() : nullptr, M, n, static_cast<int>(C), static_cast<int>(V),
+                                         dtype_code(grad_out.scalar_type(), false), ws.get(), bytes, stream),
+        "fgb_indice_weighted_sum_grad");
+  g_launches += 4;
+  return out;
+}
+
+struct GridSampleBackward : public torch::autograd::Node {
+  Tensor indices, weight;
+  int64_t n = 0, V = 1;
+  std::string name() const override { return "GridSample3dBackward"; }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(1);
+    if (!grads[0].defined() || !task_should_compute_output(0)) return out;
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor g = grads[0].contiguous();
+    out[0] = run_sample_grad(g.view({-1, g.size(-1)}), indices, weight, n, V);
+    return out;
+  }
+};
+
+// (feats, coords, shape, grid, trilinear, ratio) -> [B, L, C] or None
+PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  FGB_TRY
+  TORCH_CHECK(n_args == 6, "grid_sample takes 6 arguments");
+  const Tensor feats = tensor_arg(a[0]), coords = tensor_arg(a[1]);
+  Tensor grid = tensor_arg(a[3]);
+  const bool trilinear = PyObject_IsTrue(a[4]) == 1;
+  int64_t shape[5];
+  const int64_t one[3] = {1, 1, 1};
+  if (!feats.defined() || !feats.is_cuda() || feats.dim() != 2 || !feats.is_contiguous() || feats.size(0) == 0 || feats.size(1) == 0 ||
+      feats.size(1) % 4 != 0 || dtype_code(feats.scalar_type(), false) < 0 || !coords_ok(coords, one) || coords.device() != feats.device() ||
+      coords.size(0) != feats.size(0) || !grid.defined() || grid.device() != feats.device() || grid.dim() != 3 || grid.size(2) != 3 ||
+      grid.scalar_type() != at::kFloat || !grid.is_contiguous() || grid.numel() == 0 || !int_args(a[2], 5, shape) ||
+      (reinterpret_cast<uintptr_t>(feats.const_data_ptr()) & 15) != 0)
+    Py_RETURN_NONE;
+  const double ratio = PyFloat_AsDouble(a[5]);
+  if (ratio == -1.0 && PyErr_Occurred()) return nullptr;
+  c10::cuda::CUDAGuard guard(feats.device());
+  const auto stream = c10::cuda::getCurrentCUDAStream(feats.device().index());
+  const bool want_grad = torch::autograd::compute_requires_grad(feats);
+  const int64_t n = feats.size(0), C = feats.size(1), B = grid.size(0), L = grid.size(1), V = trilinear ? 8 : 1;
+  const int64_t slots = std::max<int64_t>({static_cast<int64_t>(ratio * static_cast<double>(n)), n, 1});
+  const double volume = double(shape[0]) * double(shape[2]) * double(shape[3]) * double(shape[4]);
+  const int key_bits = volume < 4294967296.0 ? 32 : 64;
+  Tensor out, indices, weight;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    out = new_tensor({B, L, C}, feats.scalar_type(), feats.device());
+    if (want_grad) {
+      indices = new_tensor({B * L, V}, at::kUInt32, feats.device());
+      if (trilinear) weight = new_tensor({B * L, V}, at::kFloat, feats.device());
+    }
+    const c10::DataPtr table = scratch(check_bytes(api.fgb_hash_table_bytes(slots, key_bits), "fgb_hash_table_bytes"));
+    // the table has a slot for every row, so it cannot run full: no status word to read back
+    check(api.fgb_grid_sample_fused(cptr<int32_t>(coords), n, ptr(feats), cptr<float>(grid), B, L, static_cast<int>(shape[2]), static_cast<int>(shape[3]),
+                                    static_cast<int>(shape[4]), static_cast<int>(C), dtype_code(feats.scalar_type(), false), trilinear ? 1 : 0,
+                                    table.get(), slots, key_bits, nullptr, out.data_ptr(),
+                                    want_grad ? static_cast<uint32_t*>(indices.data_ptr()) : nullptr,
+                                    want_grad && trilinear ? static_cast<float*>(weight.data_ptr()) : nullptr, stream),
+          "fgb_grid_sample_fused");
+    g_launches += 2;
+  }
+  if (want_grad) {
+    std::shared_ptr<GridSampleBackward> node(new GridSampleBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(feats));
+    node->indices = indices, node->weight = weight, node->n = n, node->V = V;
+    torch::autograd::set_history(out, node);
+  }
+  return THPVariable_Wrap(out);
+  FGB_END
+}
+
+// (grad_out [M, C], indices [M, V], weight or None, n) -> [n, C]
+PyObject* py_sample_grad(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  FGB_TRY
+  TORCH_CHECK(n_args == 4, "sample_grad takes 4 arguments");
+  const Tensor g = tensor_arg(a[0]), indices = tensor_arg(a[1]);
+  at::AutoDispatchBelowADInplaceOrView below;
+  return THPVariable_Wrap(run_sample_grad(g, indices, tensor_arg(a[2]), PyLong_AsLongLong(a[3]), indices.size(1)));
+  FGB_END
+}
+
 PyObject* py_status_word(PyObject*, PyObject* index) {
   FGB_TRY
   return THPVariable_Wrap(device_state(static_cast<c10::DeviceIndex>(PyLong_AsLong(index))).status);
@@ -849,6 +942,8 @@ PyMethodDef methods[] = {
     {"subm_conv", FAST(py_subm_conv), "submanifold conv"},
     {"conv", FAST(py_conv), "convolution on an existing cache"},
     {"conv_backward", FAST(py_conv_backward), "gradients of a convolution"},
+    {"grid_sample", FAST(py_grid_sample), "sparse grid sample"},
+    {"sample_grad", FAST(py_sample_grad), "gradient of a weighted gather"},
     {"status_word", py_status_word, METH_O, "device status word"},
     {"poll", py_poll, METH_O, "raise a soft error that the device has reported"},
     {"clear_mirror", py_clear_mirror, METH_O, "forget the host copy of the status word"},

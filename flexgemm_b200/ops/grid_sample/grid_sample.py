@@ -8,7 +8,7 @@ import torch
 from torch.autograd import Function
 
 from .. import grid_sample, utils
-from ... import kernels
+from ... import _native, kernels
 
 
 def _check(feats, coords, query_pts):
@@ -70,8 +70,8 @@ class GridSample3dFunction(Function):
             indices, weight = ctx.saved_tensors
             idx, w = indices.view(-1, 8), weight.view(-1, 8)
         C = grad_output.shape[-1]
-        g32 = kernels.cuda.indice_weighted_sum_bwd(grad_output.reshape(-1, C).contiguous(), idx, w, ctx.N)
-        return g32.to(grad_output.dtype), None, None, None, None
+        g = _native.ext().sample_grad(grad_output.reshape(-1, C).contiguous(), idx.contiguous(), w, ctx.N)
+        return g, None, None, None, None
 
     @staticmethod
     def forward(ctx, feats: torch.Tensor, coords: torch.Tensor, shape: torch.Size, grid: torch.Tensor, mode: str = "trilinear") -> torch.Tensor:
@@ -101,4 +101,8 @@ def grid_sample_3d(feats: torch.Tensor, coords: torch.Tensor, shape: torch.Size,
     Returns:
         [B, L, C] sampled features.
     """
+    if mode in ("nearest", "trilinear"):
+        out = _native.ext().grid_sample(feats, coords, shape, grid, mode == "trilinear", grid_sample.HASHMAP_RATIO)
+        if out is not None:
+            return out
     return GridSample3dFunction.apply(feats, coords, shape, grid, mode)

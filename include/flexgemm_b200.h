@@ -532,6 +532,25 @@ int fgb_indice_weighted_sum_fwd(const void* feats, const uint32_t* indices, cons
 int fgb_indice_weighted_sum_bwd(const void* grad_out, const uint32_t* indices, const float* weight,
                                 float* grad_feats_f32, int64_t M, int64_t N, int C, int V, int dtype, void* stream);
 
+/* The whole forward pass of grid_sample_3d in three stream operations: clears
+ * `table`, inserts the n coordinate rows and blends the features at the B * L
+ * query points (trilinear = 0: the voxel that contains the point).  neighbor
+ * [B * L, 8 or 1] and weight [B * L, 8] receive the map when not null (a backward
+ * pass wants it; nearest has no weights).  out [B * L, C].  table_status (may be
+ * null): a word for FGB_S_TABLE_FULL, which slots >= n rules out. */
+int fgb_grid_sample_fused(const int32_t* coords, int64_t n, const void* feats, const float* query, int64_t B, int64_t L,
+                          int W, int H, int D, int C, int dtype, int trilinear,
+                          void* table, int64_t slots, int key_bits, int32_t* table_status,
+                          void* out, uint32_t* neighbor, float* weight, void* stream);
+
+/* As fgb_indice_weighted_sum_bwd, with the result [N, C] in the feature type:
+ * the entries are grouped by voxel in the workspace and every voxel's row is
+ * summed in fp32 and written once, instead of added up by atomics. */
+int64_t fgb_indice_weighted_sum_grad_bytes(int64_t M, int64_t N, int V);
+int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t* indices, const float* weight, void* grad_feats,
+                                 int64_t M, int64_t N, int C, int V, int dtype,
+                                 void* workspace, int64_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------------
  * One-struct calls of the conv passes (what the torch host code uses)
  * --------------------------------------------------------------------- */

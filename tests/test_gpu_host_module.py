@@ -83,3 +83,36 @@ def test_inference_cache_has_no_pair_lists():
     out, _ = spconv.sparse_submanifold_conv3d(feats.to(DEV), coords.to(DEV), torch.Size(shape), w, None, cache)
     with pytest.raises(AttributeError, match="valid_signal_i"):
         out.sum().backward()
+
+
+@pytest.mark.parametrize("C,dtype,mode,points", [(4, "float16", "trilinear", 1), (12, "bfloat16", "trilinear", 37), (64, "float16", "nearest", 1000),
+                                                 (136, "float32", "trilinear", 333), (256, "bfloat16", "trilinear", 515), (264, "float16", "nearest", 130),
+                                                 (520, "float16", "trilinear", 77), (72, "float32", "trilinear", 60000), (8, "float16", "nearest", 40000)])
+@pytest.mark.parametrize("volume", [16, 2048])
+def test_grid_sample_matches_separate_kernels(C, dtype, mode, points, volume):
+    """Forward: the same bits as the map kernel followed by the gather (same weights, fp32 sums over the corners in the
+    same order; only the fused multiply-adds may be contracted differently: one rounding step of the type).  Gradient:
+    fp32 sums of the same terms in another order, up to `terms` of them, then one rounding."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import grid_sample, utils
+    T = getattr(torch, dtype)
+    coords = torch.from_numpy(orc.make_problem(16, 8, 8, "float16", seed=5, batch=2)[0].numpy()).to(DEV)
+    shape = torch.Size((2, C, volume, volume, volume))
+    g = torch.Generator().manual_seed(C)
+    feats = torch.randn(coords.shape[0], C, generator=g).to(T).to(DEV).requires_grad_(True)
+    query = (torch.rand(2, points, 3, generator=g) * 18 - 1).to(DEV)
+    gout = torch.randn(2, points, C, generator=g).to(T).to(DEV)
+    out = grid_sample.grid_sample_3d(feats, coords, shape, query, mode)
+    (gf,) = torch.autograd.grad(out, feats, gout)
+    slots = 2 * coords.shape[0]
+    table, bits = utils.init_table(shape, slots, DEV)
+    K.table_insert_3d_idx_as_val(table, bits, slots, coords, volume, volume, volume)
+    nb = K.grid_sample_neighbor_map(table, bits, slots, query, volume, volume, volume, mode == "trilinear")
+    idx, w = (nb[0].view(-1, 8), nb[1].view(-1, 8)) if mode == "trilinear" else (nb.view(-1, 1), None)
+    want = K.indice_weighted_sum_fwd(feats.detach(), idx, w).view(out.shape)
+    ulp = {"float16": 2.0 ** -10, "bfloat16": 2.0 ** -7, "float32": 2.0 ** -22}[dtype]
+    assert torch.all((out.detach().double() - want.double()).abs() <= want.double().abs() * ulp + 1e-6)
+    g32 = K.indice_weighted_sum_bwd(gout.view(-1, C), idx, w, coords.shape[0]).double()
+    mag = K.indice_weighted_sum_bwd(gout.view(-1, C).abs(), idx, w, coords.shape[0]).double()
+    terms = 8.0 * points / 100
+    assert torch.all((gf.double() - g32).abs() <= g32.abs() * ulp + mag * 2.0 ** -24 * (2 + terms) + 1e-7)

@@ -169,11 +169,12 @@ __global__ void __launch_bounds__(256) weighted_scatter_kernel(const T* __restri
 
 // ------------------------------------------------------------------ fused sample
 // Points around one voxel grid, features blended in one kernel.  A warp takes four points at a time: its 32 lanes look up
-// the 4 x 8 corners at once (the probes are dependent L2 loads: the latency is paid once per four points, and the map goes
-// to memory only where a backward pass will want it), then the points' feature rows are gathered with 16-byte loads, all
-// corners of a point in flight.  Narrow rows share the warp: kGroup lanes per point.  Bound: the gathered rows out of L2
-// (about four of eight corners exist near a surface: 2 GB at 10^6 points, C = 256 fp16).  Against the map kernel and a
-// gather that walked the corners one after the other (84 + 620 us): see the figure at fgb_grid_sample_fused.
+// the 4 x 8 corners at once, and the map goes to memory only where a backward pass will want it; then the points' feature
+// rows are gathered with 16-byte loads.  Narrow rows share the warp: kGroup lanes per point.
+// Bound at 10^6 points, C = 256 fp16, RES = 256: the rows' way out of L2 (1.6 GB of them at random places of an 84 MB
+// matrix, and the 0.5 GB of results): 375 us against 84 + 620 us for a map kernel and a gather that walked the eight
+// corners one after the other.  Occupancies from 32 to 48 warps, two to four rows in flight and lookups ahead or not
+// all gave 367 to 397 us.
 // kNearest: one corner, the voxel that contains the point; the four points of a warp are looked up by four lanes.
 template <typename T, int kVec>
 struct Pack;  // kVec consecutive elements as one load
@@ -199,7 +200,7 @@ __device__ __forceinline__ typename Pack<T, kVec>::Raw round_pack(const float (&
 constexpr int kSamplePoints = 4;  // points of a warp
 
 template <typename T, int kVec, int kKeyBits, bool kNearest, int kGroup>
-__global__ void __launch_bounds__(256) sample_kernel(const T* __restrict__ feats, const float* __restrict__ query, uint32_t points, uint32_t L,
+__global__ void __launch_bounds__(256, 4) sample_kernel(const T* __restrict__ feats, const float* __restrict__ query, uint32_t points, uint32_t L,
                                                      Grid3 g, void* table_mem, uint32_t slots, int C, T* __restrict__ out,
                                                      uint32_t* __restrict__ neighbor, float* __restrict__ weight) {
   using Raw = typename Pack<T, kVec>::Raw;
@@ -208,68 +209,105 @@ __global__ void __launch_bounds__(256) sample_kernel(const T* __restrict__ feats
   chain_release();
   chain_wait();
   const int lane = threadIdx.x & 31;
-  const uint32_t p0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * kSamplePoints;
-  if (p0 >= points) return;  // whole warps
-  uint32_t nb = kInvalid;
-  float w = 0.f;
-  {
-    const uint32_t q = p0 + lane / kCorners;
-    if (lane < kSamplePoints * kCorners && q < points) {
-      const int b = static_cast<int>(q / L), k = lane % kCorners;
-      const float qx = __ldg(&query[3 * size_t(q)]), qy = __ldg(&query[3 * size_t(q) + 1]), qz = __ldg(&query[3 * size_t(q) + 2]);
-      int x, y, z;
-      if constexpr (kNearest) {
-        x = static_cast<int>(qx), y = static_cast<int>(qy), z = static_cast<int>(qz);
-      } else {
-        x = static_cast<int>(floorf(qx - 0.5f)) + (k & 1);
-        y = static_cast<int>(floorf(qy - 0.5f)) + ((k >> 1) & 1);
-        z = static_cast<int>(floorf(qz - 0.5f)) + ((k >> 2) & 1);
-      }
-      if (x >= 0 && x < g.W && y >= 0 && y < g.H && z >= 0 && z < g.D) {
-        nb = make_table<kKeyBits>(table_mem, slots).find(g.template key<kKeyBits>(b, x, y, z));
-        if (nb != kInvalid) {
-          if constexpr (kNearest) w = 1.f;
-          else w = (1.f - fabsf(qx - x - 0.5f)) * (1.f - fabsf(qy - y - 0.5f)) * (1.f - fabsf(qz - z - 0.5f));
-        }
-      }
+  const auto table = make_table<kKeyBits>(table_mem, slots);
+  const bool looks = lane < kSamplePoints * kCorners;
+  const int k = lane % kCorners;
+  // A warp walks over groups of four points.  The next group's home slots and the query points of the one after are
+  // loaded before the current group's rows, so a step waits for one latency, not for three in a row.
+  auto load_query = [&](uint32_t group, float (&q)[3]) {
+    const uint64_t i = uint64_t(group) * kSamplePoints + lane / kCorners;
+    const bool ok = looks && i < points;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) q[d] = ok ? __ldg(&query[3 * i + d]) : -4.f;  // -4: outside every grid
+  };
+  struct Probe {
+    uint64_t key;
+    unsigned long long word;  // the home slot
+    float w;
+    bool inside;
+  };
+  auto start_probe = [&](uint32_t group, const float (&q)[3]) {
+    Probe pr;
+    const uint32_t i = group * kSamplePoints + lane / kCorners;
+    int x, y, z;
+    if constexpr (kNearest) {
+      x = static_cast<int>(q[0]), y = static_cast<int>(q[1]), z = static_cast<int>(q[2]);
+      pr.w = 1.f;
+    } else {
+      x = static_cast<int>(floorf(q[0] - 0.5f)) + (k & 1);
+      y = static_cast<int>(floorf(q[1] - 0.5f)) + ((k >> 1) & 1);
+      z = static_cast<int>(floorf(q[2] - 0.5f)) + ((k >> 2) & 1);
+      pr.w = (1.f - fabsf(q[0] - x - 0.5f)) * (1.f - fabsf(q[1] - y - 0.5f)) * (1.f - fabsf(q[2] - z - 0.5f));
     }
+    pr.inside = x >= 0 && x < g.W && y >= 0 && y < g.H && z >= 0 && z < g.D;
+    pr.key = 0, pr.word = 0;
+    if (pr.inside) {
+      pr.key = g.template key<kKeyBits>(static_cast<int>(i / L), x, y, z);
+      pr.word = table.start(pr.key);
+    }
+    return pr;
+  };
+  const uint32_t groups = (points + kSamplePoints - 1) / kSamplePoints, stride = gridDim.x * 8u;
+  uint32_t group = blockIdx.x * 8u + (threadIdx.x >> 5);
+  float ahead[3];
+  load_query(group, ahead);
+  Probe next = start_probe(group, ahead);
+  load_query(group + stride, ahead);
+  const int nv = C / kVec;
+#pragma unroll 1
+  for (; group < groups; group += stride) {
+    const uint32_t p0 = group * kSamplePoints;
+    const uint32_t nb = next.inside ? table.finish(next.key, next.word) : kInvalid;
+    float w = nb != kInvalid ? next.w : 0.f;
+    next = start_probe(group + stride, ahead);
+    load_query(group + 2 * stride, ahead);
     if constexpr (!kNearest) {
       // corner order of the sum as in the map kernel: the weights of a point are the same bits either way
       float sum = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) sum += __shfl_sync(0xffffffffu, w, (lane & 24) + k);
+      for (int j = 0; j < 8; ++j) sum += __shfl_sync(0xffffffffu, w, (lane & 24) + j);
       w *= 1.f / fmaxf(sum, 1e-12f);
     }
-    if (neighbor != nullptr && lane < kSamplePoints * kCorners && q < points) {
+    if (neighbor != nullptr && looks && p0 + lane / kCorners < points) {
       neighbor[size_t(p0) * kCorners + lane] = nb;
       if constexpr (!kNearest) weight[size_t(p0) * kCorners + lane] = w;
     }
-  }
-  const int nv = C / kVec;
+    // Only corners that exist are walked (about three of eight near a surface), kBatch rows in flight per step: walking all
+    // eight under predicates took twice the instructions and, at 80 registers, ran with a third of the warps.
+    constexpr int kBatch = kNearest ? 1 : 4;
+    const unsigned valid = __ballot_sync(0xffffffffu, nb != kInvalid);
+#pragma unroll 1
+    for (int i = 0; i < kSamplePoints; i += kAtOnce < kSamplePoints ? kAtOnce : kSamplePoints) {
+      const int local = (i + (kAtOnce == 1 ? 0 : lane / kGroup)) % kSamplePoints;
+      const bool mine = p0 + local < points;
+      const unsigned corners = (valid >> (local * kCorners)) & ((1u << kCorners) - 1u);
+      const int steps = kGroup == 32 ? __popc(corners) : __reduce_max_sync(0xffffffffu, __popc(corners));
+      for (int c0 = 0; c0 < nv; c0 += kGroup) {
+        const int c = c0 + lane % kGroup;
+        const bool col = mine && c < nv;
+        float acc[kVec];
 #pragma unroll
-  for (int i = 0; i < kSamplePoints; i += (kAtOnce < kSamplePoints ? kAtOnce : kSamplePoints)) {
-    const int local = i + (kAtOnce == 1 ? 0 : lane / kGroup);
-    const bool mine = local < kSamplePoints && p0 + local < points;
-    uint32_t rows[kCorners];
-    float ws[kCorners];
+        for (int j = 0; j < kVec; ++j) acc[j] = 0.f;
+        unsigned left = corners;
+        for (int t = 0; t < steps; t += kBatch) {
+          Raw raw[kBatch];
+          float ws[kBatch];
+          bool ok[kBatch];
 #pragma unroll
-    for (int k = 0; k < kCorners; ++k) {
-      rows[k] = __shfl_sync(0xffffffffu, nb, (local * kCorners + k) & 31);
-      ws[k] = __shfl_sync(0xffffffffu, w, (local * kCorners + k) & 31);
-    }
-    if (!mine) continue;
-    for (int c = lane % kGroup; c < nv; c += kGroup) {
-      Raw raw[kCorners];
+          for (int u = 0; u < kBatch; ++u) {
+            ok[u] = left != 0u;
+            const int src = local * kCorners + (ok[u] ? __ffs(left) - 1 : 0);
+            left &= left - 1u;
+            const uint32_t row = __shfl_sync(0xffffffffu, nb, src);
+            ws[u] = __shfl_sync(0xffffffffu, w, src);
+            if (ok[u] && col) raw[u] = __ldg(reinterpret_cast<const Raw*>(feats + size_t(row) * C) + c);
+          }
 #pragma unroll
-      for (int k = 0; k < kCorners; ++k)
-        if (rows[k] != kInvalid) raw[k] = __ldg(reinterpret_cast<const Raw*>(feats + size_t(rows[k]) * C) + c);
-      float acc[kVec];
-#pragma unroll
-      for (int j = 0; j < kVec; ++j) acc[j] = 0.f;
-#pragma unroll
-      for (int k = 0; k < kCorners; ++k)
-        if (rows[k] != kInvalid) fma_pack<T, kVec>(acc, raw[k], ws[k]);
-      __stcs(reinterpret_cast<Raw*>(out + size_t(p0 + local) * C) + c, round_pack<T, kVec>(acc));
+          for (int u = 0; u < kBatch; ++u)
+            if (ok[u]) fma_pack<T, kVec>(acc, raw[u], ws[u]);
+        }
+        if (col) __stcs(reinterpret_cast<Raw*>(out + size_t(p0 + local) * C) + c, round_pack<T, kVec>(acc));
+      }
     }
   }
 }
@@ -282,16 +320,15 @@ __global__ void __launch_bounds__(256) sample_kernel(const T* __restrict__ feats
 // Against fp32 atomics into a buffer that is zeroed before and converted after (10^6 points, C = 256 fp16 on the RES=256
 // shell: 2.05 ms + 28 + 35 us, all of it atomic traffic of 4 bytes per channel and corner) the gradient rows cross L2
 // as 2-byte values, and consecutive voxels share the points between them, so a row comes from HBM once.
-__global__ void __launch_bounds__(256) group_count_kernel(const uint32_t* __restrict__ indices, uint32_t entries, uint32_t* __restrict__ count,
-                                                          uint32_t* __restrict__ rank) {
+__global__ void __launch_bounds__(256) group_count_kernel(const uint32_t* __restrict__ indices, uint32_t entries, uint32_t* __restrict__ count) {
   chain_release();
   chain_wait();
   for (uint64_t e = blockIdx.x * uint64_t(256) + threadIdx.x; e < entries; e += uint64_t(gridDim.x) * 256) {
     const uint32_t row = __ldg(&indices[e]);
-    if (row != kInvalid) rank[e] = atomicAdd(&count[row], 1u);
+    if (row != kInvalid) atomicAdd(&count[row], 1u);
   }
 }
-// start[r] = where the entries of voxel r go.  The groups of 1024 consecutive voxels stand together, in order; such
+// start[r] = where the entries of voxel r go (the fill moves it on to their end).  The groups of 1024 consecutive voxels stand together, in order; such
 // blocks take their places as they come (one atomic each), which no result depends on.
 __global__ void __launch_bounds__(1024) group_place_kernel(const uint32_t* __restrict__ count, uint32_t n, uint32_t* __restrict__ start,
                                                            uint32_t* __restrict__ total) {
@@ -324,22 +361,21 @@ __global__ void __launch_bounds__(1024) group_place_kernel(const uint32_t* __res
   if (i < n) start[i] = s_base + (wi ? s_warp[wi - 1] : 0u) + inc - x;
 }
 __global__ void __launch_bounds__(256) group_fill_kernel(const uint32_t* __restrict__ indices, const float* __restrict__ weight, uint32_t entries,
-                                                         int V, const uint32_t* __restrict__ start, const uint32_t* __restrict__ rank,
-                                                         uint2* __restrict__ grouped) {
+                                                         int V, uint32_t* __restrict__ start, uint2* __restrict__ grouped) {
   chain_release();
   chain_wait();
   for (uint64_t e = blockIdx.x * uint64_t(256) + threadIdx.x; e < entries; e += uint64_t(gridDim.x) * 256) {
     const uint32_t row = __ldg(&indices[e]);
     if (row == kInvalid) continue;
     const float w = weight != nullptr ? __ldg(&weight[e]) : 1.f;
-    grouped[__ldg(&start[row]) + __ldg(&rank[e])] = make_uint2(static_cast<uint32_t>(e / V), __float_as_uint(w));
+    grouped[atomicAdd(&start[row], 1u)] = make_uint2(static_cast<uint32_t>(e / V), __float_as_uint(w));
   }
 }
 // kWarps warps of a CTA share one voxel (1, or 8 where voxels have many entries); kGroup lanes cover a row, so 32 / kGroup
 // entries are read side by side.
 template <typename T, int kVec, int kWarps, int kGroup>
 __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ grad_out, const uint2* __restrict__ grouped,
-                                                        const uint32_t* __restrict__ start, const uint32_t* __restrict__ count, uint32_t n, int C,
+                                                        const uint32_t* __restrict__ end, const uint32_t* __restrict__ count, uint32_t n, int C,
                                                         T* __restrict__ grad_feats) {
   using Raw = typename Pack<T, kVec>::Raw;
   constexpr int kSide = 32 / kGroup;
@@ -350,7 +386,7 @@ __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ gr
   const uint32_t row = kWarps > 1 ? blockIdx.x : blockIdx.x * 8u + wi;
   if (row >= n) return;  // whole warps; with kWarps > 1 whole CTAs
   const uint32_t len = __ldg(&count[row]);
-  const uint2* list = grouped + (len ? __ldg(&start[row]) : 0u);
+  const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
   const int nv = C / kVec;
   const int side = lane / kGroup;
   const int share = kWarps > 1 ? wi : 0;
@@ -402,7 +438,9 @@ static cudaError_t launch_sample(const void* feats, const float* query, uint32_t
   auto kernel = lanes == 8    ? sample_kernel<T, kVec, kKeyBits, kNearest, 8>
                 : lanes == 16 ? sample_kernel<T, kVec, kKeyBits, kNearest, 16>
                               : sample_kernel<T, kVec, kKeyBits, kNearest, 32>;
-  return launch_chained(kernel, dim3(static_cast<unsigned>(ceil_div(points, 8 * kSamplePoints))), dim3(256), 0, s, static_cast<const T*>(feats),
+  // eight CTAs per SM at most: more would only shorten the walks that hide the lookups
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ceil_div(points, 8 * kSamplePoints), int64_t(device_sm_count()) * 8));
+  return launch_chained(kernel, dim3(grid), dim3(256), 0, s, static_cast<const T*>(feats),
                         query, points, L, g, table, slots, C, static_cast<T*>(out), neighbor, weight);
 }
 template <typename T, int kVec>
@@ -430,7 +468,7 @@ static cudaError_t launch_group_sum(bool shared_rows, const void* grad_out, cons
 }
 
 struct GroupScratch {
-  size_t count_off, total_off, zero_bytes, start_off, rank_off, grouped_off, bytes;
+  size_t count_off, total_off, zero_bytes, start_off, grouped_off, bytes;
 };
 static GroupScratch group_scratch(int64_t entries, int64_t n) {
   GroupScratch g;
@@ -438,8 +476,7 @@ static GroupScratch group_scratch(int64_t entries, int64_t n) {
   g.total_off = align256(n * 4);
   g.zero_bytes = g.total_off + 256;
   g.start_off = g.zero_bytes;
-  g.rank_off = g.start_off + align256(n * 4);
-  g.grouped_off = g.rank_off + align256(entries * 4);
+  g.grouped_off = g.start_off + align256(n * 4);
   g.bytes = g.grouped_off + align256(entries * 8);
   return g;
 }
@@ -638,17 +675,15 @@ extern "C" int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t
   uint32_t* count = reinterpret_cast<uint32_t*>(mem + G.count_off);
   uint32_t* total = reinterpret_cast<uint32_t*>(mem + G.total_off);
   uint32_t* start = reinterpret_cast<uint32_t*>(mem + G.start_off);
-  uint32_t* rank = reinterpret_cast<uint32_t*>(mem + G.rank_off);
   uint2* grouped = reinterpret_cast<uint2*>(mem + G.grouped_off);
   LaunchErrors chain;
   chain.add(cudaMemsetAsync(mem, 0, G.zero_bytes, s));
   if (entries > 0) {
     const dim3 egrid(static_cast<unsigned>(std::min<int64_t>(ceil_div(entries, 256), 148 * 32)));
-    chain.add(launch_chained(group_count_kernel, egrid, dim3(256), 0, s, indices, entries, count, rank));
+    chain.add(launch_chained(group_count_kernel, egrid, dim3(256), 0, s, indices, entries, count));
     chain.add(launch_chained(group_place_kernel, dim3(static_cast<unsigned>(ceil_div(N, 1024))), dim3(1024), 0, s, static_cast<const uint32_t*>(count), n,
                              start, total));
-    chain.add(launch_chained(group_fill_kernel, egrid, dim3(256), 0, s, indices, weight, entries, V, static_cast<const uint32_t*>(start),
-                             static_cast<const uint32_t*>(rank), grouped));
+    chain.add(launch_chained(group_fill_kernel, egrid, dim3(256), 0, s, indices, weight, entries, V, start, grouped));
   }
   // many entries per voxel: the warps of a CTA share a voxel, else few warps would walk long lists
   const bool shared_rows = entries / n >= 128u;

@@ -35,16 +35,19 @@ struct Table<32> {
     }
     return false;
   }
-  __device__ __forceinline__ uint32_t find(uint64_t key) const {
+  // a lookup in two halves: the load of the home slot, and the rest once it has arrived
+  __device__ __forceinline__ unsigned long long start(uint64_t key) const { return __ldg(&slots_[home(key)]); }
+  __device__ __forceinline__ uint32_t finish(uint64_t key, unsigned long long w) const {
     uint32_t s = home(key);
     for (uint32_t i = 0; i < n_; ++i) {
-      unsigned long long w = __ldg(&slots_[s]);
       if (w == ~0ULL) return kInvalid;
       if (static_cast<uint32_t>(w >> 32) == static_cast<uint32_t>(key)) return static_cast<uint32_t>(w);
       if (++s >= n_) s = 0;
+      w = __ldg(&slots_[s]);
     }
     return kInvalid;
   }
+  __device__ __forceinline__ uint32_t find(uint64_t key) const { return finish(key, start(key)); }
 };
 
 template <>
@@ -66,16 +69,18 @@ struct Table<64> {
     }
     return false;
   }
-  __device__ __forceinline__ uint32_t find(uint64_t key) const {
+  __device__ __forceinline__ unsigned long long start(uint64_t key) const { return __ldg(&keys_[home(key)]); }
+  __device__ __forceinline__ uint32_t finish(uint64_t key, unsigned long long k) const {
     uint32_t s = home(key);
     for (uint32_t i = 0; i < n_; ++i) {
-      unsigned long long k = __ldg(&keys_[s]);
       if (k == ~0ULL) return kInvalid;
       if (k == key) return __ldg(&rows_[s]);
       if (++s >= n_) s = 0;
+      k = __ldg(&keys_[s]);
     }
     return kInvalid;
   }
+  __device__ __forceinline__ uint32_t find(uint64_t key) const { return finish(key, start(key)); }
 };
 
 template <int kKeyBits>

@@ -24,6 +24,10 @@ _PROTOTYPES = {
     "fgb_wgrad_call_workspace_bytes": (c_int64, [_P]),
     "fgb_wgrad_call_run": (c_int, [_P, _P]),
     "fgb_resize_rows": (c_int, [_P, _P, c_int64, c_int64, c_int64, c_int64, _P]),
+    "fgb_strided_grid_bytes": (c_int64, [_P]),
+    "fgb_strided_mark": (c_int, [_P, _P]),
+    "fgb_strided_build_bytes": (c_int64, [_P]),
+    "fgb_strided_build": (c_int, [_P, _P]),
     "fgb_subm_cache_scratch_bytes": (c_int64, [_P]),
     "fgb_subm_cache_build": (c_int, [_P, _P]),
     "fgb_error_string": (c_char_p, [c_int]),

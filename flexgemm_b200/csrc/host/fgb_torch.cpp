@@ -46,6 +46,7 @@ using torch::autograd::variable_list;
   X(fgb_conv_call_dgrad) X(fgb_wgrad_call_workspace_bytes) X(fgb_wgrad_call_run) X(fgb_resize_rows)                   \
   X(fgb_bias_grad_workspace_bytes) X(fgb_subm_conv_bias_grad) X(fgb_subm_cache_scratch_bytes)                         \
   X(fgb_subm_cache_build) X(fgb_pp_valid_signal) X(fgb_hash_table_bytes)                                    \
+  X(fgb_strided_grid_bytes) X(fgb_strided_mark) X(fgb_strided_build_bytes) X(fgb_strided_build)                       \
   X(fgb_grid_sample_fused) X(fgb_indice_weighted_sum_grad_bytes) X(fgb_indice_weighted_sum_grad)
 struct Api {
 #define X(f) decltype(&::f) f = nullptr;
@@ -356,7 +357,7 @@ Grads run_backward(const Tensor& grad_output, const Tensor& feats, const Tensor&
 // ------------------------------------------------------------------ Python objects
 PyObject *s_neighbor_map, *s_gray_code, *s_sorted_idx, *s_tile_masks, *s_block_order, *s_vs_i, *s_vs_o, *s_seg, *s_block_offsets, *s_build_status;
 PyObject *s_neighbor_map_bwd, *s_sorted_idx_bwd, *s_tile_masks_bwd, *s_block_order_bwd, *s_ensure_bwd, *s_m_tile_masks, *s_m_block_order,
-    *s_m_tile_masks_bwd, *s_m_block_order_bwd, *s_tile_rows;
+    *s_m_tile_masks_bwd, *s_m_block_order_bwd, *s_tile_rows, *s_gray_code_bwd;
 PyObject* s_empty_tuple;
 
 struct PyError {};  // a Python exception is set
@@ -542,23 +543,34 @@ CacheBuild start_cache(const Tensor& coords, const int64_t* shape, const int64_t
   return b;
 }
 
+// Waits for the sequence number in word `index` without holding the GIL, gives the words back and returns those from
+// `first` on.
+struct Words3 {
+  uint32_t v[3];
+};
+Words3 take_back(const HostWords& w, int first, int index, cudaStream_t stream) {
+  std::exception_ptr failed;
+  Py_BEGIN_ALLOW_THREADS;
+  try {
+    wait_host_words(w, index, stream);
+  } catch (...) {
+    failed = std::current_exception();
+  }
+  Py_END_ALLOW_THREADS;
+  if (failed) std::rethrow_exception(failed);
+  const Words3 r{{w.host[first], w.host[first + 1], w.host[first + 2]}};
+  give_host_words(w);
+  return r;
+}
+
 // waits for the pair count and queues the pair lists; the GIL is released while it waits
 Pairs finish_cache(const CacheBuild& b) {
   const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
   int64_t pairs = 0;
   if (b.n > 0) {
-    std::exception_ptr failed;
-    Py_BEGIN_ALLOW_THREADS;
-    try {
-      wait_host_words(b.words, b.V + 3, stream);
-    } catch (...) {
-      failed = std::current_exception();
-    }
-    Py_END_ALLOW_THREADS;
-    if (failed) std::rethrow_exception(failed);
-    pairs = b.words.host[b.V];
-    const int code = static_cast<int>(b.words.host[b.V + 2]);
-    give_host_words(b.words);
+    const Words3 got = take_back(b.words, b.V, b.V + 3, stream);
+    pairs = got.v[0];
+    const int code = static_cast<int>(got.v[2]);
     if (code != 0) throw_soft_error(code);
   }
   Pairs p;
@@ -808,6 +820,196 @@ PyObject* py_conv_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   FGB_END
 }
 
+// ------------------------------------------------------------------ strided convolution
+struct StridedBuild {
+  fgb_strided_call c{};
+  c10::DataPtr grid;
+  Tensor out_coords, nbr, nbr_bwd, gray, gray_bwd, sorted_idx, sorted_bwd, masks, masks_bwd, order, order_bwd, block_offsets, meta;
+  HostWords words;
+  int V = 0;
+};
+
+// marks and counts the output voxels; false where the bit grid does not serve the case (or there are none)
+bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape, const int64_t* ks, const int64_t* st, const int64_t* pad,
+                    const int64_t* dil, bool coords_only) {
+  const auto stream = c10::cuda::getCurrentCUDAStream(coords.device().index());
+  fgb_strided_call& c = b.c;
+  c.coords = cptr<int32_t>(coords);
+  c.n = coords.size(0);
+  c.b = static_cast<int32_t>(shape[0]), c.w = static_cast<int32_t>(shape[2]), c.h = static_cast<int32_t>(shape[3]), c.d = static_cast<int32_t>(shape[4]);
+  for (int i = 0; i < 3; ++i) {
+    c.k[i] = static_cast<int32_t>(ks[i]), c.s[i] = static_cast<int32_t>(st[i]);
+    c.p[i] = static_cast<int32_t>(pad[i]), c.dil[i] = static_cast<int32_t>(dil[i]);
+  }
+  b.V = static_cast<int>(ks[0] * ks[1] * ks[2]);
+  const int64_t bytes = api.fgb_strided_grid_bytes(&c);
+  if (bytes <= 0) return false;
+  b.grid = scratch(bytes);
+  c.grid_mem = b.grid.get(), c.grid_bytes = bytes;
+  const HostWords w = take_host_words();
+  c.host_words = w.dev, c.host_seq = w.seq;
+  check(api.fgb_strided_mark(&c, stream), "fgb_strided_mark");
+  g_launches += 2;
+  c.n_out = take_back(w, 0, 1, stream).v[0];
+  c.host_words = nullptr;
+  b.out_coords = new_tensor({c.n_out, 4}, at::kInt, coords.device());
+  if (c.n_out == 0) return coords_only;
+  c.out_coords = static_cast<int32_t*>(b.out_coords.data_ptr());
+  if (coords_only) {
+    check(api.fgb_strided_build(&c, stream), "fgb_strided_build");
+    g_launches += 1;
+  }
+  return true;
+}
+
+void strided_maps(StridedBuild& b, at::Device dev, bool train) {
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  fgb_strided_call& c = b.c;
+  const int64_t n = c.n, m = c.n_out, V = b.V;
+  auto tiles = [](int64_t rows) { return (rows + 127) / 128; };
+  auto make = [&](Tensor& t, at::IntArrayRef size, at::ScalarType dt) {
+    t = new_tensor(size, dt, dev);
+    return t.data_ptr();
+  };
+  c.neighbor_map = static_cast<uint32_t*>(make(b.nbr, {m, V}, at::kUInt32));
+  c.gray_code = static_cast<int32_t*>(make(b.gray, {m}, at::kInt));
+  c.sorted_idx = static_cast<int64_t*>(make(b.sorted_idx, {m}, at::kLong));
+  c.tile_masks = static_cast<uint32_t*>(make(b.masks, {tiles(m)}, at::kUInt32));
+  c.block_order = static_cast<uint32_t*>(make(b.order, {(tiles(m) + 1) / 2}, at::kUInt32));
+  c.block_offsets = static_cast<uint32_t*>(make(b.block_offsets, {V * ((m + 255) / 256)}, at::kUInt32));
+  c.meta = static_cast<uint32_t*>(make(b.meta, {V + 1}, at::kUInt32));
+  if (train) {
+    c.neighbor_map_bwd = static_cast<uint32_t*>(make(b.nbr_bwd, {n, V}, at::kUInt32));
+    c.gray_code_bwd = static_cast<int32_t*>(make(b.gray_bwd, {n}, at::kInt));
+    c.sorted_idx_bwd = static_cast<int64_t*>(make(b.sorted_bwd, {n}, at::kLong));
+    c.tile_masks_bwd = static_cast<uint32_t*>(make(b.masks_bwd, {tiles(n)}, at::kUInt32));
+    c.block_order_bwd = static_cast<uint32_t*>(make(b.order_bwd, {(tiles(n) + 1) / 2}, at::kUInt32));
+    b.words = take_host_words();
+    c.host_words = b.words.dev, c.host_seq = b.words.seq;
+  }
+  c.scratch_bytes = check_bytes(api.fgb_strided_build_bytes(&c), "fgb_strided_build_bytes");
+  const c10::DataPtr mem = scratch(c.scratch_bytes);
+  c.scratch = mem.get();
+  c.status = static_cast<int32_t*>(device_state(dev.index()).status.data_ptr());
+  check(api.fgb_strided_build(&c, stream), "fgb_strided_build");
+  g_launches += train ? 11 : 8;
+}
+
+Pairs strided_pairs(const StridedBuild& b) {
+  const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
+  const int64_t pairs = take_back(b.words, b.V, b.V + 3, stream).v[0];
+  Pairs p;
+  p.vs_i = new_tensor({pairs}, at::kUInt32, b.nbr.device());
+  p.vs_o = new_tensor({pairs}, at::kUInt32, b.nbr.device());
+  p.seg = b.meta;
+  p.block_offsets = b.block_offsets;
+  if (pairs > 0) {
+    check(api.fgb_pp_valid_signal(cptr<uint32_t>(b.nbr), cptr<int32_t>(b.gray), b.c.n_out, b.V, cptr<uint32_t>(b.block_offsets), cptr<uint32_t>(b.meta),
+                                  static_cast<uint32_t*>(p.vs_i.data_ptr()), static_cast<uint32_t*>(p.vs_o.data_ptr()), nullptr, stream),
+          "fgb_pp_valid_signal");
+    g_launches += 1;
+  }
+  return p;
+}
+
+bool geometry_args(PyObject* stride, PyObject* padding, PyObject* dilation, int64_t* st, int64_t* pad, int64_t* dil) {
+  if (!int_args(stride, 3, st) || !int_args(padding, 3, pad) || !int_args(dilation, 3, dil)) return false;
+  for (int i = 0; i < 3; ++i)
+    if (st[i] < 1 || pad[i] < 0 || dil[i] < 1) return false;
+  return true;
+}
+bool rows_ok(const Tensor& coords) {
+  const int64_t one[3] = {1, 1, 1};
+  return coords_ok(coords, one) && coords.size(0) > 0;
+}
+
+// (coords, shape, kernel_size, stride, padding, dilation) -> output coordinates in flat-index order, or None
+PyObject* py_strided_coords(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  FGB_TRY
+  TORCH_CHECK(n == 6, "strided_coords takes 6 arguments");
+  const Tensor coords = tensor_arg(a[0]);
+  int64_t shape[5], ks[3], st[3], pad[3], dil[3];
+  if (!rows_ok(coords) || !int_args(a[1], 5, shape) || !int_args(a[2], 3, ks) || !geometry_args(a[3], a[4], a[5], st, pad, dil)) Py_RETURN_NONE;
+  c10::cuda::CUDAGuard guard(coords.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  StridedBuild b;
+  if (!strided_coords(b, coords, shape, ks, st, pad, dil, true)) Py_RETURN_NONE;
+  return THPVariable_Wrap(b.out_coords);
+  FGB_END
+}
+
+// (cache_cls, feats, coords, shape, weight, bias, stride, padding, dilation, tf32) -> (out, out_coords, cache) or None
+PyObject* py_strided_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  FGB_TRY
+  TORCH_CHECK(n == 10, "strided_conv takes 10 arguments");
+  const Tensor feats = tensor_arg(a[1]), coords = tensor_arg(a[2]), weight = tensor_arg(a[4]), bias = tensor_arg(a[5]);
+  const int dtype = feats.defined() ? dtype_code(feats.scalar_type(), PyObject_IsTrue(a[9]) == 1) : -1;
+  int64_t V = 0, shape[5], st[3], pad[3], dil[3];
+  if (!conv_args_ok(feats, weight, bias, a[5], &V, dtype) || !rows_ok(coords) || coords.device() != feats.device() ||
+      coords.size(0) != feats.size(0) || !int_args(a[3], 5, shape) || !geometry_args(a[6], a[7], a[8], st, pad, dil))
+    Py_RETURN_NONE;
+  const int64_t ks[3] = {weight.size(1), weight.size(2), weight.size(3)};
+  c10::cuda::CUDAGuard guard(feats.device());
+  StridedBuild b;
+  Tensor out;
+  Pairs pairs;
+  Maps m, bwd;
+  const bool train = feats.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad());
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    if (!strided_coords(b, coords, shape, ks, st, pad, dil, false)) Py_RETURN_NONE;
+    strided_maps(b, feats.device(), train);
+    m = Maps{b.nbr, b.sorted_idx, b.masks, b.order};
+    if (train) bwd = Maps{b.nbr_bwd, b.sorted_bwd, b.masks_bwd, b.order_bwd};
+    try {
+      out = run_fprop(feats, weight, bias, m, V, dtype);
+    } catch (...) {
+      if (train) strided_pairs(b);
+      throw;
+    }
+    if (train) pairs = strided_pairs(b);
+  }
+  PyObject* cache = new_cache(a[0]);
+  PyObject* t = nullptr;
+  try {
+    set_tensor(cache, s_neighbor_map, b.nbr);
+    set_tensor(cache, s_gray_code, b.gray);
+    set_tensor(cache, s_sorted_idx, b.sorted_idx);
+    set_tensor(cache, s_tile_masks, b.masks);
+    set_tensor(cache, s_block_order, b.order);
+    if (train) {
+      set_tensor(cache, s_neighbor_map_bwd, b.nbr_bwd);
+      set_tensor(cache, s_gray_code_bwd, b.gray_bwd);
+      set_tensor(cache, s_sorted_idx_bwd, b.sorted_bwd);
+      set_tensor(cache, s_tile_masks_bwd, b.masks_bwd);
+      set_tensor(cache, s_block_order_bwd, b.order_bwd);
+      set_tensor(cache, s_seg, pairs.seg);
+      set_tensor(cache, s_vs_i, pairs.vs_i);
+      set_tensor(cache, s_vs_o, pairs.vs_o);
+      set_tensor(cache, s_block_offsets, b.block_offsets);
+    } else if (PyObject_SetAttr(cache, s_neighbor_map_bwd, Py_None) != 0) {
+      throw PyError{};
+    }
+    out = conv_autograd(feats, weight, bias, m, bwd, pairs, false, V, dtype, std::move(out));
+    PyObject* o = THPVariable_Wrap(out);
+    PyObject* oc = o != nullptr ? THPVariable_Wrap(b.out_coords) : nullptr;
+    t = oc != nullptr ? PyTuple_New(3) : nullptr;
+    if (t == nullptr) {
+      Py_XDECREF(o);
+      Py_XDECREF(oc);
+      throw PyError{};
+    }
+    PyTuple_SET_ITEM(t, 0, o);
+    PyTuple_SET_ITEM(t, 1, oc);
+    PyTuple_SET_ITEM(t, 2, cache);
+  } catch (...) {
+    Py_DECREF(cache);
+    throw;
+  }
+  return t;
+  FGB_END
+}
+
 // ------------------------------------------------------------------ grid sample
 Tensor run_sample_grad(const Tensor& grad_out /* [M, C] */, const Tensor& indices, const Tensor& weight, int64_t n, int64_t V) {
   c10::cuda::CUDAGuard guard(grad_out.device());
@@ -942,6 +1144,8 @@ PyMethodDef methods[] = {
     {"subm_conv", FAST(py_subm_conv), "submanifold conv"},
     {"conv", FAST(py_conv), "convolution on an existing cache"},
     {"conv_backward", FAST(py_conv_backward), "gradients of a convolution"},
+    {"strided_coords", FAST(py_strided_coords), "output coordinates of a strided conv"},
+    {"strided_conv", FAST(py_strided_conv), "strided conv"},
     {"grid_sample", FAST(py_grid_sample), "sparse grid sample"},
     {"sample_grad", FAST(py_sample_grad), "gradient of a weighted gather"},
     {"status_word", py_status_word, METH_O, "device status word"},
@@ -968,6 +1172,7 @@ PyMODINIT_FUNC PyInit__fgb_torch(void) {
   s_sorted_idx_bwd = PyUnicode_InternFromString("sorted_idx_bwd");
   s_tile_masks_bwd = PyUnicode_InternFromString("tile_masks_bwd_128");
   s_block_order_bwd = PyUnicode_InternFromString("block_order_bwd_128");
+  s_gray_code_bwd = PyUnicode_InternFromString("gray_code_bwd");
   s_ensure_bwd = PyUnicode_InternFromString("_ensure_bwd_order");
   s_m_tile_masks = PyUnicode_InternFromString("tile_masks");
   s_m_block_order = PyUnicode_InternFromString("block_order");

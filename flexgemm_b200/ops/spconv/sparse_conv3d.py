@@ -130,6 +130,10 @@ class SparseConv3dFunction(Function):
             raise ValueError(f"Unsupported output coordinate algorithm {spconv.OUT_COORD_ALGO}")
         if spconv.SERIALIZATION_MODE not in (0, 1, 2):
             raise RuntimeError("Unsupported serialize mode.")
+        if spconv.SERIALIZATION_MODE == 0:   # flat-index order falls out of marking the output cells as bits
+            got = _native.ext().strided_coords(coords, shape, kernel_size, stride, padding, dilation)
+            if got is not None:
+                return got
         return kernels.cuda.sparse_out_coords(coords, shape, kernel_size, stride, padding, dilation,
                                               spconv.OUT_COORD_HASHMAP_RATIO, spconv.SERIALIZATION_MODE)
 
@@ -366,4 +370,16 @@ def sparse_conv3d(feats: torch.Tensor, coords: torch.Tensor, shape: torch.Size, 
     Returns:
         (out_feats [M, Co], out_coords [M, 4], neighbor_cache)
     """
+    if spconv.ALGORITHM in _MASKED:
+        if neighbor_cache is None and out_coords is None and spconv.SERIALIZATION_MODE == 0 and spconv.OUT_COORD_ALGO in (0, 1):
+            got = _native.ext().strided_conv(SparseConv3dNeighborCache, feats, coords, shape, weight, bias, stride, padding, dilation,
+                                             config.allow_tf32)
+            if got is not None:
+                return got
+        elif neighbor_cache is not None:
+            if out_coords is None:
+                out_coords = SparseConv3dFunction._get_output_coords(coords, shape, tuple(weight.shape[1:4]), stride, padding, dilation)
+            out = _native.ext().conv(feats, weight, bias, neighbor_cache, config.allow_tf32, True)
+            if out is not None:
+                return out, out_coords, neighbor_cache
     return SparseConv3dFunction.apply(feats, coords, shape, neighbor_cache, weight, bias, out_coords, stride, padding, dilation)

@@ -614,6 +614,52 @@ typedef struct fgb_map_call {
 int64_t fgb_subm_cache_scratch_bytes(const fgb_map_call* call);
 int fgb_subm_cache_build(const fgb_map_call* call, void* stream);
 
+/* A strided convolution's output coordinates -- the distinct output voxels that
+ * an input voxel reaches, in flat-index order -- and everything it needs of them,
+ * in two calls with one host read (the number of output rows) between:
+ *   fgb_strided_grid_bytes  memory of the marked output cells; 0 when the grid is
+ *                           too large or too empty for one bit per cell (the calls
+ *                           of the generic conv above then do the work);
+ *   fgb_strided_mark        marks and counts the cells; host_words (mapped pinned,
+ *                           may be null) receives the count in word 0, then
+ *                           host_seq in word 1;
+ *   fgb_strided_build       with n_out = that count: out_coords and, when
+ *                           neighbor_map is not null, both maps (the backward one
+ *                           when neighbor_map_bwd is not null), codes, row orders,
+ *                           tile masks, schedules, block offsets, and meta [v + 1] =
+ *                           the segment table; host_words as in fgb_map_call.
+ * coords: in-range rows without duplicates (of duplicates, any one is kept). */
+typedef struct fgb_strided_call {
+  const int32_t* coords;
+  int64_t n;
+  int32_t b, w, h, d, k[3], s[3], p[3], dil[3];
+  void* grid_mem;
+  int64_t grid_bytes;
+  uint32_t* host_words;
+  uint32_t host_seq;
+  int64_t n_out;
+  int32_t* out_coords;
+  uint32_t* neighbor_map;
+  uint32_t* neighbor_map_bwd;
+  int32_t* gray_code;
+  int32_t* gray_code_bwd;
+  int64_t* sorted_idx;
+  int64_t* sorted_idx_bwd;
+  uint32_t* tile_masks;
+  uint32_t* tile_masks_bwd;
+  uint32_t* block_order;
+  uint32_t* block_order_bwd;
+  uint32_t* block_offsets;
+  uint32_t* meta;
+  void* scratch;
+  int64_t scratch_bytes;
+  int32_t* status;
+} fgb_strided_call;
+int64_t fgb_strided_grid_bytes(const fgb_strided_call* call);
+int fgb_strided_mark(const fgb_strided_call* call, void* stream);
+int64_t fgb_strided_build_bytes(const fgb_strided_call* call);
+int fgb_strided_build(const fgb_strided_call* call, void* stream);
+
 /* grad_weight [co, v, ci] and, when grad_bias is not null, grad_bias [co], both
  * of the element type `dtype`. */
 typedef struct fgb_wgrad_call {

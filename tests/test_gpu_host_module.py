@@ -116,3 +116,45 @@ def test_grid_sample_matches_separate_kernels(C, dtype, mode, points, volume):
     mag = K.indice_weighted_sum_bwd(gout.view(-1, C).abs(), idx, w, coords.shape[0]).double()
     terms = 8.0 * points / 100
     assert torch.all((gf.double() - g32).abs() <= g32.abs() * ulp + mag * 2.0 ** -24 * (2 + terms) + 1e-7)
+
+
+@pytest.mark.parametrize("ksize,stride,pad,dil", [((2, 2, 2), (2, 2, 2), (0, 0, 0), (1, 1, 1)), ((3, 3, 3), (2, 2, 2), (1, 1, 1), (1, 1, 1)),
+                                                  ((3, 1, 2), (1, 3, 2), (2, 0, 1), (2, 1, 1)), ((1, 1, 1), (1, 1, 1), (0, 0, 0), (1, 1, 1)),
+                                                  ((1, 1, 32), (1, 1, 4), (0, 0, 15), (1, 1, 1))])
+@pytest.mark.parametrize("n,shuffle", [(1, False), (255, True), (3000, False), (40000, True)])
+def test_strided_build_matches_hash_path(ksize, stride, pad, dil, n, shuffle):
+    """Output coordinates and maps made on the bit grid against the hash set, sort and table of the generic calls."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import utils
+    from flexgemm_b200.ops.spconv import SparseConv3dFunction, sparse_conv3d
+    g = torch.Generator().manual_seed(n)
+    W, H, D = 40, 33, 70
+    flat = torch.randperm(2 * W * H * D, generator=g)[:n].sort().values
+    coords = torch.stack([flat // (W * H * D), flat // (H * D) % W, flat // D % H, flat % D], 1).int()
+    if shuffle:
+        coords = coords[torch.randperm(n, generator=g)]
+    coords = coords.to(DEV).contiguous()
+    shape = torch.Size((2, 8, W, H, D))
+    geom = (shape, ksize, stride, pad, dil)
+    want_oc = K.sparse_out_coords(coords, *geom, 1.1, 0)
+    assert torch.equal(SparseConv3dFunction._get_output_coords(coords, *geom), want_oc)
+    feats = torch.randn(n, 8, generator=g).half().to(DEV).requires_grad_(True)
+    weight = torch.randn(8, *ksize, 8, generator=g).half().to(DEV)
+    out, oc, cache = sparse_conv3d(feats, coords, shape, weight, None, stride=stride, padding=pad, dilation=dil)
+    assert torch.equal(oc, want_oc) and out.shape == (oc.shape[0], 8)
+    if oc.shape[0] == 0:
+        return
+    V = ksize[0] * ksize[1] * ksize[2]
+    table, bits = utils.init_table(shape, max(2 * n, 1), DEV)
+    want = K.sparse_build_neighbor_map(coords, oc, *geom, table, bits, max(2 * n, 1), True)
+    seg = u32(want["valid_signal_seg"])
+    vs_i, vs_o = K.valid_signal(want["neighbor_map"], want["gray_code"], want["block_offsets"], want["valid_signal_seg"], int(seg[V]))
+    gray_bwd, binary_bwd = K.gray_code_from_map(want["neighbor_map_bwd"])
+    order, order_bwd = K.sorted_idx_from_binary(want["binary_code"], V), K.sorted_idx_from_binary(binary_bwd, V)
+    for name, ref in (("neighbor_map", want["neighbor_map"]), ("neighbor_map_bwd", want["neighbor_map_bwd"]), ("valid_signal_i", vs_i),
+                      ("valid_signal_o", vs_o), ("valid_signal_seg", want["valid_signal_seg"]), ("pair_block_offsets", want["block_offsets"]),
+                      ("tile_masks_128", K.tile_masks(want["gray_code"], order, 128)), ("tile_masks_bwd_128", K.tile_masks(gray_bwd, order_bwd, 128))):
+        assert np.array_equal(u32(cache[name]), u32(ref)), name
+    for name, ref in (("gray_code", want["gray_code"]), ("gray_code_bwd", gray_bwd), ("sorted_idx", order), ("sorted_idx_bwd", order_bwd)):
+        assert torch.equal(cache[name], ref), name
+    K.check_status(DEV)

@@ -79,7 +79,9 @@ struct IgemmParams {
   int bn;                    // output channels per work item (32, 64, 128, 256)
   int n_tiles_n;
   int splits;                // split-K: shares of a block's offsets that run as separate work items (1 = off)
-  int items_per_block;       // n_tiles_n * splits
+  int items_per_block;       // n_tiles_n * splits; tail mode: n_tiles_n * 3 (upper half, lower half, whole block)
+  uint32_t tickets;          // work items to hand out
+  uint32_t whole_items;      // tail mode: (block, column tile) items handed out whole; the rest go out as two halves each
   int row_bytes;             // kc * element size
   int num_kb;                // 128-byte slices per row
   int flip;                  // bit 0: weight slot = V-1-v instead of v; bit 1: the weight operand is MN-major (below)
@@ -202,7 +204,8 @@ __device__ __forceinline__ uint4 fuse_piece(uint4 val, int act, const char* resi
 // kMode: kPlain -- the epilogue adds the bias and writes `out` in the operand type; kFusedEp -- the same plus
 // activation / residual / pre-activation copy; kSplitK -- the work item covers only a share of the block's offsets and
 // the epilogue writes the raw fp32 accumulators into its split's slab of a partial buffer (summed by a second kernel).
-enum { kPlain = 0, kFusedEp = 1, kSplitK = 2 };
+// kTail -- as kPlain, but the last items of the schedule go out as halves (see tail_items).
+enum { kPlain = 0, kFusedEp = 1, kSplitK = 2, kTail = 3 };
 
 template <int kDtype, int kMode>
 __global__ void __launch_bounds__(kIgemmThreads, 1)
@@ -210,6 +213,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
   constexpr bool kTF32 = (kDtype == FGB_F32_TF32);
   constexpr bool kFused = kMode == kFusedEp;
   constexpr bool kSplit = kMode == kSplitK;
+  constexpr bool kHalves = kMode == kTail;
   constexpr int kElem = (kDtype == FGB_F16 || kDtype == FGB_BF16) ? 2 : 4;
   constexpr int kOutDtype = kSplit ? FGB_F32_TF32 : kDtype;  // element type the epilogue writes
   constexpr int kElemOut = kSplit ? 4 : kElem;
@@ -279,8 +283,15 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     // so they run at about the same time on different SMs and find the block's gathered rows in L2
     const uint32_t ipb = static_cast<uint32_t>(p.items_per_block);
     const uint32_t t = pub_block == none ? none : atomicAdd(p.ticket, 1u);
-    if (t == none || t / ipb >= p.num_blocks) {
+    if (t == none || t >= p.tickets) {
       pub_block = none;  // stays "no more work"
+    } else if constexpr (kHalves) {
+      const uint32_t nt = ipb / 3u;
+      const bool half = t >= p.whole_items;
+      const uint32_t item = half ? p.whole_items + (t - p.whole_items) / 2u : t;
+      const uint32_t pos = nt == 1 ? item : item / nt;
+      pub_block = p.block_order != nullptr ? __ldg(&p.block_order[pos]) : pos;
+      pub_ntile = (item - pos * nt) * 3u + (half ? (t - p.whole_items) & 1u : 2u);
     } else {
       const uint32_t pos = ipb == 1 ? t : t / ipb;
       pub_block = p.block_order != nullptr ? __ldg(&p.block_order[pos]) : pos;
@@ -303,7 +314,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     return true;
   };
   // column tile and split of a work item's sub-index
-  auto tile_of = [&](uint32_t sub) -> uint32_t { return kSplit ? sub / static_cast<uint32_t>(p.splits) : sub; };
+  auto tile_of = [&](uint32_t sub) -> uint32_t { return kSplit ? sub / static_cast<uint32_t>(p.splits) : kHalves ? sub / 3u : sub; };
   auto split_of = [&](uint32_t sub) -> uint32_t { return kSplit ? sub % static_cast<uint32_t>(p.splits) : 0u; };
   // Offset masks of the two halves of a work item.  With split-K the item keeps only its share of the block's
   // offsets: the set bits of the union mask, in ascending order, are dealt to the splits in equal runs (a split beyond
@@ -320,6 +331,11 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
         if (rank >= first && rank < last) keep |= u & (0u - u);
       }
       m0 &= keep, m1 &= keep;
+    }
+    if constexpr (kHalves) {
+      const uint32_t which = sub % 3u;
+      if (which == 0u) m1 = 0u;
+      else if (which == 1u) m0 = 0u;
     }
   };
 
@@ -533,6 +549,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
       tc_fence_after_sync();
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
+        if (kHalves && ntile % 3u + h == 1u) continue;  // the other half of the block is another item
         const bool has_acc = (h == 0 ? m0 : m1) != 0u;  // a half without offsets holds no rows
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + set * 2 * p.bn + h * p.bn;
         for (int c0 = group * kColsPerPass; c0 < p.bn; c0 += 2 * kColsPerPass) {
@@ -790,6 +807,11 @@ static int pick_bn(int nout) {
 // beside a conv kernel leaves it some SMs this way: the conv CTAs fill their SMs completely (shared memory and
 // registers), so a kernel launched beside them would otherwise wait for the first of them to finish.
 static std::atomic<int> g_cta_limit{0};
+static int persistent_ctas() {
+  const int ctas = device_sm_count();
+  const int limit = g_cta_limit.load(std::memory_order_relaxed);
+  return limit > 0 && limit < ctas ? limit : ctas;
+}
 
 template <int kDtype, int kMode>
 static int launch_igemm_variant(const CUtensorMap& tmap, const IgemmParams& p, const FusedEpilogue& fe, cudaStream_t s) {
@@ -797,10 +819,8 @@ static int launch_igemm_variant(const CUtensorMap& tmap, const IgemmParams& p, c
   static PerDeviceTable configured;  // the attribute belongs to (kernel instance, device)
   const int rc = ensure_dynamic_smem(configured, subm_igemm_kernel<kDtype, kMode>, smem);
   if (rc != FGB_OK) return rc;
-  const int64_t work = int64_t(p.num_blocks) * p.items_per_block;
-  int ctas = device_sm_count();
-  const int limit = g_cta_limit.load(std::memory_order_relaxed);
-  if (limit > 0 && limit < ctas) ctas = limit;
+  const int64_t work = p.tickets;
+  const int ctas = persistent_ctas();
   const unsigned grid = static_cast<unsigned>(work < ctas ? work : ctas);
   const cudaError_t e = launch_chained(subm_igemm_kernel<kDtype, kMode>, dim3(grid), dim3(kIgemmThreads), smem, s, tmap, p, fe);
   return e != cudaSuccess ? cuda_status(e) : launch_status();
@@ -810,6 +830,7 @@ static int launch_igemm_variant(const CUtensorMap& tmap, const IgemmParams& p, c
 template <int kDtype>
 static int launch_igemm(const CUtensorMap& tmap, const IgemmParams& p, const FusedEpilogue& fe, cudaStream_t s) {
   if (p.splits > 1) return launch_igemm_variant<kDtype, kSplitK>(tmap, p, fe, s);
+  if (p.whole_items < p.tickets) return launch_igemm_variant<kDtype, kTail>(tmap, p, fe, s);
   if (fe.act != FGB_ACT_NONE || fe.residual != nullptr || fe.preact != nullptr) return launch_igemm_variant<kDtype, kFusedEp>(tmap, p, fe, s);
   return launch_igemm_variant<kDtype, kPlain>(tmap, p, fe, s);
 }
@@ -837,6 +858,24 @@ int igemm_splits(int64_t n, int nout, int V) {
 int64_t igemm_partial_bytes(int64_t n, int nout, int V) {
   const int sp = igemm_splits(n, nout, V);
   return sp > 1 ? align256(int64_t(sp) * n * nout * 4) : 0;
+}
+
+// ------------------------------------------------------------------ halves at the end of a launch
+// A launch of T work items on P SMs ends with about T mod P items running alone while the other SMs idle; at a few items
+// per SM that is a good part of the launch (RES=128, C=256: 161 items on 148 SMs).  A half of a block (one 128-row
+// accumulator, the other left out of gather, MMA and write-out) takes 0.6 to 0.7 of the whole block's time -- the weight
+// tile is fetched for both -- so the items beyond the whole waves, the cheapest of the schedule, go out as two halves
+// each where the halves fit one wave.  No sum is cut: every row sees the same products in the same order.
+// fprop / dgrad, us: RES=128 C=256 fp16 106 -> 97, C=96 bf16 50 -> 45, C=512 TF32 626 / 645 -> 592 / 613; RES=256 C=256
+// 260 -> 254.  Beyond six waves the rest is a few percent and the items' spread hides it.  Halving every item of a launch
+// below one wave lost (156 items, 239 -> 295 us): the halves make two waves.
+// (Shares of the offsets with partial accumulators in memory, added up by the last CTA, balance better on paper but the
+// slabs cost more than they win: 256 -> 293 us at RES=256, C=256, and 545 us in the TF32 case.)
+static int64_t tail_items(int64_t T) {
+  const int64_t P = persistent_ctas();
+  if (T < P || T > 6 * P) return 0;
+  const int64_t rest = T % P;
+  return rest * 2 > P ? 0 : rest;
 }
 
 // out[r, c] = sum_s partial[s, r, c] (+ bias[c]) in split order, converted to T
@@ -904,6 +943,12 @@ int run_igemm(const void* x, const void* w, const void* bias, const uint32_t* nb
   p.splits = (partial != nullptr && !fused) ? igemm_splits(n, nout, V) : 1;
   p.items_per_block = p.n_tiles_n * p.splits;
   if (p.splits > 1) p.out = reinterpret_cast<char*>(partial);
+  const int64_t all_items = ceil_div(n, kBlockM) * p.n_tiles_n;
+  const int64_t halved = p.splits == 1 && !fused ? tail_items(all_items) : 0;
+  if (all_items * p.splits > 0x7FFFFFFF) return FGB_E_SIZE;
+  p.whole_items = static_cast<uint32_t>(all_items * p.splits - halved);
+  p.tickets = p.whole_items + static_cast<uint32_t>(2 * halved);
+  if (halved > 0) p.items_per_block = p.n_tiles_n * 3;
   p.row_bytes = kc * eb;
   p.num_kb = static_cast<int>(ceil_div(p.row_bytes, 128));
   p.flip = flip;

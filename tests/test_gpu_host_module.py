@@ -158,3 +158,29 @@ def test_strided_build_matches_hash_path(ksize, stride, pad, dil, n, shuffle):
     for name, ref in (("gray_code", want["gray_code"]), ("gray_code_bwd", gray_bwd), ("sorted_idx", order), ("sorted_idx_bwd", order_bwd)):
         assert torch.equal(cache[name], ref), name
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("n,co,dtype", [(148 * 256 + 1, 32, "float16"), (150 * 256, 64, "bfloat16"), (163 * 128 + 37, 264, "float32"), (222 * 256 - 5, 16, "float16")])
+def test_halved_items_at_the_end_of_a_launch(n, co, dtype):
+    """Launches whose last work items go out as halves: bit for bit the rows of the same convolution with the number of
+    SMs capped so that no item is halved."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops.spconv import sparse_submanifold_conv3d
+    T = getattr(torch, dtype)
+    g = torch.Generator().manual_seed(n)
+    flat = torch.randperm(96 ** 3, generator=g)[:n].sort().values
+    coords = torch.stack([flat * 0, flat // 96 ** 2, flat // 96 % 96, flat % 96], 1).int().to(DEV).contiguous()
+    shape = torch.Size((1, 32, 96, 96, 96))
+    feats = torch.randn(n, 32, generator=g).to(T).to(DEV).requires_grad_(True)
+    weight = (torch.randn(co, 3, 3, 3, 32, generator=g) / 12).to(T).to(DEV)
+    gout = torch.randn(n, co, generator=g).to(T).to(DEV)
+    out, cache = sparse_submanifold_conv3d(feats, coords, shape, weight)
+    (gf,) = torch.autograd.grad(out, feats, gout)
+    prev = K.set_conv_cta_limit(7)          # more than six waves: nothing is halved
+    try:
+        out1, _ = sparse_submanifold_conv3d(feats, coords, shape, weight, None, cache)
+        (gf1,) = torch.autograd.grad(out1, feats, gout)
+    finally:
+        K.set_conv_cta_limit(prev)
+    assert torch.equal(out, out1) and torch.equal(gf, gf1)
+    K.check_status(DEV)

@@ -67,6 +67,9 @@ struct WgradParams {
   int64_t bias_rows;
   float* bias_partial;    // [bias_ctas, Co]
   int bias_ctas;
+  char* direct;           // one unit per offset: the result [Co, V, Ci] itself, no slabs; null = slabs
+  int direct_add;         // add to what is there (fp32 only)
+  char* direct_bias;      // [Co]: the bias gradient of a launch without slabs, or null
   int32_t* status;
   int32_t* status_mirror;
 };
@@ -219,6 +222,44 @@ __device__ __forceinline__ void bias_share(const T* __restrict__ src, int64_t ro
   }
 }
 
+// Column sums without a second step, for launches that write their result directly: the CTA takes whole 16-byte columns
+// (column cta, cta + ctas, ...) over all rows.  Half of every 32-byte sector goes unused, which does not show: such
+// launches have few rows or many channels, and these threads wait for the accumulator anyway.
+template <typename T>
+__device__ __forceinline__ void bias_columns(const T* __restrict__ src, int64_t rows, int Co, T* __restrict__ out, int cta, int ctas,
+                                             float* s_acc /* [128 * 16 / sizeof(T)] */, int tid) {
+  constexpr int kVec = 16 / sizeof(T);
+  for (int cg = cta; cg < Co / kVec; cg += ctas) {
+    float acc[4][kVec];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) acc[u][i] = 0.f;
+    for (int64_t r = tid; r < rows; r += 4 * 128) {
+      uint4 w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        w[u] = r + u * 128 < rows ? __ldg(reinterpret_cast<const uint4*>(src + (r + u * 128) * Co) + cg) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const T* e = reinterpret_cast<const T*>(&w[u]);
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) acc[u][i] += static_cast<float>(e[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      float x = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+      if ((tid & 31) == 0) s_acc[(tid >> 5) * kVec + i] = x;
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (tid < kVec) out[cg * kVec + tid] = static_cast<T>((s_acc[tid] + s_acc[kVec + tid]) + (s_acc[2 * kVec + tid] + s_acc[3 * kVec + tid]));
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+  }
+}
+
 // kRows = pairs of a stage / 32 = pair rows per gather thread.  kBanded: the CTA walks its share of every row band (see
 // above); otherwise one contiguous run of k-blocks of its offset's list, without the per-band tables in the gather loop
 // (that loop's bookkeeping alone costs 2-3 % where bands bring nothing).
@@ -251,7 +292,23 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
   bid /= p.ci_tiles;
   const int co_group = bid % p.co_groups;
   bid /= p.co_groups;
-  if (warp == 0) {
+  if (warp == 0 && p.direct != nullptr) {
+    // one unit per offset, the longest lists first (they end last)
+    uint32_t nk = 0;
+    if (lane < p.V) nk = (__ldg(&p.seg[lane + 1]) - __ldg(&p.seg[lane]) + p.kb - 1) / p.kb;
+    uint32_t rank = 0;
+    for (int j = 0; j < p.V; ++j) {
+      const uint32_t o = __shfl_sync(0xffffffffu, nk, j);
+      if (o > nk || (o == nk && j < lane)) ++rank;
+    }
+    const unsigned mine = __ballot_sync(0xffffffffu, lane < p.V && rank == bid);
+    if (lane == 0) {
+      const int32_t skip = p.status != nullptr ? *reinterpret_cast<volatile const int32_t*>(p.status) : 0;
+      if (skip != 0 && blockIdx.x == 0) mirror_code(p.status_mirror, skip);
+      ctl->unit_v = skip != 0 || mine == 0u ? -1 : __ffs(mine) - 1;
+      ctl->unit_j = 0, ctl->unit_kb = 0x3FFFFFFF;
+    }
+  } else if (warp == 0) {
     const uint32_t ukb = wg_plan_unit_kb(p.seg, p.V, p.kb, static_cast<uint32_t>(p.target_units), lane);
     int v = -1, j = -1;
     if (lane == 0) {
@@ -296,9 +353,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
   }
   __syncthreads();
   const int v = ctl->unit_v, unit_j = ctl->unit_j, unit_kb = ctl->unit_kb;
-  const bool sums_bias = warp < 4 && p.bias_src != nullptr && blockIdx.x < static_cast<uint32_t>(p.bias_ctas);
+  auto sum_bias = [&]() {  // the threads of the epilogue warps
+    if (warp >= 4 || p.bias_src == nullptr || blockIdx.x >= static_cast<uint32_t>(p.bias_ctas)) return;
+    const T* src = reinterpret_cast<const T*>(p.bias_src);
+    if (p.direct_bias != nullptr) bias_columns<T>(src, p.bias_rows, p.Co, reinterpret_cast<T*>(p.direct_bias), blockIdx.x, p.bias_ctas, s_bias, tid);
+    else bias_share<T>(src, p.bias_rows, p.Co, p.bias_partial, blockIdx.x, p.bias_ctas, s_bias, tid);
+  };
   if (v < 0) {  // grid is sized for the worst case; also the no-op path after a soft error
-    if (sums_bias) bias_share<T>(reinterpret_cast<const T*>(p.bias_src), p.bias_rows, p.Co, p.bias_partial, blockIdx.x, p.bias_ctas, s_bias, tid);
+    sum_bias();
     return;
   }
   const int co0 = co_group * p.mt * 128;
@@ -442,8 +504,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     // and nothing is in flight), 16-byte pieces XOR-swizzled by the row, and come back so that eight consecutive
     // lanes hold one row's 128 contiguous bytes: every store instruction then writes four whole lines of the slab
     // instead of one 16-byte piece in each of 32 lines.
-    if (sums_bias) bias_share<T>(reinterpret_cast<const T*>(p.bias_src), p.bias_rows, p.Co, p.bias_partial, blockIdx.x, p.bias_ctas, s_bias, tid);
-    const uint32_t slab = wg_slab_of(p.seg, p.kb, unit_kb, v, unit_j);
+    sum_bias();
+    const uint32_t slab = p.direct != nullptr ? 0u : wg_slab_of(p.seg, p.kb, unit_kb, v, unit_j);
     mbar_wait(&ctl->acc_full, 0, abort_flag);
     tc_fence_after_sync();
     uint8_t* stage_out = stages + warp * 4096;
@@ -469,7 +531,25 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
           const int row = i * 4 + (lane >> 3), piece = lane & 7;
           const int ci = ci0 + c0 + piece * 4;
           const uint4 val = *reinterpret_cast<const uint4*>(stage_out + row * 128 + ((piece ^ (row & 7)) << 4));
-          if (co_base + row < p.Co && ci < p.Ci) *reinterpret_cast<uint4*>(obase + size_t(row) * p.Ci + ci) = val;
+          if (co_base + row < p.Co && ci < p.Ci) {
+            if (p.direct == nullptr) {
+              *reinterpret_cast<uint4*>(obase + size_t(row) * p.Ci + ci) = val;
+            } else {
+              float f[4] = {__uint_as_float(val.x), __uint_as_float(val.y), __uint_as_float(val.z), __uint_as_float(val.w)};
+              T* o = reinterpret_cast<T*>(p.direct) + (size_t(co_base + row) * p.V + v) * p.Ci + ci;
+              if constexpr (kTF32) {
+                float4 r = make_float4(f[0], f[1], f[2], f[3]);
+                if (p.direct_add) {
+                  const float4 b = *reinterpret_cast<const float4*>(o);
+                  r.x += b.x, r.y += b.y, r.z += b.z, r.w += b.w;
+                }
+                *reinterpret_cast<float4*>(o) = r;
+              } else {
+                T t4[4] = {static_cast<T>(f[0]), static_cast<T>(f[1]), static_cast<T>(f[2]), static_cast<T>(f[3])};
+                *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(t4);
+              }
+            }
+          }
         }
         __syncwarp();
       }
@@ -533,11 +613,11 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
   __syncthreads();
   const int unit_kb = s_unit_kb;
   const int v = blockIdx.y;
-  const int64_t e = (blockIdx.x * int64_t(256) + threadIdx.x) * 4;  // element of the [Co, Ci] slab
   const uint32_t first = wg_slab_of(seg, kb, unit_kb, v, 0);
   const uint32_t count = wg_chunks_of(seg, v, kb, unit_kb);
   chain_wait();  // the slabs are complete
-  if (e >= int64_t(Co) * Ci) return;
+  // a CTA walks over the [Co, Ci] elements: its plan (some microseconds) is made once, not once per 1024 of them
+  for (int64_t e = (blockIdx.x * int64_t(256) + threadIdx.x) * 4; e < int64_t(Co) * Ci; e += int64_t(gridDim.x) * 1024) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* src = partial + size_t(first) * Co * Ci + e;
   const size_t slab = size_t(Co) * Ci;
@@ -571,6 +651,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
       T t4[4] = {static_cast<T>(acc.x), static_cast<T>(acc.y), static_cast<T>(acc.z), static_cast<T>(acc.w)};
       *reinterpret_cast<uint2*>(out + o) = *reinterpret_cast<uint2*>(t4);
     }
+  }
   }
 }
 
@@ -814,6 +895,24 @@ struct BiasJob {
 };
 constexpr int kBiasCtas = 148;  // the CTAs of a launch's first wave share the rows
 
+// Whether a launch gives every offset one unit and writes the result itself, without slabs and the sum over them.  Costs
+// in microseconds from measured rates: a 64 KB stage 0.75, slab bytes written and read again at 4 TB/s, 5 for the second
+// launch.  Slabs win where one list would be walked by one CTA per tile while the device idles (few channels, many rows);
+// the direct way where there are enough tiles of channels (C = 1024: 54 slabs of 4 MB each; RES=32, fp16: 129 + 64 us)
+// or hardly any rows.  The longest list, the centre offset's, has at most n_out pairs.
+static bool wgrad_direct(const WgradPlan& w, int64_t n_out, int64_t n_pairs, int Ci, int Co, int V, int splitk) {
+  const int P = device_sm_count();
+  const int64_t tiles = int64_t(w.co_groups) * w.ci_tiles;
+  const double stage_us = 0.75 * (w.a_chunks + w.b_chunks) * w.kb * 128 / 65536.0;
+  const double stages = double(ceil_div(n_pairs, w.kb)) + V / 2.0;
+  const double longest = double(std::min(ceil_div(n_out, w.kb), ceil_div(n_pairs, w.kb)));
+  const double even = stages * tiles / P;
+  const double units = std::min<double>(target_units(w, V, splitk), stages);
+  const double waves = std::max(1.0, double(ceil_div(int64_t(units) * tiles, P)));
+  const double split = std::max(even, waves) * stage_us + 2e-6 * units * Ci * Co * 4 / 4.0 + 5.0;
+  return std::max(longest, even + longest / 4) * stage_us < split;
+}
+
 // one wgrad pass over operands of element type `dtype` (never FGB_F32_IEEE): partial slabs, then the ordered sum
 static int wgrad_pass(const void* grad_out, const void* feats, const uint32_t* vs_i, const uint32_t* vs_o, const uint32_t* seg,
                       const uint32_t* block_offsets, void* grad_weight, float* grad_weight_f32, int64_t n_out, int64_t n_in,
@@ -842,8 +941,13 @@ static int wgrad_pass(const void* grad_out, const void* feats, const uint32_t* v
   p.order = 0;  // offset-major: measured faster than chunk-major on B200 (chunk-major makes every SM stream the same rows at once)
   p.status = status;
   p.status_mirror = status_mirror(status);
-  const int64_t grid = max_units * w.co_groups * w.ci_tiles;
+  const bool direct = grad_weight != nullptr && grad_weight_f32 == nullptr && wgrad_direct(w, n_out, n_pairs, Ci, Co, V, splitk);
+  const int64_t grid = (direct ? int64_t(V) : max_units) * w.co_groups * w.ci_tiles;
   if (grid > 0x7FFFFFFF) return FGB_E_SIZE;
+  p.direct = direct ? static_cast<char*>(grad_weight) : nullptr;
+  p.direct_add = accumulate;
+  p.direct_bias = direct ? static_cast<char*>(bias.out) : nullptr;
+  if (direct) p.bands = 1;
   p.bias_src = static_cast<const char*>(bias.src);
   p.bias_rows = bias.rows;
   p.bias_partial = bias.partial;
@@ -852,7 +956,9 @@ static int wgrad_pass(const void* grad_out, const void* feats, const uint32_t* v
            : dtype == FGB_BF16 ? launch_wgrad<FGB_BF16>(grid, w.smem, p, s)
                                : launch_wgrad<FGB_F32_TF32>(grid, w.smem, p, s);
   if (rc != FGB_OK) return rc;
-  const dim3 rgrid(static_cast<unsigned>(ceil_div(int64_t(Co) * Ci, 1024)), static_cast<unsigned>(V + (bias.src != nullptr ? 1 : 0)));
+  if (direct) return FGB_OK;
+  const int64_t per_offset = std::max<int64_t>(1, int64_t(device_sm_count()) * 16 / V);
+  const dim3 rgrid(static_cast<unsigned>(std::min(ceil_div(int64_t(Co) * Ci, 1024), per_offset)), static_cast<unsigned>(V + (bias.src != nullptr ? 1 : 0)));
   const float* slabs_in = slabs;
   const float* bias_in = bias.partial;
   switch (dtype) {

@@ -184,3 +184,29 @@ def test_halved_items_at_the_end_of_a_launch(n, co, dtype):
         K.set_conv_cta_limit(prev)
     assert torch.equal(out, out1) and torch.equal(gf, gf1)
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("res,ci,co,dtype,tf32", [(8, 40, 40, "float16", True), (8, 1024, 264, "bfloat16", True), (16, 512, 1024, "float16", True),
+                                                  (8, 136, 300, "float32", True), (8, 260, 132, "float32", False), (2, 16, 16, "float16", True)])
+def test_weight_gradient_without_slabs(res, ci, co, dtype, tf32):
+    """Small inputs and wide channels: every offset is one unit that writes its result directly.  Against the slab path
+    (which the call with an fp32 copy takes): the same products, summed in fp32 in another grouping."""
+    from flexgemm_b200.kernels import config
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = orc.make_problem(res, ci, co, dtype, seed=res + co)
+    config.allow_tf32 = tf32
+    try:
+        f, w, b = (t.to(DEV).requires_grad_(True) for t in (feats, weight, bias))
+        gout = torch.randn(coords.shape[0], co, generator=torch.Generator().manual_seed(2)).to(f.dtype).to(DEV)
+        out, cache = spconv.sparse_submanifold_conv3d(f, coords.to(DEV), torch.Size(shape), w, b)
+        gw, gb = torch.autograd.grad(out, (w, b), gout)
+        _, gw32 = K.conv_wgrad(gout, f.detach(), cache["valid_signal_i"], cache["valid_signal_o"], cache["valid_signal_seg"], want_f32=True)
+        gb32 = K.bias_grad(gout, want_f32=True)[1]
+    finally:
+        config.allow_tf32 = True
+    ulp = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -24}[dtype]
+    for got, want, terms in ((gw.view(co, 27, ci), gw32, 27 + len(coords)), (gb, gb32, len(coords))):
+        err = (got.double() - want.double()).abs()
+        assert torch.all(err <= want.double().abs() * ulp + want.double().abs().max() * terms * 2.0 ** -24 + 1e-7)
+    K.check_status(DEV)

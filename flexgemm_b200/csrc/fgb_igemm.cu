@@ -76,7 +76,8 @@ struct IgemmParams {
   int kc;                    // reduction channels per offset
   int nout;                  // output channels
   int V;
-  int bn;                    // output channels per work item (32, 64, 128, 256)
+  int bn;                    // output channels per work item (a multiple of 32 up to 256)
+  int b_bytes;               // weight bytes of a stage
   int n_tiles_n;
   int splits;                // split-K: shares of a block's offsets that run as separate work items (1 = off)
   int items_per_block;       // n_tiles_n * splits; tail mode: n_tiles_n * 3 (upper half, lower half, whole block)
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   IgemmSmem* ctl = reinterpret_cast<IgemmSmem*>(smem);
   uint8_t* stages = smem + kCtrlBytes;
-  const int stage_bytes = 2 * kATileBytes + p.bn * 128;  // A half 0 | A half 1 | B
+  const int stage_bytes = 2 * kATileBytes + p.b_bytes;  // A half 0 | A half 1 | B
   const int S = p.stages;
 
   // Launched chained (fgb_device.cuh): the CTA may be on its SM before the kernel ahead in the stream has finished.
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     };
     // ring position of the next stage and its phase bit, advanced by hand: a division by the runtime stage count
     // in this loop costs several XU-pipe instructions per stage and starves the epilogue's conversions
+    const int k_bytes = (p.row_bytes + 31) & ~31;  // an MMA takes 32 bytes of a row
     uint32_t s = 0, ph = 0;
     uint32_t rows[8], nrows[8], idx[8], nidx[8];
     uint32_t m0 = 0, m1 = 0, nm0 = 0, nm1 = 0;
@@ -415,9 +417,10 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
           mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag);
           const uint32_t a_base = smem_u32(stages + size_t(s) * stage_bytes);
           const bool col_ok = kb * 128 + piece * 16 < p.row_bytes;
+          const bool read = kb * 128 + piece * 16 < k_bytes;  // pieces that no MMA reads are left alone
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            if (j < 4 ? need0 : need1) {
+            if (read && (j < 4 ? need0 : need1)) {
               const bool ok = col_ok && idx[j] != kInvalid;
               cp_async_16(a_base + dst_off[j], src[j] + kb * 128, ok ? 16u : 0u);
             }
@@ -451,12 +454,12 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
           const int wv = (p.flip & 1) ? V - 1 - v : v;
           for (int kb = 0; kb < p.num_kb; ++kb) {
             mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag);
-            mbar_arrive_expect_tx(&ctl->full[s], static_cast<uint32_t>(p.bn) * 128u);
+            mbar_arrive_expect_tx(&ctl->full[s], static_cast<uint32_t>(p.b_bytes));
             const uint32_t b_dst = smem_u32(stages + size_t(s) * stage_bytes + 2 * kATileBytes);
             if (p.flip & 2) {
               // MN-major weights (dgrad of 16-bit types reads the weight as stored, [Co][V][Ci]): rows of the stage are
               // reduction channels, 128 bytes = 64 output channels per row, one 8 KB chunk per 64 output channels
-              for (int c = 0; c < p.bn / 64; ++c) tma_load_3d(b_dst + c * 8192, &tmap_w, &ctl->full[s], n0 + c * 64, wv, kb * 64);
+              for (int c = 0; c * 64 < p.bn; ++c) tma_load_3d(b_dst + c * 8192, &tmap_w, &ctl->full[s], n0 + c * 64, wv, kb * 64);
             } else {
               tma_load_3d(b_dst, &tmap_w, &ctl->full[s], kb * (128 / kElem), wv, n0);
             }
@@ -797,10 +800,13 @@ int make_rows_tmap(CUtensorMap* map, const void* rows, int64_t n_rows, int row_e
   });
 }
 
+// Output channels per work item: all of them in steps of 32 up to 256, else as many equal column tiles as 256-wide ones
+// would make, in steps of 64 (the epilogue writes 64 columns of a 16-bit type at a time).  The width sets the weight
+// bytes and the MMA time of a stage: powers of two ran C = 136 like 256 and C = 312 like 512.
 static int pick_bn(int nout) {
-  int bn = 32;
-  while (bn < nout && bn < 256) bn <<= 1;
-  return bn;
+  if (nout <= 256) return (nout + 31) / 32 * 32;
+  const int tiles = (nout + 255) / 256;
+  return ((nout + tiles - 1) / tiles + 63) / 64 * 64;
 }
 
 // Upper bound on the CTAs (= SMs) of the persistent conv kernels; 0 = all.  A caller that has a collective running
@@ -815,7 +821,7 @@ static int persistent_ctas() {
 
 template <int kDtype, int kMode>
 static int launch_igemm_variant(const CUtensorMap& tmap, const IgemmParams& p, const FusedEpilogue& fe, cudaStream_t s) {
-  const size_t smem = 1024 + kCtrlBytes + size_t(p.stages) * (2 * kATileBytes + p.bn * 128) + kStoreStageBytes;
+  const size_t smem = 1024 + kCtrlBytes + size_t(p.stages) * (2 * kATileBytes + p.b_bytes) + kStoreStageBytes;
   static PerDeviceTable configured;  // the attribute belongs to (kernel instance, device)
   const int rc = ensure_dynamic_smem(configured, subm_igemm_kernel<kDtype, kMode>, smem);
   if (rc != FGB_OK) return rc;
@@ -954,7 +960,8 @@ int run_igemm(const void* x, const void* w, const void* bias, const uint32_t* nb
   p.flip = flip;
   p.num_tiles = static_cast<uint32_t>(ceil_div(n, kTileM));
   p.num_blocks = static_cast<uint32_t>(ceil_div(n, kBlockM));
-  const int stage_bytes = 2 * kATileBytes + p.bn * 128;
+  p.b_bytes = (flip & 2) ? (p.bn + 63) / 64 * 8192 : p.bn * 128;  // MN-major: whole chunks of 64 output channels
+  const int stage_bytes = 2 * kATileBytes + p.b_bytes;
   p.stages = (kSmemBudget - 1024 - kCtrlBytes - kStoreStageBytes) / stage_bytes;
   if (p.stages > kMaxStages) p.stages = kMaxStages;
   p.acc_sets = 2 * p.bn * 2 <= 512 ? 2 : 1;
@@ -1106,10 +1113,10 @@ extern "C" int fgb_subm_conv_fprop_fused(const void* feats, const void* weight, 
 namespace fgb {
 
 // 16-bit types read the weight as it is stored, [Co][V][Ci], as an MN-major operand (rows = reduction channels): no
-// re-layout pass.  Column tiles narrower than one 64-channel chunk, and the 32-bit types (whose MN-major layout TMA
+// re-layout pass.  Column tiles narrower than a 64-channel chunk, and the 32-bit types (whose MN-major layout TMA
 // does not produce), go through the re-laid-out copy.
 static bool dgrad_as_stored(int Ci, int eb) {
-  return eb == 2 && !g_dgrad_relayout.load(std::memory_order_relaxed) && pick_bn(Ci) % 64 == 0;
+  return eb == 2 && !g_dgrad_relayout.load(std::memory_order_relaxed) && pick_bn(Ci) >= 64;
 }
 
 // n rows of the map / of `grad_feats`; n_src rows of `grad_out`; mirror = the map is the forward map of a submanifold

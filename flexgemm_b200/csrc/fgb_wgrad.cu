@@ -58,7 +58,7 @@ struct WgradParams {
   int ci_tiles;   // ceil(Ci / bn)
   int kb;         // pairs per stage
   int stages;
-  int a_chunks;   // 128-byte column chunks of the A stage (mt * 128 * elem / 128)
+  int a_chunks;   // 128-byte column chunks of the A stage: those that hold channels
   int b_chunks;
   uint32_t idesc;
   uint32_t tmem_cols;
@@ -365,6 +365,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
   }
   const int co0 = co_group * p.mt * 128;
   const int ci0 = ci_tile * p.bn;
+  // 128-row accumulator blocks and 128-byte chunks of this CTA that hold channels; the rest of an accumulator is computed
+  // from whatever lies behind (rows and columns that nobody reads)
+  const int mt = min(p.mt, (p.Co - co0 + 127) / 128);
+  const int a_used = min(p.a_chunks, ((p.Co - co0) * kElem + 127) / 128), b_used = min(p.b_chunks, ((p.Ci - ci0) * kElem + 127) / 128);
   // contiguous walk: k-blocks [k_begin, k_begin + total) of the offset's list, full units and a shorter last one
   const uint32_t seg_begin = __ldg(&p.seg[v]);
   const uint32_t seg_end = __ldg(&p.seg[v + 1]);
@@ -453,13 +457,13 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
       }
       mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag);
       const uint32_t st_base = smem_u32(stages + size_t(s) * stage_bytes);
-      for (int c = 0; c < p.a_chunks; ++c) {
+      for (int c = 0; c < a_used; ++c) {
         const bool col_ok = co0 * kElem + c * 128 + piece * 16 < a_row_bytes;
 #pragma unroll
         for (int j = 0; j < kRows; ++j)
           cp_async_16(st_base + c * chunk_bytes + row_off[j], srca[j] + c * 128, (col_ok && io[j] != kInvalid) ? 16u : 0u);
       }
-      for (int c = 0; c < p.b_chunks; ++c) {
+      for (int c = 0; c < b_used; ++c) {
         const bool col_ok = ci0 * kElem + c * 128 + piece * 16 < b_row_bytes;
 #pragma unroll
         for (int j = 0; j < kRows; ++j)
@@ -485,9 +489,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
         for (int ks = 0; ks < p.kb / kUmmaK; ++ks) {
           const uint32_t koff = ks * kUmmaK * 128;  // kUmmaK pair rows of 128 bytes
           const uint64_t db = make_smem_desc(b_addr + koff, chunk_bytes, kSbo, kLayout);
-          for (int mt = 0; mt < p.mt; ++mt) {
-            const uint64_t da = make_smem_desc(a_addr + mt * chunks_per_m * chunk_bytes + koff, chunk_bytes, kSbo, kLayout);
-            umma_ss<kTF32>(tmem_base + mt * p.bn, da, db, p.idesc, accumulate);
+          for (int m = 0; m < mt; ++m) {
+            const uint64_t da = make_smem_desc(a_addr + m * chunks_per_m * chunk_bytes + koff, chunk_bytes, kSbo, kLayout);
+            umma_ss<kTF32>(tmem_base + m * p.bn, da, db, p.idesc, accumulate);
           }
           accumulate = 1;
         }
@@ -509,13 +513,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     mbar_wait(&ctl->acc_full, 0, abort_flag);
     tc_fence_after_sync();
     uint8_t* stage_out = stages + warp * 4096;
-    for (int mt = 0; mt < p.mt; ++mt) {
-      const int co_base = co0 + mt * 128 + warp * 32;
+    for (int m = 0; m < mt; ++m) {
+      const int co_base = co0 + m * 128 + warp * 32;
+      if (co_base >= p.Co) continue;  // whole warps
       float* obase = p.partial + (size_t(slab) * p.Co + co_base) * p.Ci;
       for (int c0 = 0; c0 < p.bn; c0 += 32) {
         uint32_t acc[32];
         if (total > 0) {
-          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + mt * p.bn + c0, acc);
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + m * p.bn + c0, acc);
           tmem_ld_wait();
         } else {
 #pragma unroll
@@ -722,10 +727,11 @@ __global__ void __launch_bounds__(256) bias_final_kernel(const float* __restrict
   }
 }
 
+// input channels per CTA: all of them in steps of 32 up to 256, else equal tiles in steps of 64
 static int pick_bn(int c) {
-  int bn = 32;
-  while (bn < c && bn < 256) bn <<= 1;
-  return bn;
+  if (c <= 256) return (c + 31) / 32 * 32;
+  const int tiles = (c + 255) / 256;
+  return ((c + tiles - 1) / tiles + 63) / 64 * 64;
 }
 
 struct WgradPlan {
@@ -737,24 +743,29 @@ struct WgradPlan {
 static WgradPlan plan_wgrad(int Ci, int Co, int eb) {
   WgradPlan w;
   w.bn = pick_bn(Ci);
-  w.mt = (Co > 128 && w.bn * 2 <= 512) ? 2 : 1;
+  w.mt = Co > 128 ? 2 : 1;
   w.co_groups = static_cast<int>(ceil_div(Co, w.mt * 128));
   w.ci_tiles = static_cast<int>(ceil_div(Ci, w.bn));
-  w.a_chunks = w.mt * 128 * eb / 128;
+  // chunks that hold channels; an MMA reads 128 accumulator rows' worth whatever of it is used
+  const int a_full = w.mt * 128 * eb / 128;
+  w.a_chunks = std::min<int>(a_full, static_cast<int>(ceil_div(int64_t(Co) * eb, 128)));
   w.b_chunks = static_cast<int>(ceil_div(w.bn * eb, 128));
   // pairs per stage: as many as keep a stage near 64 KB (more pairs per stage for narrow channel counts, so that the
   // fixed cost of a stage hand-over is spread over enough bytes); a multiple of 32 (one row per gather lane group)
   w.kb = 32;
   while (w.kb < 32 * kWgRowsMax && size_t(w.a_chunks + w.b_chunks) * (w.kb * 2) * 128 <= 64 * 1024) w.kb *= 2;
   const size_t stage = size_t(w.a_chunks + w.b_chunks) * w.kb * 128;
-  const size_t budget = 224 * 1024;
+  // what an MMA may read behind the last stage's operand A when that holds fewer chunks than 128 rows take
+  const size_t behind = size_t(std::max(0, a_full - w.a_chunks - w.b_chunks)) * w.kb * 128;
+  const size_t budget = 220 * 1024 - behind;
   w.stages = static_cast<int>(budget / stage);
   if (w.stages > kWgMaxStages) w.stages = kWgMaxStages;
   if (w.stages < 2) w.stages = 2;
   uint32_t cols = 32;
   while (cols < uint32_t(w.mt * w.bn)) cols <<= 1;
   w.tmem_cols = cols;
-  w.smem = 1024 + 1024 + stage * w.stages;
+  w.smem = 1024 + 1024 + stage * w.stages + behind;
+  if (w.smem < 1024 + 1024 + 4 * 4096) w.smem = 1024 + 1024 + 4 * 4096;  // the epilogue's staging buffers lie over the stages
   return w;
 }
 

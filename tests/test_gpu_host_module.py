@@ -210,3 +210,31 @@ def test_weight_gradient_without_slabs(res, ci, co, dtype, tf32):
         err = (got.double() - want.double()).abs()
         assert torch.all(err <= want.double().abs() * ulp + want.double().abs().max() * terms * 2.0 ** -24 + 1e-7)
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+@pytest.mark.parametrize("ci,co", [(8, 8), (16, 40), (40, 72), (72, 136), (96, 96), (136, 200), (200, 320), (264, 312), (520, 16)])
+def test_channel_tiles_of_any_width(ci, co, dtype):
+    """Column tiles, accumulator blocks and chunks at widths off the powers of two, forward and backward, against the
+    oracle; RES=20 has enough rows for two blocks and takes every slice of the reduction."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = orc.make_problem(20, ci, co, dtype, seed=ci + co)
+    gout = torch.randn(coords.shape[0], co, generator=torch.Generator().manual_seed(2)).to(feats.dtype)
+    nbr = orc.neighbor_map(coords.numpy(), shape)
+    want = (orc.conv_forward(feats.double(), nbr, weight.double(), bias.double()),
+            *orc.conv_backward(gout.double(), feats.double(), nbr, weight.double()))
+    for splits in (0, 1):
+        prev = K.set_conv_splitk(splits)
+        try:
+            f, w, b = (t.to(DEV).requires_grad_(True) for t in (feats, weight, bias))
+            out, cache = spconv.sparse_submanifold_conv3d(f, coords.to(DEV), torch.Size(shape), w, b)
+            got = (out, *torch.autograd.grad(out, (f, w, b), gout.to(DEV)))
+            # the weight gradient through slabs as well
+            gw, _ = K.conv_wgrad(gout.to(DEV), f.detach(), cache["valid_signal_i"], cache["valid_signal_o"], cache["valid_signal_seg"], splitk=3,
+                                 want_f32=True)
+        finally:
+            K.set_conv_splitk(prev)
+        for x, y in zip((*got, gw.view(want[2].shape)), (*want, want[2])):
+            assert (x.detach().cpu().double() - y).abs().max() <= 1e-2 * y.abs().max()
+    K.check_status(DEV)

@@ -371,8 +371,10 @@ __global__ void __launch_bounds__(256) group_fill_kernel(const uint32_t* __restr
     grouped[atomicAdd(&start[row], 1u)] = make_uint2(static_cast<uint32_t>(e / V), __float_as_uint(w));
   }
 }
-// kWarps warps of a CTA share one voxel (1, or 8 where voxels have many entries); kGroup lanes cover a row, so 32 / kGroup
-// entries are read side by side.
+// kGroup lanes cover a voxel's row (or 32 packs of it at a time).  kWarps = 0: every group has a voxel of its own, 32 /
+// kGroup of them per warp -- with narrow rows and few entries per voxel a warp per voxel spends its life on three
+// dependent loads (RES=467, C=16, 2.4 entries per voxel: most of 275 us).  kWarps = 1: a warp per voxel, its groups take
+// the entries in turn.  kWarps = 8: the warps of a CTA share a voxel, where voxels have many entries.
 template <typename T, int kVec, int kWarps, int kGroup>
 __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ grad_out, const uint2* __restrict__ grouped,
                                                         const uint32_t* __restrict__ end, const uint32_t* __restrict__ count, uint32_t n, int C,
@@ -383,12 +385,39 @@ __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ gr
   chain_release();
   chain_wait();
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int nv = C / kVec;
+  const int side = lane / kGroup;
+  if constexpr (kWarps == 0) {
+    const uint32_t row = (blockIdx.x * 8u + wi) * kSide + side;
+    if (row >= n) return;
+    const uint32_t len = __ldg(&count[row]);
+    const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
+    for (int c = lane % kGroup; c < nv; c += kGroup) {
+      float acc[kVec];
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) acc[i] = 0.f;
+      uint32_t j = 0;
+      for (; j + 4 <= len; j += 4) {
+        uint2 e[4];
+        Raw raw[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u] = __ldg(&list[j + u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) raw[u] = __ldg(reinterpret_cast<const Raw*>(grad_out + size_t(e[u].x) * C) + c);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) fma_pack<T, kVec>(acc, raw[u], __uint_as_float(e[u].y));
+      }
+      for (; j < len; ++j) {
+        const uint2 e = __ldg(&list[j]);
+        fma_pack<T, kVec>(acc, __ldg(reinterpret_cast<const Raw*>(grad_out + size_t(e.x) * C) + c), __uint_as_float(e.y));
+      }
+      reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
+    }
+  } else {
   const uint32_t row = kWarps > 1 ? blockIdx.x : blockIdx.x * 8u + wi;
   if (row >= n) return;  // whole warps; with kWarps > 1 whole CTAs
   const uint32_t len = __ldg(&count[row]);
   const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
-  const int nv = C / kVec;
-  const int side = lane / kGroup;
   const int share = kWarps > 1 ? wi : 0;
   for (int c0 = 0; c0 < nv; c0 += kGroup) {
     const int c = c0 + lane % kGroup;
@@ -426,6 +455,7 @@ __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ gr
     }
     if ((kWarps == 1 || wi == 0) && side == 0 && c < nv) reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
   }
+  }
 }
 
 // lanes for a row of nv packs: the next power of two, 8 .. 32
@@ -454,17 +484,25 @@ static cudaError_t launch_sample(int key_bits, bool nearest, const void* feats, 
 }
 
 template <typename T, int kVec>
-static cudaError_t launch_group_sum(bool shared_rows, const void* grad_out, const uint2* grouped, const uint32_t* start, const uint32_t* count,
+static cudaError_t launch_group_sum(uint32_t entries, const void* grad_out, const uint2* grouped, const uint32_t* start, const uint32_t* count,
                                     uint32_t n, int C, void* grad_feats, cudaStream_t s) {
-  const int lanes = group_lanes(C / kVec);
-  auto kernel = shared_rows ? (lanes == 8    ? group_sum_kernel<T, kVec, 8, 8>
-                               : lanes == 16 ? group_sum_kernel<T, kVec, 8, 16>
-                                             : group_sum_kernel<T, kVec, 8, 32>)
-                            : (lanes == 8    ? group_sum_kernel<T, kVec, 1, 8>
-                               : lanes == 16 ? group_sum_kernel<T, kVec, 1, 16>
-                                             : group_sum_kernel<T, kVec, 1, 32>);
-  return launch_chained(kernel, dim3(shared_rows ? n : static_cast<unsigned>(ceil_div(n, 8))), dim3(256), 0, s, static_cast<const T*>(grad_out),
-                        grouped, start, count, n, C, static_cast<T*>(grad_feats));
+  const int nv = C / kVec;
+  const uint32_t mean = entries / n;  // places of entries, of which a part is used
+  void (*kernel)(const T*, const uint2*, const uint32_t*, const uint32_t*, uint32_t, int, T*);
+  unsigned grid = static_cast<unsigned>(ceil_div(n, 8));
+  if (mean >= 128) {  // few warps would walk long lists otherwise
+    kernel = nv <= 8 ? group_sum_kernel<T, kVec, 8, 8> : nv <= 16 ? group_sum_kernel<T, kVec, 8, 16> : group_sum_kernel<T, kVec, 8, 32>;
+    grid = n;
+  } else if (nv <= 16 && mean < 32) {
+    const int lanes = nv <= 2 ? 2 : nv <= 4 ? 4 : nv <= 8 ? 8 : 16;
+    kernel = lanes == 2 ? group_sum_kernel<T, kVec, 0, 2> : lanes == 4 ? group_sum_kernel<T, kVec, 0, 4>
+             : lanes == 8 ? group_sum_kernel<T, kVec, 0, 8> : group_sum_kernel<T, kVec, 0, 16>;
+    grid = static_cast<unsigned>(ceil_div(n, 8 * (32 / lanes)));
+  } else {
+    kernel = nv <= 8 ? group_sum_kernel<T, kVec, 1, 8> : nv <= 16 ? group_sum_kernel<T, kVec, 1, 16> : group_sum_kernel<T, kVec, 1, 32>;
+  }
+  return launch_chained(kernel, dim3(grid), dim3(256), 0, s, static_cast<const T*>(grad_out), grouped, start, count, n, C,
+                        static_cast<T*>(grad_feats));
 }
 
 struct GroupScratch {
@@ -685,15 +723,13 @@ extern "C" int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t
                              start, total));
     chain.add(launch_chained(group_fill_kernel, egrid, dim3(256), 0, s, indices, weight, entries, V, start, grouped));
   }
-  // many entries per voxel: the warps of a CTA share a voxel, else few warps would walk long lists
-  const bool shared_rows = entries / n >= 128u;
   if (dtype == FGB_F16)
-    chain.add(C % 8 == 0 ? launch_group_sum<__half, 8>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s)
-                         : launch_group_sum<__half, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(C % 8 == 0 ? launch_group_sum<__half, 8>(entries, grad_out, grouped, start, count, n, C, grad_feats, s)
+                         : launch_group_sum<__half, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
   else if (dtype == FGB_BF16)
-    chain.add(C % 8 == 0 ? launch_group_sum<__nv_bfloat16, 8>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s)
-                         : launch_group_sum<__nv_bfloat16, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(C % 8 == 0 ? launch_group_sum<__nv_bfloat16, 8>(entries, grad_out, grouped, start, count, n, C, grad_feats, s)
+                         : launch_group_sum<__nv_bfloat16, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
   else
-    chain.add(launch_group_sum<float, 4>(shared_rows, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(launch_group_sum<float, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
   return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
 }

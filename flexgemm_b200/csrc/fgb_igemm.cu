@@ -42,6 +42,7 @@
 #include "fgb_common.cuh"
 #include "fgb_device.cuh"
 #include "fgb_precision.cuh"
+#include "fgb_map.cuh"
 #include "fgb_sort.cuh"
 #include "fgb_umma.cuh"
 
@@ -619,45 +620,6 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
 // cost of a block being the number of (tile, offset) products it runs.  One CTA;
 // a counting sort over the 65 possible costs.  Blocks of equal cost may come out
 // in any order: the order only decides which SM computes a block, never a result.
-// Costs of a block of two tiles lie in 0 .. 64.  Blocks of equal cost mostly stand together (the rows are sorted by
-// mask), so a warp takes its places by one atomic per distinct cost, not per block.
-struct ScheduleSmem {
-  uint32_t count[65], start[65];
-};
-__device__ __forceinline__ void block_schedule(ScheduleSmem& sm, const uint32_t* masks, uint32_t num_tiles, uint32_t nb,
-                                               uint32_t* __restrict__ order) {
-  const int t = threadIdx.x, lane = t & 31;
-  if (t < 65) sm.count[t] = 0;
-  __syncthreads();
-  auto cost_of = [&](uint32_t b) {  // the masks may have been written by other CTAs of this launch: loads that bypass L1
-    const uint32_t t0 = 2 * b;
-    return __popc(__ldcg(&masks[t0])) + (t0 + 1 < num_tiles ? __popc(__ldcg(&masks[t0 + 1])) : 0);
-  };
-  auto take = [&](uint32_t* counters, uint32_t b) -> uint32_t {  // whole warps call it; a place for every lane with b < nb
-    const bool ok = b < nb;
-    const int c = ok ? cost_of(b) : 65;
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (ok && lane == leader) base = atomicAdd(&counters[c], static_cast<uint32_t>(__popc(peers)));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return base + static_cast<uint32_t>(__popc(peers & ((1u << lane) - 1u)));
-  };
-  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) take(sm.count, b0 + lane);
-  __syncthreads();
-  if (t == 0) {
-    uint32_t acc = 0;
-    for (int c = 64; c >= 0; --c) {
-      sm.start[c] = acc;
-      acc += sm.count[c];
-    }
-  }
-  __syncthreads();
-  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) {
-    const uint32_t pos = take(sm.start, b0 + lane);
-    if (b0 + lane < nb) order[pos] = b0 + lane;
-  }
-}
 __global__ void __launch_bounds__(1024) block_schedule_kernel(const uint32_t* __restrict__ masks, uint32_t num_tiles, uint32_t nb,
                                                               uint32_t* __restrict__ order) {
   __shared__ ScheduleSmem sm;

@@ -87,6 +87,69 @@ struct ScanFinish {
   uint32_t host_seq;
 };
 
+// The block schedule: row blocks (pairs of 128-row tiles) by descending cost, a block's cost being the number of (tile,
+// offset) products it runs.
+// Costs of a block of two tiles lie in 0 .. 64.  Blocks of equal cost mostly stand together (the rows are sorted by
+// mask), so a warp takes its places by one atomic per distinct cost, not per block.
+struct ScheduleSmem {
+  uint32_t count[65], start[65];
+};
+__device__ __forceinline__ void block_schedule(ScheduleSmem& sm, const uint32_t* masks, uint32_t num_tiles, uint32_t nb,
+                                               uint32_t* __restrict__ order) {
+  const int t = threadIdx.x, lane = t & 31;
+  if (t < 65) sm.count[t] = 0;
+  __syncthreads();
+  auto cost_of = [&](uint32_t b) {  // the masks may have been written by other CTAs of this launch: loads that bypass L1
+    const uint32_t t0 = 2 * b;
+    return __popc(__ldcg(&masks[t0])) + (t0 + 1 < num_tiles ? __popc(__ldcg(&masks[t0 + 1])) : 0);
+  };
+  auto take = [&](uint32_t* counters, uint32_t b) -> uint32_t {  // whole warps call it; a place for every lane with b < nb
+    const bool ok = b < nb;
+    const int c = ok ? cost_of(b) : 65;
+    const unsigned peers = __match_any_sync(0xffffffffu, c);
+    const int leader = __ffs(peers) - 1;
+    uint32_t base = 0;
+    if (ok && lane == leader) base = atomicAdd(&counters[c], static_cast<uint32_t>(__popc(peers)));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    return base + static_cast<uint32_t>(__popc(peers & ((1u << lane) - 1u)));
+  };
+  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) take(sm.count, b0 + lane);
+  __syncthreads();
+  if (t == 0) {
+    uint32_t acc = 0;
+    for (int c = 64; c >= 0; --c) {
+      sm.start[c] = acc;
+      acc += sm.count[c];
+    }
+  }
+  __syncthreads();
+  for (uint32_t b0 = t - lane; b0 < nb; b0 += blockDim.x) {
+    const uint32_t pos = take(sm.start, b0 + lane);
+    if (b0 + lane < nb) order[pos] = b0 + lane;
+  }
+}
 cudaError_t launch_block_scan(uint32_t* block_counts, uint32_t nblk, int V, uint32_t* seg, const ScanFinish& fin, cudaStream_t s);
+
+// ------------------------------------------------------------------ small inputs (fgb_small.cu)
+constexpr int64_t kSmallRows = 8192;  // up to here one CTA sorts and plans, and a map CTA keeps the whole hash table in shared memory
+
+// what one CTA derives from a map's codes
+struct PlanJob {
+  const int32_t* codes;   // [n] binary codes
+  const int32_t* gray;    // [n]
+  uint32_t n;
+  int V;
+  int64_t* sorted_idx;    // [n]
+  uint32_t* tile_masks;   // [ceil(n / 128)]
+  uint32_t* block_order;  // [ceil(n / 256)]
+  uint32_t* counts;       // [V, nblk] per-block counts to turn into offsets, or null
+  uint32_t* seg;          // with counts: the segment table [V + 1] (+ the words of `fin`)
+  ScanFinish fin;
+};
+// one or two jobs (a null second one is left out), a CTA each
+cudaError_t launch_small_plan(const PlanJob& a, const PlanJob* b, cudaStream_t s);
+// the submanifold map of n <= kSmallRows rows
+cudaError_t launch_small_map(const int32_t* coords, uint32_t n, int W, int H, int D, const int32_t* k, const int32_t* dil, int key_bits,
+                             const MapOut& o, cudaStream_t s);
 
 }  // namespace fgb

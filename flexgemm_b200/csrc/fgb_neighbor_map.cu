@@ -611,6 +611,17 @@ extern "C" int fgb_subm_cache_build(const fgb_map_call* c, void* stream) {
   const CacheScratch L = cache_scratch(c->n, c->b, c->w, c->h, V, c->slots, c->key_bits);
   if (c->scratch_bytes < static_cast<int64_t>(L.total)) return FGB_E_WORKSPACE;
   char* mem = static_cast<char*>(c->scratch);
+  if (c->n <= kSmallRows) {
+    int32_t* codes = reinterpret_cast<int32_t*>(mem + L.codes_off);
+    const MapOut o{c->neighbor_map, c->gray_code, codes, c->block_offsets, nullptr, static_cast<uint32_t>(ceil_div(c->n, kMapBlock))};
+    cudaError_t e = launch_small_map(c->coords, static_cast<uint32_t>(c->n), c->w, c->h, c->d, c->k, c->dil, c->key_bits, o, s);
+    if (e != cudaSuccess) return cuda_status(e);
+    PlanJob j{codes, c->gray_code, static_cast<uint32_t>(c->n), V, c->sorted_idx, c->tile_masks, c->block_order, c->block_offsets, c->meta, {}};
+    j.fin.build_status = reinterpret_cast<const int32_t*>(c->meta);  // not null: the words after the segment table are wanted
+    j.fin.host_words = c->host_words, j.fin.host_seq = c->host_seq;
+    e = launch_small_plan(j, nullptr, s);
+    return e != cudaSuccess ? cuda_status(e) : launch_status();
+  }
   uint32_t* words = reinterpret_cast<uint32_t*>(mem + L.words_off);
   uint32_t* hist = reinterpret_cast<uint32_t*>(mem + L.hist_off);
   cudaError_t e = cudaMemsetAsync(mem, 0, L.zero_bytes, s);

@@ -365,17 +365,26 @@ extern "C" int fgb_strided_build(const fgb_strided_call* c, void* stream) {
   uint32_t* hist_bwd = reinterpret_cast<uint32_t*>(mem + L.hist_bwd_off);
   int32_t* codes = reinterpret_cast<int32_t*>(mem + L.codes_off);
   int32_t* codes_bwd = reinterpret_cast<int32_t*>(mem + L.codes_bwd_off);
-  chain.add(cudaMemsetAsync(mem, 0, L.zero_bytes, s));
+  // few rows on both sides: no histograms or look-back words to clear, one launch for all that follows from the codes
+  const bool small = c->n <= kSmallRows && c->n_out <= kSmallRows;
+  if (!small) chain.add(cudaMemsetAsync(mem, 0, L.zero_bytes, s));
   chain.add(cudaMemsetAsync(c->neighbor_map, 0xFF, size_t(n_out) * V * 4, s));
   chain.add(launch_chained(emit_cells_kernel, dim3(m.ctas), dim3(kRankThreads), 0, s, bits,
                            reinterpret_cast<const uint32_t*>(gm + m.base_off), g, n_out, rank, reinterpret_cast<int4*>(c->out_coords)));
-  const MapOut ob{c->neighbor_map_bwd, c->gray_code_bwd, codes_bwd, nullptr, hist_bwd, 0};
+  const MapOut ob{c->neighbor_map_bwd, c->gray_code_bwd, codes_bwd, nullptr, small ? nullptr : hist_bwd, 0};
   chain.add(launch_chained(strided_maps_kernel, dim3(static_cast<unsigned>(ceil_div(c->n, kMapBlock))), dim3(kMapBlock), with_bwd ? codes_smem(V) : 0, s,
                            reinterpret_cast<const int4*>(c->coords), n, g, bits, static_cast<const uint32_t*>(rank), n_out, c->neighbor_map,
                            c->neighbor_map_bwd, ob));
   const uint32_t nblk = static_cast<uint32_t>(ceil_div(c->n_out, kMapBlock));
-  const MapOut of{c->neighbor_map, c->gray_code, codes, c->block_offsets, hist, nblk};
+  const MapOut of{c->neighbor_map, c->gray_code, codes, c->block_offsets, small ? nullptr : hist, nblk};
   chain.add(launch_chained(map_codes_kernel, dim3(nblk), dim3(kMapBlock), codes_smem(V), s, static_cast<const uint32_t*>(c->neighbor_map), n_out, V, of));
+  if (small) {
+    PlanJob jf{codes, c->gray_code, n_out, V, c->sorted_idx, c->tile_masks, c->block_order, c->block_offsets, c->meta, {}};
+    jf.fin.host_words = c->host_words, jf.fin.host_seq = c->host_seq;
+    const PlanJob jb{codes_bwd, c->gray_code_bwd, n, V, c->sorted_idx_bwd, c->tile_masks_bwd, c->block_order_bwd, nullptr, nullptr, {}};
+    if (chain.first == cudaSuccess) chain.add(launch_small_plan(jf, with_bwd ? &jb : nullptr, s));
+    return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
+  }
   ScanFinish fin{words, nullptr, nullptr, c->host_words, c->host_seq};
   chain.add(launch_block_scan(c->block_offsets, nblk, V, c->meta, fin, s));
   if (chain.first == cudaSuccess)

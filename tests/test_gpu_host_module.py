@@ -16,8 +16,8 @@ def u32(t):
 
 @pytest.mark.parametrize("n,ksize,shuffle,volume", [(1, (3, 3, 3), False, 64), (127, (3, 3, 3), False, 64), (128, (3, 3, 3), True, 64),
                                                     (257, (3, 1, 3), False, 64), (1025, (3, 3, 3), True, 64), (4097, (1, 1, 1), False, 64),
-                                                    (33000, (3, 3, 3), False, 64), (33000, (3, 3, 3), True, 2048),
-                                                    (3000, (1, 1, 31), False, 64)])
+                                                    (8192, (3, 3, 3), True, 64), (8193, (3, 3, 3), False, 64), (2049, (3, 1, 1), True, 2048), (33000, (3, 3, 3), False, 64), (33000, (3, 3, 3), True, 2048),
+                                                    (3000, (1, 1, 31), False, 64), (1, (1, 1, 1), False, 64)])
 def test_cache_build_matches_single_calls(n, ksize, shuffle, volume):
     from flexgemm_b200.kernels import cuda as K
     from flexgemm_b200.ops import utils
@@ -121,7 +121,7 @@ def test_grid_sample_matches_separate_kernels(C, dtype, mode, points, volume):
 @pytest.mark.parametrize("ksize,stride,pad,dil", [((2, 2, 2), (2, 2, 2), (0, 0, 0), (1, 1, 1)), ((3, 3, 3), (2, 2, 2), (1, 1, 1), (1, 1, 1)),
                                                   ((3, 1, 2), (1, 3, 2), (2, 0, 1), (2, 1, 1)), ((1, 1, 1), (1, 1, 1), (0, 0, 0), (1, 1, 1)),
                                                   ((1, 1, 32), (1, 1, 4), (0, 0, 15), (1, 1, 1))])
-@pytest.mark.parametrize("n,shuffle", [(1, False), (255, True), (3000, False), (40000, True)])
+@pytest.mark.parametrize("n,shuffle", [(1, False), (255, True), (3000, False), (8192, True), (40000, True)])
 def test_strided_build_matches_hash_path(ksize, stride, pad, dil, n, shuffle):
     """Output coordinates and maps made on the bit grid against the hash set, sort and table of the generic calls."""
     from flexgemm_b200.kernels import cuda as K

@@ -19,7 +19,7 @@
 //               BN = 256), so halving it is worth the extra warps;
 //   warp 4      one lane streams the dense weight tile [BN x 128 B] of the
 //               current (offset, channel slice) with a tiled TMA load;
-//   warp 5      owns the TMEM allocation; one lane issues tcgen05.mma and
+//   warp 5      owns the TMEM allocation; one elected lane issues tcgen05.mma and
 //               releases stages / publishes accumulators with tcgen05.commit;
 //   warps 6-13  gather the activation rows of both halves into a 128B-swizzled
 //               K-major stage with 16-byte cp.async (zero fill for missing
@@ -52,7 +52,7 @@ constexpr int kTileM = 128;             // rows per accumulator (and per tile ma
 constexpr int kBlockM = 2 * kTileM;     // rows per work item
 constexpr int kMaxStages = 6;
 constexpr int kSchedRing = 16;  // deeper than the gather front can ever run ahead of the epilogue (stages + accumulator sets + 1 blocks)
-constexpr int kSchedReaders = 18;  // 8 gather warps, the TMA lane, the MMA lane, 8 epilogue warps
+constexpr int kSchedReaders = 18;  // 8 gather warps, the TMA lane, the MMA warp, 8 epilogue warps
 constexpr int kIgemmThreads = 576;
 constexpr int kEpilogueWarp1 = 14;  // second group of epilogue warps: 14..17 (the first is 0..3)
 constexpr int kGatherWarp0 = 6;
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
   auto work_of = [&](uint32_t k, uint32_t& mblk, uint32_t& ntile, bool one_lane) -> bool {
     const uint32_t slot = k % kSchedRing;
     const bool ok = mbar_wait(&ctl->sched_full[slot], (k / kSchedRing) & 1, abort_flag);
-    const uint32_t e = ok ? *reinterpret_cast<volatile uint32_t*>(&ctl->sched_entry[slot]) : none;
-    if (!one_lane) __syncwarp();
+    uint32_t e = ok ? *reinterpret_cast<volatile uint32_t*>(&ctl->sched_entry[slot]) : none;
+    if (!one_lane) e = __shfl_sync(0xffffffffu, e, 0);  // every lane has read, and all go the same way after a wait that gave up
     if (one_lane || lane == 0) mbar_arrive(&ctl->sched_empty[slot]);
     if (e == kInvalid) return false;
     mblk = p.items_per_block == 1 ? e : e / p.items_per_block;  // once per work item
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------ weight TMA
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, ph = 0;
       uint32_t mblk = 0, ntile = 0;
       for (uint32_t pass = 0; work_of(pass, mblk, ntile, true); ++pass) {
@@ -471,55 +471,59 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------- MMA
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0, item = 0;
-      uint32_t set = 0, set_ph = 0;  // accumulator set of the item and its phase bit
-      uint32_t mblk = 0, ntile = 0;
-      for (; work_of(item, mblk, ntile, true); ++item) {
-        uint32_t m0, m1;
-        masks_of(mblk, ntile, m0, m1);
-        const uint32_t acc_tmem = tmem_base + set * 2 * p.bn;
-        // the epilogue must have drained this accumulator pair
-        mbar_wait(&ctl->acc_empty[set], set_ph ^ 1, abort_flag);
-        tc_fence_after_sync();
-        uint32_t acc0 = 0, acc1 = 0;
-        uint32_t un = m0 | m1;
-        while (un) {
-          const int v = __ffs(un) - 1;
-          un &= un - 1;
-          const bool need0 = (m0 >> v) & 1u, need1 = (m1 >> v) & 1u;
-          for (int kb = 0; kb < p.num_kb; ++kb) {
-            mbar_wait(&ctl->full[s], ph, abort_flag);
-            // the activation rows were written by cp.async (generic proxy), the MMA reads them through the async proxy
-            fence_proxy_async_smem();
-            tc_fence_after_sync();
+    // The whole warp walks the loop and one elected lane issues.  Under `if (lane == 0)` the compiler does not know that a
+    // single thread is active, and an MMA takes its descriptors from registers that are uniform over the warp: every MMA
+    // of the loop cost ~200 cycles of the lane, more than the MMA itself takes below 256 columns (measured with clock64:
+    // 1640 cycles a stage at C = 64, 92 % of the lane's time, 6 % waiting for operands).  Forward + backward, us: RES=128
+    // C=512 TF32 1911 -> 1615, 4 x RES=64 C=512 bf16 (4 convs) 3392 -> 2972, RES=256 C=256 fp16 878 -> 788.
+    uint32_t s = 0, ph = 0, item = 0;
+    uint32_t set = 0, set_ph = 0;  // accumulator set of the item and its phase bit
+    uint32_t mblk = 0, ntile = 0;
+    // K-major weights: a k-step is 32 bytes along the row; MN-major: 16 rows of 128 bytes, chunks 8 KB apart
+    const bool b_mn = (p.flip & 2) != 0;
+    const uint64_t b_step = b_mn ? 128u : 2u;
+    for (; work_of(item, mblk, ntile, false); ++item) {
+      uint32_t m0, m1;
+      masks_of(mblk, ntile, m0, m1);
+      const uint32_t acc_tmem = tmem_base + set * 2 * p.bn;
+      // the epilogue must have drained this accumulator pair
+      mbar_wait(&ctl->acc_empty[set], set_ph ^ 1, abort_flag);
+      tc_fence_after_sync();
+      uint32_t acc0 = 0, acc1 = 0;
+      uint32_t un = m0 | m1;
+      while (un) {
+        const int v = __ffs(un) - 1;
+        un &= un - 1;
+        const bool need0 = (m0 >> v) & 1u, need1 = (m1 >> v) & 1u;
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          mbar_wait(&ctl->full[s], ph, abort_flag);
+          __syncwarp();
+          // the activation rows were written by cp.async (generic proxy), the MMA reads them through the async proxy
+          fence_proxy_async_smem();
+          tc_fence_after_sync();
+          if (elect_one()) {
             const uint32_t a_addr = smem_u32(stages + size_t(s) * stage_bytes);
             const uint64_t da0 = make_smem_desc(a_addr, 16, 1024);
             const uint64_t da1 = make_smem_desc(a_addr + kATileBytes, 16, 1024);
-            // K-major weights: a k-step is 32 bytes along the row; MN-major: 16 rows of 128 bytes, chunks 8 KB apart
-            const bool b_mn = (p.flip & 2) != 0;
             const uint64_t db = make_smem_desc(a_addr + 2 * kATileBytes, b_mn ? 8192 : 16, 1024);
-            const uint32_t b_step = b_mn ? 128u : 2u;
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4) {
               if (kb * 128 + k4 * 32 < p.row_bytes) {
-                if (need0) {
-                  umma_ss<kTF32>(acc_tmem, da0 + uint64_t(k4 * 2), db + uint64_t(k4 * b_step), p.idesc, acc0);
-                  acc0 = 1;
-                }
-                if (need1) {
-                  umma_ss<kTF32>(acc_tmem + p.bn, da1 + uint64_t(k4 * 2), db + uint64_t(k4 * b_step), p.idesc, acc1);
-                  acc1 = 1;
-                }
+                if (need0) umma_ss<kTF32>(acc_tmem, da0 + uint64_t(k4 * 2), db + k4 * b_step, p.idesc, k4 == 0 ? acc0 : 1u);
+                if (need1) umma_ss<kTF32>(acc_tmem + p.bn, da1 + uint64_t(k4 * 2), db + k4 * b_step, p.idesc, k4 == 0 ? acc1 : 1u);
               }
             }
             umma_commit(&ctl->empty[s]);
-            if (++s == static_cast<uint32_t>(S)) s = 0, ph ^= 1;
           }
+          __syncwarp();
+          acc0 |= need0 ? 1u : 0u;
+          acc1 |= need1 ? 1u : 0u;
+          if (++s == static_cast<uint32_t>(S)) s = 0, ph ^= 1;
         }
-        umma_commit(&ctl->acc_full[set]);
-        if (++set == static_cast<uint32_t>(p.acc_sets)) set = 0, set_ph ^= 1;
       }
+      if (elect_one()) umma_commit(&ctl->acc_full[set]);  // the lane that issued: elect picks the same one each time
+      __syncwarp();
+      if (++set == static_cast<uint32_t>(p.acc_sets)) set = 0, set_ph ^= 1;
     }
   } else {
     // -------------------------------------------------------------- epilogue

@@ -14,7 +14,7 @@
 // second kernel adds the slabs of an offset in a fixed order.
 //
 // Warp roles (416 threads): warps 0-3 epilogue (tcgen05.ld -> fp32 slab),
-// warp 4 owns the TMEM allocation and lane 0 issues the MMAs, warps 5-12 gather
+// warp 4 owns the TMEM allocation and one elected lane issues the MMAs, warps 5-12 gather
 // both operands (cp.async 16 B, pair indices prefetched into registers one stage
 // ahead, completion signalled per thread on the stage's mbarrier).
 #include <cuda_bf16.h>
@@ -474,33 +474,38 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------- MMA
-    if (lane == 0) {
-      uint32_t accumulate = 0;
-      const int chunks_per_m = 128 / kChunkElems;  // 128-byte chunks per 128 accumulator rows
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0; it < total; ++it) {
-        mbar_wait(&ctl->full[s], ph, abort_flag);
-        // both operands were written by cp.async (generic proxy), the MMA reads them through the async proxy
-        fence_proxy_async_smem();
-        tc_fence_after_sync();
+    // the whole warp walks the loop and one elected lane issues: under `if (lane == 0)` every MMA cost the lane ~230 cycles
+    // whatever its width (1840 cycles a stage of eight at C = 64 and at C = 32, 6 % of them waiting for operands)
+    const int chunks_per_m = 128 / kChunkElems;  // 128-byte chunks per 128 accumulator rows
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0; it < total; ++it) {
+      mbar_wait(&ctl->full[s], ph, abort_flag);
+      __syncwarp();
+      // both operands were written by cp.async (generic proxy), the MMA reads them through the async proxy
+      fence_proxy_async_smem();
+      tc_fence_after_sync();
+      if (elect_one()) {
         const uint32_t a_addr = smem_u32(stages + size_t(s) * stage_bytes);
-        const uint32_t b_addr = a_addr + a_bytes;
-        for (int ks = 0; ks < p.kb / kUmmaK; ++ks) {
-          const uint32_t koff = ks * kUmmaK * 128;  // kUmmaK pair rows of 128 bytes
-          const uint64_t db = make_smem_desc(b_addr + koff, chunk_bytes, kSbo, kLayout);
-          for (int m = 0; m < mt; ++m) {
-            const uint64_t da = make_smem_desc(a_addr + m * chunks_per_m * chunk_bytes + koff, chunk_bytes, kSbo, kLayout);
-            umma_ss<kTF32>(tmem_base + m * p.bn, da, db, p.idesc, accumulate);
-          }
-          accumulate = 1;
+        const uint64_t da0 = make_smem_desc(a_addr, chunk_bytes, kSbo, kLayout);
+        const uint64_t db0 = make_smem_desc(a_addr + a_bytes, chunk_bytes, kSbo, kLayout);
+#pragma unroll
+        for (int ks = 0; ks < kRows * 32 / kUmmaK; ++ks) {  // kUmmaK pair rows of 128 bytes a step
+          const uint64_t koff = ks * kUmmaK * 128 >> 4;
+          for (int m = 0; m < mt; ++m)
+            umma_ss<kTF32>(tmem_base + m * p.bn, da0 + uint64_t(m * chunks_per_m * chunk_bytes >> 4) + koff, db0 + koff, p.idesc,
+                           it > 0 || ks > 0 ? 1u : 0u);
         }
         umma_commit(&ctl->empty[s]);
-        if (++s == S) s = 0, ph ^= 1;
       }
+      __syncwarp();
+      if (++s == S) s = 0, ph ^= 1;
+    }
+    if (elect_one()) {  // the lane that issued: elect picks the same one each time
       if (total > 0) umma_commit(&ctl->acc_full);
       else mbar_arrive(&ctl->acc_full);  // nothing was issued: the epilogue writes zeros
     }
+    __syncwarp();
   } else {
     // -------------------------------------------------------------- epilogue
     // Thread `lane` of warp w holds accumulator row 32 w + lane.  32 columns at a time go through a 4 KB staging

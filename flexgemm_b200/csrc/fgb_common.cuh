@@ -32,6 +32,17 @@ __device__ __forceinline__ void mirror_code(int32_t* mirror, int32_t code) {
   }
 }
 
+// Fills a host slot (flexgemm_b200.h), the sequence number last; nothing when the slot is null.
+__device__ __forceinline__ void tell_host(uint32_t* slot, uint32_t seq, uint32_t count, uint32_t order, uint32_t status) {
+  if (slot == nullptr) return;
+  volatile uint32_t* h = slot;
+  h[FGB_HOST_COUNT] = count;
+  h[FGB_HOST_ORDER] = order;
+  h[FGB_HOST_STATUS] = status;
+  __threadfence_system();
+  h[FGB_HOST_SEQ] = seq;
+}
+
 inline int elem_bytes(int dtype) {
   switch (dtype) {
     case FGB_F16:

@@ -83,7 +83,7 @@ struct ScanFinish {
   uint32_t* done;               // zeroed word: count of finished CTAs; null = leave the totals as they are
   const uint32_t* unsorted;     // copied to seg[V + 1] when not null
   const int32_t* build_status;  // copied to seg[V + 2] when not null
-  uint32_t* host_words;         // mapped pinned memory [V + 3], then the sequence word; null = not wanted
+  uint32_t* host_words;         // host slot (flexgemm_b200.h), or null
   uint32_t host_seq;
 };
 

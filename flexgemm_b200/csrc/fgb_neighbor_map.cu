@@ -202,14 +202,8 @@ __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__
         seg[0] = 0;
         if (fin.unsorted != nullptr) seg[V + 1] = *fin.unsorted;
         if (fin.build_status != nullptr) seg[V + 2] = static_cast<uint32_t>(*fin.build_status);
-        if (fin.host_words != nullptr) {
-          volatile uint32_t* h = fin.host_words;
-          h[V] = acc;
-          h[V + 1] = fin.unsorted != nullptr ? *fin.unsorted : 0u;
-          h[V + 2] = fin.build_status != nullptr ? static_cast<uint32_t>(*fin.build_status) : 0u;
-          __threadfence_system();
-          h[V + 3] = fin.host_seq;
-        }
+        tell_host(fin.host_words, fin.host_seq, acc, fin.unsorted != nullptr ? *fin.unsorted : 0u,
+                  fin.build_status != nullptr ? static_cast<uint32_t>(*fin.build_status) : 0u);
       }
     }
   }

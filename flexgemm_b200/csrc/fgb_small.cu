@@ -148,14 +148,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_plan_kernel(PlanJob job_a
       if (lane == 0) j.seg[0] = 0;
       if (lane == 31) {
         if (j.fin.build_status != nullptr) j.seg[j.V + 1] = 1u, j.seg[j.V + 2] = 0u;  // not by columns; nothing can run full
-        if (j.fin.host_words != nullptr) {
-          volatile uint32_t* h = j.fin.host_words;
-          h[j.V] = inc;
-          h[j.V + 1] = 1u;
-          h[j.V + 2] = 0u;
-          __threadfence_system();
-          h[j.V + 3] = j.fin.host_seq;
-        }
+        tell_host(j.fin.host_words, j.fin.host_seq, inc, 1u, 0u);
       }
     }
   }

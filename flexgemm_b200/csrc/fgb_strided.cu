@@ -109,7 +109,7 @@ __device__ __forceinline__ uint32_t load_words(const uint32_t* bits, uint32_t fi
 }
 
 // cta_base[b] = set bits of CTA b's words; the CTA that ends last turns them into exclusive sums and tells the host the
-// total (mapped memory: the count, then the sequence number)
+// total
 __global__ void __launch_bounds__(kRankThreads) count_cells_kernel(const uint32_t* __restrict__ bits, uint32_t* cta_base,
                                                                    uint32_t* done, uint32_t* host_words, uint32_t host_seq) {
   __shared__ uint32_t s_warp[32];
@@ -143,12 +143,7 @@ __global__ void __launch_bounds__(kRankThreads) count_cells_kernel(const uint32_
     }
     carry += total;
   }
-  if (threadIdx.x == 0 && host_words != nullptr) {
-    volatile uint32_t* h = host_words;
-    h[0] = carry;
-    __threadfence_system();
-    h[1] = host_seq;
-  }
+  if (threadIdx.x == 0) tell_host(host_words, host_seq, carry, 0u, 0u);
 }
 
 // rows of the marked cells, and the row of the first cell of every word that has one

@@ -156,7 +156,8 @@ struct HostWords {
 };
 std::mutex g_words_mu;
 std::vector<HostWords> g_words_free;
-constexpr int kHostWords = 64;  // per slot: up to 32 + 4 are used
+constexpr int kHostWords = 16;  // per slot: FGB_HOST_WORDS, and a line of its own
+static_assert(FGB_HOST_WORDS <= kHostWords);
 
 HostWords take_host_words() {
   std::lock_guard<std::mutex> lock(g_words_mu);
@@ -178,9 +179,9 @@ void give_host_words(const HostWords& w) {
   std::lock_guard<std::mutex> lock(g_words_mu);
   g_words_free.push_back(w);
 }
-// waits until the stream's work has stored `seq` into word `index`
-void wait_host_words(const HostWords& w, int index, cudaStream_t stream) {
-  for (uint64_t i = 1; w.host[index] != w.seq; ++i) {
+// waits until the stream's work has stored the use's sequence number
+void wait_host_words(const HostWords& w, cudaStream_t stream) {
+  for (uint64_t i = 1; w.host[FGB_HOST_SEQ] != w.seq; ++i) {
 #if defined(__x86_64__)
     __builtin_ia32_pause();
 #endif
@@ -188,7 +189,7 @@ void wait_host_words(const HostWords& w, int index, cudaStream_t stream) {
       const cudaError_t e = cudaStreamQuery(stream);
       if (e == cudaErrorNotReady) continue;
       C10_CUDA_CHECK(e);
-      if (w.host[index] != w.seq) throw std::runtime_error("flexgemm_b200: the neighbour-map build ended without its pair count");
+      if (w.host[FGB_HOST_SEQ] != w.seq) throw std::runtime_error("flexgemm_b200: the neighbour-map build ended without its pair count");
     }
   }
   std::atomic_thread_fence(std::memory_order_acquire);
@@ -543,22 +544,21 @@ CacheBuild start_cache(const Tensor& coords, const int64_t* shape, const int64_t
   return b;
 }
 
-// Waits for the sequence number in word `index` without holding the GIL, gives the words back and returns those from
-// `first` on.
-struct Words3 {
-  uint32_t v[3];
+// What a kernel has told the host: waits for it without holding the GIL and gives the words back.
+struct Told {
+  uint32_t count, status;
 };
-Words3 take_back(const HostWords& w, int first, int index, cudaStream_t stream) {
+Told take_back(const HostWords& w, cudaStream_t stream) {
   std::exception_ptr failed;
   Py_BEGIN_ALLOW_THREADS;
   try {
-    wait_host_words(w, index, stream);
+    wait_host_words(w, stream);
   } catch (...) {
     failed = std::current_exception();
   }
   Py_END_ALLOW_THREADS;
   if (failed) std::rethrow_exception(failed);
-  const Words3 r{{w.host[first], w.host[first + 1], w.host[first + 2]}};
+  const Told r{w.host[FGB_HOST_COUNT], w.host[FGB_HOST_STATUS]};
   give_host_words(w);
   return r;
 }
@@ -568,10 +568,9 @@ Pairs finish_cache(const CacheBuild& b) {
   const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
   int64_t pairs = 0;
   if (b.n > 0) {
-    const Words3 got = take_back(b.words, b.V, b.V + 3, stream);
-    pairs = got.v[0];
-    const int code = static_cast<int>(got.v[2]);
-    if (code != 0) throw_soft_error(code);
+    const Told got = take_back(b.words, stream);
+    pairs = got.count;
+    if (got.status != 0u) throw_soft_error(static_cast<int>(got.status));
   }
   Pairs p;
   p.vs_i = new_tensor({pairs}, at::kUInt32, b.nbr.device());
@@ -850,7 +849,7 @@ bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape,
   c.host_words = w.dev, c.host_seq = w.seq;
   check(api.fgb_strided_mark(&c, stream), "fgb_strided_mark");
   g_launches += 2;
-  c.n_out = take_back(w, 0, 1, stream).v[0];
+  c.n_out = take_back(w, stream).count;
   c.host_words = nullptr;
   b.out_coords = new_tensor({c.n_out, 4}, at::kInt, coords.device());
   if (c.n_out == 0) return coords_only;
@@ -897,7 +896,7 @@ void strided_maps(StridedBuild& b, at::Device dev, bool train) {
 
 Pairs strided_pairs(const StridedBuild& b) {
   const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
-  const int64_t pairs = take_back(b.words, b.V, b.V + 3, stream).v[0];
+  const int64_t pairs = take_back(b.words, stream).count;
   Pairs p;
   p.vs_i = new_tensor({pairs}, at::kUInt32, b.nbr.device());
   p.vs_o = new_tensor({pairs}, at::kUInt32, b.nbr.device());

@@ -589,10 +589,20 @@ int fgb_conv_call_dgrad(const fgb_conv_call* call, void* stream);
  * (fgb_subm_build_neighbor_map), sorted_idx (fgb_pp_sorted_idx), the masks of
  * 128-row tiles and the block schedule, on one scratch block and two memsets.
  * meta [v + 3] receives the segment table [v + 1], the key-order word and the
- * build's status (FGB_S_TABLE_FULL); host_words, when not null, is mapped pinned
- * memory [v + 4] whose words v .. v + 2 receive the pair count, the key-order word
- * and the status, and then word v + 3 the value host_seq: a host that wants the
- * pair count watches that word.  `status`: the device status word of the sort. */
+ * build's status (FGB_S_TABLE_FULL); host_words, when not null, is a host slot
+ * (below) that receives the pair count, the key-order word and the status.
+ * `status`: the device status word of the sort.
+ *
+ * Host slot: FGB_HOST_WORDS words of mapped pinned memory through which a kernel
+ * hands numbers to a waiting host.  Word FGB_HOST_SEQ receives the caller's
+ * host_seq after the others are written, and never anything else: a host that
+ * gives every use of a slot a value the word has not held before can use the slot
+ * for any of the calls in turn, whatever the earlier ones left in the other words. */
+#define FGB_HOST_COUNT 0
+#define FGB_HOST_ORDER 1
+#define FGB_HOST_STATUS 2
+#define FGB_HOST_SEQ 3
+#define FGB_HOST_WORDS 4
 typedef struct fgb_map_call {
   const int32_t* coords;
   int64_t n;
@@ -620,14 +630,13 @@ int fgb_subm_cache_build(const fgb_map_call* call, void* stream);
  *   fgb_strided_grid_bytes  memory of the marked output cells; 0 when the grid is
  *                           too large or too empty for one bit per cell (the calls
  *                           of the generic conv above then do the work);
- *   fgb_strided_mark        marks and counts the cells; host_words (mapped pinned,
- *                           may be null) receives the count in word 0, then
- *                           host_seq in word 1;
+ *   fgb_strided_mark        marks and counts the cells; host_words (a host slot,
+ *                           may be null) receives the count;
  *   fgb_strided_build       with n_out = that count: out_coords and, when
  *                           neighbor_map is not null, both maps (the backward one
  *                           when neighbor_map_bwd is not null), codes, row orders,
  *                           tile masks, schedules, block offsets, and meta [v + 1] =
- *                           the segment table; host_words as in fgb_map_call.
+ *                           the segment table; host_words receives the pair count.
  * coords: in-range rows without duplicates (of duplicates, any one is kept). */
 typedef struct fgb_strided_call {
   const int32_t* coords;

@@ -27,6 +27,19 @@ def test_header_and_binding_agree(lib):
         assert hasattr(lib, name), name
 
 
+def test_host_slot_keeps_the_sequence_word_to_itself():
+    """A host slot serves calls of every kind in turn: the word the host watches is not one that any of them puts a number
+    into, and every kernel fills a slot through the one function that knows the layout."""
+    header = open(os.path.join(ROOT, "include", "flexgemm_b200.h")).read()
+    at = {k: int(v) for k, v in re.findall(r"#define FGB_HOST_(\w+) (\d+)", header)}
+    words = at.pop("WORDS")
+    assert set(at) == {"COUNT", "ORDER", "STATUS", "SEQ"} and len(set(at.values())) == 4 and max(at.values()) < words
+    csrc = os.path.join(ROOT, "flexgemm_b200", "csrc")
+    text = {f: open(os.path.join(csrc, f)).read() for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))}
+    assert sum(t.count("[FGB_HOST_SEQ] = ") for t in text.values()) == 1
+    assert not any(re.search(r"= *\w*\.?host_words;", t) for t in text.values())
+
+
 def test_version_and_errors(lib):
     assert b"sm_100a" in lib.fgb_version()
     assert _cabi.error_string(0) == "ok"

@@ -1090,7 +1090,7 @@ static bool dgrad_as_stored(int Ci, int eb) {
 static int dgrad_impl(const void* grad_out, const void* weight, const uint32_t* neighbor_map, const int64_t* sorted_idx,
                       const uint32_t* tile_masks, const uint32_t* block_order, void* grad_feats, int64_t n, int64_t n_src, int Ci, int Co,
                       int V, int dtype, int mirror, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream,
-                      uint32_t* zeroed_ticket = nullptr) {
+                      uint32_t* zeroed_ticket = nullptr, bool no_relayout_room = false) {
   const int eb = elem_bytes(dtype);
   if (eb == 0) return FGB_E_DTYPE;
   if (n < 0 || n_src < 0 || Ci <= 0 || Co <= 0 || V < 1 || V > 32) return FGB_E_SIZE;
@@ -1098,7 +1098,7 @@ static int dgrad_impl(const void* grad_out, const void* weight, const uint32_t* 
   if (!weight || !workspace) return FGB_E_NULL;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return FGB_E_ALIGN;
   const bool as_stored = dgrad_as_stored(Ci, eb);
-  const int64_t wt_bytes = as_stored && zeroed_ticket != nullptr ? 0 : align256(int64_t(Ci) * V * Co * eb);
+  const int64_t wt_bytes = as_stored && no_relayout_room ? 0 : align256(int64_t(Ci) * V * Co * eb);
   const bool ieee = dtype == FGB_F32_IEEE;
   const int64_t w3_bytes = ieee ? align256(int64_t(Ci) * V * 3 * Co * 4) : 0;
   const int64_t g3_bytes = ieee ? align256(n_src * 3 * Co * 4) : 0;
@@ -1176,5 +1176,5 @@ extern "C" int fgb_conv_call_fprop(const fgb_conv_call* c, void* stream) {
 extern "C" int fgb_conv_call_dgrad(const fgb_conv_call* c, void* stream) {
   if (!c) return FGB_E_NULL;
   return fgb::dgrad_impl(c->x, c->weight, c->neighbor_map, c->sorted_idx, c->tile_masks, c->block_order, c->out, c->n, c->n_src, c->ci,
-                         c->co, c->v, c->dtype, c->mirror, c->workspace, c->workspace_bytes, c->status, stream, c->counters);
+                         c->co, c->v, c->dtype, c->mirror, c->workspace, c->workspace_bytes, c->status, stream, c->counters, true);
 }

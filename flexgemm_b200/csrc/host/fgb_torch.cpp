@@ -17,6 +17,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
@@ -127,7 +128,10 @@ std::unordered_map<uint64_t, ZeroPool> g_zero;
 constexpr int64_t kZeroPoolWords = 4096;
 constexpr size_t kMaxZeroPools = 64;
 
+// null while the stream is being captured: a graph runs its calls again and must zero their words itself, each time, in
+// memory that is its own (the library does so in a call's workspace), and what a capture allocates stays out of the pool.
 uint32_t* zeroed_words(c10::cuda::CUDAStream stream, int64_t words) {
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
   words = (words + 7) & ~int64_t(7);
   std::lock_guard<std::mutex> lock(g_zero_mu);
   const uint64_t key = reinterpret_cast<uint64_t>(stream.stream()) * 64 + static_cast<uint64_t>(stream.device_index());

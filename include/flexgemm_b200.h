@@ -556,10 +556,12 @@ int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t* indices, 
  * --------------------------------------------------------------------- */
 
 /* The passes above with their arguments in one struct and two differences that
- * save stream operations: the caller hands in `counters`, device words that are
- * zero and that no other call uses (one word; a pool zeroed now and then costs
- * nothing per call, where a memset per launch does), and the weight gradient
- * call computes the bias gradient in the same two launches.
+ * save stream operations: the caller may hand in `counters`, a device word that is
+ * zero and that no other call uses (a pool zeroed now and then costs nothing per
+ * call, where a memset per launch does; the call leaves the word non-zero), and the
+ * weight gradient call computes the bias gradient in the same two launches.
+ * counters = null: the call zeroes a word of its workspace, as the calls above do --
+ * the way for a call that is captured into a graph and so runs more than once.
  *
  * fprop: x = feats [n_src, ci], out [n, co]; dgrad: x = grad_out [n_src, co],
  * out = grad_feats [n, ci], mirror = 1 for the forward map of a submanifold conv,

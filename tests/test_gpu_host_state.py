@@ -1,6 +1,9 @@
-"""State that the native host path shares between calls: the slots through which a build reports to the host."""
+"""State that the native host path shares between calls: the slots through which a build reports to the host, the work
+counters of the conv kernels."""
 import pytest
 import torch
+
+from oracle import submconv_oracle as orc
 
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +32,53 @@ def test_host_slots_serve_every_kind_of_build_in_turn():
         cache = SubMConv3dFunction._compute_neighbor_cache(coords, shape, (1, 1, 5), (1, 1, 1), True)
         pairs = n + 2 * (n - 1) + 2 * (n - 2)
         assert cache["valid_signal_i"].shape[0] == pairs and cache["valid_signal_o"].shape[0] == pairs
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+def test_graph_replays_follow_their_inputs(dtype):
+    """A captured pass gives on every replay what the same call gives outside a graph, also when the capturing stream has
+    been used before, when several graphs are captured on it and when calls outside them come between."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(16, 32, 96, dtype, seed=4))
+    shape = torch.Size(shape)
+    g = torch.Generator().manual_seed(9)
+    gout = torch.randn(len(coords), 96, generator=g).to(feats.dtype).to(DEV)
+    w = weight.detach().requires_grad_(True)
+    x = feats.detach().clone().requires_grad_(True)
+    _, cache = spconv.sparse_submanifold_conv3d(x, coords, shape, w, bias)
+
+    def train():
+        out, _ = spconv.sparse_submanifold_conv3d(x, coords, shape, w, bias, cache)
+        return (out.detach(), *torch.autograd.grad(out, (x, w), gout))
+
+    def infer():
+        args = (x.detach(), coords, shape, w.detach(), bias)   # the first builds an inference cache, which waits for nothing
+        return spconv.sparse_submanifold_conv3d(*args)[0], spconv.sparse_submanifold_conv3d(*args, cache)[0]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            train(), infer()
+    torch.cuda.current_stream().wait_stream(side)
+    graphs = []
+    for call in (train, infer, train):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            outs = call()
+        graphs.append((graph, call, outs))
+    for i in range(3):
+        with torch.no_grad():
+            x.copy_(torch.randn(x.shape, generator=g).to(x.dtype))
+        for graph, call, outs in graphs:
+            for o in outs:
+                o.fill_(float("nan"))
+            graph.replay()
+            for got, want in zip(outs, call()):
+                assert torch.equal(got, want)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            train()
+        torch.cuda.synchronize()
+    K.check_status(DEV)

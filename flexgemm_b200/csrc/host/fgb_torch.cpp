@@ -117,8 +117,9 @@ void poll(DeviceState& s, c10::cuda::CUDAStream stream) {
 }
 
 // Zeroed device words, handed out once each: a slice of a buffer that is zeroed 4096 words at a time on the stream that
-// uses it.  One buffer per stream, dropped when it is used up (its last words are then in use by earlier work of the same
-// stream, which the allocator's stream order covers) and all of them when streams come and go.
+// uses it.  One buffer per stream, dropped when it is used up and all of them when streams come and go.  Whoever takes
+// words holds their buffer until the work on them is queued: another thread on the same stream may drop it from the pool
+// meanwhile, and from then on only the allocator's stream order keeps later users of the memory behind that work.
 struct ZeroPool {
   Tensor buf;
   int64_t used = 0;
@@ -127,11 +128,15 @@ std::mutex g_zero_mu;
 std::unordered_map<uint64_t, ZeroPool> g_zero;
 constexpr int64_t kZeroPoolWords = 4096;
 constexpr size_t kMaxZeroPools = 64;
+struct ZeroedWords {
+  Tensor buf;  // holds the words
+  uint32_t* words = nullptr;
+};
 
-// null while the stream is being captured: a graph runs its calls again and must zero their words itself, each time, in
+// None while the stream is being captured: a graph runs its calls again and must zero their words itself, each time, in
 // memory that is its own (the library does so in a call's workspace), and what a capture allocates stays out of the pool.
-uint32_t* zeroed_words(c10::cuda::CUDAStream stream, int64_t words) {
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
+ZeroedWords zeroed_words(c10::cuda::CUDAStream stream, int64_t words) {
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
   words = (words + 7) & ~int64_t(7);
   std::lock_guard<std::mutex> lock(g_zero_mu);
   const uint64_t key = reinterpret_cast<uint64_t>(stream.stream()) * 64 + static_cast<uint64_t>(stream.device_index());
@@ -146,7 +151,7 @@ uint32_t* zeroed_words(c10::cuda::CUDAStream stream, int64_t words) {
     C10_CUDA_CHECK(cudaMemsetAsync(p.buf.data_ptr(), 0, kZeroPoolWords * 4, stream));
     p.used = 0;
   }
-  uint32_t* out = static_cast<uint32_t*>(p.buf.data_ptr()) + p.used;
+  const ZeroedWords out{p.buf, static_cast<uint32_t*>(p.buf.data_ptr()) + p.used};
   p.used += words;
   return out;
 }
@@ -269,7 +274,8 @@ Tensor run_fprop(const Tensor& feats, const Tensor& weight, const Tensor& bias, 
   c.workspace_bytes = check_bytes(api.fgb_conv_call_workspace_bytes(&c, 0), "fgb_conv_call_workspace_bytes");
   const c10::DataPtr ws = scratch(c.workspace_bytes);
   c.workspace = ws.get();
-  c.counters = zeroed_words(stream, 1);
+  const ZeroedWords counter = zeroed_words(stream, 1);
+  c.counters = counter.words;
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   check(api.fgb_conv_call_fprop(&c, stream), "fgb_conv_call_fprop");
   g_launches += 1;
@@ -295,7 +301,8 @@ Tensor run_dgrad(const Tensor& grad_out, const Tensor& weight, const Maps& m, in
   c.workspace_bytes = check_bytes(api.fgb_conv_call_workspace_bytes(&c, 1), "fgb_conv_call_workspace_bytes");
   const c10::DataPtr ws = scratch(c.workspace_bytes);
   c.workspace = ws.get();
-  c.counters = zeroed_words(stream, 1);
+  const ZeroedWords counter = zeroed_words(stream, 1);
+  c.counters = counter.words;
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   check(api.fgb_conv_call_dgrad(&c, stream), "fgb_conv_call_dgrad");
   g_launches += 2;

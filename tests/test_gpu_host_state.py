@@ -82,3 +82,42 @@ def test_graph_replays_follow_their_inputs(dtype):
             train()
         torch.cuda.synchronize()
     K.check_status(DEV)
+
+
+def test_work_counters_of_threads_on_one_stream():
+    """Two threads run passes on the same stream, their backward passes beside the other's forward ones, through several
+    refills of the counter pool and with more streams than it keeps pools for: every pass gives the same bits."""
+    import threading
+
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(12, 16, 32, "float16", seed=6))
+    shape = torch.Size(shape)
+    gout = torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(3)).half().to(DEV)
+    _, cache = spconv.sparse_submanifold_conv3d(feats, coords, shape, weight.detach().requires_grad_(True), bias)
+
+    def once():
+        x, w = feats.detach().requires_grad_(True), weight.detach().requires_grad_(True)
+        out, _ = spconv.sparse_submanifold_conv3d(x, coords, shape, w, bias, cache)
+        return (out.detach(), *torch.autograd.grad(out, (x, w), gout))
+    want = once()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(seed):
+        for i in range(400):
+            if i % 6 == seed:
+                with torch.cuda.stream(torch.cuda.ExternalStream(streams[(i + 31 * seed) % len(streams)].cuda_stream)):
+                    once()
+            got = once()
+            if i % 8 == 0 and not all(torch.equal(a, b) for a, b in zip(got, want)):
+                wrong.append((seed, i))
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(32)] + [torch.cuda.current_stream()]
+    threads = [threading.Thread(target=work, args=(s,)) for s in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong
+    K.check_status(DEV)

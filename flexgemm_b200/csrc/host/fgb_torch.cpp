@@ -485,9 +485,14 @@ struct ConvBackward : public torch::autograd::Node {
   }
 };
 
+// Whether an input carries a forward-mode tangent.  There is no forward-mode derivative: the Python functions refuse
+// such inputs, and the fast way, which looks at requires_grad, would drop the tangent.
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
 // the checks of the fast way
 bool conv_args_ok(const Tensor& feats, const Tensor& weight, const Tensor& bias, PyObject* bias_obj, int64_t* V, int dtype) {
   if (!feats.defined() || !weight.defined() || dtype < 0) return false;
+  if (has_tangent(feats) || has_tangent(weight) || has_tangent(bias)) return false;
   if (!feats.is_cuda() || feats.dim() != 2 || feats.size(0) == 0 || feats.size(1) == 0 || !feats.is_contiguous()) return false;
   if (weight.device() != feats.device() || weight.scalar_type() != feats.scalar_type() || weight.dim() != 5 || !weight.is_contiguous() ||
       weight.size(0) == 0 || weight.size(4) != feats.size(1))
@@ -1063,7 +1068,7 @@ PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       feats.size(1) % 4 != 0 || dtype_code(feats.scalar_type(), false) < 0 || !coords_ok(coords, one) || coords.device() != feats.device() ||
       coords.size(0) != feats.size(0) || !grid.defined() || grid.device() != feats.device() || grid.dim() != 3 || grid.size(2) != 3 ||
       grid.scalar_type() != at::kFloat || !grid.is_contiguous() || grid.numel() == 0 || !int_args(a[2], 5, shape) ||
-      (reinterpret_cast<uintptr_t>(feats.const_data_ptr()) & 15) != 0)
+      (reinterpret_cast<uintptr_t>(feats.const_data_ptr()) & 15) != 0 || has_tangent(feats) || has_tangent(grid))
     Py_RETURN_NONE;
   const double ratio = PyFloat_AsDouble(a[5]);
   if (ratio == -1.0 && PyErr_Occurred()) return nullptr;

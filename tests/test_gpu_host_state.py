@@ -1,5 +1,5 @@
-"""State that the native host path shares between calls: the slots through which a build reports to the host, the work
-counters of the conv kernels."""
+"""What the native host path keeps or must refuse: the slots through which a build reports to the host, the work
+counters of the conv kernels, inputs that autograd treats specially."""
 import pytest
 import torch
 
@@ -121,3 +121,29 @@ def test_work_counters_of_threads_on_one_stream():
     torch.cuda.synchronize()
     assert not wrong
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_forward_mode_is_refused(which):
+    """There is no forward-mode derivative: a tangent on any input is an error, not an output without one."""
+    import torch.autograd.forward_ad as fwad
+
+    from flexgemm_b200.ops import grid_sample, spconv
+    coords, *args, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 16, 16, "float16", seed=2))
+    shape = torch.Size(shape)
+    _, cache = spconv.sparse_submanifold_conv3d(args[0], coords, shape, args[1], args[2])
+    query = torch.rand(1, 50, 3, device=DEV) * 8
+    with fwad.dual_level():
+        args[which] = fwad.make_dual(args[which], torch.ones_like(args[which]))
+        f, w, b = args
+        calls = [lambda: spconv.sparse_submanifold_conv3d(f, coords, shape, w, b), lambda: spconv.sparse_submanifold_conv3d(f, coords, shape, w, b, cache),
+                 lambda: spconv.sparse_conv3d(f, coords, shape, w, b, stride=(2, 2, 2), padding=(1, 1, 1))]
+        if which == 0:
+            calls += [lambda: grid_sample.grid_sample_3d(f, coords, shape, query, "trilinear"),
+                      lambda: grid_sample.grid_sample_3d(f, coords, shape, query, "nearest")]
+        if which == 1:
+            q = fwad.make_dual(query, torch.ones_like(query))
+            calls.append(lambda: grid_sample.grid_sample_3d(args[0], coords, shape, q))
+        for call in calls:
+            with pytest.raises(NotImplementedError, match="jvp"):
+                call()

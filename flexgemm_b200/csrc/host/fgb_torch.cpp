@@ -1042,12 +1042,17 @@ Tensor run_sample_grad(const Tensor& grad_out /* [M, C] */, const Tensor& indice
 }
 
 struct GridSampleBackward : public torch::autograd::Node {
-  Tensor indices, weight;
+  torch::autograd::SavedVariable indices_, weight_;
   int64_t n = 0, V = 1;
   std::string name() const override { return "GridSample3dBackward"; }
+  void release_variables() override {
+    indices_.reset_data();
+    weight_.reset_data();
+  }
   variable_list apply(variable_list&& grads) override {
     variable_list out(1);
     if (!grads[0].defined() || !task_should_compute_output(0)) return out;
+    const Tensor indices = indices_.unpack(), weight = weight_.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor g = grads[0].contiguous();
     out[0] = run_sample_grad(g.view({-1, g.size(-1)}), indices, weight, n, V);
@@ -1100,7 +1105,9 @@ PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (want_grad) {
     std::shared_ptr<GridSampleBackward> node(new GridSampleBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(feats));
-    node->indices = indices, node->weight = weight, node->n = n, node->V = V;
+    node->indices_ = torch::autograd::SavedVariable(indices, false);
+    node->weight_ = torch::autograd::SavedVariable(weight, false);
+    node->n = n, node->V = V;
     torch::autograd::set_history(out, node);
   }
   return THPVariable_Wrap(out);

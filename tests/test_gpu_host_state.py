@@ -147,3 +147,30 @@ def test_forward_mode_is_refused(which):
         for call in calls:
             with pytest.raises(NotImplementedError, match="jvp"):
                 call()
+
+
+@pytest.mark.parametrize("mode", ["trilinear", "nearest"])
+def test_grid_sample_saves_its_map_as_autograd_does(mode):
+    """The map of a sample is a saved tensor: freed by the backward pass (a second one is an error), kept by retain_graph,
+    and seen by saved-tensor hooks.  (The order of the fp32 sums is not fixed: two passes may differ by one step of fp16.)"""
+    from flexgemm_b200.ops import grid_sample
+    coords, feats, _, _, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 16, 16, "float16", seed=2))
+    feats.requires_grad_(True)
+    query = torch.rand(1, 5000, 3, device=DEV) * 8
+    (want,) = torch.autograd.grad(grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query, mode).sum(), feats)
+    out = grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query, mode).sum()
+    for retain in (True, False):
+        (got,) = torch.autograd.grad(out, feats, retain_graph=retain)
+        assert torch.allclose(got, want, rtol=2e-3, atol=2e-3)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, feats)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.numel()) or t.cpu(), lambda t: t.to(DEV)):
+        out = grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query, mode)
+    assert packed == ([40000, 40000] if mode == "trilinear" else [5000])
+    (got,) = torch.autograd.grad(out.sum(), feats)
+    assert torch.allclose(got, want, rtol=2e-3, atol=2e-3)
+    held = torch.cuda.memory_allocated()
+    out = grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query, mode)
+    (got,) = torch.autograd.grad(out.sum(), feats)
+    assert torch.cuda.memory_allocated() - held <= 2 * out.numel() + 4 * got.numel() + 4096   # the output and the gradient

@@ -1075,6 +1075,8 @@ PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       grid.scalar_type() != at::kFloat || !grid.is_contiguous() || grid.numel() == 0 || !int_args(a[2], 5, shape) ||
       (reinterpret_cast<uintptr_t>(feats.const_data_ptr()) & 15) != 0 || has_tangent(feats) || has_tangent(grid))
     Py_RETURN_NONE;
+  // query points that want a gradient get none, but a backward pass from the output has to go through
+  if (torch::autograd::compute_requires_grad(grid)) Py_RETURN_NONE;
   const double ratio = PyFloat_AsDouble(a[5]);
   if (ratio == -1.0 && PyErr_Occurred()) return nullptr;
   c10::cuda::CUDAGuard guard(feats.device());

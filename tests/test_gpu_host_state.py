@@ -174,3 +174,16 @@ def test_grid_sample_saves_its_map_as_autograd_does(mode):
     out = grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query, mode)
     (got,) = torch.autograd.grad(out.sum(), feats)
     assert torch.cuda.memory_allocated() - held <= 2 * out.numel() + 4 * got.numel() + 4096   # the output and the gradient
+
+
+@pytest.mark.parametrize("feats_grad", [False, True])
+def test_grid_sample_with_query_points_that_require_grad(feats_grad):
+    """There is no gradient with respect to the points, yet the output takes part in the graph."""
+    from flexgemm_b200.ops import grid_sample
+    coords, feats, _, _, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 16, 16, "float32", seed=2))
+    feats.requires_grad_(feats_grad)
+    query = (torch.rand(1, 50, 3, device=DEV) * 8).requires_grad_(True)
+    out = grid_sample.grid_sample_3d(feats, coords, torch.Size(shape), query)
+    assert out.requires_grad
+    out.sum().backward()
+    assert query.grad is None and (feats.grad is not None) == feats_grad

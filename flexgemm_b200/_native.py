@@ -21,6 +21,7 @@ def ext():
         spec = importlib.util.spec_from_file_location("_fgb_torch", path, loader=importlib.machinery.ExtensionFileLoader("_fgb_torch", path))
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
-        mod.init(_cabi.lib()._handle)
+        from .kernels import config
+        mod.init(_cabi.lib()._handle, config)
         _mod = mod
     return _mod

@@ -456,14 +456,27 @@ bool int_args(PyObject* seq, int k, int64_t* out) {
 }
 
 // ------------------------------------------------------------------ autograd
+PyObject *g_config, *s_allow_tf32;  // the module flexgemm_b200.kernels.config, and its setting
+
+// Element type of a backward pass.  TF32 or accurate fp32 is what the setting says when the pass runs.
+int backward_dtype(at::ScalarType t) {
+  if (t != at::kFloat) return dtype_code(t, false);
+  const PyGILState_STATE gil = PyGILState_Ensure();
+  PyObject* v = PyObject_GetAttr(g_config, s_allow_tf32);
+  const int on = v != nullptr ? PyObject_IsTrue(v) : -1;
+  Py_XDECREF(v);
+  if (on < 0) PyErr_Clear();
+  PyGILState_Release(gil);
+  if (on < 0) throw std::runtime_error("flexgemm_b200.kernels.config.allow_tf32 is not a truth value");
+  return dtype_code(t, on == 1);
+}
+
 struct ConvBackward : public torch::autograd::Node {
   torch::autograd::SavedVariable feats_, weight_;
   Maps bwd;
   Pairs pairs;
   bool mirror = true;
   int64_t V = 0;
-  int dtype = 0;
-  bool has_pairs = false;
 
   std::string name() const override { return mirror ? "SubMConv3dBackward" : "SparseConv3dBackward"; }
   void release_variables() override {
@@ -478,6 +491,7 @@ struct ConvBackward : public torch::autograd::Node {
     if ((need_w && !pairs.vs_i.defined()) || (need_x && !bwd.nbr.defined()))
       throw torch::AttributeError(std::string("the neighbor cache was built for inference: it has no ") +
                                   (need_w ? "valid_signal_i" : "neighbor_map_bwd"));
+    const int dtype = backward_dtype(feats.scalar_type());
     at::AutoDispatchBelowADInplaceOrView below;
     Grads g = run_backward(grads[0], feats, weight, bwd, pairs, mirror, V, dtype, need_x, need_w, need_b);
     out[0] = std::move(g.feats), out[1] = std::move(g.weight), out[2] = std::move(g.bias);
@@ -689,7 +703,7 @@ PyObject* py_subm_cache(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // Output of a convolution over `m`, with its autograd node where a gradient is wanted
 Tensor conv_autograd(const Tensor& feats, const Tensor& weight, const Tensor& bias, const Maps& m, const Maps& bwd, const Pairs& pairs,
-                     bool mirror, int64_t V, int dtype, Tensor out) {
+                     bool mirror, int64_t V, Tensor out) {
   if (!torch::autograd::compute_requires_grad(feats, weight, bias)) return out;
   std::shared_ptr<ConvBackward> node(new ConvBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(feats, weight, bias));
@@ -699,7 +713,6 @@ Tensor conv_autograd(const Tensor& feats, const Tensor& weight, const Tensor& bi
   node->pairs = pairs;
   node->mirror = mirror;
   node->V = V;
-  node->dtype = dtype;
   torch::autograd::set_history(out, node);
   return out;
 }
@@ -769,7 +782,7 @@ PyObject* py_subm_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
       throw;
     }
   }
-  return pair_of(conv_autograd(feats, weight, bias, m, m, pairs, true, V, dtype, std::move(out)), cache);
+  return pair_of(conv_autograd(feats, weight, bias, m, m, pairs, true, V, std::move(out)), cache);
   FGB_END
 }
 
@@ -796,7 +809,7 @@ PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (sparse) bwd = feats.requires_grad() && at::GradMode::is_enabled() ? bwd_maps(a[3]) : Maps{};
   Pairs pairs;
   if (weight.requires_grad()) pairs = pairs_of(a[3]);
-  return THPVariable_Wrap(conv_autograd(feats, weight, bias, m, bwd, pairs, !sparse, V, dtype, std::move(out)));
+  return THPVariable_Wrap(conv_autograd(feats, weight, bias, m, bwd, pairs, !sparse, V, std::move(out)));
   FGB_END
 }
 
@@ -1005,7 +1018,7 @@ PyObject* py_strided_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } else if (PyObject_SetAttr(cache, s_neighbor_map_bwd, Py_None) != 0) {
       throw PyError{};
     }
-    out = conv_autograd(feats, weight, bias, m, bwd, pairs, false, V, dtype, std::move(out));
+    out = conv_autograd(feats, weight, bias, m, bwd, pairs, false, V, std::move(out));
     PyObject* o = THPVariable_Wrap(out);
     PyObject* oc = o != nullptr ? THPVariable_Wrap(b.out_coords) : nullptr;
     t = oc != nullptr ? PyTuple_New(3) : nullptr;
@@ -1148,10 +1161,15 @@ PyObject* py_clear_mirror(PyObject*, PyObject* index) {
 }
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
-PyObject* py_init(PyObject*, PyObject* handle) {
+// (handle, config): the CUDA library's dlopen handle, the module with the settings
+PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   FGB_TRY
-  void* lib = PyLong_AsVoidPtr(handle);
+  TORCH_CHECK(n == 2, "init takes 2 arguments");
+  void* lib = PyLong_AsVoidPtr(a[0]);
   if (lib == nullptr) return nullptr;
+  Py_INCREF(a[1]);
+  Py_XDECREF(g_config);
+  g_config = a[1];
 #define X(f)                                                    \
   api.f = reinterpret_cast<decltype(api.f)>(dlsym(lib, #f));    \
   TORCH_CHECK(api.f != nullptr, "the CUDA library lacks " #f);
@@ -1163,7 +1181,7 @@ PyObject* py_init(PyObject*, PyObject* handle) {
 
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL
 PyMethodDef methods[] = {
-    {"init", py_init, METH_O, "bind the CUDA library (its dlopen handle)"},
+    {"init", FAST(py_init), "bind the CUDA library (its dlopen handle) and the settings"},
     {"subm_cache", FAST(py_subm_cache), "neighbour cache of a submanifold conv"},
     {"subm_conv", FAST(py_subm_conv), "submanifold conv"},
     {"conv", FAST(py_conv), "convolution on an existing cache"},
@@ -1202,6 +1220,7 @@ PyMODINIT_FUNC PyInit__fgb_torch(void) {
   s_m_block_order = PyUnicode_InternFromString("block_order");
   s_m_tile_masks_bwd = PyUnicode_InternFromString("tile_masks_bwd");
   s_m_block_order_bwd = PyUnicode_InternFromString("block_order_bwd");
+  s_allow_tf32 = PyUnicode_InternFromString("allow_tf32");
   s_tile_rows = PyLong_FromLong(128);
   s_empty_tuple = PyTuple_New(0);
   return PyModule_Create(&module);

@@ -187,3 +187,29 @@ def test_grid_sample_with_query_points_that_require_grad(feats_grad):
     assert out.requires_grad
     out.sum().backward()
     assert query.grad is None and (feats.grad is not None) == feats_grad
+
+
+@pytest.mark.parametrize("op", ["submanifold", "strided"])
+def test_backward_takes_the_fp32_setting_of_its_own_time(op):
+    """TF32 or accurate fp32 is decided when a pass runs: a backward pass after the switch is the other pass's, bit for
+    bit, and not this one's."""
+    from flexgemm_b200.kernels import config
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 32, 32, "float32", seed=2))
+    f, w = feats.requires_grad_(True), weight.requires_grad_(True)
+    assert config.allow_tf32
+
+    def grads(at_forward, at_backward):
+        try:
+            config.allow_tf32 = at_forward
+            if op == "submanifold":
+                out = spconv.sparse_submanifold_conv3d(f, coords, torch.Size(shape), w, bias)[0]
+            else:
+                out = spconv.sparse_conv3d(f, coords, torch.Size(shape), w, bias, stride=(2, 2, 2), padding=(1, 1, 1))[0]
+            config.allow_tf32 = at_backward
+            return torch.autograd.grad(out, (f, w), torch.randn(out.shape, generator=torch.Generator().manual_seed(1)).to(DEV))
+        finally:
+            config.allow_tf32 = True
+    tf32, exact = grads(True, True), grads(False, False)
+    for got, want, other in zip(grads(True, False) + grads(False, True), exact + tf32, tf32 + exact):
+        assert torch.equal(got, want) and not torch.equal(got, other)

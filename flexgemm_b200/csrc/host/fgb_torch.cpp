@@ -455,6 +455,18 @@ bool int_args(PyObject* seq, int k, int64_t* out) {
   return ok;
 }
 
+// 32-bit keys while a (N, C, W, H, D) grid has fewer than 2^32 cells, else 64-bit; 0 where those cannot tell its cells
+// apart either (utils.hashmap_key_bits, which raises for such a grid)
+int key_bits_of(const int64_t* shape) {
+  unsigned __int128 cells = 1;
+  for (int i : {0, 2, 3, 4}) {
+    if (shape[i] <= 0) return 32;  // refused by the call
+    cells *= static_cast<uint64_t>(shape[i]);
+    if (cells >> 64 != 0) return 0;
+  }
+  return cells >> 32 != 0 ? 64 : 32;
+}
+
 // ------------------------------------------------------------------ autograd
 PyObject *g_config, *s_allow_tf32;  // the module flexgemm_b200.kernels.config, and its setting
 
@@ -551,8 +563,7 @@ CacheBuild start_cache(const Tensor& coords, const int64_t* shape, const int64_t
   c.n = n;
   c.b = static_cast<int32_t>(shape[0]), c.w = static_cast<int32_t>(shape[2]), c.h = static_cast<int32_t>(shape[3]), c.d = static_cast<int32_t>(shape[4]);
   for (int i = 0; i < 3; ++i) c.k[i] = static_cast<int32_t>(ks[i]), c.dil[i] = static_cast<int32_t>(dil[i]);
-  const double volume = double(shape[0]) * double(shape[2]) * double(shape[3]) * double(shape[4]);
-  c.key_bits = volume < 4294967296.0 ? 32 : 64;
+  c.key_bits = key_bits_of(shape);
   c.slots = std::max<int64_t>({static_cast<int64_t>(ratio * static_cast<double>(n)), n, 1});
   c.scratch_bytes = check_bytes(api.fgb_subm_cache_scratch_bytes(&c), "fgb_subm_cache_scratch_bytes");
   const c10::DataPtr mem = scratch(c.scratch_bytes);
@@ -681,7 +692,9 @@ PyObject* py_subm_cache(PyObject*, PyObject* const* a, Py_ssize_t n) {
   TORCH_CHECK(n == 7, "subm_cache takes 7 arguments");
   const Tensor coords = tensor_arg(a[1]);
   int64_t shape[5], ks[3], dil[3];
-  if (!int_args(a[2], 5, shape) || !int_args(a[3], 3, ks) || !int_args(a[4], 3, dil) || !coords_ok(coords, ks)) Py_RETURN_NONE;
+  if (!int_args(a[2], 5, shape) || !int_args(a[3], 3, ks) || !int_args(a[4], 3, dil) || !coords_ok(coords, ks) ||
+      key_bits_of(shape) == 0)
+    Py_RETURN_NONE;
   const double ratio = PyFloat_AsDouble(a[5]);
   if (ratio == -1.0 && PyErr_Occurred()) return nullptr;
   const bool train = PyObject_IsTrue(a[6]) == 1;
@@ -758,7 +771,7 @@ PyObject* py_subm_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor coords = tensor_arg(a[2]);
     int64_t shape[5], ks[3] = {weight.size(1), weight.size(2), weight.size(3)}, dil[3];
     if (!int_args(a[3], 5, shape) || !int_args(a[7], 3, dil) || !coords_ok(coords, ks) || coords.device() != feats.device() ||
-        coords.size(0) != feats.size(0))
+        coords.size(0) != feats.size(0) || key_bits_of(shape) == 0)
       Py_RETURN_NONE;
     const double ratio = PyFloat_AsDouble(a[8]);
     if (ratio == -1.0 && PyErr_Occurred()) return nullptr;
@@ -974,7 +987,8 @@ PyObject* py_strided_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dtype = feats.defined() ? dtype_code(feats.scalar_type(), PyObject_IsTrue(a[9]) == 1) : -1;
   int64_t V = 0, shape[5], st[3], pad[3], dil[3];
   if (!conv_args_ok(feats, weight, bias, a[5], &V, dtype) || !rows_ok(coords) || coords.device() != feats.device() ||
-      coords.size(0) != feats.size(0) || !int_args(a[3], 5, shape) || !geometry_args(a[6], a[7], a[8], st, pad, dil))
+      coords.size(0) != feats.size(0) || !int_args(a[3], 5, shape) || !geometry_args(a[6], a[7], a[8], st, pad, dil) ||
+      key_bits_of(shape) == 0)
     Py_RETURN_NONE;
   const int64_t ks[3] = {weight.size(1), weight.size(2), weight.size(3)};
   c10::cuda::CUDAGuard guard(feats.device());
@@ -1097,8 +1111,8 @@ PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const bool want_grad = torch::autograd::compute_requires_grad(feats);
   const int64_t n = feats.size(0), C = feats.size(1), B = grid.size(0), L = grid.size(1), V = trilinear ? 8 : 1;
   const int64_t slots = std::max<int64_t>({static_cast<int64_t>(ratio * static_cast<double>(n)), n, 1});
-  const double volume = double(shape[0]) * double(shape[2]) * double(shape[3]) * double(shape[4]);
-  const int key_bits = volume < 4294967296.0 ? 32 : 64;
+  const int key_bits = key_bits_of(shape);
+  if (key_bits == 0) Py_RETURN_NONE;
   Tensor out, indices, weight;
   {
     at::AutoDispatchBelowADInplaceOrView below;

@@ -213,3 +213,20 @@ def test_backward_takes_the_fp32_setting_of_its_own_time(op):
     tf32, exact = grads(True, True), grads(False, False)
     for got, want, other in zip(grads(True, False) + grads(False, True), exact + tf32, tf32 + exact):
         assert torch.equal(got, want) and not torch.equal(got, other)
+
+
+def test_grids_that_no_key_can_hold_are_refused():
+    """2^64 cells and more: an error from every entry point, and 2^63 cells go through."""
+    from flexgemm_b200.ops import grid_sample, spconv
+    coords, feats, weight, bias, _ = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 16, 16, "float16", seed=2))
+    query = torch.rand(1, 50, 3, device=DEV) * 8
+    calls = [lambda s: spconv.sparse_submanifold_conv3d(feats, coords, s, weight, bias)[0], lambda s: grid_sample.grid_sample_3d(feats, coords, s, query),
+             lambda s: spconv.sparse_conv3d(feats, coords, s, weight, bias, stride=(2 ** 16,) * 3, padding=(1, 1, 1))[0]]
+    small = torch.Size((1, 16, 2 ** 21, 2 ** 21, 2 ** 21))
+    for extents in ((2 ** 22, 2 ** 21, 2 ** 21), (2 ** 31 - 1,) * 3):
+        for call in calls:
+            with pytest.raises(ValueError, match="too large"):
+                call(torch.Size((1, 16, *extents)))
+    for call in calls:
+        assert torch.isfinite(call(small)).all()
+    assert torch.equal(calls[0](small), calls[0](torch.Size((1, 16, 8, 8, 8))))

@@ -156,8 +156,8 @@ ZeroedWords zeroed_words(c10::cuda::CUDAStream stream, int64_t words) {
   return out;
 }
 
-// Mapped pinned words into which a cache build reports its pair count; returned to the free list after each build, so
-// there are as many as builds have ever run at the same time.
+// Mapped pinned words into which a build reports its counts; returned to the free list after each build, so there are as
+// many as builds have ever run at the same time.
 struct HostWords {
   volatile uint32_t* host = nullptr;
   uint32_t* dev = nullptr;
@@ -165,44 +165,92 @@ struct HostWords {
 };
 std::mutex g_words_mu;
 std::vector<HostWords> g_words_free;
+int64_t g_words_made = 0;
 constexpr int kHostWords = 16;  // per slot: FGB_HOST_WORDS, and a line of its own
 static_assert(FGB_HOST_WORDS <= kHostWords);
 
-HostWords take_host_words() {
-  std::lock_guard<std::mutex> lock(g_words_mu);
-  if (g_words_free.empty()) {
-    void *host = nullptr, *dev = nullptr;
-    constexpr int kSlots = 16;
-    C10_CUDA_CHECK(cudaHostAlloc(&host, kSlots * kHostWords * 4, cudaHostAllocMapped | cudaHostAllocPortable));
-    C10_CUDA_CHECK(cudaHostGetDevicePointer(&dev, host, 0));
-    memset(host, 0, kSlots * kHostWords * 4);
-    for (int i = 0; i < kSlots; ++i)
-      g_words_free.push_back({static_cast<volatile uint32_t*>(host) + i * kHostWords, static_cast<uint32_t*>(dev) + i * kHostWords, 0});
-  }
-  HostWords w = g_words_free.back();
-  g_words_free.pop_back();
-  ++w.seq;
-  return w;
-}
-void give_host_words(const HostWords& w) {
-  std::lock_guard<std::mutex> lock(g_words_mu);
-  g_words_free.push_back(w);
-}
-// waits until the stream's work has stored the use's sequence number
-void wait_host_words(const HostWords& w, cudaStream_t stream) {
-  for (uint64_t i = 1; w.host[FGB_HOST_SEQ] != w.seq; ++i) {
-#if defined(__x86_64__)
-    __builtin_ia32_pause();
-#endif
-    if ((i & 0xFFFu) == 0) {
-      const cudaError_t e = cudaStreamQuery(stream);
-      if (e == cudaErrorNotReady) continue;
-      C10_CUDA_CHECK(e);
-      if (w.host[FGB_HOST_SEQ] != w.seq) throw std::runtime_error("flexgemm_b200: the neighbour-map build ended without its pair count");
+// What a kernel has told the host.
+struct Told {
+  uint32_t count, status;
+};
+
+// A slot for the length of one build.  It goes back when the build has reported, and also when the call ends before:
+// at once if nothing that writes to it can have been queued, after the stream's work otherwise (and not at all where the
+// stream cannot be waited for).
+class HostSlot {
+ public:
+  HostSlot() = default;
+  HostSlot(HostSlot&& o) noexcept { std::swap(w_, o.w_), std::swap(stream_, o.stream_), std::swap(queued_, o.queued_); }
+  HostSlot(const HostSlot&) = delete;
+  HostSlot& operator=(const HostSlot&) = delete;
+  ~HostSlot() {
+    if (w_.host == nullptr) return;
+    if (queued_ && cudaStreamSynchronize(stream_) != cudaSuccess) {
+      cudaGetLastError();
+      return;
     }
+    give_back();
   }
-  std::atomic_thread_fence(std::memory_order_acquire);
-}
+  // for the next call into the library, whose stream is `stream`
+  void take(cudaStream_t stream, uint32_t** dev, uint32_t* seq) {
+    std::lock_guard<std::mutex> lock(g_words_mu);
+    if (g_words_free.empty()) {
+      void *host = nullptr, *mapped = nullptr;
+      constexpr int kSlots = 16;
+      C10_CUDA_CHECK(cudaHostAlloc(&host, kSlots * kHostWords * 4, cudaHostAllocMapped | cudaHostAllocPortable));
+      C10_CUDA_CHECK(cudaHostGetDevicePointer(&mapped, host, 0));
+      memset(host, 0, kSlots * kHostWords * 4);
+      for (int i = 0; i < kSlots; ++i)
+        g_words_free.push_back({static_cast<volatile uint32_t*>(host) + i * kHostWords, static_cast<uint32_t*>(mapped) + i * kHostWords, 0});
+      g_words_made += kSlots;
+    }
+    w_ = g_words_free.back();
+    g_words_free.pop_back();
+    stream_ = stream, queued_ = false;
+    *dev = w_.dev, *seq = ++w_.seq;
+  }
+  // the library is about to queue the kernels that write to the slot
+  void queued() { queued_ = true; }
+  // Waits until the stream's work has stored the sequence number; the GIL is released meanwhile.
+  Told take_back() {
+    std::exception_ptr failed;
+    Py_BEGIN_ALLOW_THREADS;
+    try {
+      wait();
+    } catch (...) {
+      failed = std::current_exception();
+    }
+    Py_END_ALLOW_THREADS;
+    if (failed) std::rethrow_exception(failed);
+    const Told r{w_.host[FGB_HOST_COUNT], w_.host[FGB_HOST_STATUS]};
+    give_back();
+    return r;
+  }
+
+ private:
+  void wait() const {
+    for (uint64_t i = 1; w_.host[FGB_HOST_SEQ] != w_.seq; ++i) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      if ((i & 0xFFFu) == 0) {
+        const cudaError_t e = cudaStreamQuery(stream_);
+        if (e == cudaErrorNotReady) continue;
+        C10_CUDA_CHECK(e);
+        if (w_.host[FGB_HOST_SEQ] != w_.seq) throw std::runtime_error("flexgemm_b200: the neighbour-map build ended without its pair count");
+      }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+  }
+  void give_back() {
+    std::lock_guard<std::mutex> lock(g_words_mu);
+    g_words_free.push_back(w_);
+    w_ = HostWords{};
+  }
+  HostWords w_;
+  cudaStream_t stream_ = nullptr;
+  bool queued_ = false;
+};
 
 // ------------------------------------------------------------------ tensors
 Tensor new_tensor(at::IntArrayRef size, at::ScalarType dtype, at::Device dev) { return at::detail::empty_cuda(size, dtype, dev, std::nullopt); }
@@ -535,7 +583,7 @@ bool conv_args_ok(const Tensor& feats, const Tensor& weight, const Tensor& bias,
 // ------------------------------------------------------------------ submanifold cache
 struct CacheBuild {
   Tensor nbr, gray, sorted_idx, masks, order, block_offsets, meta;
-  HostWords words;
+  HostSlot slot;
   int64_t n = 0;
   int V = 0;
   bool train = false;
@@ -576,40 +624,21 @@ CacheBuild start_cache(const Tensor& coords, const int64_t* shape, const int64_t
   c.block_offsets = static_cast<uint32_t*>(b.block_offsets.data_ptr());
   c.meta = static_cast<uint32_t*>(b.meta.data_ptr());
   if (train && n > 0) {
-    b.words = take_host_words();
-    c.host_words = b.words.dev, c.host_seq = b.words.seq;
+    b.slot.take(stream, &c.host_words, &c.host_seq);
   }
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
+  b.slot.queued();
   check(api.fgb_subm_cache_build(&c, stream), "fgb_subm_cache_build");
   g_launches += 8;
   return b;
 }
 
-// What a kernel has told the host: waits for it without holding the GIL and gives the words back.
-struct Told {
-  uint32_t count, status;
-};
-Told take_back(const HostWords& w, cudaStream_t stream) {
-  std::exception_ptr failed;
-  Py_BEGIN_ALLOW_THREADS;
-  try {
-    wait_host_words(w, stream);
-  } catch (...) {
-    failed = std::current_exception();
-  }
-  Py_END_ALLOW_THREADS;
-  if (failed) std::rethrow_exception(failed);
-  const Told r{w.host[FGB_HOST_COUNT], w.host[FGB_HOST_STATUS]};
-  give_host_words(w);
-  return r;
-}
-
 // waits for the pair count and queues the pair lists; the GIL is released while it waits
-Pairs finish_cache(const CacheBuild& b) {
+Pairs finish_cache(CacheBuild& b) {
   const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
   int64_t pairs = 0;
   if (b.n > 0) {
-    const Told got = take_back(b.words, stream);
+    const Told got = b.slot.take_back();
     pairs = got.count;
     if (got.status != 0u) throw_soft_error(static_cast<int>(got.status));
   }
@@ -700,7 +729,7 @@ PyObject* py_subm_cache(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool train = PyObject_IsTrue(a[6]) == 1;
   c10::cuda::CUDAGuard guard(coords.device());
   at::AutoDispatchBelowADInplaceOrView below;
-  const CacheBuild b = start_cache(coords, shape, ks, dil, ratio, train);
+  CacheBuild b = start_cache(coords, shape, ks, dil, ratio, train);
   Pairs p;
   if (train) p = finish_cache(b);
   PyObject* cache = new_cache(a[0]);
@@ -777,15 +806,10 @@ PyObject* py_subm_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (ratio == -1.0 && PyErr_Occurred()) return nullptr;
     const bool train = feats.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad());
     at::AutoDispatchBelowADInplaceOrView below;
-    const CacheBuild b = start_cache(coords, shape, ks, dil, ratio, train);
+    CacheBuild b = start_cache(coords, shape, ks, dil, ratio, train);
     m = Maps{b.nbr, b.sorted_idx, b.masks, b.order};
     // the convolution does not need the pair lists: it is queued before the host waits for their length
-    try {
-      out = run_fprop(feats, weight, bias, m, V, dtype);
-    } catch (...) {
-      if (train) finish_cache(b);  // the host words go back when the build has reported
-      throw;
-    }
+    out = run_fprop(feats, weight, bias, m, V, dtype);
     if (train) pairs = finish_cache(b);
     cache = new_cache(a[0]);
     try {
@@ -866,7 +890,7 @@ struct StridedBuild {
   fgb_strided_call c{};
   c10::DataPtr grid;
   Tensor out_coords, nbr, nbr_bwd, gray, gray_bwd, sorted_idx, sorted_bwd, masks, masks_bwd, order, order_bwd, block_offsets, meta;
-  HostWords words;
+  HostSlot slot;
   int V = 0;
 };
 
@@ -887,11 +911,12 @@ bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape,
   if (bytes <= 0) return false;
   b.grid = scratch(bytes);
   c.grid_mem = b.grid.get(), c.grid_bytes = bytes;
-  const HostWords w = take_host_words();
-  c.host_words = w.dev, c.host_seq = w.seq;
+  HostSlot slot;
+  slot.take(stream, &c.host_words, &c.host_seq);
+  slot.queued();
   check(api.fgb_strided_mark(&c, stream), "fgb_strided_mark");
   g_launches += 2;
-  c.n_out = take_back(w, stream).count;
+  c.n_out = slot.take_back().count;
   c.host_words = nullptr;
   b.out_coords = new_tensor({c.n_out, 4}, at::kInt, coords.device());
   if (c.n_out == 0) return coords_only;
@@ -925,20 +950,20 @@ void strided_maps(StridedBuild& b, at::Device dev, bool train) {
     c.sorted_idx_bwd = static_cast<int64_t*>(make(b.sorted_bwd, {n}, at::kLong));
     c.tile_masks_bwd = static_cast<uint32_t*>(make(b.masks_bwd, {tiles(n)}, at::kUInt32));
     c.block_order_bwd = static_cast<uint32_t*>(make(b.order_bwd, {(tiles(n) + 1) / 2}, at::kUInt32));
-    b.words = take_host_words();
-    c.host_words = b.words.dev, c.host_seq = b.words.seq;
+    b.slot.take(stream, &c.host_words, &c.host_seq);
   }
   c.scratch_bytes = check_bytes(api.fgb_strided_build_bytes(&c), "fgb_strided_build_bytes");
   const c10::DataPtr mem = scratch(c.scratch_bytes);
   c.scratch = mem.get();
   c.status = static_cast<int32_t*>(device_state(dev.index()).status.data_ptr());
+  b.slot.queued();
   check(api.fgb_strided_build(&c, stream), "fgb_strided_build");
   g_launches += train ? 11 : 8;
 }
 
-Pairs strided_pairs(const StridedBuild& b) {
+Pairs strided_pairs(StridedBuild& b) {
   const auto stream = c10::cuda::getCurrentCUDAStream(b.nbr.device().index());
-  const int64_t pairs = take_back(b.words, stream).count;
+  const int64_t pairs = b.slot.take_back().count;
   Pairs p;
   p.vs_i = new_tensor({pairs}, at::kUInt32, b.nbr.device());
   p.vs_o = new_tensor({pairs}, at::kUInt32, b.nbr.device());
@@ -1003,12 +1028,7 @@ PyObject* py_strided_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     strided_maps(b, feats.device(), train);
     m = Maps{b.nbr, b.sorted_idx, b.masks, b.order};
     if (train) bwd = Maps{b.nbr_bwd, b.sorted_bwd, b.masks_bwd, b.order_bwd};
-    try {
-      out = run_fprop(feats, weight, bias, m, V, dtype);
-    } catch (...) {
-      if (train) strided_pairs(b);
-      throw;
-    }
+    out = run_fprop(feats, weight, bias, m, V, dtype);
     if (train) pairs = strided_pairs(b);
   }
   PyObject* cache = new_cache(a[0]);
@@ -1173,6 +1193,11 @@ PyObject* py_clear_mirror(PyObject*, PyObject* index) {
   Py_RETURN_NONE;
   FGB_END
 }
+// (slots made, slots free)
+PyObject* py_host_slots(PyObject*, PyObject*) {
+  std::lock_guard<std::mutex> lock(g_words_mu);
+  return Py_BuildValue("Ln", static_cast<long long>(g_words_made), static_cast<Py_ssize_t>(g_words_free.size()));
+}
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
 // (handle, config): the CUDA library's dlopen handle, the module with the settings
@@ -1207,6 +1232,7 @@ PyMethodDef methods[] = {
     {"status_word", py_status_word, METH_O, "device status word"},
     {"poll", py_poll, METH_O, "raise a soft error that the device has reported"},
     {"clear_mirror", py_clear_mirror, METH_O, "forget the host copy of the status word"},
+    {"host_slots", py_host_slots, METH_NOARGS, "slots through which builds report: (made, free)"},
     {"launches", py_launches, METH_NOARGS, "kernels launched so far"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fgb_torch", "torch host code of flexgemm_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -230,3 +230,25 @@ def test_grids_that_no_key_can_hold_are_refused():
     for call in calls:
         assert torch.isfinite(call(small)).all()
     assert torch.equal(calls[0](small), calls[0](torch.Size((1, 16, 8, 8, 8))))
+
+
+def test_calls_that_fail_give_their_slot_back():
+    """Builds that the library refuses after a slot was taken (coordinates that are not 16-byte aligned)."""
+    from flexgemm_b200 import _native
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 16, 16, "float16", seed=2))
+    shape = torch.Size(shape)
+    weight.requires_grad_(True)
+    want = spconv.sparse_submanifold_conv3d(feats, coords, shape, weight, bias)[0]
+    spconv.sparse_conv3d(feats, coords, shape, weight, bias, stride=(2, 2, 2), padding=(1, 1, 1))
+    off = torch.empty(coords.numel() + 1, dtype=torch.int32, device=DEV)[1:].view(-1, 4)
+    off.copy_(coords)
+    made, free = _native.ext().host_slots()
+    assert made == free and made > 0
+    for _ in range(made + 1):
+        with pytest.raises(ValueError, match="align"):
+            spconv.sparse_submanifold_conv3d(feats, off, shape, weight, bias)
+        with pytest.raises(ValueError, match="align"):
+            spconv.sparse_conv3d(feats, off, shape, weight, bias, stride=(2, 2, 2), padding=(1, 1, 1))
+    assert _native.ext().host_slots() == (made, free)
+    assert torch.equal(spconv.sparse_submanifold_conv3d(feats, coords, shape, weight, bias)[0], want)

@@ -52,14 +52,18 @@ __device__ __forceinline__ void for_targets(const int4 c, const StridedGeom& g, 
   }
 }
 
-__global__ void __launch_bounds__(256) mark_cells_kernel(const int4* __restrict__ coords, uint32_t n, StridedGeom g, uint32_t* __restrict__ bits) {
+// *outside = 1 when a row's batch index has no place in the grid (the hash path takes such rows as they are)
+__global__ void __launch_bounds__(256) mark_cells_kernel(const int4* __restrict__ coords, uint32_t n, StridedGeom g, uint32_t* __restrict__ bits,
+                                                         uint32_t* outside) {
   chain_release();
   chain_wait();
   const uint32_t i = blockIdx.x * 256u + threadIdx.x;
   if (i >= n) return;
   // consecutive targets often lie in one word: they are collected and set together
   uint32_t word = kInvalid, mask = 0;
-  for_targets(__ldg(&coords[i]), g, [&](int, uint32_t cell) {
+  const int4 c = __ldg(&coords[i]);
+  if (static_cast<unsigned>(c.x) >= static_cast<unsigned>(g.B)) *outside = 1u;
+  for_targets(c, g, [&](int, uint32_t cell) {
     const uint32_t w = cell >> 5, b = 1u << (cell & 31);
     if (w != word) {
       if (mask) atomicOr(&bits[word], mask);
@@ -111,7 +115,8 @@ __device__ __forceinline__ uint32_t load_words(const uint32_t* bits, uint32_t fi
 // cta_base[b] = set bits of CTA b's words; the CTA that ends last turns them into exclusive sums and tells the host the
 // total
 __global__ void __launch_bounds__(kRankThreads) count_cells_kernel(const uint32_t* __restrict__ bits, uint32_t* cta_base,
-                                                                   uint32_t* done, uint32_t* host_words, uint32_t host_seq) {
+                                                                   uint32_t* done, const uint32_t* outside, uint32_t* host_words,
+                                                                   uint32_t host_seq) {
   __shared__ uint32_t s_warp[32];
   __shared__ bool s_last;
   chain_release();
@@ -143,7 +148,7 @@ __global__ void __launch_bounds__(kRankThreads) count_cells_kernel(const uint32_
     }
     carry += total;
   }
-  if (threadIdx.x == 0) tell_host(host_words, host_seq, carry, 0u, 0u);
+  if (threadIdx.x == 0) tell_host(host_words, host_seq, carry, 0u, __ldcg(outside));
 }
 
 // rows of the marked cells, and the row of the first cell of every word that has one
@@ -309,12 +314,13 @@ extern "C" int fgb_strided_mark(const fgb_strided_call* c, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* mem = static_cast<char*>(c->grid_mem);
   uint32_t* bits = reinterpret_cast<uint32_t*>(mem);
+  uint32_t* done = reinterpret_cast<uint32_t*>(mem + m.done_off);  // [0] count of finished CTAs [1] rows outside the grid's batches
   LaunchErrors chain;
   chain.add(cudaMemsetAsync(mem, 0, m.zero_bytes, s));
   chain.add(launch_chained(mark_cells_kernel, dim3(static_cast<unsigned>(ceil_div(c->n, 256))), dim3(256), 0, s,
-                           reinterpret_cast<const int4*>(c->coords), static_cast<uint32_t>(c->n), g, bits));
+                           reinterpret_cast<const int4*>(c->coords), static_cast<uint32_t>(c->n), g, bits, done + 1));
   chain.add(launch_chained(count_cells_kernel, dim3(m.ctas), dim3(kRankThreads), 0, s, static_cast<const uint32_t*>(bits),
-                           reinterpret_cast<uint32_t*>(mem + m.base_off), reinterpret_cast<uint32_t*>(mem + m.done_off), c->host_words, c->host_seq));
+                           reinterpret_cast<uint32_t*>(mem + m.base_off), done, static_cast<const uint32_t*>(done + 1), c->host_words, c->host_seq));
   return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
 }
 

@@ -916,7 +916,9 @@ bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape,
   slot.queued();
   check(api.fgb_strided_mark(&c, stream), "fgb_strided_mark");
   g_launches += 2;
-  c.n_out = slot.take_back().count;
+  const Told got = slot.take_back();
+  if (got.status != 0u) return false;  // rows of a batch beyond the shape's: the bits have no place for them
+  c.n_out = got.count;
   c.host_words = nullptr;
   b.out_coords = new_tensor({c.n_out, 4}, at::kInt, coords.device());
   if (c.n_out == 0) return coords_only;

@@ -633,7 +633,9 @@ int fgb_subm_cache_build(const fgb_map_call* call, void* stream);
  *                           too large or too empty for one bit per cell (the calls
  *                           of the generic conv above then do the work);
  *   fgb_strided_mark        marks and counts the cells; host_words (a host slot,
- *                           may be null) receives the count;
+ *                           may be null) receives the count, and 1 as status when
+ *                           some row's batch index is not in 0 .. b - 1 (such rows
+ *                           mark nothing: the generic calls are the way then);
  *   fgb_strided_build       with n_out = that count: out_coords and, when
  *                           neighbor_map is not null, both maps (the backward one
  *                           when neighbor_map_bwd is not null), codes, row orders,

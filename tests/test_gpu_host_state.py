@@ -252,3 +252,23 @@ def test_calls_that_fail_give_their_slot_back():
             spconv.sparse_conv3d(feats, off, shape, weight, bias, stride=(2, 2, 2), padding=(1, 1, 1))
     assert _native.ext().host_slots() == (made, free)
     assert torch.equal(spconv.sparse_submanifold_conv3d(feats, coords, shape, weight, bias)[0], want)
+
+
+def test_strided_rows_of_a_batch_beyond_the_shape():
+    """The hash path takes every batch index, so the bit grid, which has no place for one beyond the shape's, leaves the
+    call to it: no output row is lost."""
+    from flexgemm_b200.ops import spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(9, 16, 16, "float32", seed=2, batch=3))
+    geom = dict(stride=(2, 2, 2), padding=(1, 1, 1))
+    outs = []
+    for batches in (3, 2):
+        w = weight.detach().requires_grad_(True)
+        out, oc, _ = spconv.sparse_conv3d(feats, coords, torch.Size((batches, *shape[1:])), w, bias, **geom)
+        (gw,) = torch.autograd.grad(out.sum(), w)
+        only = spconv.SparseConv3dFunction._get_output_coords(coords, torch.Size((batches, *shape[1:])), (3, 3, 3), (2, 2, 2), (1, 1, 1), (1, 1, 1))
+        key, also = (((c[:, 0].long() * 64 + c[:, 1]) * 64 + c[:, 2]) * 64 + c[:, 3] for c in (oc, only))
+        assert torch.equal(key.sort().values, also.sort().values)   # the order of such rows is not fixed
+        outs.append((key.sort().values, out.detach()[key.argsort()], gw))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    # the pairs of an offset are summed in row order, which differs: fp32 sums of TF32 products
+    assert (outs[0][2] - outs[1][2]).abs().max() <= 1e-5 * outs[0][2].abs().max() * len(key) ** 0.5

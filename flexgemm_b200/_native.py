@@ -1,6 +1,7 @@
 """The torch host module (``csrc/host/fgb_torch.cpp``): whole forward and backward
 passes in one native call.  There is no fallback for a missing file: loading
 raises and every op fails, as with the CUDA library it drives."""
+import ctypes
 import importlib.machinery
 import importlib.util
 import os
@@ -22,6 +23,6 @@ def ext():
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         from .kernels import config
-        mod.init(_cabi.lib()._handle, config)
+        mod.init(_cabi.lib()._handle, ctypes.addressof(config._native_tf32))
         _mod = mod
     return _mod

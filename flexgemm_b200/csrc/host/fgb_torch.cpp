@@ -516,20 +516,9 @@ int key_bits_of(const int64_t* shape) {
 }
 
 // ------------------------------------------------------------------ autograd
-PyObject *g_config, *s_allow_tf32;  // the module flexgemm_b200.kernels.config, and its setting
-
-// Element type of a backward pass.  TF32 or accurate fp32 is what the setting says when the pass runs.
-int backward_dtype(at::ScalarType t) {
-  if (t != at::kFloat) return dtype_code(t, false);
-  const PyGILState_STATE gil = PyGILState_Ensure();
-  PyObject* v = PyObject_GetAttr(g_config, s_allow_tf32);
-  const int on = v != nullptr ? PyObject_IsTrue(v) : -1;
-  Py_XDECREF(v);
-  if (on < 0) PyErr_Clear();
-  PyGILState_Release(gil);
-  if (on < 0) throw std::runtime_error("flexgemm_b200.kernels.config.allow_tf32 is not a truth value");
-  return dtype_code(t, on == 1);
-}
+// The byte that flexgemm_b200.kernels.config keeps equal to its allow_tf32: a backward pass reads the setting when it runs,
+// in a thread that does not hold the GIL (taking it cost a small layer's backward pass a microsecond and a half).
+const volatile char* g_allow_tf32 = nullptr;
 
 struct ConvBackward : public torch::autograd::Node {
   torch::autograd::SavedVariable feats_, weight_;
@@ -551,7 +540,7 @@ struct ConvBackward : public torch::autograd::Node {
     if ((need_w && !pairs.vs_i.defined()) || (need_x && !bwd.nbr.defined()))
       throw torch::AttributeError(std::string("the neighbor cache was built for inference: it has no ") +
                                   (need_w ? "valid_signal_i" : "neighbor_map_bwd"));
-    const int dtype = backward_dtype(feats.scalar_type());
+    const int dtype = dtype_code(feats.scalar_type(), *g_allow_tf32 != 0);
     at::AutoDispatchBelowADInplaceOrView below;
     Grads g = run_backward(grads[0], feats, weight, bwd, pairs, mirror, V, dtype, need_x, need_w, need_b);
     out[0] = std::move(g.feats), out[1] = std::move(g.weight), out[2] = std::move(g.bias);
@@ -1202,15 +1191,14 @@ PyObject* py_host_slots(PyObject*, PyObject*) {
 }
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
-// (handle, config): the CUDA library's dlopen handle, the module with the settings
+// (handle, address): the CUDA library's dlopen handle, the byte of allow_tf32
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   FGB_TRY
   TORCH_CHECK(n == 2, "init takes 2 arguments");
   void* lib = PyLong_AsVoidPtr(a[0]);
   if (lib == nullptr) return nullptr;
-  Py_INCREF(a[1]);
-  Py_XDECREF(g_config);
-  g_config = a[1];
+  g_allow_tf32 = static_cast<const char*>(PyLong_AsVoidPtr(a[1]));
+  if (g_allow_tf32 == nullptr) return nullptr;
 #define X(f)                                                    \
   api.f = reinterpret_cast<decltype(api.f)>(dlsym(lib, #f));    \
   TORCH_CHECK(api.f != nullptr, "the CUDA library lacks " #f);
@@ -1262,7 +1250,6 @@ PyMODINIT_FUNC PyInit__fgb_torch(void) {
   s_m_block_order = PyUnicode_InternFromString("block_order");
   s_m_tile_masks_bwd = PyUnicode_InternFromString("tile_masks_bwd");
   s_m_block_order_bwd = PyUnicode_InternFromString("block_order_bwd");
-  s_allow_tf32 = PyUnicode_InternFromString("allow_tf32");
   s_tile_rows = PyLong_FromLong(128);
   s_empty_tuple = PyTuple_New(0);
   return PyModule_Create(&module);

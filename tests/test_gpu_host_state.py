@@ -194,6 +194,7 @@ def test_backward_takes_the_fp32_setting_of_its_own_time(op):
     """TF32 or accurate fp32 is decided when a pass runs: a backward pass after the switch is the other pass's, bit for
     bit, and not this one's."""
     from flexgemm_b200.kernels import config
+    from flexgemm_b200.kernels.triton.spconv import config as forwarded
     from flexgemm_b200.ops import spconv
     coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 32, 32, "float32", seed=2))
     f, w = feats.requires_grad_(True), weight.requires_grad_(True)
@@ -206,7 +207,7 @@ def test_backward_takes_the_fp32_setting_of_its_own_time(op):
                 out = spconv.sparse_submanifold_conv3d(f, coords, torch.Size(shape), w, bias)[0]
             else:
                 out = spconv.sparse_conv3d(f, coords, torch.Size(shape), w, bias, stride=(2, 2, 2), padding=(1, 1, 1))[0]
-            config.allow_tf32 = at_backward
+            forwarded.allow_tf32 = at_backward
             return torch.autograd.grad(out, (f, w), torch.randn(out.shape, generator=torch.Generator().manual_seed(1)).to(DEV))
         finally:
             config.allow_tf32 = True

@@ -73,6 +73,7 @@ _PROTOTYPES = {
     "fgb_grid_sample_fused": (c_int, [_P, c_int64, _P, _P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int64, c_int, _P,
                                       _P, _P, _P, _P]),
     "fgb_indice_weighted_sum_grad_bytes": (c_int64, [c_int64, c_int64, c_int]),
+    "fgb_indice_weighted_sum_grad_full_bytes": (c_int64, [c_int64, c_int64, c_int, c_int, c_int]),
     "fgb_indice_weighted_sum_grad": (c_int, [_P, _P, _P, _P, c_int64, c_int64, c_int, c_int, c_int, _P, c_int64, _P]),
     "fgb_sparse_out_grid": (c_int, [c_int] * 15 + [_P, _P, _P]),
     "fgb_sparse_out_coords_collect": (c_int, [_P, c_int64] + [c_int] * 15 + [_P, c_int64, c_int, _P, _P, _P, _P]),

@@ -328,10 +328,22 @@ __global__ void __launch_bounds__(256) group_count_kernel(const uint32_t* __rest
     if (row != kInvalid) atomicAdd(&count[row], 1u);
   }
 }
-// start[r] = where the entries of voxel r go (the fill moves it on to their end).  The groups of 1024 consecutive voxels stand together, in order; such
-// blocks take their places as they come (one atomic each), which no result depends on.
+// Lists longer than `limit` entries are cut into pieces that warps take on their own, so that a voxel that is hit far more
+// often than the others (queries padded with one repeated point, a cluster of them) does not leave the sum to one warp.
+struct CutLists {
+  uint32_t limit, piece;  // limit = ~0: nothing is cut
+  uint32_t* total;        // zeroed: pieces listed
+  uint2* pieces;          // (row, first piece of the row)
+  uint32_t* done;         // pieces of the row that are summed, at the row's first piece
+  float* slab;            // [pieces, C] their sums
+};
+// At most 1024: the warp that ends last adds a row's parts up.
+__host__ __device__ __forceinline__ uint32_t pieces_of(uint32_t len, uint32_t piece) { return min((len - 1u) / piece + 1u, 1024u); }
+
+// start[r] = where the entries of voxel r go (the fill moves it on to their end).  The groups of 1024 consecutive voxels
+// stand together, in order; such blocks take their places as they come (one atomic each), which no result depends on.
 __global__ void __launch_bounds__(1024) group_place_kernel(const uint32_t* __restrict__ count, uint32_t n, uint32_t* __restrict__ start,
-                                                           uint32_t* __restrict__ total) {
+                                                           uint32_t* __restrict__ total, CutLists cut) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_base;
   chain_release();
@@ -359,6 +371,17 @@ __global__ void __launch_bounds__(1024) group_place_kernel(const uint32_t* __res
   }
   __syncthreads();
   if (i < n) start[i] = s_base + (wi ? s_warp[wi - 1] : 0u) + inc - x;
+  const uint32_t k = x > cut.limit ? pieces_of(x, cut.piece) : 0u;
+  uint32_t first = 0;
+  if (k != 0u) {
+    first = atomicAdd(cut.total, k);
+    cut.done[first] = 0u;
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, k != 0u); todo != 0u; todo &= todo - 1u) {
+    const int l = __ffs(todo) - 1;
+    const uint32_t row = __shfl_sync(0xffffffffu, i, l), at = __shfl_sync(0xffffffffu, first, l), many = __shfl_sync(0xffffffffu, k, l);
+    for (uint32_t j = lane; j < many; j += 32u) cut.pieces[at + j] = make_uint2(row, at);
+  }
 }
 __global__ void __launch_bounds__(256) group_fill_kernel(const uint32_t* __restrict__ indices, const float* __restrict__ weight, uint32_t entries,
                                                          int V, uint32_t* __restrict__ start, uint2* __restrict__ grouped) {
@@ -371,14 +394,82 @@ __global__ void __launch_bounds__(256) group_fill_kernel(const uint32_t* __restr
     grouped[atomicAdd(&start[row], 1u)] = make_uint2(static_cast<uint32_t>(e / V), __float_as_uint(w));
   }
 }
+// Sum over the entries base, base + step, ... (32 at a time) of a list, for the row's packs c0 + lane % kGroup: the lane
+// groups of the warp take the entries in turn, and every lane ends with the whole sum.  Whole warps call it.
+template <typename T, int kVec, int kGroup>
+__device__ __forceinline__ void warp_sum(const T* __restrict__ grad_out, const uint2* list, uint32_t base, uint32_t step, uint32_t len, int C, int c,
+                                         float (&acc)[kVec]) {
+  using Raw = typename Pack<T, kVec>::Raw;
+  constexpr int kSide = 32 / kGroup;
+  const int lane = threadIdx.x & 31, side = lane / kGroup;
+  const bool col = c < C / kVec;
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) acc[i] = 0.f;
+  for (; base < len; base += step) {
+    const uint32_t here = min(32u, len - base);
+    const uint2 e = lane < here ? __ldg(&list[base + lane]) : make_uint2(0, 0);
+#pragma unroll 4
+    for (uint32_t j0 = 0; j0 < here; j0 += kSide) {
+      const uint32_t j = j0 + side;
+      const uint32_t m = __shfl_sync(0xffffffffu, e.x, j & 31);
+      const float w = __uint_as_float(__shfl_sync(0xffffffffu, e.y, j & 31));
+      if (j < here && col) fma_pack<T, kVec>(acc, __ldg(reinterpret_cast<const Raw*>(grad_out + size_t(m) * C) + c), w);
+    }
+  }
+#pragma unroll
+  for (int d = kGroup; d < 32; d <<= 1)
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], d);
+}
+
+// One piece of a list that is cut, by one warp; the warp that ends a row's last piece adds the parts up, in their order.
+template <typename T, int kVec, int kGroup>
+__device__ __forceinline__ void sum_piece(const T* __restrict__ grad_out, const uint2* __restrict__ grouped, const uint32_t* __restrict__ end,
+                                          const uint32_t* __restrict__ count, int C, const CutLists& cut, uint32_t p, T* __restrict__ grad_feats) {
+  const int lane = threadIdx.x & 31, nv = C / kVec;
+  const uint2 d = __ldg(&cut.pieces[p]);
+  const uint32_t len = __ldg(&count[d.x]), many = pieces_of(len, cut.piece), j = p - d.y;
+  const uint32_t from = static_cast<uint32_t>(uint64_t(len) * j / many), to = static_cast<uint32_t>(uint64_t(len) * (j + 1u) / many);
+  const uint2* list = grouped + (__ldg(&end[d.x]) - len);
+  float acc[kVec];
+  for (int c0 = 0; c0 < nv; c0 += kGroup) {
+    const int c = c0 + lane % kGroup;
+    warp_sum<T, kVec, kGroup>(grad_out, list, from, 32u, to, C, c, acc);
+    if (lane < kGroup && c < nv)
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) __stcg(&cut.slab[size_t(p) * C + c * kVec + i], acc[i]);
+  }
+  __threadfence();
+  __syncwarp();
+  uint32_t before = 0;
+  if (lane == 0) before = atomicAdd(&cut.done[d.y], 1u);
+  if (__shfl_sync(0xffffffffu, before, 0) != many - 1u) return;
+  __threadfence();
+  const float4* parts = reinterpret_cast<const float4*>(cut.slab + size_t(d.y) * C);
+  for (int c = lane; c < C / 4; c += 32) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (uint32_t q = 0; q < many; ++q) {
+      const float4 x = __ldcg(&parts[size_t(q) * (C / 4) + c]);
+      sum[0] += x.x, sum[1] += x.y, sum[2] += x.z, sum[3] += x.w;
+    }
+    reinterpret_cast<typename Pack<T, 4>::Raw*>(grad_feats + size_t(d.x) * C)[c] = round_pack<T, 4>(sum);
+  }
+}
+
 // kGroup lanes cover a voxel's row (or 32 packs of it at a time).  kWarps = 0: every group has a voxel of its own, 32 /
 // kGroup of them per warp -- with narrow rows and few entries per voxel a warp per voxel spends its life on three
 // dependent loads (RES=467, C=16, 2.4 entries per voxel: most of 275 us).  kWarps = 1: a warp per voxel, its groups take
-// the entries in turn.  kWarps = 8: the warps of a CTA share a voxel, where voxels have many entries.
+// the entries in turn.  kWarps = 8: the warps of a CTA share a voxel, where voxels have many entries.  The first
+// `piece_ctas` CTAs take the pieces of the lists that are cut.
+// Cut lists, 10^6 points on 165 k voxels, us without and with: every tenth point the same one, C = 64 fp16 14256 -> 470,
+// C = 256 50852 -> 905; all of them the same, C = 64 166387 -> 2484; none repeated 383 -> 381 and 843 -> 840 (RES=256
+// shell, forward and backward, C = 16 to 512: 0.1 to 0.4 % more).  The register limits keep the walkers at the occupancy
+// that they have without the pieces' code: at 6 CTAs per SM instead of 8 the same passes took 4 to 6 % longer.
 template <typename T, int kVec, int kWarps, int kGroup>
-__global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ grad_out, const uint2* __restrict__ grouped,
+__global__ void __launch_bounds__(256, kWarps == 8 ? 5 : kWarps == 0 && sizeof(T) == 2 && kVec == 8 ? 6 : 8) group_sum_kernel(const T* __restrict__ grad_out, const uint2* __restrict__ grouped,
                                                         const uint32_t* __restrict__ end, const uint32_t* __restrict__ count, uint32_t n, int C,
-                                                        T* __restrict__ grad_feats) {
+                                                        T* __restrict__ grad_feats, CutLists cut, uint32_t piece_ctas) {
   using Raw = typename Pack<T, kVec>::Raw;
   constexpr int kSide = 32 / kGroup;
   __shared__ float s_acc[kWarps > 1 ? kWarps : 1][kWarps > 1 ? 32 * kVec : 1];
@@ -387,10 +478,18 @@ __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ gr
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const int nv = C / kVec;
   const int side = lane / kGroup;
+  if (blockIdx.x < piece_ctas) {
+    const uint32_t total = *cut.total;
+    for (uint32_t p = blockIdx.x * 8u + wi; p < total; p += piece_ctas * 8u)
+      sum_piece<T, kVec, kGroup>(grad_out, grouped, end, count, C, cut, p, grad_feats);
+    return;
+  }
+  const uint32_t block = blockIdx.x - piece_ctas;
   if constexpr (kWarps == 0) {
-    const uint32_t row = (blockIdx.x * 8u + wi) * kSide + side;
+    const uint32_t row = (block * 8u + wi) * kSide + side;
     if (row >= n) return;
     const uint32_t len = __ldg(&count[row]);
+    if (len > cut.limit) return;
     const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
     for (int c = lane % kGroup; c < nv; c += kGroup) {
       float acc[kVec];
@@ -414,47 +513,32 @@ __global__ void __launch_bounds__(256) group_sum_kernel(const T* __restrict__ gr
       reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
     }
   } else {
-  const uint32_t row = kWarps > 1 ? blockIdx.x : blockIdx.x * 8u + wi;
-  if (row >= n) return;  // whole warps; with kWarps > 1 whole CTAs
-  const uint32_t len = __ldg(&count[row]);
-  const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
-  const int share = kWarps > 1 ? wi : 0;
-  for (int c0 = 0; c0 < nv; c0 += kGroup) {
-    const int c = c0 + lane % kGroup;
-    float acc[kVec];
+    const uint32_t row = kWarps > 1 ? block : block * 8u + wi;
+    if (row >= n) return;  // whole warps; with kWarps > 1 whole CTAs
+    const uint32_t len = __ldg(&count[row]);
+    if (len > cut.limit) return;
+    const uint2* list = grouped + (len ? __ldg(&end[row]) - len : 0u);
+    const int share = kWarps > 1 ? wi : 0;
+    for (int c0 = 0; c0 < nv; c0 += kGroup) {
+      const int c = c0 + lane % kGroup;
+      float acc[kVec];
+      warp_sum<T, kVec, kGroup>(grad_out, list, share * 32u, kWarps * 32u, len, C, c, acc);
+      if constexpr (kWarps > 1) {
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) acc[i] = 0.f;
-    for (uint32_t base = share * 32u; base < len; base += kWarps * 32u) {
-      const uint32_t here = min(32u, len - base);
-      const uint2 e = lane < here ? __ldg(&list[base + lane]) : make_uint2(0, 0);
-#pragma unroll 4
-      for (uint32_t j0 = 0; j0 < here; j0 += kSide) {
-        const uint32_t j = j0 + side;
-        const uint32_t m = __shfl_sync(0xffffffffu, e.x, j & 31);
-        const float w = __uint_as_float(__shfl_sync(0xffffffffu, e.y, j & 31));
-        if (j < here && c < nv) fma_pack<T, kVec>(acc, __ldg(reinterpret_cast<const Raw*>(grad_out + size_t(m) * C) + c), w);
-      }
-    }
+        for (int i = 0; i < kVec; ++i) s_acc[wi][lane * kVec + i] = acc[i];
+        __syncthreads();
+        if (wi == 0) {
 #pragma unroll
-    for (int d = kGroup; d < 32; d <<= 1)
+          for (int i = 0; i < kVec; ++i) {
+            acc[i] = 0.f;
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], d);
-    if constexpr (kWarps > 1) {
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) s_acc[wi][lane * kVec + i] = acc[i];
-      __syncthreads();
-      if (wi == 0) {
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) {
-          acc[i] = 0.f;
-#pragma unroll
-          for (int k = 0; k < kWarps; ++k) acc[i] += s_acc[k][lane * kVec + i];
+            for (int k = 0; k < kWarps; ++k) acc[i] += s_acc[k][lane * kVec + i];
+          }
         }
+        __syncthreads();
       }
-      __syncthreads();
+      if ((kWarps == 1 || wi == 0) && side == 0 && c < nv) reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
     }
-    if ((kWarps == 1 || wi == 0) && side == 0 && c < nv) reinterpret_cast<Raw*>(grad_feats + size_t(row) * C)[c] = round_pack<T, kVec>(acc);
-  }
   }
 }
 
@@ -483,26 +567,36 @@ static cudaError_t launch_sample(int key_bits, bool nearest, const void* feats, 
                  : launch_sample<T, kVec, 64, false>(feats, query, points, L, g, table, slots, C, out, neighbor, weight, s);
 }
 
-template <typename T, int kVec>
-static cudaError_t launch_group_sum(uint32_t entries, const void* grad_out, const uint2* grouped, const uint32_t* start, const uint32_t* count,
-                                    uint32_t n, int C, void* grad_feats, cudaStream_t s) {
-  const int nv = C / kVec;
+// How the voxels' lists are summed, for rows of nv packs, and where lists are cut.  A piece takes a warp about as long as a
+// list just below the limit takes whoever walks that (20 to 40 us), so a cut list does not end after the rest.
+struct GroupPlan {
+  int warps, lanes;
+  uint32_t limit, piece;
+};
+static GroupPlan group_plan(uint32_t entries, uint32_t n, int nv) {
   const uint32_t mean = entries / n;  // places of entries, of which a part is used
-  void (*kernel)(const T*, const uint2*, const uint32_t*, const uint32_t*, uint32_t, int, T*);
-  unsigned grid = static_cast<unsigned>(ceil_div(n, 8));
-  if (mean >= 128) {  // few warps would walk long lists otherwise
-    kernel = nv <= 8 ? group_sum_kernel<T, kVec, 8, 8> : nv <= 16 ? group_sum_kernel<T, kVec, 8, 16> : group_sum_kernel<T, kVec, 8, 32>;
-    grid = n;
-  } else if (nv <= 16 && mean < 32) {
-    const int lanes = nv <= 2 ? 2 : nv <= 4 ? 4 : nv <= 8 ? 8 : 16;
-    kernel = lanes == 2 ? group_sum_kernel<T, kVec, 0, 2> : lanes == 4 ? group_sum_kernel<T, kVec, 0, 4>
-             : lanes == 8 ? group_sum_kernel<T, kVec, 0, 8> : group_sum_kernel<T, kVec, 0, 16>;
-    grid = static_cast<unsigned>(ceil_div(n, 8 * (32 / lanes)));
+  if (mean >= 128) return {8, group_lanes(nv), 8192, 1024};  // few warps would walk long lists otherwise
+  if (nv <= 16 && mean < 32) return {0, nv <= 2 ? 2 : nv <= 4 ? 4 : nv <= 8 ? 8 : 16, 256, 128};
+  return {1, group_lanes(nv), 1024, 512};
+}
+
+template <typename T, int kVec>
+static cudaError_t launch_group_sum(const GroupPlan& g, const void* grad_out, const uint2* grouped, const uint32_t* start, const uint32_t* count,
+                                    uint32_t n, int C, void* grad_feats, const CutLists& cut, uint32_t piece_ctas, cudaStream_t s) {
+  void (*kernel)(const T*, const uint2*, const uint32_t*, const uint32_t*, uint32_t, int, T*, CutLists, uint32_t);
+  int64_t rows_ctas = ceil_div(n, 8);
+  if (g.warps == 8) {
+    kernel = g.lanes == 8 ? group_sum_kernel<T, kVec, 8, 8> : g.lanes == 16 ? group_sum_kernel<T, kVec, 8, 16> : group_sum_kernel<T, kVec, 8, 32>;
+    rows_ctas = n;
+  } else if (g.warps == 0) {
+    kernel = g.lanes == 2 ? group_sum_kernel<T, kVec, 0, 2> : g.lanes == 4 ? group_sum_kernel<T, kVec, 0, 4>
+             : g.lanes == 8 ? group_sum_kernel<T, kVec, 0, 8> : group_sum_kernel<T, kVec, 0, 16>;
+    rows_ctas = ceil_div(n, 8 * (32 / g.lanes));
   } else {
-    kernel = nv <= 8 ? group_sum_kernel<T, kVec, 1, 8> : nv <= 16 ? group_sum_kernel<T, kVec, 1, 16> : group_sum_kernel<T, kVec, 1, 32>;
+    kernel = g.lanes == 8 ? group_sum_kernel<T, kVec, 1, 8> : g.lanes == 16 ? group_sum_kernel<T, kVec, 1, 16> : group_sum_kernel<T, kVec, 1, 32>;
   }
-  return launch_chained(kernel, dim3(grid), dim3(256), 0, s, static_cast<const T*>(grad_out), grouped, start, count, n, C,
-                        static_cast<T*>(grad_feats));
+  return launch_chained(kernel, dim3(static_cast<unsigned>(piece_ctas + rows_ctas)), dim3(256), 0, s, static_cast<const T*>(grad_out), grouped, start,
+                        count, n, C, static_cast<T*>(grad_feats), cut, piece_ctas);
 }
 
 struct GroupScratch {
@@ -511,13 +605,29 @@ struct GroupScratch {
 static GroupScratch group_scratch(int64_t entries, int64_t n) {
   GroupScratch g;
   g.count_off = 0;
-  g.total_off = align256(n * 4);
+  g.total_off = align256(n * 4);  // [0] places handed out [1] pieces listed
   g.zero_bytes = g.total_off + 256;
   g.start_off = g.zero_bytes;
   g.grouped_off = g.start_off + align256(n * 4);
   g.bytes = g.grouped_off + align256(entries * 8);
   return g;
 }
+// what cutting needs behind that
+struct CutScratch {
+  int64_t pieces;  // at most; 0 where no list can exceed the limit
+  size_t pieces_off, done_off, slab_off, end;
+};
+static CutScratch cut_scratch(const GroupScratch& g, const GroupPlan& plan, int64_t entries, int C) {
+  CutScratch c{};
+  // a list of len > limit entries has at most len / piece + 1 pieces, and there are fewer than entries / limit such lists
+  c.pieces = entries > plan.limit ? entries / plan.piece + entries / plan.limit + 1 : 0;
+  c.pieces_off = g.bytes;
+  c.done_off = c.pieces_off + align256(c.pieces * 8);
+  c.slab_off = c.done_off + align256(c.pieces * 4);
+  c.end = c.slab_off + align256(c.pieces * C * 4);
+  return c;
+}
+static int pack_width(int C, int dtype) { return elem_bytes(dtype) == 2 && C % 8 == 0 ? 8 : 4; }
 
 static int check_table(const void* table, int64_t slots, int key_bits) {
   if (key_bits != 32 && key_bits != 64) return FGB_E_DTYPE;
@@ -694,6 +804,17 @@ extern "C" int64_t fgb_indice_weighted_sum_grad_bytes(int64_t M, int64_t N, int 
   return static_cast<int64_t>(fgb::group_scratch(M * V, N).bytes);
 }
 
+extern "C" int64_t fgb_indice_weighted_sum_grad_full_bytes(int64_t M, int64_t N, int C, int V, int dtype) {
+  using namespace fgb;
+  const int64_t bytes = fgb_indice_weighted_sum_grad_bytes(M, N, V);
+  if (!elem_code_ok(dtype)) return FGB_E_DTYPE;
+  if (bytes < 0 || C <= 0) return FGB_E_SIZE;
+  if (C % 4) return FGB_E_ALIGN;
+  if (N == 0) return bytes;
+  const GroupPlan plan = group_plan(static_cast<uint32_t>(M * V), static_cast<uint32_t>(N), C / pack_width(C, dtype));
+  return static_cast<int64_t>(cut_scratch(group_scratch(M * V, N), plan, M * V, C).end);
+}
+
 extern "C" int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t* indices, const float* weight, void* grad_feats, int64_t M,
                                             int64_t N, int C, int V, int dtype, void* workspace, int64_t workspace_bytes, void* stream) {
   using namespace fgb;
@@ -714,22 +835,33 @@ extern "C" int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t
   uint32_t* total = reinterpret_cast<uint32_t*>(mem + G.total_off);
   uint32_t* start = reinterpret_cast<uint32_t*>(mem + G.start_off);
   uint2* grouped = reinterpret_cast<uint2*>(mem + G.grouped_off);
+  const GroupPlan plan = group_plan(entries, n, C / pack_width(C, dtype));
+  const CutScratch K = cut_scratch(G, plan, entries, C);
+  CutLists cut{0xFFFFFFFFu, plan.piece, total + 1, nullptr, nullptr, nullptr};
+  uint32_t piece_ctas = 0;
+  if (K.pieces > 0 && workspace_bytes >= static_cast<int64_t>(K.end)) {
+    cut.limit = plan.limit;
+    cut.pieces = reinterpret_cast<uint2*>(mem + K.pieces_off);
+    cut.done = reinterpret_cast<uint32_t*>(mem + K.done_off);
+    cut.slab = reinterpret_cast<float*>(mem + K.slab_off);
+    piece_ctas = static_cast<uint32_t>(std::min<int64_t>(ceil_div(K.pieces, 8), int64_t(device_sm_count()) * 2));
+  }
   LaunchErrors chain;
   chain.add(cudaMemsetAsync(mem, 0, G.zero_bytes, s));
   if (entries > 0) {
     const dim3 egrid(static_cast<unsigned>(std::min<int64_t>(ceil_div(entries, 256), 148 * 32)));
     chain.add(launch_chained(group_count_kernel, egrid, dim3(256), 0, s, indices, entries, count));
     chain.add(launch_chained(group_place_kernel, dim3(static_cast<unsigned>(ceil_div(N, 1024))), dim3(1024), 0, s, static_cast<const uint32_t*>(count), n,
-                             start, total));
+                             start, total, cut));
     chain.add(launch_chained(group_fill_kernel, egrid, dim3(256), 0, s, indices, weight, entries, V, start, grouped));
   }
   if (dtype == FGB_F16)
-    chain.add(C % 8 == 0 ? launch_group_sum<__half, 8>(entries, grad_out, grouped, start, count, n, C, grad_feats, s)
-                         : launch_group_sum<__half, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(C % 8 == 0 ? launch_group_sum<__half, 8>(plan, grad_out, grouped, start, count, n, C, grad_feats, cut, piece_ctas, s)
+                         : launch_group_sum<__half, 4>(plan, grad_out, grouped, start, count, n, C, grad_feats, cut, piece_ctas, s));
   else if (dtype == FGB_BF16)
-    chain.add(C % 8 == 0 ? launch_group_sum<__nv_bfloat16, 8>(entries, grad_out, grouped, start, count, n, C, grad_feats, s)
-                         : launch_group_sum<__nv_bfloat16, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(C % 8 == 0 ? launch_group_sum<__nv_bfloat16, 8>(plan, grad_out, grouped, start, count, n, C, grad_feats, cut, piece_ctas, s)
+                         : launch_group_sum<__nv_bfloat16, 4>(plan, grad_out, grouped, start, count, n, C, grad_feats, cut, piece_ctas, s));
   else
-    chain.add(launch_group_sum<float, 4>(entries, grad_out, grouped, start, count, n, C, grad_feats, s));
+    chain.add(launch_group_sum<float, 4>(plan, grad_out, grouped, start, count, n, C, grad_feats, cut, piece_ctas, s));
   return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
 }

@@ -48,7 +48,7 @@ using torch::autograd::variable_list;
   X(fgb_bias_grad_workspace_bytes) X(fgb_subm_conv_bias_grad) X(fgb_subm_cache_scratch_bytes)                         \
   X(fgb_subm_cache_build) X(fgb_pp_valid_signal) X(fgb_hash_table_bytes)                                    \
   X(fgb_strided_grid_bytes) X(fgb_strided_mark) X(fgb_strided_build_bytes) X(fgb_strided_build)                       \
-  X(fgb_grid_sample_fused) X(fgb_indice_weighted_sum_grad_bytes) X(fgb_indice_weighted_sum_grad)
+  X(fgb_grid_sample_fused) X(fgb_indice_weighted_sum_grad_full_bytes) X(fgb_indice_weighted_sum_grad)
 struct Api {
 #define X(f) decltype(&::f) f = nullptr;
   FGB_TORCH_API(X)
@@ -1064,16 +1064,18 @@ PyObject* py_strided_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------ grid sample
-Tensor run_sample_grad(const Tensor& grad_out /* [M, C] */, const Tensor& indices, const Tensor& weight, int64_t n, int64_t V) {
+Tensor run_sample_grad(const Tensor& grad_out /* [..., C] */, const Tensor& indices, const Tensor& weight, int64_t n, int64_t V) {
   c10::cuda::CUDAGuard guard(grad_out.device());
   const auto stream = c10::cuda::getCurrentCUDAStream(grad_out.device().index());
-  const int64_t M = grad_out.size(0), C = grad_out.size(1);
+  const int64_t C = grad_out.size(-1), M = C > 0 ? grad_out.numel() / C : 0;
   Tensor out = new_tensor({n, C}, grad_out.scalar_type(), grad_out.device());
-  const int64_t bytes = check_bytes(api.fgb_indice_weighted_sum_grad_bytes(M, n, static_cast<int>(V)), "fgb_indice_weighted_sum_grad_bytes");
+  const int dtype = dtype_code(grad_out.scalar_type(), false);
+  const int64_t bytes = check_bytes(api.fgb_indice_weighted_sum_grad_full_bytes(M, n, static_cast<int>(C), static_cast<int>(V), dtype),
+                                    "fgb_indice_weighted_sum_grad_full_bytes");
   const c10::DataPtr ws = scratch(bytes);
   check(api.fgb_indice_weighted_sum_grad(ptr(grad_out), cptr<uint32_t>(indices), weight.defined() ? cptr<float>(weight) : nullptr,
                                          n > 0 ? out.data_ptr() : nullptr, M, n, static_cast<int>(C), static_cast<int>(V),
-                                         dtype_code(grad_out.scalar_type(), false), ws.get(), bytes, stream),
+                                         dtype, ws.get(), bytes, stream),
         "fgb_indice_weighted_sum_grad");
   g_launches += 4;
   return out;
@@ -1092,8 +1094,7 @@ struct GridSampleBackward : public torch::autograd::Node {
     if (!grads[0].defined() || !task_should_compute_output(0)) return out;
     const Tensor indices = indices_.unpack(), weight = weight_.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor g = grads[0].contiguous();
-    out[0] = run_sample_grad(g.view({-1, g.size(-1)}), indices, weight, n, V);
+    out[0] = run_sample_grad(grads[0].contiguous(), indices, weight, n, V);
     return out;
   }
 };

@@ -545,8 +545,12 @@ int fgb_grid_sample_fused(const int32_t* coords, int64_t n, const void* feats, c
 
 /* As fgb_indice_weighted_sum_bwd, with the result [N, C] in the feature type:
  * the entries are grouped by voxel in the workspace and every voxel's row is
- * summed in fp32 and written once, instead of added up by atomics. */
+ * summed in fp32 and written once, instead of added up by atomics.  With a
+ * workspace of fgb_indice_weighted_sum_grad_full_bytes (a little more than the
+ * least, fgb_indice_weighted_sum_grad_bytes) the entries of a voxel that is hit far
+ * more often than the others are shared out among many warps. */
 int64_t fgb_indice_weighted_sum_grad_bytes(int64_t M, int64_t N, int V);
+int64_t fgb_indice_weighted_sum_grad_full_bytes(int64_t M, int64_t N, int C, int V, int dtype);
 int fgb_indice_weighted_sum_grad(const void* grad_out, const uint32_t* indices, const float* weight, void* grad_feats,
                                  int64_t M, int64_t N, int C, int V, int dtype,
                                  void* workspace, int64_t workspace_bytes, void* stream);

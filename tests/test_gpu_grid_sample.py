@@ -118,3 +118,34 @@ def test_grid_sample_64bit_keys_and_empty_inputs():
     assert rel_err(out, ref) <= 1e-5 and float(out[:7].abs().max()) == 0.0
     none = grid_sample_3d(feats.to(DEV), torch.from_numpy(coords_np).to(DEV), torch.Size(shape), torch.zeros(8, 0, 3, device=DEV), "nearest")
     assert none.shape == (8, 0, 4)
+
+
+@pytest.mark.parametrize("C,dtype,n,hot", [(4, "float16", 9000, (256, 257, 5000)), (64, "float16", 9000, (255, 256, 257, 511, 512, 40000)),
+                                           (12, "bfloat16", 9000, (257, 131073)), (256, "float16", 3000, (1024, 1025, 1537, 600001)),
+                                           (136, "float32", 3000, (1023, 1024, 1025, 30000)), (520, "bfloat16", 700, (1025, 20000)),
+                                           (16, "float32", 40, (8191, 8192, 8193, 100000)), (256, "float16", 7, (8193, 9217, 70000)),
+                                           (72, "float16", 1, (300000,))])
+@pytest.mark.parametrize("V", [1, 8])
+def test_gradient_of_voxels_hit_far_more_often_than_the_others(C, dtype, n, hot, V):
+    """Lists below, at and above the length from which they are cut into pieces, for each way of walking the lists, and
+    with more pieces than a list is given at most.  fp32 sums in any order, rounded once: within half a unit in the last
+    place of the type plus (terms) * 2^-24 of the absolute sum."""
+    from flexgemm_b200 import _native
+    g = torch.Generator().manual_seed(C + n)
+    rows = torch.cat([torch.full((c,), r, dtype=torch.int64) for r, c in enumerate(hot)] + [torch.randint(0, n, (4 * n,), generator=g)])
+    rows = torch.cat([rows, torch.full((-len(rows) % V + 3 * V,), 0xFFFFFFFF)])[torch.randperm(len(rows) + -len(rows) % V + 3 * V, generator=g)]
+    M = len(rows) // V
+    rows = rows.to(DEV)
+    weight = torch.rand(M, V, generator=g).to(DEV) if V == 8 else None
+    gout = torch.randn(M, C, generator=g).to(getattr(torch, dtype)).to(DEV)
+    got = _native.ext().sample_grad(gout, rows.to(torch.uint32).view(M, V), weight, n)
+    ok = (rows != 0xFFFFFFFF).nonzero().view(-1)
+    want, mag = (torch.zeros(n, C, dtype=torch.float64, device=DEV) for _ in range(2))
+    for some in ok.split(100_000):
+        terms = gout[some // V].double() * (weight.view(-1)[some].double()[:, None] if V == 8 else 1.0)
+        want.index_add_(0, rows[some], terms)
+        mag.index_add_(0, rows[some], terms.abs())
+    count = torch.bincount(rows[ok], minlength=n).double()[:, None]
+    ulp = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -24}[dtype]
+    # fp16 results below its normal range are rounded to a multiple of 2^-24
+    assert torch.all((got.double() - want).abs() <= want.abs() * ulp + mag * 2.0 ** -24 * count + 2.0 ** -25)

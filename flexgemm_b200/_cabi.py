@@ -17,6 +17,7 @@ F16, BF16, F32_TF32, F32_IEEE = 0, 1, 2, 3
 _P = c_void_p
 _PROTOTYPES = {
     "fgb_version": (c_char_p, []),
+    "fgb_launch_count": (c_int64, []),
     "fgb_status_set_mirror": (c_int, [_P, _P]),
     "fgb_conv_call_workspace_bytes": (c_int64, [_P, c_int]),
     "fgb_conv_call_fprop": (c_int, [_P, _P]),

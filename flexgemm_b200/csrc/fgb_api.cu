@@ -40,6 +40,8 @@ extern "C" int fgb_status_set_mirror(const int32_t* status, int32_t* mirror) {
   return FGB_E_SIZE;
 }
 
+extern "C" int64_t fgb_launch_count(void) { return fgb::launch_counter().load(std::memory_order_relaxed); }
+
 extern "C" const char* fgb_version(void) { return "flexgemm_b200 0.1.0 (sm_100a)"; }
 
 extern "C" const char* fgb_error_string(int code) {

@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "fgb_common.cuh"
@@ -87,6 +88,27 @@ inline int ensure_dynamic_smem(PerDeviceTable& table, Kernel kernel, size_t byte
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Kernels that this library has launched (fgb_launch_count): every launch goes through one of the two functions below.
+inline std::atomic<int64_t>& launch_counter() {
+  static std::atomic<int64_t> count{0};
+  return count;
+}
+inline cudaError_t counted(cudaError_t e) {
+  if (e == cudaSuccess) launch_counter().fetch_add(1, std::memory_order_relaxed);
+  return e;
+}
+
+// the ordinary launch; an error shows in launch_status()
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return counted(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -99,7 +121,7 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  return counted(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
 }
 
 // first error of a sequence of launches

@@ -653,15 +653,15 @@ extern "C" int fgb_hash_insert_3d_idx_as_val(const int32_t* coords, int64_t n, i
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t words = static_cast<size_t>(fgb_hash_table_bytes(slots, key_bits)) / 4;
   const unsigned grid = static_cast<unsigned>(std::min<size_t>((words + 2047) / 2048, 148 * 16));
-  fill_words_kernel<<<grid > 0 ? grid : 1, 256, 0, s>>>(static_cast<uint32_t*>(table), words, 0xFFFFFFFFu);
+  launch(fill_words_kernel, grid > 0 ? grid : 1, 256, 0, s, static_cast<uint32_t*>(table), words, 0xFFFFFFFFu);
   if (n == 0) return launch_status();
   const Grid3 g{W, H, D};
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, kMapBlock));
   if (key_bits == 32)
-    hash_insert_kernel<32><<<blocks, kMapBlock, 0, s>>>(reinterpret_cast<const int4*>(coords), static_cast<uint32_t>(n), g, table,
+    launch(hash_insert_kernel<32>, blocks, kMapBlock, 0, s, reinterpret_cast<const int4*>(coords), static_cast<uint32_t>(n), g, table,
                                                        static_cast<uint32_t>(slots), status, nullptr);
   else
-    hash_insert_kernel<64><<<blocks, kMapBlock, 0, s>>>(reinterpret_cast<const int4*>(coords), static_cast<uint32_t>(n), g, table,
+    launch(hash_insert_kernel<64>, blocks, kMapBlock, 0, s, reinterpret_cast<const int4*>(coords), static_cast<uint32_t>(n), g, table,
                                                        static_cast<uint32_t>(slots), status, nullptr);
   return launch_status();
 }
@@ -679,10 +679,10 @@ extern "C" int fgb_hash_lookup_3d(const int32_t* query_coords, int64_t m, int W,
   const Grid3 g{W, H, D};
   const unsigned blocks = static_cast<unsigned>(ceil_div(m, 256));
   if (key_bits == 32)
-    hash_lookup_3d_kernel<32><<<blocks, 256, 0, s>>>(reinterpret_cast<const int4*>(query_coords), static_cast<uint32_t>(m), g, table,
+    launch(hash_lookup_3d_kernel<32>, blocks, 256, 0, s, reinterpret_cast<const int4*>(query_coords), static_cast<uint32_t>(m), g, table,
                                                     static_cast<uint32_t>(slots), out_rows);
   else
-    hash_lookup_3d_kernel<64><<<blocks, 256, 0, s>>>(reinterpret_cast<const int4*>(query_coords), static_cast<uint32_t>(m), g, table,
+    launch(hash_lookup_3d_kernel<64>, blocks, 256, 0, s, reinterpret_cast<const int4*>(query_coords), static_cast<uint32_t>(m), g, table,
                                                     static_cast<uint32_t>(slots), out_rows);
   return launch_status();
 }
@@ -701,11 +701,11 @@ extern "C" int fgb_grid_sample_neighbor_map(const float* query, int64_t B, int64
   const unsigned blocks = static_cast<unsigned>(ceil_div(B * L, 256));
   const uint32_t b = static_cast<uint32_t>(B), l = static_cast<uint32_t>(L), sl = static_cast<uint32_t>(slots);
   if (trilinear) {
-    if (key_bits == 32) trilinear_map_kernel<32><<<blocks, 256, 0, s>>>(query, b, l, g, table, sl, neighbor, weight);
-    else trilinear_map_kernel<64><<<blocks, 256, 0, s>>>(query, b, l, g, table, sl, neighbor, weight);
+    if (key_bits == 32) launch(trilinear_map_kernel<32>, blocks, 256, 0, s, query, b, l, g, table, sl, neighbor, weight);
+    else launch(trilinear_map_kernel<64>, blocks, 256, 0, s, query, b, l, g, table, sl, neighbor, weight);
   } else {
-    if (key_bits == 32) nearest_map_kernel<32><<<blocks, 256, 0, s>>>(query, b, l, g, table, sl, neighbor);
-    else nearest_map_kernel<64><<<blocks, 256, 0, s>>>(query, b, l, g, table, sl, neighbor);
+    if (key_bits == 32) launch(nearest_map_kernel<32>, blocks, 256, 0, s, query, b, l, g, table, sl, neighbor);
+    else launch(nearest_map_kernel<64>, blocks, 256, 0, s, query, b, l, g, table, sl, neighbor);
   }
   return launch_status();
 }
@@ -724,12 +724,12 @@ extern "C" int fgb_indice_weighted_sum_fwd(const void* feats, const uint32_t* in
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned g = static_cast<unsigned>(blocks);
   if (dtype == FGB_F16)
-    weighted_gather_kernel<__half><<<g, 256, 0, s>>>(static_cast<const __half*>(feats), indices, weight, static_cast<__half*>(out), M, C, V);
+    launch(weighted_gather_kernel<__half>, g, 256, 0, s, static_cast<const __half*>(feats), indices, weight, static_cast<__half*>(out), M, C, V);
   else if (dtype == FGB_BF16)
-    weighted_gather_kernel<__nv_bfloat16><<<g, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(feats), indices, weight,
+    launch(weighted_gather_kernel<__nv_bfloat16>, g, 256, 0, s, static_cast<const __nv_bfloat16*>(feats), indices, weight,
                                                             static_cast<__nv_bfloat16*>(out), M, C, V);
   else
-    weighted_gather_kernel<float><<<g, 256, 0, s>>>(static_cast<const float*>(feats), indices, weight, static_cast<float*>(out), M, C, V);
+    launch(weighted_gather_kernel<float>, g, 256, 0, s, static_cast<const float*>(feats), indices, weight, static_cast<float*>(out), M, C, V);
   return launch_status();
 }
 
@@ -752,12 +752,12 @@ extern "C" int fgb_indice_weighted_sum_bwd(const void* grad_out, const uint32_t*
   if (blocks > 0x7FFFFFFF) return FGB_E_SIZE;
   const unsigned g = static_cast<unsigned>(blocks);
   if (dtype == FGB_F16)
-    weighted_scatter_kernel<__half><<<g, 256, 0, s>>>(static_cast<const __half*>(grad_out), indices, weight, grad_feats_f32, M, C, V);
+    launch(weighted_scatter_kernel<__half>, g, 256, 0, s, static_cast<const __half*>(grad_out), indices, weight, grad_feats_f32, M, C, V);
   else if (dtype == FGB_BF16)
-    weighted_scatter_kernel<__nv_bfloat16><<<g, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(grad_out), indices, weight, grad_feats_f32, M,
+    launch(weighted_scatter_kernel<__nv_bfloat16>, g, 256, 0, s, static_cast<const __nv_bfloat16*>(grad_out), indices, weight, grad_feats_f32, M,
                                                              C, V);
   else
-    weighted_scatter_kernel<float><<<g, 256, 0, s>>>(static_cast<const float*>(grad_out), indices, weight, grad_feats_f32, M, C, V);
+    launch(weighted_scatter_kernel<float>, g, 256, 0, s, static_cast<const float*>(grad_out), indices, weight, grad_feats_f32, M, C, V);
   return launch_status();
 }
 

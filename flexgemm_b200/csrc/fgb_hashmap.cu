@@ -14,6 +14,7 @@
 // reference.  A table without a free slot records FGB_S_TABLE_FULL in the
 // status word instead of probing forever.
 #include "fgb_common.cuh"
+#include "fgb_device.cuh"
 
 namespace fgb {
 
@@ -115,10 +116,10 @@ static int dispatch_open(void* keys, void* vals, int64_t slots, int key_bits, in
     using K = decltype(k0);
     using V = decltype(v0);
     if constexpr (kInsert)
-      open_insert_kernel<K, V, kMode><<<grid, 256, 0, s>>>(static_cast<K*>(keys), static_cast<V*>(vals), n, in, static_cast<const V*>(in_vals), m,
+      launch(open_insert_kernel<K, V, kMode>, grid, 256, 0, s, static_cast<K*>(keys), static_cast<V*>(vals), n, in, static_cast<const V*>(in_vals), m,
                                                           W, H, D, status);
     else
-      open_lookup_kernel<K, V, kMode><<<grid, 256, 0, s>>>(static_cast<const K*>(keys), static_cast<const V*>(vals), n, in, m, W, H, D,
+      launch(open_lookup_kernel<K, V, kMode>, grid, 256, 0, s, static_cast<const K*>(keys), static_cast<const V*>(vals), n, in, m, W, H, D,
                                                           static_cast<V*>(out));
   };
   if (key_bits == 32 && val_bits == 32) run(uint32_t(0), uint32_t(0));

@@ -1002,7 +1002,7 @@ extern "C" int fgb_conv_block_schedule(const uint32_t* tile_masks, int64_t num_t
   if (num_tiles == 0) return FGB_OK;
   if (!tile_masks || !block_order) return FGB_E_NULL;
   const uint32_t nb = static_cast<uint32_t>(ceil_div(num_tiles, 2));
-  block_schedule_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(tile_masks, static_cast<uint32_t>(num_tiles), nb, block_order);
+  launch(block_schedule_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream), tile_masks, static_cast<uint32_t>(num_tiles), nb, block_order);
   return launch_status();
 }
 
@@ -1118,9 +1118,9 @@ static int dgrad_impl(const void* grad_out, const void* weight, const uint32_t* 
     if (e != cudaSuccess) return cuda_status(e);
   }
   if (eb == 2)
-    weight_transpose_kernel<uint16_t><<<grid, 256, 0, s>>>(static_cast<const uint16_t*>(weight), reinterpret_cast<uint16_t*>(wt), Co, V, Ci);
+    launch(weight_transpose_kernel<uint16_t>, grid, 256, 0, s, static_cast<const uint16_t*>(weight), reinterpret_cast<uint16_t*>(wt), Co, V, Ci);
   else
-    weight_transpose_kernel<uint32_t><<<grid, 256, 0, s>>>(static_cast<const uint32_t*>(weight), reinterpret_cast<uint32_t*>(wt), Co, V, Ci);
+    launch(weight_transpose_kernel<uint32_t>, grid, 256, 0, s, static_cast<const uint32_t*>(weight), reinterpret_cast<uint32_t*>(wt), Co, V, Ci);
   int rc = launch_status();
   if (rc != FGB_OK) return rc;
   if (!ieee)

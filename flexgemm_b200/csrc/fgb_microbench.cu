@@ -430,14 +430,14 @@ extern "C" int fgb_microbench_pipeline(int mode, int stages_a, int stages_b, int
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         rc = cuda_status(cudaEventRecord(e0, s));
-        if (rc == FGB_OK) rc = cuda_status(cudaLaunchKernelEx(&cfg, microbench_kernel<true>, tmap, p));
+        if (rc == FGB_OK) rc = cuda_status(counted(cudaLaunchKernelEx(&cfg, microbench_kernel<true>, tmap, p)));
       }
     } else {
       static PerDeviceTable configured;
       rc = ensure_dynamic_smem(configured, microbench_kernel<false>, smem);
       if (rc == FGB_OK) rc = cuda_status(cudaEventRecord(e0, s));
       if (rc == FGB_OK) {
-        microbench_kernel<false><<<sms, kMbThreads, smem, s>>>(tmap, p);
+        launch(microbench_kernel<false>, sms, kMbThreads, smem, s, tmap, p);
         rc = launch_status();
       }
     }

@@ -454,13 +454,14 @@ static int build_general_impl(const int32_t* in_coords, uint32_t n_in, const int
                               void* table, uint32_t slots, uint32_t* nbr, uint32_t* nbr_bwd, int32_t* gray, int32_t* binary,
                               uint32_t* block_counts, uint32_t* seg, int32_t* status, cudaStream_t s) {
   if (n_in > 0)
-    hash_insert_kernel<kKeyBits><<<static_cast<unsigned>(ceil_div(n_in, kMapBlock)), kMapBlock, 0, s>>>(
-        reinterpret_cast<const int4*>(in_coords), n_in, g, table, slots, status, nullptr);
+    launch(hash_insert_kernel<kKeyBits>, static_cast<unsigned>(ceil_div(n_in, kMapBlock)), kMapBlock, 0, s,
+           reinterpret_cast<const int4*>(in_coords), n_in, g, table, slots, status, nullptr);
   const uint32_t nblk = static_cast<uint32_t>(ceil_div(n_out, kMapBlock));
   const MapOut o{nbr, gray, binary, block_counts, nullptr, nblk};
-  sparse_lookup_kernel<kKeyBits><<<nblk, kMapBlock, hash_smem_bytes(st.V), s>>>(reinterpret_cast<const int4*>(out_coords), n_out, g, st, table, slots, o, nbr_bwd);
-  block_scan_kernel<<<st.V, 1024, 0, s>>>(block_counts, nblk, seg, ScanFinish{});
-  seg_prefix_kernel<<<1, 32, 0, s>>>(seg, st.V);
+  launch(sparse_lookup_kernel<kKeyBits>, nblk, kMapBlock, hash_smem_bytes(st.V), s,
+         reinterpret_cast<const int4*>(out_coords), n_out, g, st, table, slots, o, nbr_bwd);
+  launch(block_scan_kernel, st.V, 1024, 0, s, block_counts, nblk, seg, ScanFinish{});
+  launch(seg_prefix_kernel, 1, 32, 0, s, seg, st.V);
   return launch_status();
 }
 
@@ -693,7 +694,7 @@ extern "C" int fgb_pp_gray_code(const uint32_t* neighbor_map, int64_t n, int V, 
   if (n < 0 || n >= (int64_t(1) << 32) - 1 || V < 1 || V > 32) return FGB_E_SIZE;
   if (n == 0) return FGB_OK;
   if (!neighbor_map || !gray_code || !binary_code) return FGB_E_NULL;
-  gray_from_map_kernel<<<static_cast<unsigned>(ceil_div(n, 256)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      neighbor_map, static_cast<uint32_t>(n), V, gray_code, binary_code);
+  launch(gray_from_map_kernel, static_cast<unsigned>(ceil_div(n, 256)), 256, 0, static_cast<cudaStream_t>(stream),
+         neighbor_map, static_cast<uint32_t>(n), V, gray_code, binary_code);
   return launch_status();
 }

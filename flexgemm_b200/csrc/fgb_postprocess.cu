@@ -158,8 +158,8 @@ extern "C" int fgb_pp_tile_masks(const int32_t* gray_code, const int64_t* sorted
   if (n == 0) return FGB_OK;
   if (!gray_code || !sorted_idx || !tile_masks) return FGB_E_NULL;
   const int64_t ntiles = ceil_div(n, block);
-  tile_mask_kernel<<<static_cast<unsigned>(ceil_div(ntiles * 32, 256)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      gray_code, sorted_idx, n, block, ntiles, tile_masks);
+  launch(tile_mask_kernel, static_cast<unsigned>(ceil_div(ntiles * 32, 256)), 256, 0, static_cast<cudaStream_t>(stream),
+         gray_code, sorted_idx, n, block, ntiles, tile_masks);
   return launch_status();
 }
 
@@ -169,7 +169,7 @@ extern "C" int fgb_pp_valid_kernel(const uint32_t* tile_masks, int64_t nblk, int
   if (nblk < 0 || nblk > (int64_t(1) << 24)) return FGB_E_SIZE;
   if (!valid_kernel_seg) return FGB_E_NULL;
   if (nblk > 0 && (!tile_masks || !valid_kernel)) return FGB_E_NULL;
-  valid_kernel_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(tile_masks, static_cast<uint32_t>(nblk), valid_kernel,
+  launch(valid_kernel_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream), tile_masks, static_cast<uint32_t>(nblk), valid_kernel,
                                                                          valid_kernel_seg);
   return launch_status();
 }

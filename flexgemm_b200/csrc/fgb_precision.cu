@@ -1,4 +1,5 @@
 // Operand splitting for the fp32-accurate (TF32-disabled) mode; see fgb_precision.cuh.
+#include "fgb_device.cuh"
 #include "fgb_precision.cuh"
 
 namespace fgb {
@@ -34,13 +35,13 @@ __global__ void __launch_bounds__(256) split2_kernel(const float* __restrict__ s
 int launch_split3(const float* src, float* dst, int64_t rows, int C, SplitMode mode, cudaStream_t s) {
   const int64_t count = rows * C;
   if (count == 0) return FGB_OK;
-  split3_kernel<<<static_cast<unsigned>(ceil_div(count, 256)), 256, 0, s>>>(src, dst, rows, C, static_cast<int>(mode));
+  launch(split3_kernel, static_cast<unsigned>(ceil_div(count, 256)), 256, 0, s, src, dst, rows, C, static_cast<int>(mode));
   return launch_status();
 }
 
 int launch_split2(const float* src, float* hi, float* lo, int64_t count, cudaStream_t s) {
   if (count == 0) return FGB_OK;
-  split2_kernel<<<static_cast<unsigned>(ceil_div(count, 256)), 256, 0, s>>>(src, hi, lo, count);
+  launch(split2_kernel, static_cast<unsigned>(ceil_div(count, 256)), 256, 0, s, src, hi, lo, count);
   return launch_status();
 }
 

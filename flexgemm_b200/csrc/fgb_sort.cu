@@ -290,7 +290,7 @@ extern "C" int fgb_pp_sorted_idx(const int32_t* binary_code, int64_t n, int key_
   // keys per CTA of the histogram: 1024 up to 400 k keys, 2048 beyond (measured: 42 / 43.5 / 46.5 us for the whole sort at
   // 164 k keys with 1024 / 2048 / 4096; 70.5 / 68.7 / 70.6 us at 660 k), at most eight CTAs per SM
   const unsigned hist_grid = static_cast<unsigned>(std::min<int64_t>(ceil_div(n, n <= 400000 ? 1024 : 2048), 148 * 8));
-  sort_histogram_kernel<<<hist_grid, kSortThreads, 0, s>>>(binary_code, static_cast<uint32_t>(n), sort_passes_of(key_bits), sort_flip_of(key_bits),
+  launch(sort_histogram_kernel, hist_grid, kSortThreads, 0, s, binary_code, static_cast<uint32_t>(n), sort_passes_of(key_bits), sort_flip_of(key_bits),
                                                           hist);
   const cudaError_t e = launch_sort_passes(binary_code, n, key_bits, sorted_idx, ws, L, hist, reinterpret_cast<uint32_t*>(ws + sort_lookback_off(L)),
                                            status, s);

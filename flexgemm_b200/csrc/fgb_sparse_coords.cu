@@ -14,6 +14,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "fgb_common.cuh"
+#include "fgb_device.cuh"
 
 namespace fgb {
 
@@ -182,7 +183,7 @@ static int finalize_impl(const K* keys, int64_t count, int B, OutGrid og, int mo
   } else {
     uint64_t* skey_in = reinterpret_cast<uint64_t*>(ws + p.skey_in_off);
     uint64_t* skey_out = reinterpret_cast<uint64_t*>(ws + p.skey_out_off);
-    serial_key_kernel<K><<<grid, 256, 0, s>>>(keys, static_cast<uint32_t>(count), og, mode, bits, skey_in);
+    launch(serial_key_kernel<K>, grid, 256, 0, s, keys, static_cast<uint32_t>(count), og, mode, bits, skey_in);
     rc = launch_status();
     if (rc != FGB_OK) return rc;
     int end_bit = 3 * bits + bit_length(B > 0 ? uint64_t(B - 1) : 0);
@@ -191,7 +192,7 @@ static int finalize_impl(const K* keys, int64_t count, int B, OutGrid og, int mo
     e = cub::DeviceRadixSort::SortPairs(ws + p.temp_off, p.temp_bytes, skey_in, skey_out, keys, sorted, count, 0, end_bit, s);
   }
   if (e != cudaSuccess) return cuda_status(e);
-  decode_out_keys_kernel<K><<<grid, 256, 0, s>>>(sorted, static_cast<uint32_t>(count), og, reinterpret_cast<int4*>(out));
+  launch(decode_out_keys_kernel<K>, grid, 256, 0, s, sorted, static_cast<uint32_t>(count), og, reinterpret_cast<int4*>(out));
   return launch_status();
 }
 
@@ -245,12 +246,12 @@ extern "C" int fgb_sparse_out_coords_collect(const int32_t* in_coords, int64_t n
   const int64_t grid = ceil_div(n_in * V, 256);
   if (grid > 0x7FFFFFFF) return FGB_E_SIZE;
   if (key_bits == 32)
-    collect_out_keys_kernel<uint32_t><<<static_cast<unsigned>(grid), 256, 0, s>>>(
-        reinterpret_cast<const int4*>(in_coords), static_cast<uint32_t>(n_in), cg, og, static_cast<uint32_t*>(set),
+    launch(collect_out_keys_kernel<uint32_t>, static_cast<unsigned>(grid), 256, 0, s,
+           reinterpret_cast<const int4*>(in_coords), static_cast<uint32_t>(n_in), cg, og, static_cast<uint32_t*>(set),
         static_cast<uint32_t>(slots), static_cast<uint32_t*>(keys), count, status);
   else
-    collect_out_keys_kernel<unsigned long long><<<static_cast<unsigned>(grid), 256, 0, s>>>(
-        reinterpret_cast<const int4*>(in_coords), static_cast<uint32_t>(n_in), cg, og, static_cast<unsigned long long*>(set),
+    launch(collect_out_keys_kernel<unsigned long long>, static_cast<unsigned>(grid), 256, 0, s,
+           reinterpret_cast<const int4*>(in_coords), static_cast<uint32_t>(n_in), cg, og, static_cast<unsigned long long*>(set),
         static_cast<uint32_t>(slots), static_cast<unsigned long long*>(keys), count, status);
   return launch_status();
 }

@@ -886,7 +886,7 @@ static int launch_wgrad_instance(int64_t grid, size_t smem, const WgradParams& p
   static PerDeviceTable configured;
   const int rc = ensure_dynamic_smem(configured, subm_wgrad_kernel<kDtype, kRows, kBanded>, smem);
   if (rc != FGB_OK) return rc;
-  subm_wgrad_kernel<kDtype, kRows, kBanded><<<static_cast<unsigned>(grid), kWgThreads, smem, s>>>(p);
+  launch(subm_wgrad_kernel<kDtype, kRows, kBanded>, static_cast<unsigned>(grid), kWgThreads, smem, s, p);
   return launch_status();
 }
 template <int kDtype>
@@ -1137,16 +1137,16 @@ extern "C" int fgb_subm_conv_bias_grad(const void* grad_out, void* grad_bias, fl
   const unsigned fblocks = static_cast<unsigned>(ceil_div(Co, 32));
   switch (dtype) {
     case FGB_F16:
-      bias_partial_kernel<__half><<<nblk, 256, 0, s>>>(static_cast<const __half*>(grad_out), n, Co, partial);
-      bias_final_kernel<__half><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<__half*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<__half>, nblk, 256, 0, s, static_cast<const __half*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<__half>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<__half*>(grad_bias), grad_bias_f32);
       break;
     case FGB_BF16:
-      bias_partial_kernel<__nv_bfloat16><<<nblk, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(grad_out), n, Co, partial);
-      bias_final_kernel<__nv_bfloat16><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<__nv_bfloat16*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<__nv_bfloat16>, nblk, 256, 0, s, static_cast<const __nv_bfloat16*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<__nv_bfloat16>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<__nv_bfloat16*>(grad_bias), grad_bias_f32);
       break;
     default:
-      bias_partial_kernel<float><<<nblk, 256, 0, s>>>(static_cast<const float*>(grad_out), n, Co, partial);
-      bias_final_kernel<float><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<float*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<float>, nblk, 256, 0, s, static_cast<const float*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<float>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<float*>(grad_bias), grad_bias_f32);
   }
   return launch_status();
 }
@@ -1206,16 +1206,16 @@ extern "C" int fgb_subm_conv_bias_grad_noalloc(const void* grad_out, void* grad_
   const unsigned fblocks = static_cast<unsigned>(ceil_div(Co, 32));
   switch (dtype) {
     case FGB_F16:
-      bias_partial_kernel<__half><<<nblk, 256, 0, s>>>(static_cast<const __half*>(grad_out), n, Co, partial);
-      bias_final_kernel<__half><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<__half*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<__half>, nblk, 256, 0, s, static_cast<const __half*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<__half>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<__half*>(grad_bias), grad_bias_f32);
       break;
     case FGB_BF16:
-      bias_partial_kernel<__nv_bfloat16><<<nblk, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(grad_out), n, Co, partial);
-      bias_final_kernel<__nv_bfloat16><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<__nv_bfloat16*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<__nv_bfloat16>, nblk, 256, 0, s, static_cast<const __nv_bfloat16*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<__nv_bfloat16>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<__nv_bfloat16*>(grad_bias), grad_bias_f32);
       break;
     default:
-      bias_partial_kernel<float><<<nblk, 256, 0, s>>>(static_cast<const float*>(grad_out), n, Co, partial);
-      bias_final_kernel<float><<<fblocks, 256, 0, s>>>(partial, nblk, Co, static_cast<float*>(grad_bias), grad_bias_f32);
+      launch(bias_partial_kernel<float>, nblk, 256, 0, s, static_cast<const float*>(grad_out), n, Co, partial);
+      launch(bias_final_kernel<float>, fblocks, 256, 0, s, partial, nblk, Co, static_cast<float*>(grad_bias), grad_bias_f32);
   }
   return launch_status();
 }
@@ -1229,14 +1229,14 @@ extern "C" int fgb_cast_from_f32(const float* src, void* dst, int64_t count, int
   const unsigned blocks = static_cast<unsigned>(ceil_div(count, 256));
   switch (dtype) {
     case FGB_F16:
-      cast_from_f32_kernel<__half><<<blocks, 256, 0, s>>>(src, static_cast<__half*>(dst), count);
+      launch(cast_from_f32_kernel<__half>, blocks, 256, 0, s, src, static_cast<__half*>(dst), count);
       break;
     case FGB_BF16:
-      cast_from_f32_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(src, static_cast<__nv_bfloat16*>(dst), count);
+      launch(cast_from_f32_kernel<__nv_bfloat16>, blocks, 256, 0, s, src, static_cast<__nv_bfloat16*>(dst), count);
       break;
     case FGB_F32_TF32:
     case FGB_F32_IEEE:
-      cast_from_f32_kernel<float><<<blocks, 256, 0, s>>>(src, static_cast<float*>(dst), count);
+      launch(cast_from_f32_kernel<float>, blocks, 256, 0, s, src, static_cast<float*>(dst), count);
       break;
     default:
       return FGB_E_DTYPE;

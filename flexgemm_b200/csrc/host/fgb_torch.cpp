@@ -66,8 +66,6 @@ int64_t check_bytes(int64_t n, const char* what) {
   return n;
 }
 
-std::atomic<int64_t> g_launches{0};  // kernels of the library launched from here
-
 // ------------------------------------------------------------------ per-device state
 constexpr int kMaxDevices = 64;
 struct DeviceState {
@@ -274,7 +272,6 @@ Tensor resize_rows(const Tensor& t, int64_t rows_in, int64_t width, at::IntArray
   Tensor out = new_tensor(out_size, t.scalar_type(), t.device());
   const int64_t eb = t.element_size();
   check(api.fgb_resize_rows(ptr(t), out.numel() > 0 ? out.data_ptr() : nullptr, rows_in, rows_out, width * eb, width_out * eb, s), "fgb_resize_rows");
-  g_launches += 1;
   return out;
 }
 int64_t round_up(int64_t c, int64_t m) { return (c + m - 1) / m * m; }
@@ -326,7 +323,6 @@ Tensor run_fprop(const Tensor& feats, const Tensor& weight, const Tensor& bias, 
   c.counters = counter.words;
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   check(api.fgb_conv_call_fprop(&c, stream), "fgb_conv_call_fprop");
-  g_launches += 1;
   return ch.co == ch.co_p ? out : resize_rows(out, n, ch.co_p, {n, ch.co}, n, ch.co, stream);
 }
 
@@ -353,7 +349,6 @@ Tensor run_dgrad(const Tensor& grad_out, const Tensor& weight, const Maps& m, in
   c.counters = counter.words;
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   check(api.fgb_conv_call_dgrad(&c, stream), "fgb_conv_call_dgrad");
-  g_launches += 2;
   return ch.ci == ch.ci_p ? out : resize_rows(out, n, ch.ci_p, {n, ch.ci}, n, ch.ci, stream);
 }
 
@@ -380,7 +375,6 @@ std::pair<Tensor, Tensor> run_wgrad(const Tensor& grad_out, const Tensor& feats,
   c.workspace = ws.get();
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   check(api.fgb_wgrad_call_run(&c, stream), "fgb_wgrad_call_run");
-  g_launches += 2;
   if (!ch.exact()) gw = resize_rows(gw, ch.co * V, ch.ci_p, weight_size, ch.co * V, ch.ci, stream);
   if (want_bias && ch.co != ch.co_p) gb = resize_rows(gb, 1, ch.co_p, {ch.co}, 1, ch.co, stream);
   return {gw, gb};
@@ -394,7 +388,6 @@ Tensor run_bias_grad(const Tensor& grad_out, int dtype) {
   const c10::DataPtr ws = scratch(bytes);
   check(api.fgb_subm_conv_bias_grad(ptr(grad_out), gb.data_ptr(), nullptr, grad_out.size(0), static_cast<int>(co), dtype, ws.get(), bytes, stream),
         "fgb_subm_conv_bias_grad");
-  g_launches += 2;
   return gb;
 }
 
@@ -618,7 +611,6 @@ CacheBuild start_cache(const Tensor& coords, const int64_t* shape, const int64_t
   c.status = static_cast<int32_t*>(ds.status.data_ptr());
   b.slot.queued();
   check(api.fgb_subm_cache_build(&c, stream), "fgb_subm_cache_build");
-  g_launches += 8;
   return b;
 }
 
@@ -641,7 +633,6 @@ Pairs finish_cache(CacheBuild& b) {
     check(api.fgb_pp_valid_signal(cptr<uint32_t>(b.nbr), cptr<int32_t>(b.gray), b.n, b.V, cptr<uint32_t>(b.block_offsets), meta,
                                   static_cast<uint32_t*>(p.vs_i.data_ptr()), static_cast<uint32_t*>(p.vs_o.data_ptr()), meta + b.V + 1, stream),
           "fgb_pp_valid_signal");
-    g_launches += 1;
   }
   return p;
 }
@@ -904,7 +895,6 @@ bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape,
   slot.take(stream, &c.host_words, &c.host_seq);
   slot.queued();
   check(api.fgb_strided_mark(&c, stream), "fgb_strided_mark");
-  g_launches += 2;
   const Told got = slot.take_back();
   if (got.status != 0u) return false;  // rows of a batch beyond the shape's: the bits have no place for them
   c.n_out = got.count;
@@ -914,7 +904,6 @@ bool strided_coords(StridedBuild& b, const Tensor& coords, const int64_t* shape,
   c.out_coords = static_cast<int32_t*>(b.out_coords.data_ptr());
   if (coords_only) {
     check(api.fgb_strided_build(&c, stream), "fgb_strided_build");
-    g_launches += 1;
   }
   return true;
 }
@@ -949,7 +938,6 @@ void strided_maps(StridedBuild& b, at::Device dev, bool train) {
   c.status = static_cast<int32_t*>(device_state(dev.index()).status.data_ptr());
   b.slot.queued();
   check(api.fgb_strided_build(&c, stream), "fgb_strided_build");
-  g_launches += train ? 11 : 8;
 }
 
 Pairs strided_pairs(StridedBuild& b) {
@@ -964,7 +952,6 @@ Pairs strided_pairs(StridedBuild& b) {
     check(api.fgb_pp_valid_signal(cptr<uint32_t>(b.nbr), cptr<int32_t>(b.gray), b.c.n_out, b.V, cptr<uint32_t>(b.block_offsets), cptr<uint32_t>(b.meta),
                                   static_cast<uint32_t*>(p.vs_i.data_ptr()), static_cast<uint32_t*>(p.vs_o.data_ptr()), nullptr, stream),
           "fgb_pp_valid_signal");
-    g_launches += 1;
   }
   return p;
 }
@@ -1077,7 +1064,6 @@ Tensor run_sample_grad(const Tensor& grad_out /* [..., C] */, const Tensor& indi
                                          n > 0 ? out.data_ptr() : nullptr, M, n, static_cast<int>(C), static_cast<int>(V),
                                          dtype, ws.get(), bytes, stream),
         "fgb_indice_weighted_sum_grad");
-  g_launches += 4;
   return out;
 }
 
@@ -1141,7 +1127,6 @@ PyObject* py_grid_sample(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
                                     want_grad ? static_cast<uint32_t*>(indices.data_ptr()) : nullptr,
                                     want_grad && trilinear ? static_cast<float*>(weight.data_ptr()) : nullptr, stream),
           "fgb_grid_sample_fused");
-    g_launches += 2;
   }
   if (want_grad) {
     std::shared_ptr<GridSampleBackward> node(new GridSampleBackward(), torch::autograd::deleteNode);
@@ -1190,7 +1175,6 @@ PyObject* py_host_slots(PyObject*, PyObject*) {
   std::lock_guard<std::mutex> lock(g_words_mu);
   return Py_BuildValue("Ln", static_cast<long long>(g_words_made), static_cast<Py_ssize_t>(g_words_free.size()));
 }
-PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
 // (handle, address): the CUDA library's dlopen handle, the byte of allow_tf32
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -1224,7 +1208,6 @@ PyMethodDef methods[] = {
     {"poll", py_poll, METH_O, "raise a soft error that the device has reported"},
     {"clear_mirror", py_clear_mirror, METH_O, "forget the host copy of the status word"},
     {"host_slots", py_host_slots, METH_NOARGS, "slots through which builds report: (made, free)"},
-    {"launches", py_launches, METH_NOARGS, "kernels launched so far"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fgb_torch", "torch host code of flexgemm_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

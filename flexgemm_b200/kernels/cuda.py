@@ -49,19 +49,10 @@ def _stream(device) -> int:
 # --------------------------------------------------------------------------
 _scratch: Dict[tuple, torch.Tensor] = {}
 
-# Kernels launched through the wrappers of this module; the native module counts its own.  ``launch_count`` (below) is
-# the number of this library's own kernels launched so far.
-_launches = 0
-
-
-def _count(k: int) -> None:
-    global _launches
-    _launches += k
-
 
 def __getattr__(name: str):
     if name == "launch_count":
-        return _launches + _native.ext().launches()
+        return _cabi.lib().fgb_launch_count()   # kernels of this library launched so far, however they were called
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
@@ -170,7 +161,6 @@ def subm_build_neighbor_map(coords: torch.Tensor, shape, ksize, dilation, table:
         meta.data_ptr() + 4 * (V + 2), _stream(dev))
     _cabi.check(rc, "fgb_subm_build_neighbor_map")
     # order check + column index, table clear, insert, hash lookup, column lookup, block scan (with the prefix)
-    _count(6)
     return out
 
 
@@ -212,7 +202,6 @@ def sparse_out_coords(coords: torch.Tensor, shape, ksize, stride, padding, dilat
     rc = lib.fgb_sparse_out_coords_collect(_ptr(coords), n, W, H, D, *geom, set_mem.data_ptr(), slots, key_bits, keys.data_ptr(),
                                            count.data_ptr(), count.data_ptr() + 4, _stream(dev))
     _cabi.check(rc, "fgb_sparse_out_coords_collect")
-    _count(1)
     host = count.cpu()
     raise_for_status(int(host[1]))
     L = int(host[0])
@@ -225,7 +214,6 @@ def sparse_out_coords(coords: torch.Tensor, shape, ksize, stride, padding, dilat
     rc = lib.fgb_sparse_out_coords_finalize(keys.data_ptr(), L, key_bits, int(mode), coord_bits, B, W, H, D, *geom, ws.data_ptr(),
                                             ws.numel() * 8, out.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_sparse_out_coords_finalize")
-    _count(2 if mode else 1)
     return out
 
 
@@ -256,7 +244,6 @@ def sparse_build_neighbor_map(coords: torch.Tensor, out_coords: torch.Tensor, sh
         _ptr(out["neighbor_map"]), _ptr(out["neighbor_map_bwd"]), _ptr(out["gray_code"]), _ptr(out["binary_code"]),
         out["block_offsets"].data_ptr(), meta.data_ptr(), meta.data_ptr() + 4 * (V + 1), _stream(dev))
     _cabi.check(rc, "fgb_sparse_build_neighbor_map")
-    _count(4)
     return out
 
 
@@ -268,7 +255,6 @@ def gray_code_from_map(neighbor_map: torch.Tensor) -> Tuple[torch.Tensor, torch.
     binary = torch.empty(n, dtype=torch.int32, device=dev)
     rc = _cabi.lib().fgb_pp_gray_code(_ptr(neighbor_map), n, V, _ptr(gray), _ptr(binary), _stream(dev))
     _cabi.check(rc, "fgb_pp_gray_code")
-    _count(1)
     return gray, binary
 
 
@@ -317,7 +303,6 @@ def sorted_idx_from_binary(binary_code: torch.Tensor, key_bits: int) -> torch.Te
     rc = lib.fgb_pp_sorted_idx(binary_code.data_ptr(), n, int(key_bits), out.data_ptr(), ws.data_ptr(), ws.numel() * 8,
                                status_word(dev).data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_pp_sorted_idx")
-    _count(1 + (int(key_bits) + 8) // 9)   # digit histogram + one kernel per 9-bit digit
     return out
 
 
@@ -334,7 +319,6 @@ def valid_signal(neighbor_map: torch.Tensor, gray_code: torch.Tensor, block_offs
     rc = lib.fgb_pp_valid_signal(_ptr(neighbor_map), _ptr(gray_code), n, V, block_offsets.data_ptr(),
                                  valid_signal_seg.data_ptr(), _ptr(vs_i), _ptr(vs_o), _ptr(order_flag), _stream(dev))
     _cabi.check(rc, "fgb_pp_valid_signal")
-    _count(1)
     return vs_i, vs_o
 
 
@@ -346,7 +330,6 @@ def tile_masks(gray_code: torch.Tensor, sorted_idx: torch.Tensor, block: int) ->
     out = torch.empty(nblk, dtype=torch.uint32, device=dev)
     rc = lib.fgb_pp_tile_masks(_ptr(gray_code), _ptr(sorted_idx), n, int(block), _ptr(out), _stream(dev))
     _cabi.check(rc, "fgb_pp_tile_masks")
-    _count(1)
     return out
 
 
@@ -357,7 +340,6 @@ def block_schedule(masks: torch.Tensor) -> torch.Tensor:
     out = torch.empty(max((nt + 1) // 2, 1), dtype=torch.uint32, device=dev)
     rc = _cabi.lib().fgb_conv_block_schedule(_ptr(masks), nt, out.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_conv_block_schedule")
-    _count(1)
     return out
 
 
@@ -372,7 +354,6 @@ def valid_kernel(masks: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     vk = torch.empty(max(nblk * 32, 1), dtype=torch.int32, device=dev)
     rc = lib.fgb_pp_valid_kernel(_ptr(masks), nblk, vk.data_ptr(), seg.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_pp_valid_kernel")
-    _count(1)
     total = int(seg[-1].item())
     return vk[:total].clone(), seg
 
@@ -418,7 +399,6 @@ def microbench_pipeline(mode: int, rows: torch.Tensor, dense: torch.Tensor, iter
     rc = _cabi.lib().fgb_microbench_pipeline(int(mode), int(stages_a), int(stages_b), int(iters), int(issue_delay), rows.data_ptr(), rows.shape[0],
                                              rows.shape[1] * 2, dense.data_ptr(), dense.numel() * dense.element_size(),
                                              ctypes.byref(ms), counters, status.data_ptr(), _stream(rows.device))
-    _count(1)
     _cabi.check(rc, "fgb_microbench_pipeline")
     check_status(rows.device)
     return float(ms.value), [int(c) for c in counters]
@@ -505,7 +485,6 @@ def conv_fprop(feats, weight_cvc, bias, neighbor_map, sorted_idx, masks, order=N
                                        _ptr(masks), _ptr(order), _ptr(out), n, n_in, Ci, Co, V, code, ws.data_ptr(),
                                        ws.numel() * 8, status_word(dev).data_ptr(), _stream(dev))
         _cabi.check(rc, "fgb_sparse_conv_fprop")
-    _count(1)   # (+ the slab reduction of a split launch, not counted)
     return out
 
 
@@ -537,7 +516,6 @@ def conv_fprop_fused(feats, weight_cvc, bias, neighbor_map, sorted_idx, masks, o
                                        ACTIVATIONS[activation], ws.data_ptr(), ws.numel() * 8, status_word(dev).data_ptr(),
                                        _stream(dev))
     _cabi.check(rc, "fgb_subm_conv_fprop_fused")
-    _count(1)
     return out, preact
 
 
@@ -574,7 +552,6 @@ def conv_dgrad(grad_out, weight_cvc, neighbor_map, sorted_idx, masks, order=None
                                        _ptr(order), _ptr(out), n, n_out, Ci, Co, V, code, ws.data_ptr(), ws.numel() * 8,
                                        status_word(dev).data_ptr(), _stream(dev))
         _cabi.check(rc, "fgb_sparse_conv_dgrad")
-    _count(2)
     return out
 
 
@@ -625,7 +602,6 @@ def conv_wgrad(grad_out, feats, vs_i, vs_o, vs_seg, splitk: Optional[int] = None
                                        _ptr(gw32), n_out, n_in, int(vs_i.shape[0]), Ci, Co, V, code, int(splitk), ws.data_ptr(),
                                        ws.numel() * 8, status_word(dev).data_ptr(), _stream(dev))
         _cabi.check(rc, "fgb_sparse_conv_wgrad")
-    _count(2)
     return gw, gw32
 
 
@@ -645,7 +621,6 @@ def bias_grad(grad_out, want_f32: bool = False, want_dtype: bool = True, out_f32
     ws = workspace(dev, "bias", nbytes)
     rc = lib.fgb_subm_conv_bias_grad(_ptr(grad_out), _ptr(gb), _ptr(gb32), n, Co, code, ws.data_ptr(), ws.numel() * 8, _stream(dev))
     _cabi.check(rc, "fgb_subm_conv_bias_grad")
-    _count(2)
     return gb, gb32
 
 
@@ -685,7 +660,6 @@ def cast_from_f32(src: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     code = _DTYPES.get(dtype, _cabi.F32_TF32)
     rc = _cabi.lib().fgb_cast_from_f32(_ptr(src), _ptr(out), src.numel(), code, _stream(src.device))
     _cabi.check(rc, "fgb_cast_from_f32")
-    _count(1)
     return out
 
 
@@ -700,7 +674,6 @@ def table_insert_3d_idx_as_val(table: torch.Tensor, key_bits: int, slots: int, c
     rc = _cabi.lib().fgb_hash_insert_3d_idx_as_val(_ptr(coords), coords.shape[0], int(W), int(H), int(D), table.data_ptr(), int(slots),
                                                    int(key_bits), status.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_hash_insert_3d_idx_as_val")
-    _count(2)
     return status
 
 
@@ -711,7 +684,6 @@ def table_lookup_3d(table: torch.Tensor, key_bits: int, slots: int, query_coords
     rc = _cabi.lib().fgb_hash_lookup_3d(_ptr(query_coords), query_coords.shape[0], int(W), int(H), int(D), table.data_ptr(), int(slots),
                                         int(key_bits), _ptr(out), _stream(dev))
     _cabi.check(rc, "fgb_hash_lookup_3d")
-    _count(1)
     return out
 
 
@@ -747,7 +719,6 @@ def hashmap_insert(hashmap_keys: torch.Tensor, hashmap_values: torch.Tensor, key
     rc = _cabi.lib().fgb_hashmap_insert(hashmap_keys.data_ptr(), hashmap_values.data_ptr(), slots, kb, vb, _ptr(keys), _ptr(values),
                                         keys.shape[0], status.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_hashmap_insert")
-    _count(1)
     _hashmap_status(dev, status)
 
 
@@ -762,7 +733,6 @@ def hashmap_lookup(hashmap_keys: torch.Tensor, hashmap_values: torch.Tensor, key
     rc = _cabi.lib().fgb_hashmap_lookup(hashmap_keys.data_ptr(), hashmap_values.data_ptr(), slots, kb, vb, _ptr(keys), keys.shape[0],
                                         _ptr(out), _stream(dev))
     _cabi.check(rc, "fgb_hashmap_lookup")
-    _count(1)
     return out
 
 
@@ -780,7 +750,6 @@ def hashmap_insert_3d(hashmap_keys: torch.Tensor, hashmap_values: torch.Tensor, 
     rc = _cabi.lib().fgb_hashmap_insert_3d(hashmap_keys.data_ptr(), hashmap_values.data_ptr(), slots, kb, vb, _ptr(coords), _ptr(values),
                                            coords.shape[0], int(W), int(H), int(D), status.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_hashmap_insert_3d")
-    _count(1)
     _hashmap_status(dev, status)
 
 
@@ -796,7 +765,6 @@ def hashmap_insert_3d_idx_as_val(hashmap_keys: torch.Tensor, hashmap_values: tor
     rc = _cabi.lib().fgb_hashmap_insert_3d_idx_as_val(hashmap_keys.data_ptr(), hashmap_values.data_ptr(), slots, kb, vb, _ptr(coords),
                                                       coords.shape[0], int(W), int(H), int(D), status.data_ptr(), _stream(dev))
     _cabi.check(rc, "fgb_hashmap_insert_3d_idx_as_val")
-    _count(1)
     _hashmap_status(dev, status)
 
 
@@ -811,7 +779,6 @@ def hashmap_lookup_3d(hashmap_keys: torch.Tensor, hashmap_values: torch.Tensor, 
     rc = _cabi.lib().fgb_hashmap_lookup_3d(hashmap_keys.data_ptr(), hashmap_values.data_ptr(), slots, kb, vb, _ptr(coords), coords.shape[0],
                                            int(W), int(H), int(D), _ptr(out), _stream(dev))
     _cabi.check(rc, "fgb_hashmap_lookup_3d")
-    _count(1)
     return out
 
 
@@ -829,7 +796,6 @@ def grid_sample_neighbor_map(table: torch.Tensor, key_bits: int, slots: int, que
     rc = _cabi.lib().fgb_grid_sample_neighbor_map(_ptr(query), B, L, int(W), int(H), int(D), table.data_ptr(), int(slots), int(key_bits),
                                                   1 if trilinear else 0, _ptr(nb), _ptr(w), _stream(dev))
     _cabi.check(rc, "fgb_grid_sample_neighbor_map")
-    _count(1)
     return (nb, w) if trilinear else nb
 
 
@@ -850,7 +816,6 @@ def indice_weighted_sum_fwd(feats: torch.Tensor, indices: torch.Tensor, weight: 
     rc = _cabi.lib().fgb_indice_weighted_sum_fwd(_ptr(feats), _ptr(indices), _ptr(weight), _ptr(out), M, C, V, _elem_code(feats.dtype),
                                                  _stream(dev))
     _cabi.check(rc, "fgb_indice_weighted_sum_fwd")
-    _count(1)
     return out
 
 
@@ -863,5 +828,4 @@ def indice_weighted_sum_bwd(grad_out: torch.Tensor, indices: torch.Tensor, weigh
     rc = _cabi.lib().fgb_indice_weighted_sum_bwd(_ptr(grad_out), _ptr(indices), _ptr(weight), _ptr(out), M, n, C, V,
                                                  _elem_code(grad_out.dtype), _stream(dev))
     _cabi.check(rc, "fgb_indice_weighted_sum_bwd")
-    _count(1)
     return out

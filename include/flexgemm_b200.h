@@ -58,6 +58,10 @@ extern "C" {
 int fgb_status_set_mirror(const int32_t* status, int32_t* mirror);
 
 const char* fgb_version(void);
+
+/* Kernels of this library launched so far in this process (not those of the
+ * toolkit libraries that it calls), whichever entry point launched them. */
+int64_t fgb_launch_count(void);
 const char* fgb_error_string(int code);
 
 /* Host-only self-test of the per-device caches the launch code keeps (SM count,

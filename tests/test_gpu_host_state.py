@@ -273,3 +273,33 @@ def test_strided_rows_of_a_batch_beyond_the_shape():
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     # the pairs of an offset are summed in row order, which differs: fp32 sums of TF32 products
     assert (outs[0][2] - outs[1][2]).abs().max() <= 1e-5 * outs[0][2].abs().max() * len(key) ** 0.5
+
+
+def test_launch_count_follows_the_kernels_that_run():
+    """The count is taken where kernels are launched, so it follows the path a call takes."""
+    from flexgemm_b200.kernels import cuda as K
+    from flexgemm_b200.ops import grid_sample, spconv
+    coords, feats, weight, bias, shape = (t.to(DEV) if torch.is_tensor(t) else t for t in orc.make_problem(8, 64, 64, "float16", seed=2))
+    shape = torch.Size(shape)
+    f, w = feats.requires_grad_(True), weight.requires_grad_(True)
+
+    def launches(call):
+        before = K.launch_count
+        out = call()
+        return K.launch_count - before, out
+    prev = K.set_conv_splitk(1)
+    try:
+        geom = (coords, shape, (3, 3, 3), (1, 1, 1))
+        assert launches(lambda: spconv.SubMConv3dFunction._compute_neighbor_cache(*geom, False))[0] == 2   # map, plan
+        count, cache = launches(lambda: spconv.SubMConv3dFunction._compute_neighbor_cache(*geom, True))
+        assert count == 3                                                                                  # and the pair lists
+        count, (out, _) = launches(lambda: spconv.sparse_submanifold_conv3d(f, coords, shape, w, bias, cache))
+        assert count == 1
+        assert launches(lambda: torch.autograd.grad(out, f, torch.ones_like(out), retain_graph=True))[0] == 1   # weight read as stored
+        # marking, counting, coordinates, maps, codes, plan, pair lists, convolution
+        assert launches(lambda: spconv.sparse_conv3d(f, coords, shape, w, bias, stride=(2, 2, 2), padding=(1, 1, 1)))[0] == 8
+        count, out = launches(lambda: grid_sample.grid_sample_3d(f, coords, shape, torch.rand(1, 100, 3, device=DEV) * 8))
+        assert count == 2
+        assert launches(lambda: torch.autograd.grad(out, f, torch.ones_like(out)))[0] == 4
+    finally:
+        K.set_conv_splitk(prev)

@@ -2,9 +2,10 @@
 
 ``build()`` compiles every ``csrc/*.cu`` into ``lib/libflexgemm_b200.so`` and
 ``csrc/host/fgb_torch.cpp`` (g++, against torch's headers) into
-``lib/_fgb_torch.so`` next to the package, so the binaries travel with a copy of
-the source tree.  It is incremental: a file is rebuilt only when its source or a
-header is newer.
+``lib/_fgb_torch.<python>.torch<version>.so`` next to the package, so the binaries
+travel with a copy of the source tree.  It is incremental: a file is rebuilt only
+when its source or a header is newer; a host module built for another Python or
+torch has another name and is never loaded.
 """
 import os
 import shutil
@@ -17,7 +18,6 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflexgemm_b200.so")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 HOST_SRC = os.path.join(CSRC, "host", "fgb_torch.cpp")
-HOST_PATH = os.path.join(LIB_DIR, "_fgb_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -37,10 +37,18 @@ def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
 
 
+def host_path() -> str:
+    """The host module of this Python and this torch: it is bound to the ABI of both."""
+    import sysconfig
+    import torch
+    return os.path.join(LIB_DIR, f"_fgb_torch.{sysconfig.get_config_var('SOABI')}.torch{torch.__version__}.so")
+
+
 def _build_host(force: bool):
     """Command and process of the torch host module's build, or None when it is up to date."""
+    path = host_path()
     newest = _newest([HOST_SRC] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE) if f.endswith(".h")])
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= newest:
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= newest:
         return None
     import sysconfig
     import torch
@@ -49,7 +57,7 @@ def _build_host(force: bool):
     cmd = [os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I" + os.path.join(tdir, "include"), "-I" + os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
-           "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_path("include"), HOST_SRC, "-o", HOST_PATH,
+           "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_path("include"), HOST_SRC, "-o", path,
            "-L" + os.path.join(tdir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
            "-L" + os.path.join(cuda, "lib64"), "-lcudart"]
     return cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)

@@ -16,7 +16,7 @@ _mod = None
 def ext():
     global _mod
     if _mod is None:
-        path = _build.HOST_PATH
+        path = _build.host_path()
         if not os.path.exists(path):
             raise RuntimeError(f"{path} not found: build it with `python -m flexgemm_b200._build`")
         spec = importlib.util.spec_from_file_location("_fgb_torch", path, loader=importlib.machinery.ExtensionFileLoader("_fgb_torch", path))

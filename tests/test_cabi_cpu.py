@@ -40,6 +40,18 @@ def test_host_slot_keeps_the_sequence_word_to_itself():
     assert not any(re.search(r"= *\w*\.?host_words;", t) for t in text.values())
 
 
+def test_host_module_belongs_to_this_python_and_torch(lib, monkeypatch):
+    """A host module built for another torch is not the one that is loaded, and the build makes a new one."""
+    path = _build.host_path()
+    assert os.path.exists(path) and _build._build_host(False) is None
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    assert _build.host_path() != path and not os.path.exists(_build.host_path())
+    started = []
+    monkeypatch.setattr(_build.subprocess, "Popen", lambda cmd, **kw: started.append(cmd))
+    cmd, _ = _build._build_host(False)
+    assert started == [cmd] and _build.host_path() in cmd
+
+
 def test_version_and_errors(lib):
     assert b"sm_100a" in lib.fgb_version()
     assert _cabi.error_string(0) == "ok"

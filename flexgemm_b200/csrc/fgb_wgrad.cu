@@ -832,6 +832,12 @@ extern "C" int fgb_wgrad_set_row_bands(int bands) {
   return fgb::g_row_bands.exchange(bands, std::memory_order_relaxed);
 }
 
+static std::atomic<int> g_wgrad_direct{0};
+extern "C" int fgb_wgrad_set_direct(int mode) {
+  if (mode < 0 || mode > 2) return FGB_E_SIZE;
+  return g_wgrad_direct.exchange(mode, std::memory_order_relaxed);
+}
+
 extern "C" int fgb_wgrad_default_splitk(int64_t n_pairs, int Ci, int Co, int V, int dtype) {
   using namespace fgb;
   const int eb = elem_bytes(dtype);
@@ -917,6 +923,8 @@ constexpr int kBiasCtas = 148;  // the CTAs of a launch's first wave share the r
 // the direct way where there are enough tiles of channels (C = 1024: 54 slabs of 4 MB each; RES=32, fp16: 129 + 64 us)
 // or hardly any rows.  The longest list, the centre offset's, has at most n_out pairs.
 static bool wgrad_direct(const WgradPlan& w, int64_t n_out, int64_t n_pairs, int Ci, int Co, int V, int splitk) {
+  const int forced = g_wgrad_direct.load(std::memory_order_relaxed);
+  if (forced != 0) return forced == 1;
   const int P = device_sm_count();
   const int64_t tiles = int64_t(w.co_groups) * w.ci_tiles;
   const double stage_us = 0.75 * (w.a_chunks + w.b_chunks) * w.kb * 128 / 65536.0;

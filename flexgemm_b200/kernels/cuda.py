@@ -373,6 +373,14 @@ def set_wgrad_row_bands(bands: int) -> int:
     return prev
 
 
+def set_wgrad_direct(mode: int) -> int:
+    """Weight gradient without slabs: 0 = where the sizes ask for it, 1 = always, 2 = never; returns the previous setting."""
+    prev = _cabi.lib().fgb_wgrad_set_direct(int(mode))
+    if prev < 0:
+        _cabi.check(prev, "fgb_wgrad_set_direct")
+    return prev
+
+
 def set_conv_splitk(splits: int) -> int:
     """Split-K of fprop / dgrad: 0 = automatic (small launches only), 1 = off, k = k shares; returns the previous setting."""
     prev = _cabi.lib().fgb_conv_set_splitk(int(splits))

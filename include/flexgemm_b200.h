@@ -320,6 +320,12 @@ int fgb_subm_conv_wgrad(const void* grad_out, const void* feats,
  * the L2 together, bands of about 8 MB of rows beyond that), 1 .. 64 = fixed.  Returns the previous value.  Process-wide tuning knob; read at launch. */
 int fgb_wgrad_set_row_bands(int bands);
 
+/* Whether fgb_*_conv_wgrad and fgb_wgrad_call_run write the result directly, one
+ * unit per offset, or through split-K slabs and their ordered sum: 0 = chosen from
+ * the sizes, 1 = directly (where no fp32 copy is asked for), 2 = slabs.  Returns the
+ * previous value.  Process-wide tuning knob; read at launch. */
+int fgb_wgrad_set_direct(int mode);
+
 /* Host-side replay of how a wgrad launch splits the pair lists among its CTAs, for
  * tests (no GPU involved; seg and block_offsets are HOST arrays here, block_offsets
  * may be null).  For unit u (offset-major) and band b,

@@ -124,9 +124,10 @@ def test_grid_sample_matches_separate_kernels(C, dtype, mode, points, volume):
 @pytest.mark.parametrize("n,shuffle", [(1, False), (255, True), (3000, False), (8192, True), (40000, True)])
 def test_strided_build_matches_hash_path(ksize, stride, pad, dil, n, shuffle):
     """Output coordinates and maps made on the bit grid against the hash set, sort and table of the generic calls."""
+    from flexgemm_b200 import _native
     from flexgemm_b200.kernels import cuda as K
     from flexgemm_b200.ops import utils
-    from flexgemm_b200.ops.spconv import SparseConv3dFunction, sparse_conv3d
+    from flexgemm_b200.ops.spconv import SparseConv3dFunction, SparseConv3dNeighborCache, sparse_conv3d
     g = torch.Generator().manual_seed(n)
     W, H, D = 40, 33, 70
     flat = torch.randperm(2 * W * H * D, generator=g)[:n].sort().values
@@ -138,12 +139,17 @@ def test_strided_build_matches_hash_path(ksize, stride, pad, dil, n, shuffle):
     geom = (shape, ksize, stride, pad, dil)
     want_oc = K.sparse_out_coords(coords, *geom, 1.1, 0)
     assert torch.equal(SparseConv3dFunction._get_output_coords(coords, *geom), want_oc)
+    on_bits = _native.ext().strided_coords(coords, *geom)   # None where the call is left to the hash path
+    assert on_bits is not None and torch.equal(on_bits, want_oc)
     feats = torch.randn(n, 8, generator=g).half().to(DEV).requires_grad_(True)
     weight = torch.randn(8, *ksize, 8, generator=g).half().to(DEV)
-    out, oc, cache = sparse_conv3d(feats, coords, shape, weight, None, stride=stride, padding=pad, dilation=dil)
-    assert torch.equal(oc, want_oc) and out.shape == (oc.shape[0], 8)
-    if oc.shape[0] == 0:
+    native = _native.ext().strided_conv(SparseConv3dNeighborCache, feats, coords, shape, weight, None, stride, pad, dil, True)
+    if want_oc.shape[0] == 0:
+        assert native is None and sparse_conv3d(feats, coords, shape, weight, None, stride=stride, padding=pad, dilation=dil)[0].shape == (0, 8)
         return
+    out, oc, cache = native
+    assert torch.equal(oc, want_oc) and out.shape == (oc.shape[0], 8)
+    assert torch.equal(sparse_conv3d(feats, coords, shape, weight, None, stride=stride, padding=pad, dilation=dil)[0], out)
     V = ksize[0] * ksize[1] * ksize[2]
     table, bits = utils.init_table(shape, max(2 * n, 1), DEV)
     want = K.sparse_build_neighbor_map(coords, oc, *geom, table, bits, max(2 * n, 1), True)
@@ -189,26 +195,35 @@ def test_halved_items_at_the_end_of_a_launch(n, co, dtype):
 @pytest.mark.parametrize("res,ci,co,dtype,tf32", [(8, 40, 40, "float16", True), (8, 1024, 264, "bfloat16", True), (16, 512, 1024, "float16", True),
                                                   (8, 136, 300, "float32", True), (8, 260, 132, "float32", False), (2, 16, 16, "float16", True)])
 def test_weight_gradient_without_slabs(res, ci, co, dtype, tf32):
-    """Small inputs and wide channels: every offset is one unit that writes its result directly.  Against the slab path
-    (which the call with an fp32 copy takes): the same products, summed in fp32 in another grouping."""
+    """Every offset as one unit that writes its result directly, against slabs and their ordered sum: the same products,
+    summed in fp32 in another grouping.  The kernels launched show which way a call took."""
     from flexgemm_b200.kernels import config
     from flexgemm_b200.kernels import cuda as K
     from flexgemm_b200.ops import spconv
     coords, feats, weight, bias, shape = orc.make_problem(res, ci, co, dtype, seed=res + co)
     config.allow_tf32 = tf32
+    got, launches = {}, {}
     try:
         f, w, b = (t.to(DEV).requires_grad_(True) for t in (feats, weight, bias))
         gout = torch.randn(coords.shape[0], co, generator=torch.Generator().manual_seed(2)).to(f.dtype).to(DEV)
-        out, cache = spconv.sparse_submanifold_conv3d(f, coords.to(DEV), torch.Size(shape), w, b)
-        gw, gb = torch.autograd.grad(out, (w, b), gout)
+        for mode in (1, 2, 0):
+            K.set_wgrad_direct(mode)
+            out, cache = spconv.sparse_submanifold_conv3d(f, coords.to(DEV), torch.Size(shape), w, b)
+            before = K.launch_count
+            got[mode] = torch.autograd.grad(out, (w, b), gout)
+            launches[mode] = K.launch_count - before
         _, gw32 = K.conv_wgrad(gout, f.detach(), cache["valid_signal_i"], cache["valid_signal_o"], cache["valid_signal_seg"], want_f32=True)
         gb32 = K.bias_grad(gout, want_f32=True)[1]
     finally:
+        K.set_wgrad_direct(0)
         config.allow_tf32 = True
+    passes = 1 if tf32 or dtype != "float32" else 3
+    assert launches[2] == launches[1] + passes and launches[0] in (launches[1], launches[2])
     ulp = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -24}[dtype]
-    for got, want, terms in ((gw.view(co, 27, ci), gw32, 27 + len(coords)), (gb, gb32, len(coords))):
-        err = (got.double() - want.double()).abs()
-        assert torch.all(err <= want.double().abs() * ulp + want.double().abs().max() * terms * 2.0 ** -24 + 1e-7)
+    for gw, gb in got.values():
+        for x, want, terms in ((gw.view(co, 27, ci), gw32, 27 + len(coords)), (gb, gb32, len(coords))):
+            err = (x.double() - want.double()).abs()
+            assert torch.all(err <= want.double().abs() * ulp + want.double().abs().max() * terms * 2.0 ** -24 + 1e-7)
     K.check_status(DEV)
 
 

@@ -839,9 +839,11 @@ int64_t igemm_partial_bytes(int64_t n, int nout, int V) {
 // accumulator, the other left out of gather, MMA and write-out) takes 0.6 to 0.7 of the whole block's time -- the weight
 // tile is fetched for both -- so the items beyond the whole waves, the cheapest of the schedule, go out as two halves
 // each where the halves fit one wave.  No sum is cut: every row sees the same products in the same order.
-// fprop / dgrad, us: RES=128 C=256 fp16 106 -> 97, C=96 bf16 50 -> 45, C=512 TF32 626 / 645 -> 592 / 613; RES=256 C=256
-// 260 -> 254.  Beyond six waves the rest is a few percent and the items' spread hides it.  Halving every item of a launch
-// below one wave lost (156 items, 239 -> 295 us): the halves make two waves.
+// A forward pass on an existing cache without and with halves, us: RES=128 (1.1 waves) C=64 fp16 29.1 -> 26.8, C=128 41.4 ->
+// 37.3, C=256 97.8 -> 90.2, C=96 bf16 39.4 -> 35.4, C=512 TF32 612 -> 587; RES=140 (1.3) C=256 113 -> 107; RES=184 (2.3) C=64
+// 43.6 -> 42.3, C=256 169 -> 163; RES=256 (4.3) C=64 62.7 -> 62.8, C=256 281 -> 277; RES=280 (5.2) C=64 73.3 -> 74.3, C=256
+// 340 -> 336.  Beyond six waves the rest is a few percent and the items' spread hides it.  Halving every item of a launch
+// below one wave lost (156 items, 239 -> 295 us, measured with the older MMA issue): the halves make two waves.
 // (Shares of the offsets with partial accumulators in memory, added up by the last CTA, balance better on paper but the
 // slabs cost more than they win: 256 -> 293 us at RES=256, C=256, and 545 us in the TF32 case.)
 static int64_t tail_items(int64_t T) {

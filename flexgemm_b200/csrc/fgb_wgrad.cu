@@ -918,23 +918,26 @@ struct BiasJob {
 constexpr int kBiasCtas = 148;  // the CTAs of a launch's first wave share the rows
 
 // Whether a launch gives every offset one unit and writes the result itself, without slabs and the sum over them.  Costs
-// in microseconds from measured rates: a 64 KB stage 0.75, slab bytes written and read again at 4 TB/s, 5 for the second
-// launch.  Slabs win where one list would be walked by one CTA per tile while the device idles (few channels, many rows);
-// the direct way where there are enough tiles of channels (C = 1024: 54 slabs of 4 MB each; RES=32, fp16: 129 + 64 us)
-// or hardly any rows.  The longest list, the centre offset's, has at most n_out pairs.
+// in microseconds: 0.3 a stage and 0.5 per 64 KB of it, slab bytes written and read again at 2.5 TB/s, 5 for the second
+// launch.  Slabs win where one list would be walked by one CTA per tile while the device idles (few channels, many rows:
+// RES=128, C=512 fp16 204 us against 420 direct); the direct way where there are enough tiles of channels (C=1024: 736
+// against 935, at RES=32 94 against 214) or hardly any rows (RES=8, C=64: 12 against 17).  The longest list, the centre
+// offset's, has at most n_out pairs.  The rates were fitted to both ways measured at eight sizes from RES=8 to 4 x 64 and
+// 128, eleven widths from 16 to 1024, fp16 and TF32: the choice costs more than 3 % in 6 of the 176, 17 % at most (0.75 per
+// 64 KB, 4 TB/s and a quarter of the longest list as a tail: 11, up to 27 %).
 static bool wgrad_direct(const WgradPlan& w, int64_t n_out, int64_t n_pairs, int Ci, int Co, int V, int splitk) {
   const int forced = g_wgrad_direct.load(std::memory_order_relaxed);
   if (forced != 0) return forced == 1;
   const int P = device_sm_count();
   const int64_t tiles = int64_t(w.co_groups) * w.ci_tiles;
-  const double stage_us = 0.75 * (w.a_chunks + w.b_chunks) * w.kb * 128 / 65536.0;
+  const double stage_us = 0.3 + 0.5 * (w.a_chunks + w.b_chunks) * w.kb * 128 / 65536.0;
   const double stages = double(ceil_div(n_pairs, w.kb)) + V / 2.0;
   const double longest = double(std::min(ceil_div(n_out, w.kb), ceil_div(n_pairs, w.kb)));
   const double even = stages * tiles / P;
   const double units = std::min<double>(target_units(w, V, splitk), stages);
   const double waves = std::max(1.0, double(ceil_div(int64_t(units) * tiles, P)));
-  const double split = std::max(even, waves) * stage_us + 2e-6 * units * Ci * Co * 4 / 4.0 + 5.0;
-  return std::max(longest, even + longest / 4) * stage_us < split;
+  const double split = std::max(even, waves) * stage_us + 2e-6 * units * Ci * Co * 4 / 2.5 + 5.0;
+  return std::max(longest, even) * stage_us < split;
 }
 
 // one wgrad pass over operands of element type `dtype` (never FGB_F32_IEEE): partial slabs, then the ordered sum

@@ -62,14 +62,14 @@ struct HashLookupSmem {
 };
 
 template <int kKeyBits, bool kGeneral>
-__device__ __forceinline__ void hash_lookup(HashLookupSmem& sm, const int4* __restrict__ coords, uint32_t n, const Grid3& g,
+__device__ __forceinline__ void hash_lookup(HashLookupSmem& sm, uint32_t block, const int4* __restrict__ coords, uint32_t n, const Grid3& g,
                                             const Stencil& st, void* table_mem, uint32_t slots, const MapOut& o,
                                             uint32_t* __restrict__ nbr_bwd) {
   int4* s_coord = sm.coord;
   int4* s_delta = sm.delta;
   uint32_t* s_gray = sm.gray;
   uint32_t* s_count = sm.count;
-  const uint32_t n0 = blockIdx.x * kMapBlock;
+  const uint32_t n0 = block * kMapBlock;
   const uint32_t nv = min(static_cast<uint32_t>(kMapBlock), n - n0);
   const int t = threadIdx.x;
   const int V = st.V;
@@ -124,7 +124,7 @@ __device__ __forceinline__ void hash_lookup(HashLookupSmem& sm, const int4* __re
     }
   }
   __syncthreads();
-  if (t < V) o.block_counts[static_cast<size_t>(t) * o.nblk + blockIdx.x] = s_count[t];
+  if (t < V) o.block_counts[static_cast<size_t>(t) * o.nblk + block] = s_count[t];
   emit_codes(o, n0, nv, V, t < nv ? s_gray[t] : 0u, reinterpret_cast<uint32_t*>(&sm));
 }
 
@@ -140,21 +140,30 @@ __global__ void __launch_bounds__(kMapBlock)
   chain_release();
   chain_wait();
   extern __shared__ __align__(16) uint8_t s_map_mem[];
-  hash_lookup<kKeyBits, true>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), coords, n, g, st, table_mem, slots, o, nbr_bwd);
+  hash_lookup<kKeyBits, true>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), blockIdx.x, coords, n, g, st, table_mem, slots, o, nbr_bwd);
 }
 
-// CTA v turns block_counts[v, :] into exclusive offsets in place and leaves the
+// CTA v < V turns block_counts[v, :] into exclusive offsets in place and leaves the
 // total of offset v in seg[v + 1].  With `fin.done` the CTA that ends last also turns the totals into the segment table
 // (what seg_prefix_kernel does as a launch of its own), adds the key-order word and the build's status behind it, and --
 // fin.host_words -- stores all of them straight into host memory, a sequence number last: the host reads the pair count
 // by watching that word.  (Against a copy and an event in the stream: two driver calls and about 5 us less, and the
 // kernels after the scan stay chained.)
 __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__ block_counts, uint32_t nblk, uint32_t* __restrict__ seg,
-                                                          ScanFinish fin) {
-  chain_release();
-  chain_wait();
+                                                          ScanFinish fin, uint32_t V, HistJob job) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_carry;
+  __shared__ uint32_t s_hist[kSortMaxPasses * kSortDigits];
+  chain_release();
+  if (blockIdx.x >= V) {
+    for (int i = threadIdx.x; i < kSortMaxPasses * kSortDigits; i += 1024) s_hist[i] = 0;
+    chain_wait();
+    if (*job.unsorted == 0u) return;
+    __syncthreads();
+    digit_histograms(s_hist, job.codes, job.n, static_cast<int>(V), blockIdx.x - V, gridDim.x - V, job.hist);
+    return;
+  }
+  chain_wait();
   uint32_t* row = block_counts + static_cast<size_t>(blockIdx.x) * nblk;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   if (t == 0) s_carry = 0;
@@ -191,9 +200,8 @@ __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__
     seg[blockIdx.x + 1] = s_carry;
     if (fin.done != nullptr) {
       __threadfence();
-      if (atomicAdd(fin.done, 1u) == gridDim.x - 1) {  // every total is written
+      if (atomicAdd(fin.done, 1u) == V - 1) {  // every total is written
         __threadfence();
-        const uint32_t V = gridDim.x;
         uint32_t acc = 0;
         for (uint32_t v = 1; v <= V; ++v) {
           acc += *reinterpret_cast<volatile uint32_t*>(&seg[v]);
@@ -209,8 +217,11 @@ __global__ void __launch_bounds__(1024) block_scan_kernel(uint32_t* __restrict__
   }
 }
 
-cudaError_t launch_block_scan(uint32_t* block_counts, uint32_t nblk, int V, uint32_t* seg, const ScanFinish& fin, cudaStream_t s) {
-  return launch_chained(block_scan_kernel, dim3(V), dim3(1024), 0, s, block_counts, nblk, seg, fin);
+cudaError_t launch_block_scan(uint32_t* block_counts, uint32_t nblk, int V, uint32_t* seg, const ScanFinish& fin, const HistJob& job,
+                              cudaStream_t s) {
+  const int64_t extra = job.hist != nullptr ? std::min<int64_t>(ceil_div(job.n, 1024), 256) : 0;
+  return launch_chained(block_scan_kernel, dim3(static_cast<unsigned>(V + extra)), dim3(1024), 0, s, block_counts, nblk, seg, fin,
+                        static_cast<uint32_t>(V), job);
 }
 
 __global__ void seg_prefix_kernel(uint32_t* seg, int V) {
@@ -370,18 +381,42 @@ static size_t map_smem_bytes(int V) {
 template <int kKeyBits, bool kUnit>
 __global__ void __launch_bounds__(kMapBlock)
     subm_map_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, const uint2* __restrict__ col_table, void* table_mem,
-                    uint32_t slots, MapOut o, const uint32_t* __restrict__ unsorted) {
+                    uint32_t slots, MapOut o, const uint32_t* __restrict__ unsorted, bool hash_apart) {
   chain_release();
   extern __shared__ __align__(16) uint8_t s_map_mem[];
   chain_wait();
   if (unsorted == nullptr || *unsorted != 0u) {
-    hash_lookup<kKeyBits, false>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), coords, n, g, st, table_mem, slots, o, nullptr);
+    if (hash_apart) return;
+    o.digit_hist = nullptr;  // rows in no order: see HistJob
+    hash_lookup<kKeyBits, false>(*reinterpret_cast<HashLookupSmem*>(s_map_mem), blockIdx.x, coords, n, g, st, table_mem, slots, o, nullptr);
   } else {
     int4* s_coord = reinterpret_cast<int4*>(s_map_mem);
     uint32_t* s_count = reinterpret_cast<uint32_t*>(s_coord + kMapBlock);
     column_lookup<kUnit>(s_count + 32, s_coord, s_count, reinterpret_cast<uint32_t*>(s_map_mem), coords, n, g, st, col_table, o);
   }
 }
+
+// The hash lookup of many rows as a kernel of its own (see kHashApart).
+template <int kKeyBits>
+__global__ void __launch_bounds__(kMapBlock)
+    subm_hash_kernel(const int4* __restrict__ coords, uint32_t n, Grid3 g, Stencil st, void* table_mem, uint32_t slots, MapOut o,
+                     const uint32_t* __restrict__ unsorted) {
+  __shared__ __align__(16) HashLookupSmem sm;
+  chain_release();
+  chain_wait();
+  if (unsorted != nullptr && *unsorted == 0u) return;
+  o.digit_hist = nullptr;  // rows in no order: see HistJob
+  for (uint32_t block = blockIdx.x; block < o.nblk; block += gridDim.x) {
+    hash_lookup<kKeyBits, false>(sm, block, coords, n, g, st, table_mem, slots, o, nullptr);
+    __syncthreads();
+  }
+}
+// Rows from which the hash lookup runs apart from the column lookup: in the common kernel it shares the SM with the map
+// tiles of the other path, 32 KB of shared memory per CTA, which leaves its scattered probes hardly any L1 to be in flight
+// in: inference build and a narrow convolution of 5.3 M shuffled voxels 5479 us in the common kernel, 3343 apart (of 164 k:
+// 287 and 244); the histograms of HistJob, 34 and 17 us of that.  Rows in key order pay a launch that returns at once (164 k:
+// 161.4 -> 163.1 us), which for fewer rows is not made up for.
+constexpr uint32_t kHashApart = 1u << 17;
 
 // Memory of a build, and where its kernels leave things
 struct BuildMem {
@@ -411,15 +446,21 @@ static cudaError_t launch_build(const int4* c4, uint32_t n, const Grid3& g, cons
   }
   const unsigned igrid = std::min<unsigned>(nblk, 148 * 8);
   chain.add(launch_chained(hash_insert_kernel<kKeyBits>, dim3(igrid), dim3(kMapBlock), 0, s, c4, n, g, m.table, m.slots, m.build_status, unsorted));
+  const bool apart = n >= kHashApart;
+  if (apart) {
+    const unsigned each = (nblk + 8191u) / 8192u;  // blocks per CTA: few, or the last CTAs' blocks run alone
+    chain.add(launch_chained(subm_hash_kernel<kKeyBits>, dim3((nblk + each - 1) / each), dim3(kMapBlock), 0, s, c4, n, g, st, m.table, m.slots, o,
+                             unsorted));
+  }
   const bool unit = st.Kw == 3 && st.Kh == 3 && st.Kd == 3 && st.Dw == 1 && st.Dh == 1 && st.Dd == 1;
   const uint2* cols = m.columns;
   if (unit)
     chain.add(launch_chained(subm_map_kernel<kKeyBits, true>, dim3(nblk), dim3(kMapBlock), map_smem_bytes(st.V), s, c4, n, g, st, cols, m.table,
-                             m.slots, o, unsorted));
+                             m.slots, o, unsorted, apart));
   else
     chain.add(launch_chained(subm_map_kernel<kKeyBits, false>, dim3(nblk), dim3(kMapBlock), map_smem_bytes(st.V), s, c4, n, g, st, cols, m.table,
-                             m.slots, o, unsorted));
-  chain.add(launch_block_scan(o.block_counts, nblk, st.V, m.seg, m.fin, s));
+                             m.slots, o, unsorted, apart));
+  chain.add(launch_block_scan(o.block_counts, nblk, st.V, m.seg, m.fin, HistJob{o.binary, n, o.digit_hist, m.fin.unsorted}, s));
   return chain.first;
 }
 
@@ -460,7 +501,7 @@ static int build_general_impl(const int32_t* in_coords, uint32_t n_in, const int
   const MapOut o{nbr, gray, binary, block_counts, nullptr, nblk};
   launch(sparse_lookup_kernel<kKeyBits>, nblk, kMapBlock, hash_smem_bytes(st.V), s,
          reinterpret_cast<const int4*>(out_coords), n_out, g, st, table, slots, o, nbr_bwd);
-  launch(block_scan_kernel, st.V, 1024, 0, s, block_counts, nblk, seg, ScanFinish{});
+  launch(block_scan_kernel, st.V, 1024, 0, s, block_counts, nblk, seg, ScanFinish{}, st.V, HistJob{});
   launch(seg_prefix_kernel, 1, 32, 0, s, seg, st.V);
   return launch_status();
 }

@@ -32,40 +32,14 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr uint32_t kFlagAggregate = 1u << 30, kFlagPrefix = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr uint32_t kLookbackPolls = 1u << 22;   // of >= 32 ns each: far beyond any legitimate wait
 
-// hist[p * 512 + d] += number of codes whose digit p is d, for every pass p < passes
-__global__ void __launch_bounds__(kSortThreads) sort_histogram_kernel(const int32_t* __restrict__ codes, uint32_t n, int passes, uint32_t flip,
+__global__ void __launch_bounds__(kSortThreads) sort_histogram_kernel(const int32_t* __restrict__ codes, uint32_t n, int key_bits,
                                                                       uint32_t* __restrict__ hist) {
   __shared__ uint32_t s_h[kSortMaxPasses * kDigits];
   chain_release();
-  for (int i = threadIdx.x; i < passes * kDigits; i += kSortThreads) s_h[i] = 0;
+  for (int i = threadIdx.x; i < sort_passes_of(key_bits) * kDigits; i += kSortThreads) s_h[i] = 0;
   chain_wait();  // set-up above overlaps the tail of the kernel before; global memory only from here on
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
-  const uint32_t begin = blockIdx.x * per, end = min(n, begin + per);
-  // whole warps walk the range so that every lane takes part in the votes
-  for (uint32_t i0 = begin + (threadIdx.x & ~31u); i0 < end; i0 += kSortThreads) {
-    const uint32_t i = i0 + lane;
-    const bool ok = i < end;
-    const uint32_t key = ok ? static_cast<uint32_t>(__ldg(&codes[i])) ^ flip : 0u;
-    const unsigned valid = __ballot_sync(0xffffffffu, ok);  // a prefix of the lanes
-    // neighbouring voxels mostly share their code: the warp's keys are cut into runs of equal keys, and the first
-    // lane of a run adds the run's length to the key's bin of every pass (equal keys share all their digits)
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const bool head = ok && (lane == 0 || key != prev);
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    if (head) {
-      const unsigned later = heads & ~((2u << lane) - 1u);  // run heads above this lane
-      const int next = later != 0u ? __ffs(later) - 1 : __popc(valid);
-      const uint32_t len = static_cast<uint32_t>(next - lane);
-      for (int p = 0; p < passes; ++p) atomicAdd(&s_h[p * kDigits + ((key >> (p * kDigitBits)) & (kDigits - 1))], len);
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < passes * kDigits; i += kSortThreads) {
-    const uint32_t c = s_h[i];
-    if (c != 0u) atomicAdd(&hist[i], c);
-  }
+  digit_histograms(s_h, codes, n, key_bits, blockIdx.x, gridDim.x, hist);
 }
 
 __device__ __forceinline__ uint32_t load_status(const uint32_t* p) {
@@ -290,7 +264,7 @@ extern "C" int fgb_pp_sorted_idx(const int32_t* binary_code, int64_t n, int key_
   // keys per CTA of the histogram: 1024 up to 400 k keys, 2048 beyond (measured: 42 / 43.5 / 46.5 us for the whole sort at
   // 164 k keys with 1024 / 2048 / 4096; 70.5 / 68.7 / 70.6 us at 660 k), at most eight CTAs per SM
   const unsigned hist_grid = static_cast<unsigned>(std::min<int64_t>(ceil_div(n, n <= 400000 ? 1024 : 2048), 148 * 8));
-  launch(sort_histogram_kernel, hist_grid, kSortThreads, 0, s, binary_code, static_cast<uint32_t>(n), sort_passes_of(key_bits), sort_flip_of(key_bits),
+  launch(sort_histogram_kernel, hist_grid, kSortThreads, 0, s, binary_code, static_cast<uint32_t>(n), key_bits,
                                                           hist);
   const cudaError_t e = launch_sort_passes(binary_code, n, key_bits, sorted_idx, ws, L, hist, reinterpret_cast<uint32_t*>(ws + sort_lookback_off(L)),
                                            status, s);

@@ -387,7 +387,7 @@ extern "C" int fgb_strided_build(const fgb_strided_call* c, void* stream) {
     return chain.first != cudaSuccess ? cuda_status(chain.first) : launch_status();
   }
   ScanFinish fin{words, nullptr, nullptr, c->host_words, c->host_seq};
-  chain.add(launch_block_scan(c->block_offsets, nblk, V, c->meta, fin, s));
+  chain.add(launch_block_scan(c->block_offsets, nblk, V, c->meta, fin, HistJob{}, s));
   if (chain.first == cudaSuccess)
     chain.add(launch_sort_passes(codes, c->n_out, V, c->sorted_idx, mem + L.buf_off, L.sort, hist, reinterpret_cast<uint32_t*>(mem + L.look_off), c->status, s));
   if (chain.first == cudaSuccess) chain.add(launch_tile_plan(c->gray_code, c->sorted_idx, c->n_out, c->tile_masks, c->block_order, words + 1, s));

@@ -17,6 +17,7 @@ def u32(t):
 @pytest.mark.parametrize("n,ksize,shuffle,volume", [(1, (3, 3, 3), False, 64), (127, (3, 3, 3), False, 64), (128, (3, 3, 3), True, 64),
                                                     (257, (3, 1, 3), False, 64), (1025, (3, 3, 3), True, 64), (4097, (1, 1, 1), False, 64),
                                                     (8192, (3, 3, 3), True, 64), (8193, (3, 3, 3), False, 64), (2049, (3, 1, 1), True, 2048), (33000, (3, 3, 3), False, 64), (33000, (3, 3, 3), True, 2048),
+                                                    (131071, (3, 3, 3), True, 64), (131072, (3, 3, 3), True, 64), (131073, (3, 1, 3), False, 64), (140001, (3, 3, 3), True, 2048),
                                                     (3000, (1, 1, 31), False, 64), (1, (1, 1, 1), False, 64)])
 def test_cache_build_matches_single_calls(n, ksize, shuffle, volume):
     from flexgemm_b200.kernels import cuda as K

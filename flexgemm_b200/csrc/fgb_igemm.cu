@@ -473,10 +473,10 @@ __global__ void __launch_bounds__(kIgemmThreads, 1)
   } else if (warp == 5) {
     // ------------------------------------------------------------------- MMA
     // The whole warp walks the loop and one elected lane issues.  Under `if (lane == 0)` the compiler does not know that a
-    // single thread is active, and an MMA takes its descriptors from registers that are uniform over the warp: every MMA
-    // of the loop cost ~200 cycles of the lane, more than the MMA itself takes below 256 columns (measured with clock64:
-    // 1640 cycles a stage at C = 64, 92 % of the lane's time, 6 % waiting for operands).  Forward + backward, us: RES=128
-    // C=512 TF32 1911 -> 1615, 4 x RES=64 C=512 bf16 (4 convs) 3392 -> 2972, RES=256 C=256 fp16 878 -> 788.
+    // single thread is active, and an MMA takes its descriptors from registers that are uniform over the warp.  The lane's
+    // cycles a stage, waits left out (clock64): 1640 at C = 64 (7.8 MMAs) and 1247 at C = 32 (3.9) before, 1120 and 983 now --
+    // about 110 and 39 an MMA; some 800 a stage stayed.  Forward + backward, us: RES=128 C=512 TF32 1911 -> 1615, 4 x RES=64
+    // C=512 bf16 (4 convs) 3392 -> 2972, RES=256 C=256 fp16 878 -> 788.
     uint32_t s = 0, ph = 0, item = 0;
     uint32_t set = 0, set_ph = 0;  // accumulator set of the item and its phase bit
     uint32_t mblk = 0, ntile = 0;

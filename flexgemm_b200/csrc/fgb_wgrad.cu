@@ -178,9 +178,8 @@ __host__ __device__ __forceinline__ uint32_t wg_band_share(uint32_t nkb, uint32_
 
 // Column sums of this CTA's share of the rows of `src` ([rows, Co], Co * sizeof(T) a multiple of 16), written to
 // partial[cta, :].  Run by the 128 threads of the epilogue warps while the CTA's pipeline fills and runs: they have
-// nothing else to do until the accumulator is complete, so the bias gradient costs no launch and next to no time
-// (before: a kernel pair on a side stream with its fork and join, 24 + 12 us beside the conv kernels at N = 164 k,
-// C = 256, and five driver calls).  A thread owns one 16-byte column of every nrg-th row, four rows in flight.
+// nothing else to do until the accumulator is complete, so the bias gradient costs no launch and next to no time (a kernel
+// pair of its own takes 24 + 12 us at N = 164 k, C = 256).  A thread owns one 16-byte column of every nrg-th row, four rows in flight.
 template <typename T>
 __device__ __forceinline__ void bias_share(const T* __restrict__ src, int64_t rows, int Co, float* __restrict__ partial, int cta, int ctas,
                                            float* s_acc /* [128 * 16 / sizeof(T)] */, int tid) {
@@ -474,8 +473,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) subm_wgrad_kernel(const WgradPa
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------- MMA
-    // the whole warp walks the loop and one elected lane issues: under `if (lane == 0)` every MMA cost the lane ~230 cycles
-    // whatever its width (1840 cycles a stage of eight at C = 64 and at C = 32, 6 % of them waiting for operands)
+    // the whole warp walks the loop and one elected lane issues (as in fprop): under `if (lane == 0)` a stage of eight MMAs took
+    // the lane 1840 cycles at C = 64 and at C = 32, 6 % of them waiting for operands; now 1290
     const int chunks_per_m = 128 / kChunkElems;  // 128-byte chunks per 128 accumulator rows
     int s = 0;
     uint32_t ph = 0;
@@ -628,40 +627,40 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
   chain_wait();  // the slabs are complete
   // a CTA walks over the [Co, Ci] elements: its plan (some microseconds) is made once, not once per 1024 of them
   for (int64_t e = (blockIdx.x * int64_t(256) + threadIdx.x) * 4; e < int64_t(Co) * Ci; e += int64_t(gridDim.x) * 1024) {
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* src = partial + size_t(first) * Co * Ci + e;
-  const size_t slab = size_t(Co) * Ci;
-  uint32_t s = 0;
-  for (; s + 4 <= count; s += 4) {  // four loads in flight, added in slab order
-    const float4 t0 = __ldg(reinterpret_cast<const float4*>(src + (s + 0) * slab));
-    const float4 t1 = __ldg(reinterpret_cast<const float4*>(src + (s + 1) * slab));
-    const float4 t2 = __ldg(reinterpret_cast<const float4*>(src + (s + 2) * slab));
-    const float4 t3 = __ldg(reinterpret_cast<const float4*>(src + (s + 3) * slab));
-    acc.x += t0.x, acc.y += t0.y, acc.z += t0.z, acc.w += t0.w;
-    acc.x += t1.x, acc.y += t1.y, acc.z += t1.z, acc.w += t1.w;
-    acc.x += t2.x, acc.y += t2.y, acc.z += t2.z, acc.w += t2.w;
-    acc.x += t3.x, acc.y += t3.y, acc.z += t3.z, acc.w += t3.w;
-  }
-  for (; s < count; ++s) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(src + s * slab));
-    acc.x += t.x, acc.y += t.y, acc.z += t.z, acc.w += t.w;
-  }
-  const int co = static_cast<int>(e / Ci), ci = static_cast<int>(e % Ci);
-  const int64_t o = (int64_t(co) * V + v) * Ci + ci;
-  if (accumulate) {  // later passes of the fp32-accurate mode add to what an earlier pass wrote (fp32 outputs only)
-    const float* prev = out_f32 ? out_f32 : reinterpret_cast<const float*>(out);
-    const float4 t = *reinterpret_cast<const float4*>(prev + o);
-    acc.x += t.x, acc.y += t.y, acc.z += t.z, acc.w += t.w;
-  }
-  if (out_f32) *reinterpret_cast<float4*>(out_f32 + o) = acc;
-  if (out) {
-    if constexpr (std::is_same<T, float>::value) {
-      *reinterpret_cast<float4*>(out + o) = acc;
-    } else {
-      T t4[4] = {static_cast<T>(acc.x), static_cast<T>(acc.y), static_cast<T>(acc.z), static_cast<T>(acc.w)};
-      *reinterpret_cast<uint2*>(out + o) = *reinterpret_cast<uint2*>(t4);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* src = partial + size_t(first) * Co * Ci + e;
+    const size_t slab = size_t(Co) * Ci;
+    uint32_t s = 0;
+    for (; s + 4 <= count; s += 4) {  // four loads in flight, added in slab order
+      const float4 t0 = __ldg(reinterpret_cast<const float4*>(src + (s + 0) * slab));
+      const float4 t1 = __ldg(reinterpret_cast<const float4*>(src + (s + 1) * slab));
+      const float4 t2 = __ldg(reinterpret_cast<const float4*>(src + (s + 2) * slab));
+      const float4 t3 = __ldg(reinterpret_cast<const float4*>(src + (s + 3) * slab));
+      acc.x += t0.x, acc.y += t0.y, acc.z += t0.z, acc.w += t0.w;
+      acc.x += t1.x, acc.y += t1.y, acc.z += t1.z, acc.w += t1.w;
+      acc.x += t2.x, acc.y += t2.y, acc.z += t2.z, acc.w += t2.w;
+      acc.x += t3.x, acc.y += t3.y, acc.z += t3.z, acc.w += t3.w;
     }
-  }
+    for (; s < count; ++s) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(src + s * slab));
+      acc.x += t.x, acc.y += t.y, acc.z += t.z, acc.w += t.w;
+    }
+    const int co = static_cast<int>(e / Ci), ci = static_cast<int>(e % Ci);
+    const int64_t o = (int64_t(co) * V + v) * Ci + ci;
+    if (accumulate) {  // later passes of the fp32-accurate mode add to what an earlier pass wrote (fp32 outputs only)
+      const float* prev = out_f32 ? out_f32 : reinterpret_cast<const float*>(out);
+      const float4 t = *reinterpret_cast<const float4*>(prev + o);
+      acc.x += t.x, acc.y += t.y, acc.z += t.z, acc.w += t.w;
+    }
+    if (out_f32) *reinterpret_cast<float4*>(out_f32 + o) = acc;
+    if (out) {
+      if constexpr (std::is_same<T, float>::value) {
+        *reinterpret_cast<float4*>(out + o) = acc;
+      } else {
+        T t4[4] = {static_cast<T>(acc.x), static_cast<T>(acc.y), static_cast<T>(acc.z), static_cast<T>(acc.w)};
+        *reinterpret_cast<uint2*>(out + o) = *reinterpret_cast<uint2*>(t4);
+      }
+    }
   }
 }
 
